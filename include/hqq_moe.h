@@ -118,15 +118,17 @@ int hqm_scratch_init(void* scratch, void* stream);
 /* Bytes of scratch hqm_linear needs for M rows of this layer (0 if none). */
 size_t hqm_linear_scratch_bytes(int64_t M, const hqm_weight* w);
 
+/* The same for the fastest launch: with less, hqm_linear at five or more rows of a 2- or 4-bit layer spreads over fewer
+ * SMs.  At least hqm_linear_scratch_bytes(). */
+size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w);
+
 /* HQQLinearTritonSavable.forward / forward_triton (custom_layers.py:49-92) with the
  * kernels of triton_kernels.py:37-191 (4-bit), :225-380 (2-bit), :414-564 (3-bit)
  * and the per-call 8-bit scale/zero decode fused in:
  *   y[M, N] = x[M, K] . W_est^T (+ bias[N]),  fp32 accumulation, bf16 in/out.
  * bias may be NULL.  scratch may be NULL when hqm_linear_scratch_bytes() is 0.
- * Rows 1..16 take the weight-streaming kernels, 17 and more (5 and more for 3-bit layers) the tcgen05 kernels;
- * HQM_GEMM_TMA=0 in the environment at load time keeps the 2- and 4-bit many-row path on its first-generation
- * kernel (operand tiles filled by threads instead of TMA), HQM_FORCE_GENERIC=1 routes everything through the
- * shape-agnostic kernel. */
+ * Rows 1..4 take the weight-streaming kernels, 5 and more the tcgen05 kernels; HQM_FORCE_GENERIC=1 in the environment
+ * at load time routes everything through the shape-agnostic kernel. */
 int hqm_linear(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias,
                void* scratch, size_t scratch_bytes, void* stream);
 
@@ -194,6 +196,15 @@ size_t hqm_moe_decode_scratch_bytes(int32_t E, const hqm_weight* w1, const hqm_w
 int hqm_moe_decode(uint16_t* out, uint16_t* router_logits, const uint16_t* x, const uint16_t* gate_w, int32_t E,
                    const void* table, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3,
                    void* scratch, size_t scratch_bytes, void* stream);
+
+/* The whole of SparseMoeWrapper.forward (custom_layers.py:272-314) for T tokens when every expert is resident on the
+ * device: router, per-expert row lists, the active experts' FFNs and the weighted sums.  The row counts never leave the
+ * device: both GEMM launches cover all experts and read the counts there.  table: as for hqm_moe_decode.  x and out
+ * (T, hidden) bf16, router_logits (T, E) bf16.  The scratch size is 0 where the shapes are not supported. */
+size_t hqm_moe_forward_scratch_bytes(int64_t T, int32_t E, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3);
+int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, const uint16_t* gate_w, int64_t T, int32_t E,
+                    const void* table, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3, void* scratch,
+                    size_t scratch_bytes, void* stream);
 
 /* ---- the attention half of a decoder layer, one token ---------------------- */
 /* The reference takes this step from the Hugging Face Mixtral decoder layer (build_model.py:166-241 builds the

@@ -76,6 +76,7 @@ SIGNATURES = {
     "hqm_scratch_header_bytes": (C.c_size_t, []),
     "hqm_scratch_init": (C.c_int, [_P, _P]),
     "hqm_linear_scratch_bytes": (C.c_size_t, [_I64, _WP]),
+    "hqm_linear_scratch_preferred": (C.c_size_t, [_I64, _WP]),
     "hqm_linear": (C.c_int, [_P, _P, _I64, _WP, _P, _P, C.c_size_t, _P]),
     "hqm_static_scratch_capacity": (C.c_size_t, []),
     "hqm_linear_static_scratch": (C.c_int, [_P, _P, _I64, _WP, _P, _P]),
@@ -85,6 +86,8 @@ SIGNATURES = {
     "hqm_expert_table_build": (C.c_int, [_P, _WP, _I32]),
     "hqm_moe_decode_scratch_bytes": (C.c_size_t, [_I32, _WP, _WP, _WP]),
     "hqm_moe_decode": (C.c_int, [_P, _P, _P, _P, _I32, _P, _WP, _WP, _WP, _P, C.c_size_t, _P]),
+    "hqm_moe_forward_scratch_bytes": (C.c_size_t, [_I64, _I32, _WP, _WP, _WP]),
+    "hqm_moe_forward": (C.c_int, [_P, _P, _P, _P, _I64, _I32, _P, _WP, _WP, _WP, _P, C.c_size_t, _P]),
     "hqm_attn_decode_scratch_bytes": (C.c_size_t, [C.POINTER(HqmAttnLayer)]),
     "hqm_attn_decode": (C.c_int, [_P, _P, _P, C.POINTER(HqmAttnLayer), _P, _P, C.c_size_t, _P]),
     "hqm_decode_layer_scratch_bytes": (C.c_size_t, [C.POINTER(HqmDecoderLayer)]),

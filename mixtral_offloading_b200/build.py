@@ -2,8 +2,8 @@
 
     python -m mixtral_offloading_b200.build [--force]
 
-One nvcc invocation, no build system: the sources are few and compile in
-seconds.  The output, libhqq_moe_b200.so, sits beside this file.
+One nvcc invocation per source, in parallel, no build system.  The output,
+libhqq_moe_b200.so, sits beside this file.
 """
 from __future__ import annotations
 
@@ -11,39 +11,52 @@ import glob
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhqq_moe_b200.so")
 
 NVCC_FLAGS = [
-    "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-Xcompiler", "-fPIC",
 ]
+OBJ = os.path.join(HERE, "..", "build", "obj")
 
 
 def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cpp")))
 
 
-def _stale():
-    if not os.path.exists(LIB):
-        return True
-    t = os.path.getmtime(LIB)
-    deps = sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
-    return any(os.path.getmtime(p) > t for p in deps)
+def _headers():
+    return glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not _stale():
-        return LIB
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB] + sources()
+def _stale(target, deps):
+    return not os.path.exists(target) or any(os.path.getmtime(p) > os.path.getmtime(target) for p in deps)
+
+
+def _run(cmd, verbose=False):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
     if verbose:
         print(res.stderr)
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Compiles what is out of date (one object per source, in parallel) and links the library."""
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    os.makedirs(OBJ, exist_ok=True)
+    jobs = []
+    for src in sources():
+        obj = os.path.join(OBJ, os.path.basename(src) + ".o")
+        if force or _stale(obj, [src] + _headers()):
+            jobs.append([nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-c", "-o", obj, src])
+    with ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        list(pool.map(lambda cmd: _run(cmd, verbose), jobs))
+    objs = [os.path.join(OBJ, os.path.basename(src) + ".o") for src in sources()]
+    if jobs or _stale(LIB, objs):
+        _run([nvcc] + NVCC_FLAGS + ["-shared", "-o", LIB] + objs)
     return LIB
 
 

@@ -5,6 +5,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "gemm_grouped.cuh"
 #include "kernels.cuh"
 
 namespace hqm {
@@ -71,18 +72,34 @@ int set_overlap(int on) {
     return prev;
 }
 
-size_t linear_scratch_bytes(int64_t M, const hqm_weight* w) {
+// Rows from which a 2- or 4-bit layer goes to the tensor-core kernel (gemm_grouped.cu); below, the streaming kernels,
+// whose work per weight grows with the rows, are faster.
+static bool use_gg(const hqm_weight* w, int G, int C, int64_t M) { return M >= GG_MIN_ROWS && M <= (1 << 22) && gg_supported(w, G, C); }
+
+size_t linear_scratch_bytes(int64_t M, const hqm_weight* w, bool preferred) {
     int G, C;
     StreamPlan plan;
     if (M <= 0 || check_weight(w, &G, &C) != HQM_OK) return 0;
     if (force_generic()) return 0;
-    if (M >= TC_MIN_ROWS && gemm_tc_supported(w, G, C, M)) return ((size_t)M * w->N * sizeof(float) + 255) / 256 * 256;
+    if (use_gg(w, G, C, M)) {
+        const GgRows rows = gg_linear_layout(M, w).rows;
+        return gg_stage_bytes(rows.padded(), w->K, true) + (preferred ? gg_scratch_bytes(rows.n) : gg_scratch_least(rows.n, w));
+    }
     if (gemm_tc3_supported(w, G, C, M)) return gemm_tc3_scratch_bytes(w, G, M);
     Stream3Plan plan3;
     if (gemv_stream3_plan(w, G, C, M, &plan3)) return gemv_stream3_scratch_bytes(plan3, M, w->N);
     const hqm_weight* one[1] = {w};
     if (!gemv_stream_plan(one, 1, M, &plan, /*chained=*/false)) return 0;
     return (gemv_stream_scratch_bytes(plan, M) + 255) / 256 * 256;
+}
+
+static int need_scratch(void* scratch, size_t have, size_t need) {
+    if (scratch == nullptr || have < need) {
+        set_error("linear: scratch of %zu bytes given, %zu needed", have, need);
+        return HQM_ERR_SCRATCH;
+    }
+    HQM_CHECK_ARG((reinterpret_cast<uintptr_t>(scratch) & 15u) == 0, "linear: scratch must be 16-byte aligned");
+    return HQM_OK;
 }
 
 int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t M, const hqm_weight* w,
@@ -94,44 +111,39 @@ int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t 
     StreamPlan plan;
     const bool x_ok = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     if (!x_ok || force_generic()) return launch_linear_generic(y, x, x_idx, M, w, G, C, bias, st);
-    if (M >= TC_MIN_ROWS && gemm_tc_supported(w, G, C, M)) {
-        const size_t need = (size_t)M * w->N * sizeof(float);
-        if (scratch == nullptr || scratch_bytes < need) {
-            set_error("linear: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
-            return HQM_ERR_SCRATCH;
-        }
-        HQM_CHECK_ARG((reinterpret_cast<uintptr_t>(scratch) & 15u) == 0, "linear: scratch must be 16-byte aligned");
-        rc = launch_gemm_tc((float*)scratch, x, x_idx, M, w, nullptr, G, C, st);
+    if (use_gg(w, G, C, M)) {
+        const GgLayout layout = gg_linear_layout(M, w);
+        const int64_t xt_rows = layout.rows.padded();
+        const size_t staged = gg_stage_bytes(xt_rows, w->K, true);
+        rc = need_scratch(scratch, scratch_bytes, staged + gg_scratch_least(layout.rows.n, w));
         if (rc != HQM_OK) return rc;
-        return launch_rows_from_sums(y, (const float*)scratch, bias, M, w->N, st);
+        const GgStaged xs = gg_staged(scratch, xt_rows, w->K, true);
+        rc = launch_gg_stage(xs, x, 0, x_idx, nullptr, 1, M, w->K, st);
+        if (rc != HQM_OK) return rc;
+        GgJob job{};
+        job.problems = 1;
+        job.w0[0] = w;
+        job.rows = (int)M;
+        job.layout = layout;
+        job.x = xs;
+        job.mode = GG_LINEAR;
+        job.y[0] = y;
+        job.bias[0] = bias;
+        return launch_gg(job, counters, (uint8_t*)scratch + staged, scratch_bytes - staged, st);
     }
     if (gemm_tc3_supported(w, G, C, M)) {
-        const size_t need = gemm_tc3_scratch_bytes(w, G, M);
-        if (scratch == nullptr || scratch_bytes < need) {
-            set_error("linear: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
-            return HQM_ERR_SCRATCH;
-        }
-        HQM_CHECK_ARG((reinterpret_cast<uintptr_t>(scratch) & 15u) == 0, "linear: scratch must be 16-byte aligned");
-        return launch_gemm_tc3(y, scratch, x, x_idx, M, w, bias, G, C, st);
+        rc = need_scratch(scratch, scratch_bytes, gemm_tc3_scratch_bytes(w, G, M));
+        return rc != HQM_OK ? rc : launch_gemm_tc3(y, scratch, x, x_idx, M, w, bias, G, C, st);
     }
     Stream3Plan plan3;
     if (gemv_stream3_plan(w, G, C, M, &plan3)) {
-        const size_t need = gemv_stream3_scratch_bytes(plan3, M, w->N);
-        if (scratch == nullptr || scratch_bytes < need) {
-            set_error("linear: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
-            return HQM_ERR_SCRATCH;
-        }
-        HQM_CHECK_ARG((reinterpret_cast<uintptr_t>(scratch) & 15u) == 0, "linear: scratch must be 16-byte aligned");
-        return launch_gemv_stream3(y, (float*)scratch, x, x_idx, M, w, bias, G, C, plan3, st);
+        rc = need_scratch(scratch, scratch_bytes, gemv_stream3_scratch_bytes(plan3, M, w->N));
+        return rc != HQM_OK ? rc : launch_gemv_stream3(y, (float*)scratch, x, x_idx, M, w, bias, G, C, plan3, st);
     }
     const hqm_weight* one[1] = {w};
     if (gemv_stream_plan(one, 1, M, &plan, /*chained=*/false)) {
-        const size_t need = gemv_stream_scratch_bytes(plan, M);
-        if (scratch == nullptr || scratch_bytes < need) {
-            set_error("linear: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
-            return HQM_ERR_SCRATCH;
-        }
-        HQM_CHECK_ARG((reinterpret_cast<uintptr_t>(scratch) & 15u) == 0, "linear: scratch must be 16-byte aligned");
+        rc = need_scratch(scratch, scratch_bytes, gemv_stream_scratch_bytes(plan, M));
+        if (rc != HQM_OK) return rc;
         StreamJob job{};
         job.w[0] = w;
         job.counters = counters;
@@ -167,6 +179,11 @@ int hqm_scratch_init(void* scratch, void* stream) {
 
 size_t hqm_linear_scratch_bytes(int64_t M, const hqm_weight* w) {
     const size_t inner = hqm::linear_scratch_bytes(M, w);
+    return inner ? inner + hqm::SCRATCH_HEADER : 0;
+}
+
+size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w) {
+    const size_t inner = hqm::linear_scratch_bytes(M, w, /*preferred=*/true);
     return inner ? inner + hqm::SCRATCH_HEADER : 0;
 }
 

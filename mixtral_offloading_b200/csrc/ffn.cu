@@ -3,6 +3,7 @@
 // (MixtralBLockSparseTop2MLP_HQQ.forward and the per-expert body of
 // SparseMoeWrapper.forward in the reference's custom_layers.py).
 #include "common.cuh"
+#include "gemm_grouped.cuh"
 #include "kernels.cuh"
 
 namespace hqm {
@@ -41,26 +42,25 @@ static bool same_format(const hqm_weight* a, const hqm_weight* b) {
            a->meta_group == b->meta_group;
 }
 
-// The tensor-core path for a whole expert (many rows): [w1; w3] GEMM -> silu * mul -> w2 GEMM -> scatter.
-struct TcPlan {
-    int G1, C1, G2, C2;
-    size_t up_bytes, h_bytes, down_bytes;
-    size_t gather_bytes;      // the routed rows of x made contiguous (the TMA-staged GEMM copies x by tiles)
+// The tensor-core path: x staged, [w1; w3] with the gate fused into its epilogue (h staged for the next launch), w2.
+// One expert (hqm_expert_ffn) or all experts of a block (hqm_moe_forward: `rows` = tokens, two list entries each).
+struct GgPlan {
+    int64_t xt_rows;
+    size_t x_bytes, h_bytes, part_bytes;
+    size_t total() const { return x_bytes + h_bytes + part_bytes; }
 };
-static bool tc_plan(int64_t M, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3, const void* x,
-                    TcPlan* tp) {
-    if (force_generic() || M < TC_MIN_ROWS || !same_format(w1, w3)) return false;
-    if (check_weight(w1, &tp->G1, &tp->C1) != HQM_OK || check_weight(w3, &tp->G1, &tp->C1) != HQM_OK ||
-        check_weight(w2, &tp->G2, &tp->C2) != HQM_OK)
+static bool gg_plan(int64_t entries, int lists, int64_t most, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3,
+                    GgPlan* gp) {
+    int G1, C1, G2, C2;
+    if (force_generic() || !same_format(w1, w3) || entries > (1 << 22)) return false;
+    if (check_weight(w1, &G1, &C1) != HQM_OK || check_weight(w3, &G1, &C1) != HQM_OK || check_weight(w2, &G2, &C2) != HQM_OK)
         return false;
-    if (x && (reinterpret_cast<uintptr_t>(x) & 15u) != 0) return false;
-    if (!gemm_tc_supported(w1, tp->G1, tp->C1, M) || !gemm_tc_supported(w3, tp->G1, tp->C1, M) ||
-        !gemm_tc_supported(w2, tp->G2, tp->C2, M))
-        return false;
-    tp->up_bytes = align_up((size_t)M * 2 * w1->N * sizeof(float), 256);
-    tp->h_bytes = align_up((size_t)M * w1->N * 2, 256);
-    tp->down_bytes = align_up((size_t)M * w2->N * sizeof(float), 256);
-    tp->gather_bytes = gemm_tma_supported(w1, tp->G1, tp->C1, M) ? align_up((size_t)M * w1->K * 2, 256) : 0;
+    if (!gg_supported(w1, G1, C1) || !gg_supported(w3, G1, C1) || !gg_supported(w2, G2, C2)) return false;
+    if (w1->nbits != 2 || w1->group_size != 16 || w2->nbits != 2 || w2->group_size != 16) return false;   // tiles of two parts
+    gp->xt_rows = gg_padded_rows(entries, lists);
+    gp->x_bytes = gg_stage_bytes(gp->xt_rows, w1->K, true);
+    gp->h_bytes = gg_stage_bytes(gp->xt_rows, w1->N, false);
+    gp->part_bytes = gg_scratch_bytes((int)(most > GG_MAX_ROWS ? GG_MAX_ROWS : (most + 15) / 16 * 16));
     return true;
 }
 
@@ -93,8 +93,8 @@ extern "C" {
 size_t hqm_expert_ffn_scratch_bytes(int64_t M, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3) {
     if (!w1 || !w2 || !w3 || M <= 0) return 0;
     const size_t H = hqm::SCRATCH_HEADER;
-    hqm::TcPlan tp;
-    if (hqm::tc_plan(M, w1, w2, w3, nullptr, &tp)) return H + tp.up_bytes + tp.h_bytes + tp.down_bytes + tp.gather_bytes;
+    hqm::GgPlan gp;
+    if (M >= hqm::GG_MIN_ROWS && hqm::gg_plan(M, 1, M, w1, w2, w3, &gp)) return H + gp.total();
     hqm::FusedPlan fp;
     if (hqm::fused_plan(M, w1, w2, w3, nullptr, &fp)) return H + fp.up_bytes + fp.h_bytes + fp.down_bytes;
     const size_t a = hqm::align_up((size_t)M * (size_t)w1->N * 2, 256);
@@ -127,26 +127,32 @@ int hqm_expert_ffn(uint16_t* out, const uint16_t* x, int64_t M, const int32_t* t
     const int F = w1->N, H = w2->N;
     uint32_t* counters = (uint32_t*)scratch;
     uint8_t* p = (uint8_t*)scratch + SCRATCH_HEADER;
-    TcPlan tp;
-    if (tc_plan(M, w1, w2, w3, x, &tp)) {
-        float* up = (float*)p;
-        uint16_t* h = (uint16_t*)(p + tp.up_bytes);
-        float* down = (float*)(p + tp.up_bytes + tp.h_bytes);
-        int rc;
-        if (token_idx && tp.gather_bytes) {
-            uint16_t* xg = (uint16_t*)(p + tp.up_bytes + tp.h_bytes + tp.down_bytes);
-            rc = launch_gather_rows(xg, x, token_idx, M, w1->K, st);
-            if (rc != HQM_OK) return rc;
-            rc = launch_gemm_tc(up, xg, nullptr, M, w1, w3, tp.G1, tp.C1, st);
-        } else {
-            rc = launch_gemm_tc(up, x, token_idx, M, w1, w3, tp.G1, tp.C1, st);
-        }
+    GgPlan gp;
+    if (M >= GG_MIN_ROWS && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && gg_plan(M, 1, M, w1, w2, w3, &gp)) {
+        // 3 launches: x staged -> h = silu(w1 x) * w3 x, staged -> w2 h, weighted, into out
+        uint8_t *xt = p, *ht = p + gp.x_bytes, *parts = ht + gp.h_bytes;
+        const GgStaged xs = gg_staged(xt, gp.xt_rows, w1->K, true), hs = gg_staged(ht, gp.xt_rows, w1->N, false);
+        int rc = launch_gg_stage(xs, x, 0, token_idx, nullptr, 1, M, w1->K, st);
         if (rc != HQM_OK) return rc;
-        rc = launch_silu_mul_from_sums(h, up, M, F, st);
+        GgJob up{}, down{};
+        up.problems = down.problems = 1;
+        up.rows = down.rows = (int)M;
+        up.layout = down.layout = gg_expert_layout(M);
+        up.mode = GG_UP;
+        up.w0[0] = w1;
+        up.w1[0] = w3;
+        up.x = xs;
+        up.ht = ht;
+        rc = launch_gg(up, counters, parts, gp.part_bytes, st);
         if (rc != HQM_OK) return rc;
-        rc = launch_gemm_tc(down, h, nullptr, M, w2, nullptr, tp.G2, tp.C2, st);
-        if (rc != HQM_OK) return rc;
-        return launch_scatter_from_sums(out, down, token_idx, route_w, accumulate, M, H, st);
+        down.mode = GG_DOWN;
+        down.w0[0] = w2;
+        down.x = hs;
+        down.out = out;
+        down.out_idx = token_idx;
+        down.row_w = route_w;
+        down.accumulate = accumulate;
+        return launch_gg(down, counters, parts, gp.part_bytes, st);
     }
     FusedPlan fp;
     if (fused_plan(M, w1, w2, w3, x, &fp)) {
@@ -188,6 +194,117 @@ int hqm_expert_ffn(uint16_t* out, const uint16_t* x, int64_t M, const int32_t* t
     const int64_t nh = M * H;
     scale_scatter_kernel<<<(int)((nh + 255) / 256 > 148 * 8 ? 148 * 8 : (nh + 255) / 256), 256, 0, st>>>(
         out, c, token_idx, route_w, M, H, accumulate);
+    HQM_LAUNCH_CHECK();
+    return HQM_OK;
+}
+
+// ---- MoE block of many tokens with every expert resident: no host read-back, seven launches --------------------------
+}  // extern "C"
+
+namespace hqm {
+// out[t] = bf16(y[i] + y[j]) of the two list entries of token t (each already weighted and rounded to bf16).
+__global__ void __launch_bounds__(256) moe_combine_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ y,
+                                                          const int32_t* __restrict__ entry_of, int64_t tokens, int H8) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int64_t total = tokens * H8;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t t = i / H8;
+        const int c = (int)(i - t * H8);
+        const uint4 a = reinterpret_cast<const uint4*>(y)[(int64_t)entry_of[2 * t] * H8 + c];
+        const uint4 b = reinterpret_cast<const uint4*>(y)[(int64_t)entry_of[2 * t + 1] * H8 + c];
+        const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float lo = __uint_as_float(av[j] << 16) + __uint_as_float(bv[j] << 16);
+            const float hi = __uint_as_float(av[j] & 0xffff0000u) + __uint_as_float(bv[j] & 0xffff0000u);
+            o[j] = (uint32_t)float_to_bf16_bits(lo) | ((uint32_t)float_to_bf16_bits(hi) << 16);
+        }
+        reinterpret_cast<uint4*>(out)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
+struct MoePlan {
+    GgPlan gg;
+    size_t route_bytes, y_bytes;
+    size_t total() const { return route_bytes + gg.total() + y_bytes; }
+};
+static bool moe_plan(int64_t T, int E, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3, MoePlan* mp) {
+    if (T < 1 || T > (1 << 20) || E < 2 || E > GG_MAX_PROBLEMS || w2->N % 8 != 0 || w2->N != w1->K || w2->K != w1->N) return false;
+    if (!gg_plan(2 * T, E, T, w1, w2, w3, &mp->gg)) return false;
+    mp->route_bytes = align_up((size_t)T * 2 * 4 * 5 + (size_t)(2 * E + 1) * 4, 1024);
+    mp->y_bytes = align_up((size_t)T * 2 * w2->N * 2, 1024);
+    return true;
+}
+}  // namespace hqm
+
+extern "C" {
+
+size_t hqm_moe_forward_scratch_bytes(int64_t T, int32_t E, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3) {
+    if (!w1 || !w2 || !w3) return 0;
+    hqm::MoePlan mp;
+    return hqm::moe_plan(T, E, w1, w2, w3, &mp) ? hqm::SCRATCH_HEADER + mp.total() : 0;
+}
+
+int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, const uint16_t* gate_w, int64_t T, int32_t E,
+                    const void* table, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3, void* scratch,
+                    size_t scratch_bytes, void* stream) {
+    using namespace hqm;
+    HQM_CHECK_ARG(out && router_logits && x && gate_w && table && w1 && w2 && w3, "moe_forward: null pointer");
+    HQM_CHECK_ARG(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0, "moe_forward: x and out must be 16-byte aligned");
+    MoePlan mp;
+    HQM_CHECK_ARG(moe_plan(T, E, w1, w2, w3, &mp), "moe_forward: %lld tokens, %d experts of these shapes are not supported", (long long)T, E);
+    if (scratch == nullptr || scratch_bytes < SCRATCH_HEADER + mp.total()) {
+        set_error("moe_forward: scratch of %zu bytes given, %zu needed", scratch_bytes, SCRATCH_HEADER + mp.total());
+        return HQM_ERR_SCRATCH;
+    }
+    HQM_CHECK_ARG((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "moe_forward: scratch must be 256-byte aligned");
+    cudaStream_t st = (cudaStream_t)stream;
+    uint32_t* counters = (uint32_t*)scratch;
+    uint8_t* p = (uint8_t*)scratch + SCRATCH_HEADER;
+    float* topk_w = (float*)p;                                        // [T][2]
+    int32_t* topk_idx = (int32_t*)(topk_w + 2 * T);                   // [T][2]
+    int32_t* entry_of = topk_idx + 2 * T;                             // [T][2]: list entries of a token
+    int32_t* token_idx = entry_of + 2 * T;                            // [2T]
+    float* token_w = (float*)(token_idx + 2 * T);                     // [2T]
+    int32_t* counts = (int32_t*)(token_w + 2 * T);                    // [E]
+    int32_t* offsets = counts + E;                                    // [E + 1]
+    uint8_t* xt = p + mp.route_bytes;
+    uint8_t* ht = xt + mp.gg.x_bytes;
+    uint8_t* parts = ht + mp.gg.h_bytes;
+    uint16_t* y = (uint16_t*)(parts + mp.gg.part_bytes);
+    int rc = launch_router_top2(router_logits, topk_w, topk_idx, x, gate_w, T, w1->K, E, st);
+    if (rc != HQM_OK) return rc;
+    rc = launch_router_lists(counts, offsets, token_idx, token_w, entry_of, topk_w, topk_idx, T, E, st);
+    if (rc != HQM_OK) return rc;
+    const GgStaged xs = gg_staged(xt, mp.gg.xt_rows, w1->K, true), hs = gg_staged(ht, mp.gg.xt_rows, w1->N, false);
+    rc = launch_gg_stage(xs, x, 0, token_idx, counts, E, 2 * T, w1->K, st);
+    if (rc != HQM_OK) return rc;
+    GgJob up{}, down{};
+    up.problems = down.problems = E;
+    up.table = down.table = static_cast<const StreamEntry*>(table);
+    up.counts = down.counts = counts;
+    up.rows = down.rows = (int)T;
+    up.mode = GG_UP;
+    up.shape = w1;
+    up.which0 = 0;
+    up.which1 = 2;
+    up.x = xs;
+    up.ht = ht;
+    rc = launch_gg(up, counters, parts, mp.gg.part_bytes, st);
+    if (rc != HQM_OK) return rc;
+    down.mode = GG_DOWN;
+    down.shape = w2;
+    down.which0 = down.which1 = 1;
+    down.x = hs;
+    down.out = y;
+    down.row_w = token_w;
+    rc = launch_gg(down, counters, parts, mp.gg.part_bytes, st);
+    if (rc != HQM_OK) return rc;
+    const int64_t work = T * (w2->N / 8);
+    launch_overlapped(moe_combine_kernel, (int)((work + 255) / 256 > 148 * 8 ? 148 * 8 : (work + 255) / 256), 256, 0, st, out,
+                      (const uint16_t*)y, (const int32_t*)entry_of, T, (int)(w2->N / 8));
     HQM_LAUNCH_CHECK();
     return HQM_OK;
 }

@@ -1,0 +1,1440 @@
+// Quantized GEMM on the 5th-generation tensor cores: sums[m, n] = sum_k x[m, k] * W_est[n, k] for one weight or for
+// all experts of a MoE block in one launch, each with its own list of rows whose length only the device knows.
+// Replaces the reference's Triton kernels (triton_kernels.py:37-131, 225-319), its per-call scale / zero decode
+// (custom_layers.py:62-66) and, with the epilogues below, the per-expert loop around them (custom_layers.py:243-256,
+// 295-312) for more than a few rows.
+//
+// The weight is the MMA's A operand: 128 output rows per tile, the rows of x are its N dimension (any multiple of 16
+// up to 256: no padding to a fixed tile).  What bounds the kernel is the dequantisation on the CUDA cores, not the
+// tensor core and not HBM, so everything is arranged around it:
+//
+//   * A lives in TMEM.  A dequantised pair of weights goes from registers to tensor memory (tcgen05.st), never
+//     through shared memory; `tcgen05.mma` reads it there.  (16 KB per 128 x 64 tile written to and read from shared
+//     memory would cost 256 of the ~260 cycles that HBM needs for a tile of 128 columns.)
+//   * The 16x256b store shape gives a thread 4 rows x 16 columns of a 32-row quadrant.  Rows are dealt so that its 4
+//     rows are members of ONE quantisation group: one (s, -z*s) pair per column serves four weights.
+//   * The order of k inside a 64-column block is free as long as x follows it.  A thread takes 16 neighbouring bytes of
+//     a storage row (one 128-bit shared-memory load) and pairs columns (k, k+2), which one AND isolates; x is staged
+//     in the matching order (tile_pos below).
+//   * fp16: a field of a byte, left where it is, IS an fp16 denormal c * 2^(p-24); one fused multiply-add with
+//     s * 2^(24-p-2) and -z*s * 2^-2 gives a quarter of the weight.  One AND and one FMA per two weights; the sums are
+//     multiplied by 4 at the end.  Where s * 2^(22-p) leaves the fp16 range (s >= 1/4), the warp takes the longer way
+//     for that unit: OR into 1024, exact subtract, FMA.  x is staged as fp16 with a power-of-two factor per row.
+//   * bf16 (down projections of more than 16 rows: h has no factor per row and may exceed fp16): OR into 128, exact
+//     subtract, FMA.
+//
+// Measured on B200 (148 SMs): LOP3 / SHF / PRMT and HFMA2 both issue every second cycle per scheduler but on two
+// pipes; tcgen05.st of a 128 x 64 tile takes 65 cycles; tcgen05.mma (K = 16, A in TMEM) 15 / 32 / 64 / 128 cycles at
+// N = 16 / 64 / 128 / 256 when issued from warp-uniform code (45 when one lane of a diverged warp issues it).
+//
+// A unit of work is 128 columns of a tile.  Roles of the 24 warps of a CTA (one CTA per SM, persistent):
+//   warps 0-15   four groups of four warps; group u % 4 dequantises unit u, warp q of it the TMEM lanes 32q .. 32q+31.
+//                A warp decodes the scales and zeros of its own rows into a private corner of shared memory: no barrier
+//                between warps.
+//   warps 16-19  epilogue
+//   warps 20, 21 copies of the packed codes, scale bytes and zero bytes of a unit (tiled TMA, 6 to a unit)
+//   warp 22      copies of the staged rows of x (untiled: a tile's rows are contiguous and already swizzled)
+//   warp 23      issues the MMAs
+//
+// Work split: the units of all tiles of all problems follow each other, weighted by what a unit costs with its list's
+// row count, and every CTA takes an equal contiguous share.  A tile cut by a share's boundary is summed from fp32
+// pieces in scratch memory by whichever CTA arrives last, in CTA order (no atomics on results, deterministic).
+//
+// Measured (one launch; before: the same layers through a kernel that staged A in shared memory, expert by expert):
+// up + gate of 8 experts, 4096 -> 14336, 33 tokens: 201 us, down 102 us; the whole block 943 -> 316 us.  One expert with
+// 512 rows 325 -> 238 us.  A unit takes ~930 cycles (2440 warp instructions) at few rows: without the decoding of scales
+// and zeros, the weights' arithmetic and the MMAs the same pipeline runs at ~430.  At 256 rows it is the staged x that
+// bounds it (64 KB per unit into every SM).
+//
+// Every wait is bounded; a wait that runs out sets the error flag, all roles leave, TMEM is freed.
+#include <cuda.h>
+#include <type_traits>
+
+#include "gemm_grouped.cuh"
+
+#include <algorithm>
+#include "tc_common.cuh"
+
+namespace hqm {
+
+bool stream_cached_maps(const hqm_weight* w, int G, void* out3);      // gemv_tma.cu
+
+namespace gg {
+using namespace tc;
+
+constexpr int GROUPS = 4;                  // dequantising groups of four warps
+constexpr int WARP_EPI = 4 * GROUPS, WARP_RAW = WARP_EPI + 4, WARP_B = WARP_RAW + 2, WARP_MMA = WARP_B + 1;
+constexpr int NTHREADS = (WARP_MMA + 1) * 32;
+// Registers per thread after the roles have split (80 at the launch): 16 x 96 + 4 x 64 + 4 x 32 = 24 x 80.
+constexpr int REGS_DEQUANT = 96, REGS_EPI = 64, REGS_ISSUE = 32;
+template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+constexpr int MAX_B_STAGES = 16, MAX_RAW = 2 * GROUPS;
+// Cycles of 128 columns of a tile with n rows (measured: 930 at 16, 1060 at 64, 1400 at 128, 2660 at 256), the weights of
+// the work split.
+__host__ __device__ constexpr int unit_cycles(bool f16, int n) {
+    return n > 128 ? n * 10 + (f16 ? 0 : 200) : (f16 ? 900 : 1170) + 4 * n;
+}
+constexpr int NA = 6;                      // A slots of 128 columns (64 TMEM columns each) at most
+// raw full, raw empty, A full, A empty (even and odd rounds of the slots), B full, B empty, accumulator full, empty
+constexpr int N_BARS = 2 * MAX_RAW + 3 * NA + 2 * MAX_B_STAGES + 4;
+constexpr int TILE_BYTES = 16 * 128 * 2;   // 16 rows of a finished tile, 16 bit; two of them
+constexpr int EPI_BYTES = 2 * TILE_BYTES + 3 * GG_MAX_ROWS * 4;     // and per row of a chunk: factor, weight, output row
+constexpr float F16_SCALE = 4.f;           // A holds a quarter of the weight in fp16 mode
+
+struct Weight {                            // one layer on the device
+    const uint16_t* meta[4];               // ms_scale, mz_scale, ms_zero, mz_zero
+    const CUtensorMap* maps;               // codes, scale bytes, zero bytes
+};
+struct Problem {
+    Weight w[2];                           // [1]: w3 of GG_UP
+    int cnt, n, chunks, cost;              // rows; rows per chunk (padded); chunks; cost of a unit
+    int row0, list0;                       // first row in the staged x, first entry in the row list
+    int tiles, G, P, C;
+    int f16;
+};
+
+// How a list's rows share the ring of staged x: a stage holds 256 columns of all rows of a chunk (128 beyond 64 rows, 64
+// beyond 128), as a wait, an expectation and a copy together cost the copying warp about 340 cycles.
+struct BClass {
+    int bytes, stages, blocks;             // bytes reserved per stage, stages in the ring, 64-column blocks in a stage
+    __device__ __forceinline__ static BClass of(int n, int ring) {
+        BClass c;
+        c.blocks = n > 128 ? 1 : (n > 64 ? 2 : 4);
+        const int rows = n <= 16 ? 16 : (n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : 256)));
+        c.bytes = rows * 128 * c.blocks;
+        c.stages = min(MAX_B_STAGES, ring / c.bytes);
+        return c;
+    }
+};
+// TMEM columns: up to 64 rows per chunk in the whole launch, D in two buffers of 64 and six A slots behind them;
+// otherwise D in two buffers of 128 (or one of 256) and four A slots.
+struct TmemMap {
+    uint32_t d_step, a_base;
+    int slots;
+    __device__ __forceinline__ static TmemMap of(int n_max) {
+        return n_max <= 64 ? TmemMap{64u, 128u, 6} : TmemMap{128u, 256u, 4};
+    }
+};
+
+struct HostProblem {
+    CUtensorMap maps[2][3];
+    const uint16_t* meta[2][4];
+    int G, P, C, tiles;
+    void* y;
+    const uint16_t* bias;
+};
+
+struct Params {
+    HostProblem hp[4];
+    int problems, K, units_k, subs_k;      // units and 64-column blocks of K
+    int chunks;                            // row chunks of n_max rows (one list shared by all problems)
+    int N;                                 // output rows of a problem (table mode: common to all)
+    const StreamEntry* table;
+    int which0, which1;
+    const int32_t* counts;
+    int rows;
+    const unsigned char* xt;
+    int64_t xt_rows;
+    const float* row_scale;                // of the staged rows (null: 1)
+    int mode;
+    int y_f16;
+    unsigned char* ht;
+    void* out;
+    int out_f16;
+    const int32_t* out_idx;
+    const float* row_w;
+    int accumulate;
+    float* parts;                          // [grid][2][n_max][128]
+    int n_max;
+    uint32_t* counters;
+    int* error_flag;
+};
+
+// ---- the split of a launch's units over its CTAs -------------------------------------------------------------------
+struct Shared {
+    Problem pr[GG_MAX_PROBLEMS];
+    int ubase[GG_MAX_PROBLEMS + 1];        // first unit of each problem
+    unsigned long long cbase[GG_MAX_PROBLEMS + 1];     // cost in front of each problem
+    int begin[256];                        // first unit of each CTA ([grid]: all units)
+    int last;                              // epilogue: this CTA completes the tile
+    uint32_t tmem;
+    volatile int failed;
+};
+
+template <int NBITS_, int GS_>
+struct Fmt {
+    static constexpr int NBITS = NBITS_, GS = GS_;
+    static constexpr int PER = codes_per_word(NBITS);
+    static constexpr int PARTS = 128 / (PER * GS);         // storage-row residues of a tile (GG_UP: one of w1, one of w3)
+    static_assert(PARTS * PER * GS == 128, "a tile holds whole groups");
+    // Columns of a unit.  What a warp does once per unit (waits, decoding, hand-over) takes about as long as the weights of
+    // 128 columns of a 2-bit tile, and those layers are large; 4-bit layers decode little and may be small.
+    static constexpr int UK = 128;
+    static constexpr int HALVES = UK / 128;                // A slots of a unit
+    static constexpr int BLOCKS = UK / 64;
+    static constexpr int SLW = (GS == 16) ? 2 : 1;         // rows of scales a warp needs (GS = 16: one of either part)
+    static constexpr int CODE_PART = GS * 128;             // packed bytes of a part of 128 columns
+    static constexpr int CODE_HALF = PARTS * CODE_PART;
+    static constexpr int SZ_PART = PER * 128;
+    static constexpr int SQ_OFF = HALVES * CODE_HALF, ZQ_OFF = SQ_OFF + HALVES * PARTS * SZ_PART;
+    static constexpr int RAW_TX = ZQ_OFF + HALVES * PARTS * SZ_PART;
+    static constexpr int RAW_BYTES = (RAW_TX + 1023) / 1024 * 1024;
+    static constexpr int DC = UK * SLW / 32;               // columns a lane decodes
+    static constexpr int ST_WARP = SLW * UK * 4;           // s and t of a warp's rows
+    static constexpr int ST_BLOCK = 2 * SLW * 64, ST_T = BLOCKS * ST_BLOCK;
+    // Launches of up to 64 rows per chunk need few staged rows in flight and many packed bytes, others the reverse.
+    __host__ __device__ static constexpr int b_ring(int n_max) { return n_max <= 64 ? 64 * 1024 : 128 * 1024; }
+    __host__ __device__ static constexpr int n_raw(int n_max) { return 2 * GROUPS; }
+    static constexpr int ST_OFF = 0, EPI_OFF = ST_OFF + 4 * GROUPS * ST_WARP, BAR_OFF = EPI_OFF + EPI_BYTES, RING_OFF = BAR_OFF + 1024;
+    __host__ __device__ static constexpr int smem(int n_max) {
+        return (RING_OFF + 1023) / 1024 * 1024 + b_ring(n_max) + n_raw(n_max) * RAW_BYTES + 1024;
+    }
+    static_assert(smem(64) + (int)sizeof(Shared) <= 227 * 1024 && smem(256) + (int)sizeof(Shared) <= 227 * 1024, "shared memory");
+    // Which row of the tile TMEM lane 32 q + 8 j + g holds (q: warp of a group, j = 0..3): part, slot of the byte, member.
+    // A thread of the 16x256b store shape holds j = 0..3 at one g: four members of one quantisation group.
+    __device__ __forceinline__ static int part_of(int q, int g) { return GS == 16 ? (g & 1) : (PARTS == 2 ? q >> 1 : 0); }
+    __device__ __forceinline__ static int slot_of(int q) { return NBITS == 2 ? q : q & 1; }
+    __device__ __forceinline__ static int member_of(int q, int g, int j) {
+        if (GS == 16) return (g >> 1) + 4 * j;
+        const int low = (g >> 1) | ((g & 1) << 2);         // neighbouring g: rows 4 apart, on other banks after the swizzle
+        return low + 8 * j + (GS == 64 ? 32 * (q >> 1) : 0);
+    }
+};
+
+// Position of column k of a 64-column block in the staged order (and in the A tile).
+__host__ __device__ constexpr int tile_pos(int k) {
+    const int c = k >> 4, i = (k >> 2) & 3, e = k & 3;                  // thread column, word, byte
+    return 16 * i + 4 * c + ((e & 1) << 1 | (e >> 1));                  // bytes in the order 0, 2, 1, 3
+}
+
+__device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait for a phase; false when the limit ran out.  try_wait suspends the warp for a while by itself.
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < (1u << 18); ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+// The same as straight-line code (the loop is inside the assembly), for the warps whose values have to stay uniform in the
+// compiler's eyes: a branch on a wait's outcome would move every operand of the copies and MMAs behind it to vector
+// registers.  `limit`: polls left; 0 once a wait has run out, and every later one then returns at once.
+__device__ __forceinline__ void wait_limited(uint32_t bar, uint32_t parity, uint32_t& limit) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\t"
+        "mov.u32 n, %0;\n\t"
+        "GG_WAIT:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra.uni GG_DONE;\n\t"
+        "setp.eq.u32 p, n, 0;\n\t"
+        "@p bra.uni GG_OUT;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "bra.uni GG_WAIT;\n\t"
+        "GG_OUT:\n\t"
+        "mov.u32 %0, 0;\n\t"
+        "GG_DONE:\n\t}"
+        : "+r"(limit)
+        : "r"(bar), "r"(parity)
+        : "memory");
+}
+constexpr uint32_t WAIT_LIMIT = 1u << 18;
+// A look at a phase without waiting, and the wait that is skipped when the look found it complete: the ~90 cycles of the
+// look pass under whatever is issued between the two.
+__device__ __forceinline__ uint32_t peek(uint32_t bar, uint32_t parity) {
+    uint32_t ready;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ready)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ready;
+}
+__device__ __forceinline__ void wait_peeked(uint32_t bar, uint32_t parity, uint32_t ready, uint32_t& limit) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .u32 n;\n\t"
+        "setp.ne.u32 p, %3, 0;\n\t"
+        "@p bra.uni GG_DONE;\n\t"
+        "mov.u32 n, %0;\n\t"
+        "GG_WAIT:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra.uni GG_DONE;\n\t"
+        "setp.eq.u32 p, n, 0;\n\t"
+        "@p bra.uni GG_OUT;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "bra.uni GG_WAIT;\n\t"
+        "GG_OUT:\n\t"
+        "mov.u32 %0, 0;\n\t"
+        "GG_DONE:\n\t}"
+        : "+r"(limit)
+        : "r"(bar), "r"(parity), "r"(ready)
+        : "memory");
+}
+__device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// Four K = 16 steps of one 64-column block; A in TMEM (8 columns per step), B in shared memory (32 bytes per step).
+#define GG_MMA4(A, B) \
+    "add.u32 a, " A ", 8;\n\tadd.u64 b, " B ", 2;\n\t" \
+    "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, q;\n\t" \
+    "add.u32 a, a, 8;\n\tadd.u64 b, b, 2;\n\t" \
+    "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, q;\n\t" \
+    "add.u32 a, a, 8;\n\tadd.u64 b, b, 2;\n\t" \
+    "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, q;\n\t"
+__device__ __forceinline__ void mma_block(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 a;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        GG_MMA4("%1", "%2") "}"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// The two blocks of a unit: the second one's rows of x lie `step` descriptor units further on.
+__device__ __forceinline__ void mma_unit(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint64_t step) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 a, a2;\n\t.reg .b64 b, b2;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"
+        "add.u32 a2, %1, 32;\n\tadd.u64 b2, %2, %5;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        GG_MMA4("%1", "%2")
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, q;\n\t"
+        GG_MMA4("a2", "b2") "}"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "l"(step)
+        : "memory");
+}
+#undef GG_MMA4
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t h2fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2sub(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2mul(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t perm(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+__device__ __forceinline__ float half_at(uint32_t pair, int hi) { return f16_bits_to_float((uint16_t)(hi ? pair >> 16 : pair)); }
+__device__ __forceinline__ float byte_at(uint32_t v, int i) {           // 2^23 + b is exact
+    return __uint_as_float(perm(v, 0x4B000000u, 0x7650u + (uint32_t)i)) - 8388608.f;
+}
+__device__ __forceinline__ uint32_t bf2(float lo, float hi) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+}
+
+// A run of this CTA's units inside one tile.
+struct Seg {
+    int p, tile, chunk, k0, k1;            // problem, tile, row chunk, 128-column units [k0, k1)
+    int u0;                                // first unit, counted from the CTA's first
+};
+__device__ __forceinline__ bool next_seg(const Shared& sh, int ubegin, int uend, int at, int units_k, Seg& s) {
+    const int u = ubegin + at;
+    if (u >= uend) return false;
+    int p = s.p;
+    while (u >= sh.ubase[p + 1]) ++p;
+    const int rel = u - sh.ubase[p];
+    const int item = rel / units_k;
+    s.p = p;
+    s.k0 = rel - item * units_k;
+    s.k1 = min(units_k, s.k0 + (uend - u));
+    const int chunks = sh.pr[p].chunks;
+    s.tile = item / chunks;
+    s.chunk = item - s.tile * chunks;
+    s.u0 = at;
+    return true;
+}
+
+template <int NBITS, int GS, int MODE>
+__global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__ Params prm) {
+    using F = Fmt<NBITS, GS>;
+    constexpr int PER = F::PER, PARTS = F::PARTS, SLW = F::SLW, UK = F::UK, HALVES = F::HALVES, BLOCKS = F::BLOCKS, DC = F::DC;
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ Shared sh;
+    const uint32_t raw0 = smem_u32(smem_raw);
+    unsigned char* base = smem_raw + ((1024u - (raw0 & 1023u)) & 1023u);
+    const uint32_t sbase = smem_u32(base);
+    const int n_raw = F::n_raw(prm.n_max), ring = F::b_ring(prm.n_max);
+    const uint32_t b_ring = sbase + (F::RING_OFF + 1023) / 1024 * 1024, raw_ring = b_ring + ring;
+    const uint32_t bars = sbase + F::BAR_OFF;
+    const uint32_t raw_full = bars, raw_empty = raw_full + 8 * MAX_RAW, a_full = raw_empty + 8 * MAX_RAW, a_empty = a_full + 8 * NA,
+                   b_full = a_empty + 16 * NA, b_empty = b_full + 8 * MAX_B_STAGES, acc_full = b_empty + 8 * MAX_B_STAGES,
+                   acc_empty = acc_full + 16;
+    static_assert(N_BARS * 8 <= 1024, "barrier area");
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int K = prm.K, units_k = prm.units_k;
+    const int grid = (int)gridDim.x, cta = (int)blockIdx.x;
+    const bool counted = prm.counts != nullptr;
+
+    grid_launch_dependents();
+    // ---- set-up: barriers, TMEM, problems side by side on three warps
+    if (warp == WARP_RAW) {
+        for (int i = lane; i < N_BARS; i += 32) {
+            // a slot of packed bytes is released, an A slot filled, by the four warps of a group, an accumulator by four warps
+            const bool four = (i >= MAX_RAW && i < 2 * MAX_RAW + NA) || i >= N_BARS - 2;
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8 * i), "r"(four ? 4u : 1u));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == WARP_MMA) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem)), "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (lane == 0) sh.failed = 0;
+    }
+    // the row counts come from a kernel in front; without them the copies of the weights may start at once
+    if (counted) grid_dependency_wait();
+    if (warp == 0) {
+        // lane e: problem e, its units and their cost; prefix sums over the lanes
+        const int e = lane;
+        int cnt = 0, units = 0, rows = 0, cost = 0;
+        if (e < prm.problems) {
+            Problem& p = sh.pr[e];
+            const HostProblem& h = prm.hp[prm.table ? 0 : e];
+            cnt = counted ? __ldcg(prm.counts + e) : prm.rows;
+#pragma unroll
+            for (int l = 0; l < 2; ++l) {
+                if (prm.table) {
+                    const StreamEntry* en = prm.table + 3 * e + (l ? prm.which1 : prm.which0);
+                    p.w[l].meta[0] = en->w.ms_scale;
+                    p.w[l].meta[1] = en->w.mz_scale;
+                    p.w[l].meta[2] = en->w.ms_zero;
+                    p.w[l].meta[3] = en->w.mz_zero;
+                    p.w[l].maps = reinterpret_cast<const CUtensorMap*>(en->maps);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) p.w[l].meta[i] = h.meta[l][i];
+                    p.w[l].maps = h.maps[l];
+                }
+            }
+            p.G = h.G;
+            p.P = h.P;
+            p.C = h.C;
+            p.tiles = h.tiles;
+            p.cnt = cnt;
+            const GgRows r = counted ? GgRows::of(cnt) : GgRows{prm.chunks, prm.n_max};
+            p.n = r.n;
+            p.chunks = r.chunks;
+            p.f16 = (MODE != GG_DOWN || cnt <= GG_F16_ROWS) ? 1 : 0;
+            // cycles of 128 columns: the dequantisation, or the MMAs (4 per row)
+            cost = unit_cycles(p.f16, p.n);
+            p.cost = cost;
+            rows = r.padded();
+            units = h.tiles * r.chunks * units_k;
+        }
+        int row1 = rows, list1 = cnt, u1 = units;
+        unsigned long long c1 = (unsigned long long)units * (unsigned)cost;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, row1, o), b = __shfl_up_sync(0xffffffffu, list1, o), c = __shfl_up_sync(0xffffffffu, u1, o);
+            const unsigned long long d = __shfl_up_sync(0xffffffffu, c1, o);
+            if (lane >= o) {
+                row1 += a;
+                list1 += b;
+                u1 += c;
+                c1 += d;
+            }
+        }
+        if (e < prm.problems) {
+            sh.pr[e].row0 = counted ? row1 - rows : 0;
+            sh.pr[e].list0 = counted ? list1 - cnt : 0;
+            sh.ubase[e + 1] = u1;
+            sh.cbase[e + 1] = c1;
+        }
+        if (e == 0) {
+            sh.ubase[0] = 0;
+            sh.cbase[0] = 0;
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if ((int)threadIdx.x <= grid) {
+        const unsigned long long total = sh.cbase[prm.problems];
+        const unsigned long long at = total * (unsigned long long)threadIdx.x / (unsigned)grid;
+        int e = 0;
+        while (e < prm.problems - 1 && at >= sh.cbase[e + 1]) ++e;
+        const unsigned long long rel = at - sh.cbase[e];
+        const unsigned cost = (unsigned)max(1, sh.pr[e].cost);
+        sh.begin[threadIdx.x] = (int)threadIdx.x == grid ? sh.ubase[prm.problems] : sh.ubase[e] + (int)((rel + cost - 1) / cost);
+    }
+    __syncthreads();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem, 0);
+    const int ub = sh.begin[cta], ue = sh.begin[cta + 1];
+    const TmemMap tmap = TmemMap::of(prm.n_max);
+    const int slots = tmap.slots;
+
+    if (warp < WARP_EPI) {
+        regs_up<REGS_DEQUANT>();
+        // =========================== dequantisation ===========================
+        const int group = warp >> 2, q = warp & 3, g = lane >> 2, c = lane & 3;
+        const int part = F::part_of(q, g), slot = F::slot_of(q);
+        // the row of scales / zeros this lane decodes: DC columns of it
+        const int dpart = (SLW == 2) ? lane >> 4 : part;
+        const int dcol = DC * (lane & (UK / DC - 1));
+        const int dhalf = dcol >> 7;
+        // The field of the warp's slot inside a byte.  2 bit: slots 0, 1 at bits 7-6, 5-4, slots 2, 3 at 3-2, 1-0; 4 bit: 7-4 or
+        // 3-0.  `upper`: it lies in the upper half of the byte; fpos: its first bit inside that half.
+        const bool upper = (NBITS == 2) ? q < 2 : (q & 1) == 0;
+        const int fpos = (NBITS == 2) ? ((q & 1) ? 0 : 2) : 0;
+        const uint32_t field = (NBITS == 2) ? 3u : 15u;
+        const uint32_t mask_hi = (field << (4 + fpos)) * 0x00010001u;      // field in bits 7-4 of each half
+        const uint32_t mask_lo = (field << fpos) * 0x00010001u;            // field in bits 3-0 of each half
+        // s / t of the warp: [block][half][part][thread column][8 values], s first; 16-byte pieces, so that the eight lanes of
+        // a load phase touch 128 contiguous bytes
+        const uint32_t st_area = sbase + F::ST_OFF + warp * F::ST_WARP;
+        const uint32_t st_read = st_area + ((SLW == 2) ? (g & 1) * 64 : 0) + c * 16;
+        // this thread's bytes of a staged row: 16 of a 64-column block, members j = 0, 1 (the 128-byte swizzle)
+        uint32_t code_off[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int m = F::member_of(q, g, j);
+            code_off[j] = (uint32_t)(part * F::CODE_PART + m * 128 + ((c ^ (m & 7)) << 4));
+        }
+        constexpr int J2 = (GS == 16 ? 8 : 16) * 128;                      // from members j = 0, 1 to j = 2, 3
+
+        Seg s;
+        s.p = 0;
+        int at = 0;
+        bool ok = true;
+        // meta values (fp16 scale / zero of the 8-bit scale and zero bytes), requested a unit ahead
+        uint32_t mt[4][DC / 2];
+        int mcol = 0, mC = 1, mstep = 0;
+        const uint16_t* mp[4] = {nullptr, nullptr, nullptr, nullptr};
+        auto load_meta = [&]() {
+            if ((mC & 7) == 0) {
+#pragma unroll
+                for (int h = 0; h < (DC + 7) / 8; ++h) {
+                    int col = mcol + 8 * h;
+                    if (col >= mC) col -= mC;
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        if constexpr (DC >= 8) {
+                            const uint4 v = __ldg(reinterpret_cast<const uint4*>(mp[a] + col));
+                            mt[a][4 * h] = v.x; mt[a][4 * h + 1] = v.y; mt[a][4 * h + 2] = v.z; mt[a][4 * h + 3] = v.w;
+                        } else {
+                            const uint2 v = __ldg(reinterpret_cast<const uint2*>(mp[a] + col));
+                            mt[a][0] = v.x; mt[a][1] = v.y;
+                        }
+                    }
+                }
+            } else {                                          // a run of columns may wrap around anywhere: one by one
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int j = 0; j < DC / 2; ++j) {
+                        const uint32_t lo = __ldg(mp[a] + (mcol + 2 * j) % mC), hi = __ldg(mp[a] + (mcol + 2 * j + 1) % mC);
+                        mt[a][j] = lo | (hi << 16);
+                    }
+            }
+        };
+        int r = group, v = group * HALVES;                    // slots of this group's next unit: packed bytes; A, and its phase
+        uint32_t r_par = 0, v_round = 0;
+        while (v >= slots) {
+            v -= slots;
+            ++v_round;
+        }
+        while (ok && next_seg(sh, ub, ue, at, units_k, s)) {
+            const int n_seg = s.k1 - s.k0;
+            at += n_seg;
+            int first = group - s.u0 % GROUPS;                // first unit of the run that is this group's
+            if (first < 0) first += GROUPS;
+            if (first >= n_seg) continue;
+            const Problem& pr = sh.pr[s.p];
+            const bool f16 = pr.f16 != 0;
+            const int wsel = (MODE == GG_UP) ? dpart : 0;
+            const int rho = (MODE == GG_UP) ? s.tile : s.tile * PARTS + dpart;
+            const int res = min(PER * rho + slot, pr.G - 1);  // (a tile's second part may lie past the last residue)
+            mC = pr.C;
+#pragma unroll
+            for (int a = 0; a < 4; ++a) mp[a] = pr.w[wsel].meta[a];
+            mcol = (int)(((uint64_t)res * (uint32_t)K + (uint32_t)((s.k0 + first) * UK + dcol)) % (uint32_t)mC);
+            mstep = (GROUPS * UK) % mC;
+            load_meta();
+            for (int k = s.k0 + first; k < s.k1; k += GROUPS) {
+                if (!wait(raw_full + 8 * r, r_par)) ok = false;
+                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                const uint32_t rw = raw_ring + r * F::RAW_BYTES;
+                uint4 wv[4];
+                auto load_codes = [&](int sub) {
+                    const uint32_t at0 = rw + (sub >> 1) * F::CODE_HALF;
+                    const uint32_t c0 = at0 + (code_off[0] ^ (64u * (sub & 1))), c1 = at0 + (code_off[1] ^ (64u * (sub & 1)));
+                    wv[0] = lds128(c0);
+                    wv[1] = lds128(c1);
+                    wv[2] = lds128(c0 + J2);
+                    wv[3] = lds128(c1 + J2);
+                };
+                // ---- scale and zero of the warp's rows
+                bool big = false;
+                {
+                    const uint32_t sqa = rw + F::SQ_OFF + (dhalf * PARTS + dpart) * F::SZ_PART + slot * 128 + (dcol & 127);
+                    constexpr int ZS = F::ZQ_OFF - F::SQ_OFF;
+                    uint32_t sq[DC / 4], zq[DC / 4];
+                    if constexpr (DC == 16) {
+                        const uint4 a = lds128(sqa), b = lds128(sqa + ZS);
+                        sq[0] = a.x; sq[1] = a.y; sq[2] = a.z; sq[3] = a.w;
+                        zq[0] = b.x; zq[1] = b.y; zq[2] = b.z; zq[3] = b.w;
+                    } else if constexpr (DC == 8) {
+                        const uint2 a = lds64(sqa), b = lds64(sqa + ZS);
+                        sq[0] = a.x; sq[1] = a.y; zq[0] = b.x; zq[1] = b.y;
+                    } else {
+                        sq[0] = lds32(sqa);
+                        zq[0] = lds32(sqa + ZS);
+                    }
+                    load_codes(0);                            // on their way while the scales are decoded
+                    uint32_t S[DC / 2], T[DC / 2];            // per four columns: pair (0, 2), pair (1, 3)
+                    if (f16) {
+                        // s * 2^(22 - p) and -z * s / 4, p = 4 + fpos the field's first bit
+#pragma unroll
+                        for (int j = 0; j < DC / 4; ++j) {
+                            uint32_t s2[2], z2[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const uint32_t sel = e ? 0x4342u : 0x4140u;
+                                const uint32_t qs = h2sub(perm(sq[j], 0x64646464u, sel), 0x64006400u);
+                                const uint32_t qz = h2sub(perm(zq[j], 0x64646464u, sel), 0x64006400u);
+                                s2[e] = h2mul(h2sub(qs, mt[1][2 * j + e]), mt[0][2 * j + e]);
+                                z2[e] = h2mul(h2sub(qz, mt[3][2 * j + e]), mt[2][2 * j + e]);
+                            }
+                            // to the order (0, 2), (1, 3)
+                            S[2 * j] = perm(s2[0], s2[1], 0x5410u);
+                            S[2 * j + 1] = perm(s2[0], s2[1], 0x7632u);
+                            T[2 * j] = h2mul(perm(z2[0], z2[1], 0x5410u), h2mul(S[2 * j], 0xB400B400u));          // -z * (s / 4)
+                            T[2 * j + 1] = h2mul(perm(z2[0], z2[1], 0x7632u), h2mul(S[2 * j + 1], 0xB400B400u));
+                        }
+                        // |s| * 2^(18 - fpos) must stay finite: |s| < 1/4 (fpos = 2: < 1)
+                        uint32_t mx = 0;
+#pragma unroll
+                        for (int j = 0; j < DC / 2; ++j) mx = __vmaxu2(mx, S[j] & 0x7FFF7FFFu);
+                        big = __any_sync(0xffffffffu, (mx & 0xffffu) > 0x33FFu || (mx >> 16) > 0x33FFu);           // 1/4 and more
+                        // * 2^(18 - fpos), exact; big: the field will be read as c * 2^(4 + fpos), so s / 4 / 2^(4 + fpos)
+                        const uint32_t f1 = big ? 0x3C003C00u : 0x64006400u;
+                        const uint32_t f2 = big ? (fpos ? 0x1C001C00u : 0x24002400u) : (fpos ? 0x54005400u : 0x5C005C00u);
+#pragma unroll
+                        for (int j = 0; j < DC / 2; ++j) S[j] = h2mul(h2mul(S[j], f1), f2);
+                    } else {
+                        // bf16: s * 2^-fpos and -z * s, computed in fp32
+                        const float down = fpos ? 0.25f : 1.f;
+#pragma unroll
+                        for (int j = 0; j < DC / 4; ++j) {
+                            float sc[4], tt[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int i = 2 * j + (e >> 1);
+                                sc[e] = (byte_at(sq[j], e) - half_at(mt[1][i], e & 1)) * half_at(mt[0][i], e & 1);
+                                const float z = (byte_at(zq[j], e) - half_at(mt[3][i], e & 1)) * half_at(mt[2][i], e & 1);
+                                tt[e] = -z * sc[e];
+                                sc[e] *= down;
+                            }
+                            S[2 * j] = bf2(sc[0], sc[2]);
+                            S[2 * j + 1] = bf2(sc[1], sc[3]);
+                            T[2 * j] = bf2(tt[0], tt[2]);
+                            T[2 * j + 1] = bf2(tt[1], tt[3]);
+                        }
+                    }
+                    // publish to the warp
+#pragma unroll
+                    for (int h = 0; h < (DC + 7) / 8; ++h) {
+                        const int w64 = (dcol + 8 * h) & 63, blk = (dcol + 8 * h) >> 6;
+                        const uint32_t dst = st_area + blk * F::ST_BLOCK + ((w64 >> 3) & 1) * (SLW * 64) + ((SLW == 2) ? dpart * 64 : 0) +
+                                             (w64 >> 4) * 16 + (w64 & 7) * 2;
+                        if constexpr (DC >= 8) {
+                            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(S[4 * h]), "r"(S[4 * h + 1]), "r"(S[4 * h + 2]), "r"(S[4 * h + 3]) : "memory");
+                            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + F::ST_T), "r"(T[4 * h]), "r"(T[4 * h + 1]), "r"(T[4 * h + 2]), "r"(T[4 * h + 3]) : "memory");
+                        } else {
+                            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst), "r"(S[0]), "r"(S[1]) : "memory");
+                            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst + F::ST_T), "r"(T[0]), "r"(T[1]) : "memory");
+                        }
+                    }
+                }
+                if (k + GROUPS < s.k1) {                      // the next unit's meta values
+                    mcol += mstep;
+                    if (mcol >= mC) mcol -= mC;
+                    load_meta();
+                }
+                __syncwarp();
+                // ---- the weights, 64 columns at a time
+                const int subs = min(BLOCKS, prm.subs_k - BLOCKS * k);
+#pragma unroll
+                for (int half = 0; half < HALVES; ++half) {
+                    const int av = v + half, aslot = av >= slots ? av - slots : av;
+                    const uint32_t round = v_round + (av >= slots ? 1u : 0u);
+                    // The A slot's tile of the round before has been read by its MMAs.  (A parity only tells the last phase from
+                    // the one before it, and with two slots to a unit a group may be two rounds behind when it comes to wait:
+                    // even and odd rounds have barriers of their own.)
+                    if (round > 0 && !wait(a_empty + 8 * (aslot + ((round & 1) ? 0 : NA)), ((round - 1) >> 1) & 1)) ok = false;
+                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t ta = tmem + tmap.a_base + 64 * aslot + ((uint32_t)(32 * q) << 16);
+#pragma unroll
+                    for (int sub2 = 0; sub2 < 2; ++sub2) {
+                        const int sub = 2 * half + sub2;
+                        if (sub < subs) {
+                            const uint32_t sa = st_read + sub * F::ST_BLOCK;
+                            const uint4 S0 = lds128(sa), S1 = lds128(sa + SLW * 64), T0 = lds128(sa + F::ST_T), T1 = lds128(sa + F::ST_T + SLW * 64);
+                            if (sub) load_codes(sub);
+                            const uint32_t SS[8] = {S0.x, S0.y, S0.z, S0.w, S1.x, S1.y, S1.z, S1.w};
+                            const uint32_t TT[8] = {T0.x, T0.y, T0.z, T0.w, T1.x, T1.y, T1.z, T1.w};
+                            // one pair of weights per (member, word i, e): fields of bytes (0, 2) and (1, 3) of the word
+                            auto all = [&](auto&& pair_lo, auto&& pair_hi) {
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    uint32_t o[16];
+#pragma unroll
+                                    for (int b = 0; b < 2; ++b) {
+                                        const uint4 vv = wv[2 * h + b];
+                                        const uint32_t w[4] = {vv.x, vv.y, vv.z, vv.w};
+#pragma unroll
+                                        for (int i = 0; i < 4; ++i) {
+                                            o[4 * i + 2 * b] = pair_lo(w[i], SS[2 * i], TT[2 * i]);
+                                            o[4 * i + 2 * b + 1] = pair_hi(w[i], SS[2 * i + 1], TT[2 * i + 1]);
+                                        }
+                                    }
+                                    asm volatile(
+                                        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                                        ::"r"(ta + 32 * sub2 + ((uint32_t)(16 * h) << 16)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]),
+                                        "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]),
+                                        "r"(o[14]), "r"(o[15])
+                                        : "memory");
+                                }
+                            };
+                            // (the shift to the left is written as a product: it then runs beside the ANDs, on the other pipe)
+                            if (f16 && !big) {
+                                if (upper)
+                                    all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(x & mask_hi, S, T); },
+                                        [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x >> 8) & mask_hi, S, T); });
+                                else
+                                    all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x * 16u) & mask_hi, S, T); },
+                                        [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x >> 4) & mask_hi, S, T); });
+                            } else if (f16) {
+                                const uint32_t magic = 0x64006400u, mul = upper ? 1u : 16u, sh = upper ? 8u : 4u;      // 1024
+                                all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x * mul, mask_hi, magic), magic), S, T); },
+                                    [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x >> sh, mask_hi, magic), magic), S, T); });
+                            } else {
+                                const uint32_t magic = 0x43004300u, sl = upper ? 4u : 0u;                               // 128
+                                all([&](uint32_t x, uint32_t S, uint32_t T) { return bf2_fma(bf2_sub(lop_and_or(x >> sl, mask_lo, magic), magic), S, T); },
+                                    [&](uint32_t x, uint32_t S, uint32_t T) { return bf2_fma(bf2_sub(lop_and_or(x >> (sl + 8u), mask_lo, magic), magic), S, T); });
+                            }
+                        }
+                    }
+                    if (half == HALVES - 1) {
+                        // The staged bytes have been read.  (Only here: what was loaded has been used by every lane.)
+                        __syncwarp();
+                        if (lane == 0) arrive(raw_empty + 8 * r);
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    if (lane == 0) arrive(a_full + 8 * aslot);
+                }
+                if (!ok) break;
+                r += GROUPS;
+                if (r >= n_raw) {
+                    r -= n_raw;
+                    r_par ^= 1u;
+                }
+                v += GROUPS * HALVES;
+                while (v >= slots) {
+                    v -= slots;
+                    ++v_round;
+                }
+            }
+        }
+        if (!ok) sh.failed = 1;
+    } else if (warp >= WARP_RAW) {
+        regs_down<REGS_ISSUE>();
+        // The copying and the MMA-issuing warps: all lanes run the same code on the same values and an elected one issues, so
+        // that the operands live in uniform registers (a tiled copy then costs 30 cycles, 100 when lanes issue one each).
+        const bool leader = elect_one();
+        uint32_t limit = WAIT_LIMIT;
+        Seg s;
+        s.p = 0;
+        int at = 0;
+        if (warp < WARP_B) {
+            // =========================== packed weights: two warps, every other unit each ===========================
+            const int turn = warp - WARP_RAW;
+            int fenced = -1;
+            while (next_seg(sh, ub, ue, at, units_k, s)) {
+                at += s.k1 - s.k0;
+                const Problem& pr = sh.pr[s.p];
+                const CUtensorMap* maps[2] = {pr.w[0].maps, pr.w[MODE == GG_UP ? 1 : 0].maps};
+                const int rho0 = (MODE == GG_UP) ? s.tile : s.tile * PARTS;
+                if (prm.table && fenced != s.p) {             // tensor maps in global memory
+                    fenced = s.p;
+#pragma unroll
+                    for (int i = 0; i < 3 * (MODE == GG_UP ? 2 : 1); ++i)
+                        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(maps[i / 3] + i % 3) : "memory");
+                }
+                for (int k = s.k0 + ((s.u0 ^ turn) & 1); k < s.k1; k += 2) {
+                    const int u = s.u0 + (k - s.k0), r = u & (n_raw - 1);         // n_raw is 4 or 8
+                    wait_limited(raw_empty + 8 * r, ((n_raw == 8 ? u >> 3 : u >> 2) & 1) ^ 1, limit);
+                    const uint32_t bar = raw_full + 8 * r, dst = raw_ring + r * F::RAW_BYTES;
+                    if (leader) {
+                        expect_tx(bar, F::RAW_TX);
+#pragma unroll
+                        for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+                            for (int p = 0; p < PARTS; ++p) {
+                                const int rho = (MODE == GG_UP) ? rho0 : rho0 + p, col = k * UK + 128 * h;
+#pragma unroll
+                                for (int b = 0; b < GS / 16; ++b)
+                                    tma_3d(dst + h * F::CODE_HALF + p * F::CODE_PART + b * 2048, maps[p], col, rho, 16 * b, bar);
+                                tma_3d(dst + F::SQ_OFF + (h * PARTS + p) * F::SZ_PART, maps[p] + 1, col, PER * rho, 0, bar);
+                                tma_3d(dst + F::ZQ_OFF + (h * PARTS + p) * F::SZ_PART, maps[p] + 2, col, PER * rho, 0, bar);
+                            }
+                    }
+                }
+            }
+        } else if (warp == WARP_B) {
+            // =========================== rows of x ===========================
+            // Where the stage size changes the ring is emptied first, so that both sides start over at stage 0.
+            if (!counted) grid_dependency_wait();
+            int cls = 0, st = 0, filled = 0;                  // filled: stages that have been used since the last change
+            uint32_t par = 0xffffffffu;                       // bit i: parity that a wait for "stage i is free" expects
+            while (next_seg(sh, ub, ue, at, units_k, s)) {
+                at += s.k1 - s.k0;
+                const Problem& pr = sh.pr[s.p];
+                const BClass bc = BClass::of(pr.n, ring);
+                if (bc.bytes != cls) {
+                    for (int i = 0; i < filled; ++i) wait_limited(b_empty + 8 * i, (par >> i) & 1, limit);       // its last use has been read
+                    // (the stage's next fill waits for the same phase again, and finds it complete)
+                    cls = bc.bytes;
+                    st = 0;
+                    filled = 0;
+                }
+                const uint32_t bytes = (uint32_t)pr.n * 128u;
+                const unsigned char* src = prm.xt + ((int64_t)(BLOCKS * s.k0) * prm.xt_rows + pr.row0 + s.chunk * pr.n) * 128;
+                const int64_t step = prm.xt_rows * 128;
+                const int b1 = min(BLOCKS * s.k1, prm.subs_k);
+                for (int b = BLOCKS * s.k0; b < b1; b += bc.blocks) {
+                    wait_limited(b_empty + 8 * st, (par >> st) & 1, limit);
+                    par ^= 1u << st;
+                    const int blocks = min(bc.blocks, b1 - b);
+                    if (leader) {
+                        const uint32_t dst = b_ring + (uint32_t)st * (uint32_t)bc.bytes, bar = b_full + 8 * st;
+                        expect_tx(bar, bytes * (uint32_t)blocks);
+                        for (int i = 0; i < blocks; ++i) bulk_load(dst + bytes * (uint32_t)i, src + step * i, bytes, bar);
+                    }
+                    src += step * bc.blocks;
+                    if (st + 1 > filled) filled = st + 1;
+                    st = (st + 1 == bc.stages) ? 0 : st + 1;
+                }
+            }
+        } else {
+            // =========================== MMAs ===========================
+            const uint32_t a_first = tmem + tmap.a_base, a_end = a_full + 8 * (uint32_t)slots;
+            uint32_t a_bar = a_full, a_tmem = a_first, a_par = 0;            // the A slot of the next 128 columns
+            uint32_t par = 0;                                 // bit i: parity that a wait for "stage i is filled" expects
+            int cls = 0, st = 0, seg = 0;
+            bool prev_wide = false;
+            uint32_t ready = 0;
+            while (next_seg(sh, ub, ue, at, units_k, s)) {
+                at += s.k1 - s.k0;
+                const Problem& pr = sh.pr[s.p];
+                const int n = pr.n;
+                const bool wide = n > 128;
+                const BClass bc = BClass::of(n, ring);
+                if (bc.bytes != cls) {
+                    cls = bc.bytes;
+                    st = 0;
+                }
+                const uint32_t idesc = (1u << 4) | (pr.f16 ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
+                const int buf = wide ? 0 : seg & 1;
+                // the accumulator is free: the run before last has been read; next to a run of more than 128 rows, the last one
+                const int need = (wide || prev_wide) ? seg - 1 : seg - 2;
+                if (need >= 0) wait_limited(acc_empty + 8 * (need & 1), (need >> 1) & 1, limit);
+                prev_wide = wide;
+                const uint32_t d = tmem + tmap.d_step * (uint32_t)buf;
+                const uint32_t sub_step = (uint32_t)n * 8u;   // descriptor units of a 64-column block: (n rows * 128 bytes) / 16
+                const uint64_t desc = (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+                uint32_t acc = 0;
+                int left = 0;                                 // units of the current stage of x still to be used
+                uint64_t bd = 0;
+                for (int k = s.k0; k < s.k1; ++k) {
+                    const uint32_t bar = a_bar, ta = a_tmem, a_done = a_bar + (a_par ? 16 * NA : 8 * NA);
+                    wait_peeked(bar, a_par, ready, limit);
+                    a_bar += 8;
+                    a_tmem += 64;
+                    if (a_bar == a_end) {
+                        a_bar = a_full;
+                        a_tmem = a_first;
+                        a_par ^= 1u;
+                    }
+                    ready = peek(a_bar, a_par);               // of the next unit, while this one's MMAs are issued
+                    const bool two = 2 * k + 1 < prm.subs_k;  // (K may be an odd number of blocks)
+                    if (!wide) {
+                        if (left == 0) {
+                            wait_limited(b_full + 8 * st, (par >> st) & 1, limit);
+                            par ^= 1u << st;
+                            left = min(bc.blocks >> 1, s.k1 - k);
+                            bd = desc | (((b_ring + (uint32_t)st * (uint32_t)bc.bytes) & 0x3FFFFu) >> 4);
+                        }
+                        --left;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (leader) {
+                            if (two) mma_unit(d, ta, bd, idesc, acc, sub_step);
+                            else mma_block(d, ta, bd, idesc, acc);
+                            commit(a_done);
+                            if (left == 0) commit(b_empty + 8 * st);
+                        }
+                        bd += 2 * sub_step;
+                        if (left == 0) st = (st + 1 == bc.stages) ? 0 : st + 1;
+                    } else {                                  // a stage is one block
+                        for (int i = 0; i < (two ? 2 : 1); ++i) {
+                            wait_limited(b_full + 8 * st, (par >> st) & 1, limit);
+                            par ^= 1u << st;
+                            bd = desc | (((b_ring + (uint32_t)st * (uint32_t)bc.bytes) & 0x3FFFFu) >> 4);
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            if (leader) {
+                                mma_block(d, ta + 32 * i, bd, idesc, i ? 1u : acc);
+                                commit(b_empty + 8 * st);
+                            }
+                            st = (st + 1 == bc.stages) ? 0 : st + 1;
+                        }
+                        if (leader) commit(a_done);
+                    }
+                    acc = 1;
+                }
+                if (leader) commit(acc_full + 8 * (seg & 1));
+                ++seg;
+            }
+        }
+        if (limit == 0) sh.failed = 1;
+    } else {
+        regs_down<REGS_EPI>();
+        // =========================== epilogue ===========================
+        if (!counted) grid_dependency_wait();
+        const int q = warp & 3, g = lane & 7, j4 = lane >> 3;         // TMEM lane 32 q + 8 j4 + g
+        const int et = threadIdx.x - WARP_EPI * 32;                   // thread of the epilogue
+        const int part = F::part_of(q, g), slot = F::slot_of(q), member = F::member_of(q, g, j4);
+        constexpr int RUN = PARTS * PER;                              // neighbouring output rows of a member in a tile
+        unsigned char* epi = base + F::EPI_OFF;
+        float* s_scale = reinterpret_cast<float*>(epi + 2 * TILE_BYTES);      // per row of the chunk: factor of the sums,
+        float* s_weight = s_scale + GG_MAX_ROWS;                              // routing weight,
+        int* s_row = reinterpret_cast<int*>(s_weight + GG_MAX_ROWS);          // output row
+        auto epi_sync = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+        Seg s;
+        s.p = 0;
+        int at = 0, seg = 0, turn = 0;
+        bool ok = true;
+        while (next_seg(sh, ub, ue, at, units_k, s)) {
+            at += s.k1 - s.k0;
+            const Problem& pr = sh.pr[s.p];
+            const int n = pr.n, cnt = pr.cnt;
+            const bool wide = n > 128;
+            const int buf = wide ? 0 : seg & 1;
+            const bool whole = s.k0 == 0 && s.k1 == units_k;
+            const int rows_here = min(n, cnt - s.chunk * n);          // rows of this chunk that exist
+            const int list = pr.list0 + s.chunk * n;                  // list entry of the chunk's first row
+            const int rho0 = (MODE == GG_UP) ? s.tile : s.tile * PARTS;
+            const int rho = (MODE == GG_UP) ? s.tile : rho0 + part;
+            // what the rows need is fetched while the sums are still being formed
+            for (int i = et; i < rows_here; i += 128) {
+                s_scale[i] = (pr.f16 ? F16_SCALE : 1.f) * (prm.row_scale ? __ldcg(prm.row_scale + pr.row0 + s.chunk * n + i) : 1.f);
+                if (MODE == GG_DOWN) {
+                    s_weight[i] = prm.row_w ? __ldcg(prm.row_w + list + i) : 1.f;
+                    s_row[i] = prm.out_idx ? __ldcg(prm.out_idx + list + i) : list + i;
+                }
+            }
+            float bias = 0.f;
+            if (MODE == GG_LINEAR) {
+                const uint16_t* bp = prm.hp[s.p].bias;
+                if (bp && rho < pr.P) bias = bf16_bits_to_float(bp[member * pr.G + PER * rho + slot]);
+            }
+            if (!wait(acc_full + 8 * (seg & 1), (seg >> 1) & 1)) ok = false;
+            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t td = tmem + tmap.d_step * (uint32_t)buf + ((uint32_t)(32 * q) << 16);
+            auto load16 = [&](int c0, float (&v)[16]) {
+                uint32_t r[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                    : "r"(td + (uint32_t)c0));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+            };
+            auto release = [&] {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) arrive(acc_empty + 8 * (seg & 1));
+            };
+            int c_first = cta, c_last = cta;
+            bool finish = true;
+            if (!whole) {
+                // the tile's units are cut over the CTAs c_first .. c_last: leave this CTA's piece, the last one to arrive adds them
+                const int t0 = ub + s.u0 - s.k0;
+                while (c_first > 0 && sh.begin[c_first] > t0) --c_first;
+                int parts_n = 0;
+                while (c_last + 1 < grid && sh.begin[c_last + 1] < t0 + units_k) ++c_last;
+                for (int c = c_first; c <= c_last; ++c) parts_n += sh.begin[c + 1] > sh.begin[c] ? 1 : 0;
+                // [4 rows of x][128 tile rows][4]: a warp writes and reads 512 contiguous bytes at a time
+                float4* mine = reinterpret_cast<float4*>(prm.parts) + (size_t)(2 * cta + (s.k0 == 0 ? 1 : 0)) * prm.n_max * 32 + 32 * q + lane;
+                for (int c0 = 0; c0 < rows_here; c0 += 16) {
+                    float v[16];
+                    load16(c0, v);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        __stcg(mine + (size_t)(c0 / 4 + i) * 128, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+                }
+                release();
+                __threadfence();
+                epi_sync();
+                if (et == 0) {
+                    const unsigned arrived = atomicAdd(prm.counters + c_first, 1u);
+                    if (arrived >= (unsigned)parts_n && prm.error_flag) atomicExch(prm.error_flag, 3);
+                    sh.last = arrived == (unsigned)(parts_n - 1);
+                    if (sh.last) prm.counters[c_first] = 0u;
+                    __threadfence();
+                }
+                epi_sync();
+                finish = sh.last != 0;
+                __threadfence();
+            } else {
+                epi_sync();                                           // s_scale and the others are complete
+            }
+            if (finish) {
+                // 8 rows of the sum of the pieces, in CTA order (a CTA without a unit has none), four pieces on their way at
+                // once: what a tile of many short pieces costs is their latency
+                auto add_pieces = [&](int r0, float* v) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] = 0.f;
+                    for (int cb = c_first; cb <= c_last; cb += 4) {
+                        float4 f[4][2];
+#pragma unroll
+                        for (int d = 0; d < 4; ++d) {
+                            const int c = cb + d;
+                            const bool has = c <= c_last && sh.begin[c + 1] > sh.begin[c];
+                            const float4* src = reinterpret_cast<const float4*>(prm.parts) + ((size_t)(2 * c + (c == c_first ? 1 : 0)) * prm.n_max + r0) * 32 + 32 * q + lane;
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) f[d][i] = has ? __ldcg(src + (size_t)i * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+#pragma unroll
+                        for (int d = 0; d < 4; ++d)
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                v[4 * i] += f[d][i].x;
+                                v[4 * i + 1] += f[d][i].y;
+                                v[4 * i + 2] += f[d][i].z;
+                                v[4 * i + 3] += f[d][i].w;
+                            }
+                    }
+                };
+                for (int c0 = 0; c0 < rows_here; c0 += 16) {
+                    float v[16];
+                    if (whole) {
+                        load16(c0, v);
+                        if (c0 + 16 >= rows_here) release();
+                    } else {
+                        add_pieces(c0, v);
+                        add_pieces(c0 + 8, v + 8);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 f = *reinterpret_cast<const float4*>(s_scale + c0 + 4 * i);
+                        v[4 * i] *= f.x;
+                        v[4 * i + 1] *= f.y;
+                        v[4 * i + 2] *= f.z;
+                        v[4 * i + 3] *= f.w;
+                    }
+                    uint16_t* tb = reinterpret_cast<uint16_t*>(epi + turn * TILE_BYTES);
+                    turn ^= 1;                                        // two buffers: one barrier per 16 rows
+                    if constexpr (MODE == GG_UP) {
+                        // neighbouring lanes hold the gate (even) and the up (odd) sums of one row of h; each finishes 8 rows of x
+                        const bool up = (lane & 1) != 0;
+                        uint16_t hv[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const float give = up ? v[i] : v[i + 8];
+                            const float other = __shfl_xor_sync(0xffffffffu, give, 1);
+                            const float a = round_bf16(up ? other : v[i]), b = round_bf16(up ? v[i + 8] : other);
+                            const float hh = round_bf16(round_bf16(__fdividef(a, 1.f + __expf(-a))) * b);
+                            hv[i] = cnt <= GG_F16_ROWS ? __half_as_ushort(__float2half_rn(hh)) : float_to_bf16_bits(hh);
+                        }
+                        // [row][member][slot in the order 0, 2, 1, 3]
+                        const int so = ((slot & 1) << 1) | (slot >> 1);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) tb[(i + (up ? 8 : 0)) * 64 + member * 4 + so] = hv[i];
+                        epi_sync();
+#pragma unroll
+                        for (int jj = 0; jj < 2; ++jj) {
+                            const int t = (et >> 4) + 8 * jj, m = et & 15;
+                            if (c0 + t < rows_here) {
+                                const int col = m * pr.G + PER * rho;         // four neighbouring columns of h, staged at pos .. pos + 3
+                                const int row = pr.row0 + s.chunk * n + c0 + t;
+                                const int pos = tile_pos(col & 63);
+                                unsigned char* dst = prm.ht + ((int64_t)(col >> 6) * prm.xt_rows + row) * 128 +
+                                                     ((((pos >> 3) ^ (row & 7)) << 4) | ((pos & 7) * 2));
+                                *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(tb + t * 64 + m * 4);
+                            }
+                        }
+                    } else {
+                        const int idx = member * RUN + part * PER + slot;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            uint16_t o;
+                            if (MODE == GG_LINEAR) {
+                                const float y = v[i] + bias;
+                                o = prm.y_f16 ? __half_as_ushort(__float2half_rn(y)) : float_to_bf16_bits(y);
+                            } else {
+                                o = float_to_bf16_bits(round_bf16(v[i]) * s_weight[c0 + i]);
+                            }
+                            tb[i * 128 + idx] = o;
+                        }
+                        epi_sync();
+                        constexpr int MEMBERS = 128 / RUN;
+                        const int valid = min(PARTS, pr.P - rho0) * PER;      // neighbouring rows that exist
+                        const int64_t ld = (MODE == GG_LINEAR) ? pr.G * GS : prm.N;
+                        uint16_t* out = reinterpret_cast<uint16_t*>(MODE == GG_LINEAR ? prm.hp[s.p].y : prm.out);
+#pragma unroll 2
+                        for (int j = et; j < 16 * MEMBERS; j += 128) {
+                            const int t = j / MEMBERS, m = j % MEMBERS;
+                            if (c0 + t >= rows_here) continue;
+                            const uint16_t* src = tb + t * 128 + m * RUN;
+                            const int64_t row = MODE == GG_DOWN ? s_row[c0 + t] : list + c0 + t;
+                            uint16_t* dst = out + row * ld + (int64_t)m * pr.G + PER * rho0;
+                            if (MODE == GG_DOWN && (prm.accumulate || prm.out_f16)) {
+                                for (int x = 0; x < valid; ++x) {
+                                    float val = bf16_bits_to_float(src[x]);
+                                    if (prm.accumulate) val += bf16_bits_to_float(dst[x]);
+                                    dst[x] = prm.out_f16 ? __half_as_ushort(__float2half_rn(val)) : float_to_bf16_bits(val);
+                                }
+                            } else if (valid == RUN && (((uintptr_t)dst) & (RUN * 2 - 1)) == 0) {
+                                if constexpr (RUN == 8) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+                                else if constexpr (RUN == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
+                                else *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(src);
+                            } else {
+                                for (int x = 0; x < valid; ++x) dst[x] = src[x];
+                            }
+                        }
+                    }
+                }
+            }
+            epi_sync();                                               // the row values are replaced by the next run's
+            ++seg;
+        }
+        if (!ok) sh.failed = 1;
+    }
+    // ---- teardown
+    if (sh.failed) {                          // copies may still be in flight towards this CTA's shared memory
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == WARP_MMA) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+    if (threadIdx.x == 0 && sh.failed && prm.error_flag) atomicExch(prm.error_flag, 1);
+}
+
+// Rows of x -> staged tiles [K / 64][row][64] in fp16: the rows of a chunk are contiguous, columns in tile_pos order,
+// 16-byte pieces swizzled by the row as the MMA's shared-memory descriptor expects.  A row is scaled by a power of two
+// so that its largest value lies in [16, 32): every bf16 row then fits fp16 without loss (values 2^-18 and more below the
+// largest become fp16 denormals), the epilogue multiplies by the inverse.  One CTA per row.
+template <bool X_F16>
+__global__ void __launch_bounds__(256) gg_stage_kernel(unsigned char* __restrict__ xt, float* __restrict__ row_scale, int64_t xt_rows,
+                                                       const uint16_t* __restrict__ x, const int32_t* __restrict__ idx,
+                                                       const int32_t* __restrict__ counts, int lists, int K) {
+    __shared__ float s_max[8];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int li = blockIdx.x;
+    int row = li;
+    if (counts) {
+        int list0 = 0, row0 = 0, e = 0;
+        for (; e < lists; ++e) {
+            const int c = __ldcg(counts + e);
+            if (li < list0 + c) break;
+            list0 += c;
+            row0 += GgRows::of(c).padded();
+        }
+        if (e == lists) return;                       // the lists together are shorter than the grid
+        row = row0 + (li - list0);
+    }
+    const uint16_t* src = x + (int64_t)(idx ? __ldcg(idx + li) : li) * K;
+    auto pair = [](uint32_t v, float& lo, float& hi) {
+        if (X_F16) {
+            lo = half_at(v, 0);
+            hi = half_at(v, 1);
+        } else {
+            lo = __uint_as_float(v << 16);
+            hi = __uint_as_float(v & 0xffff0000u);
+        }
+    };
+    float mx = 0.f;
+    for (int i = threadIdx.x; i < K / 8; i += 256) {
+        const uint4 v = *reinterpret_cast<const uint4*>(src + 8 * i);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float lo, hi;
+            pair(w[j], lo, hi);
+            mx = fmaxf(mx, fmaxf(fabsf(lo), fabsf(hi)));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    mx = s_max[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, s_max[w]);
+    // 2^(exponent of mx - 4); zero, tiny and infinite rows keep a finite factor
+    const int e = min(max((int)(__float_as_uint(mx) >> 23), 30), 250) - 4;
+    const float down = __uint_as_float((uint32_t)(254 - e) << 23);
+    if (threadIdx.x == 0) row_scale[row] = __uint_as_float((uint32_t)e << 23);
+    for (int i = threadIdx.x; i < K / 8; i += 256) {
+        const int b = i >> 3, ch = i & 7;
+        // piece ch of the staged block: words (thread column 2 (ch & 1), word ch >> 1) and the next thread column
+        const int k0 = b * 64 + 32 * (ch & 1) + 4 * (ch >> 1);
+        const uint2 a = *reinterpret_cast<const uint2*>(src + k0), d = *reinterpret_cast<const uint2*>(src + k0 + 16);
+        const uint32_t o[4] = {perm(a.x, a.y, 0x5410u), perm(a.x, a.y, 0x7632u), perm(d.x, d.y, 0x5410u), perm(d.x, d.y, 0x7632u)};
+        uint32_t h[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            float lo, hi;
+            pair(o[w], lo, hi);
+            const __half2 v = __floats2half2_rn(lo * down, hi * down);
+            h[w] = *reinterpret_cast<const uint32_t*>(&v);
+        }
+        *reinterpret_cast<uint4*>(xt + ((int64_t)b * xt_rows + row) * 128 + ((ch ^ (row & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+}
+
+}  // namespace gg
+
+// --------------------------------------------------------------------------- host side
+static int gg_sm_count() {
+    static int counts[MAX_DEVICES];
+    int& c = counts[current_device_slot()];
+    if (c == 0) {
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            sms <= 0)
+            sms = 148;
+        c = sms > 255 ? 255 : sms;
+    }
+    return c;
+}
+
+static constexpr int UK_MIN = 128;
+bool gg_supported(const hqm_weight* w, int G, int C) {
+    if ((w->nbits != 2 && w->nbits != 4) || !meta_uniform(w) || tma_encode_entry() == nullptr) return false;
+    const int per = codes_per_word(w->nbits), g = w->group_size;
+    if (!((w->nbits == 2 && (g == 16 || g == 32)) || (w->nbits == 4 && (g == 32 || g == 64)))) return false;
+    if (G % per != 0 || w->K % 64 != 0 || w->K < UK_MIN || C < 1) return false;
+    if ((int64_t)G * w->K >= ((int64_t)1 << 31)) return false;
+    auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    return a16(w->W_q) && a16(w->scale_q) && a16(w->zero_q) && a16(w->ms_scale) && a16(w->mz_scale) && a16(w->ms_zero) &&
+           a16(w->mz_zero);
+}
+
+static int gg_n_max(int64_t rows) {
+    const int64_t n = (rows + 15) / 16 * 16;
+    return (int)(n < 16 ? 16 : (n > GG_MAX_ROWS ? GG_MAX_ROWS : n));
+}
+static size_t gg_piece_bytes(int n) { return (size_t)2 * n * 128 * sizeof(float); }      // of one CTA
+size_t gg_scratch_bytes(int n) { return (size_t)gg_sm_count() * gg_piece_bytes(n); }
+static int64_t gg_tiles(const hqm_weight* w) {
+    const int per = codes_per_word(w->nbits), parts = 128 / (per * w->group_size);
+    return (w->N / w->group_size / per + parts - 1) / parts;
+}
+// (a layer with a tile for every SM is not worth running on a third of them)
+size_t gg_scratch_least(int n, const hqm_weight* w) {
+    return (size_t)(gg_tiles(w) >= gg_sm_count() ? gg_sm_count() : GG_LEAST_CTAS) * gg_piece_bytes(n);
+}
+
+GgLayout gg_expert_layout(int64_t M) { return GgLayout{GgRows::of((int)M), gg_sm_count()}; }
+// Rows per chunk and CTAs of a linear layer, by what a launch costs in cycles of its longest CTA:
+//   its units of 128 columns:  unit_cycles
+//   a finished tile, per 16 rows:  ~250, or 1500 + 400 p where the last CTA to arrive reads p pieces back
+// Wide chunks dequantise the weights less often; narrow ones give every SM work without cutting a tile into many pieces.
+// (4-bit 1024 x 4096, 500 rows: 51 us as four chunks of 125 rows over 148 SMs, 27 us as sixteen of 32.)
+GgLayout gg_linear_layout(int64_t M, const hqm_weight* w) {
+    const int64_t tiles = gg_tiles(w), units_k = (w->K + 127) / 128, sms = gg_sm_count();
+    GgLayout best{};
+    int64_t best_cost = INT64_MAX;
+    for (int cap = 16; cap <= GG_MAX_ROWS; cap *= 2) {
+        const GgRows r = GgRows::of((int)M, cap);
+        const int64_t units = tiles * r.chunks * units_k, unit = gg::unit_cycles(true, r.n);
+        for (int64_t share = (units + sms - 1) / sms, step = 0; step < 3 && share <= units_k; ++step, share *= 2) {
+            const int64_t pieces = share >= units_k ? 1 : (units_k + share - 1) / share + 1;
+            const int64_t cost = share * unit + r.n / 16 * (pieces > 1 ? 1500 + 400 * pieces : 250);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = GgLayout{r, (int)std::min<int64_t>(sms, (units + share - 1) / share)};
+            }
+        }
+        const int64_t share = (units + sms - 1) / sms;
+        if (share > units_k) {               // a tile and more per CTA: cut in two at most
+            const int64_t cost = share * unit + (share + units_k - 1) / units_k * (r.n / 16) * 250 + r.n / 16 * 2300;
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = GgLayout{r, (int)sms};
+            }
+        }
+        if (r.chunks == 1) break;
+    }
+    return best;
+}
+
+int launch_gg_stage(const GgStaged& to, const void* x, int x_f16, const int32_t* idx, const int32_t* counts, int lists, int64_t rows,
+                    int K, cudaStream_t st) {
+    auto kern = x_f16 ? gg::gg_stage_kernel<true> : gg::gg_stage_kernel<false>;
+    launch_overlapped(kern, (int)rows, 256, 0, st, (unsigned char*)to.data, to.scale, to.rows, (const uint16_t*)x, idx, counts, lists, K);
+    HQM_LAUNCH_CHECK();
+    return HQM_OK;
+}
+
+template <int NBITS, int GS, int MODE>
+static int gg_launch_one(const gg::Params& p, int grid, cudaStream_t st) {
+    using F = gg::Fmt<NBITS, GS>;
+    auto kern = gg::gg_kernel<NBITS, GS, MODE>;
+    static bool attr_done[MAX_DEVICES];
+    bool& done = attr_done[current_device_slot()];
+    if (!done) {
+        HQM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem(64) > F::smem(256) ? F::smem(64) : F::smem(256)));
+        done = true;
+    }
+    launch_overlapped(kern, grid, gg::NTHREADS, F::smem(p.n_max), st, p);
+    HQM_LAUNCH_CHECK();
+    return HQM_OK;
+}
+
+int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st) {
+    gg::Params p{};
+    const int host_problems = job.table ? 1 : job.problems;
+    const hqm_weight* first = job.table ? job.shape : job.w0[0];
+    const int nbits = first->nbits, gs = first->group_size, per = codes_per_word(nbits);
+    const int parts = 128 / (per * gs);
+    HQM_CHECK_ARG(job.problems >= 1 && job.problems <= GG_MAX_PROBLEMS && host_problems <= 4, "gemm: %d problems in a launch", job.problems);
+    HQM_CHECK_ARG(job.mode != GG_UP || parts == 2, "gemm: the fused gate needs tiles of two parts");
+    int64_t tiles_all = 0;
+    for (int i = 0; i < host_problems; ++i) {
+        gg::HostProblem& h = p.hp[i];
+        for (int l = 0; l < 2; ++l) {
+            const hqm_weight* w = job.table ? job.shape : (l && job.mode == GG_UP ? job.w1[i] : job.w0[i]);
+            int G, C;
+            const int rc = check_weight(w, &G, &C);
+            if (rc != HQM_OK) return rc;
+            h.G = G;
+            h.C = C;
+            h.P = G / per;
+            h.tiles = job.mode == GG_UP ? h.P : (h.P + parts - 1) / parts;
+            if (!job.table) {
+                h.meta[l][0] = w->ms_scale;
+                h.meta[l][1] = w->mz_scale;
+                h.meta[l][2] = w->ms_zero;
+                h.meta[l][3] = w->mz_zero;
+                if ((l == 0 || job.mode == GG_UP) && !stream_cached_maps(w, G, h.maps[l])) {
+                    set_error("gemm: cuTensorMapEncodeTiled failed for a %dx%d %d-bit layer", w->N, w->K, w->nbits);
+                    return HQM_ERR_CUDA;
+                }
+            }
+        }
+        h.y = job.y[i];
+        h.bias = job.bias[i];
+        tiles_all += h.tiles;
+    }
+    if (job.table) tiles_all *= job.problems;
+    p.problems = job.problems;
+    p.K = first->K;
+    p.subs_k = p.K / 64;
+    p.units_k = (p.subs_k + 1) / 2;
+    p.N = first->N;
+    p.table = job.table;
+    p.which0 = job.which0;
+    p.which1 = job.which1;
+    p.counts = job.counts;
+    p.rows = job.rows;
+    p.xt = (const unsigned char*)job.x.data;
+    p.row_scale = job.x.scale;
+    p.xt_rows = job.x.rows;
+    p.mode = job.mode;
+    p.y_f16 = job.y_f16;
+    p.ht = (unsigned char*)job.ht;
+    p.out = job.out;
+    p.out_f16 = job.out_f16;
+    p.out_idx = job.out_idx;
+    p.row_w = job.row_w;
+    p.accumulate = job.accumulate;
+    p.parts = (float*)scratch;
+    p.n_max = job.counts ? gg_n_max(job.rows) : job.layout.rows.n;
+    p.chunks = job.layout.rows.chunks;
+    p.counters = counters;
+    p.error_flag = tc_error_ptr();
+    int64_t grid = job.counts ? gg_sm_count() : job.layout.grid;
+    const size_t least_bytes = job.counts ? gg_scratch_bytes(p.n_max) : std::min((size_t)grid * gg_piece_bytes(p.n_max), gg_scratch_least(p.n_max, first));
+    if (scratch == nullptr || counters == nullptr || scratch_bytes < least_bytes) {
+        set_error("gemm: scratch of %zu bytes given, %zu needed", scratch_bytes, least_bytes);
+        return HQM_ERR_SCRATCH;
+    }
+    grid = std::min<int64_t>(grid, (int64_t)(scratch_bytes / gg_piece_bytes(p.n_max)));
+#define HQM_GG(B, S, M) \
+    if (nbits == B && gs == S && job.mode == M) return gg_launch_one<B, S, M>(p, (int)grid, st);
+    HQM_GG(2, 16, GG_LINEAR) HQM_GG(2, 16, GG_UP) HQM_GG(2, 16, GG_DOWN)
+    HQM_GG(2, 32, GG_LINEAR) HQM_GG(2, 32, GG_DOWN)
+    HQM_GG(4, 32, GG_LINEAR) HQM_GG(4, 32, GG_DOWN)
+    HQM_GG(4, 64, GG_LINEAR) HQM_GG(4, 64, GG_DOWN)
+#undef HQM_GG
+    set_error("gemm: no kernel for nbits=%d group_size=%d mode=%d", nbits, gs, (int)job.mode);
+    return HQM_ERR_ARG;
+}
+
+}  // namespace hqm

@@ -1,0 +1,95 @@
+// Quantized GEMM on the 5th-generation tensor cores for several weights and row lists at once (gemm_grouped.cu).
+#pragma once
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace hqm {
+
+constexpr int GG_MAX_PROBLEMS = 32;
+constexpr int GG_MAX_ROWS = 256;          // rows of x per pass over a weight (the MMA's N)
+constexpr int GG_LEAST_CTAS = 48;
+constexpr int GG_F16_ROWS = 16;           // up to here h of an expert is staged as fp16, beyond it as bf16
+
+// How a launch's rows are laid out in the staged copy of x ("tiles": [K / 64][row][64], see gemm_grouped.cu): a row
+// list of `cnt` rows is cut into equal chunks of at most GG_MAX_ROWS rows, padded to a multiple of 16.
+struct GgRows {
+    int chunks, n;                        // n = rows per chunk
+    __host__ __device__ static GgRows of(int cnt, int cap = GG_MAX_ROWS) {
+        GgRows r;
+        r.chunks = (cnt + cap - 1) / cap;
+        r.n = r.chunks == 0 ? 0 : ((cnt + r.chunks - 1) / r.chunks + 15) / 16 * 16;
+        return r;
+    }
+    __host__ __device__ int padded() const { return chunks * n; }
+};
+struct GgLayout {                         // of a launch whose row count the host knows
+    GgRows rows;
+    int grid;
+};
+// Upper bound of the padded rows of `rows` rows spread over `lists` lists.
+inline int64_t gg_padded_rows(int64_t rows, int lists) {
+    return (rows + 16 * ((int64_t)lists + rows / GG_MAX_ROWS + 1) + 15) / 16 * 16;
+}
+
+// A staged copy of x or h.
+struct GgStaged {
+    void* data;                           // [K / 64][rows][64]
+    float* scale;                         // power-of-two factor of every row (null: 1)
+    int64_t rows;
+};
+inline size_t gg_align(size_t v) { return (v + 1023) / 1024 * 1024; }
+inline size_t gg_stage_bytes(int64_t rows, int K, bool scaled) {
+    return gg_align((size_t)rows * (size_t)K * 2) + (scaled ? gg_align((size_t)rows * 4) : 0);
+}
+inline GgStaged gg_staged(void* at, int64_t rows, int K, bool scaled) {
+    return GgStaged{at, scaled ? (float*)((uint8_t*)at + gg_align((size_t)rows * (size_t)K * 2)) : nullptr, rows};
+}
+
+// What happens to a finished sum.
+enum GgMode {
+    GG_LINEAR = 0,       // y[row, n] = sum (+ bias[n])
+    GG_UP = 1,           // h = silu(gate) * up, staged as the next launch's x
+    GG_DOWN = 2,         // out[row] (+)= weight * sum
+};
+
+struct GgJob {
+    int problems;                         // weights (GG_LINEAR, one expert) or experts of the table
+    const hqm_weight* w0[4];              // host descriptors of the problems (no table), GG_UP: w1
+    const hqm_weight* w1[4];              // GG_UP: w3
+    const StreamEntry* table;             // device table, entries 3 * e + which; shape[] then only gives the shapes
+    const hqm_weight* shape;
+    int which0, which1;
+    const int32_t* counts;                // device: rows of every problem; null: `rows` rows, shared by all problems
+    int rows;                             // rows (counts == null), or the most all lists hold together
+    GgLayout layout;                      // (counts == null)
+    GgStaged x;                           // the staged rows
+    GgMode mode;
+    // GG_LINEAR
+    void* y[4];                           // (rows, N) of each problem
+    const uint16_t* bias[4];
+    int y_f16;                            // y is fp16 instead of bf16
+    // GG_UP
+    void* ht;                             // staged h
+    // GG_DOWN
+    void* out;                            // (*, H)
+    int out_f16;
+    const int32_t* out_idx;               // row of `out` of list entry i (null: i)
+    const float* row_w;                   // weight of list entry i (null: 1)
+    int accumulate;
+};
+
+bool gg_supported(const hqm_weight* w, int G, int C);
+GgLayout gg_linear_layout(int64_t M, const hqm_weight* w);
+GgLayout gg_expert_layout(int64_t M);
+// Bytes of scratch (partial tiles) of a launch with up to n rows per chunk: with a CTA on every SM, and the least a launch
+// without `counts` works with (it then uses fewer CTAs).
+size_t gg_scratch_bytes(int n);
+size_t gg_scratch_least(int n, const hqm_weight* w);
+int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st);
+
+// Stages rows of x (bf16 or fp16).  counts == null: one list of `rows` rows, else `lists` lists of together at most `rows`;
+// idx: row of x of list entry i (null: i).
+int launch_gg_stage(const GgStaged& to, const void* x, int x_f16, const int32_t* idx, const int32_t* counts, int lists, int64_t rows,
+                    int K, cudaStream_t st);
+
+}  // namespace hqm

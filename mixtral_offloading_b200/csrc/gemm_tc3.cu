@@ -15,7 +15,7 @@
 //      and one fused multiply-add with the row's (S, T) pairs give the dequantised weights, stored
 //      as one 16-byte chunk of the K-major, 128-byte-swizzled A tile.  The tokens are the MMA's N
 //      dimension (64 or 128), the accumulator lives in TMEM; ring of stages, full / empty
-//      mbarriers with bounded waits, exactly as in gemm_tc.cu.
+//      mbarriers with bounded waits.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "tc_common.cuh"

@@ -612,15 +612,18 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-bool tma_shape_ok(const hqm_weight* w, int G, int C) {
+// Layers whose tensor maps can be encoded.
+bool maps_ok(const hqm_weight* w, int G) {
     if ((w->nbits != 2 && w->nbits != 4) || !meta_uniform(w)) return false;
     const int per = codes_per_word(w->nbits);
-    if (w->group_size % 16 != 0 || w->K % KC != 0 || C % KC != 0 || G % per != 0) return false;
+    if (w->group_size % 16 != 0 || w->K % 16 != 0 || w->K < KC || G % per != 0) return false;
     if (w->group_size > 256 || (int64_t)G * w->K >= ((int64_t)1 << 31)) return false;
     auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     return a16(w->W_q) && a16(w->scale_q) && a16(w->zero_q) && a16(w->ms_scale) && a16(w->mz_scale) && a16(w->ms_zero) &&
            a16(w->mz_zero);
 }
+// Layers this file's kernel takes: whole passes whose meta columns do not wrap.
+bool tma_shape_ok(const hqm_weight* w, int G, int C) { return maps_ok(w, G) && w->K % KC == 0 && C % KC == 0; }
 
 // The three tensor maps of a layer: codes as (K, P, group_size) bytes with box (128, 1, 16) and the 128-byte
 // swizzle; scale_q and zero_q as (K, G, 1) bytes with box (128, PER, 1).
@@ -754,6 +757,11 @@ bool prepare_kernel(size_t smem) {
 }
 
 }  // namespace
+
+// The tensor maps of a layer for the other TMA users (three CUtensorMaps; the codes' box is 128 columns x 16 members).
+bool stream_cached_maps(const hqm_weight* w, int G, void* out3) {
+    return maps_ok(w, G) && cached_maps(w, G, static_cast<CUtensorMap*>(out3));
+}
 
 // cuTensorMapEncodeTiled of the installed driver (null when it cannot be had), for the other TMA users.
 void* tma_encode_entry() { return (void*)encode_fn(); }
@@ -925,7 +933,7 @@ int hqm_expert_table_build(void* host_out, const hqm_weight* weights, int32_t n_
         int G, C;
         const int rc = check_weight(&weights[i], &G, &C);
         if (rc != HQM_OK) return rc;
-        if (!tma_disabled() && encode_fn() != nullptr && tma_shape_ok(&weights[i], G, C) &&
+        if (encode_fn() != nullptr && maps_ok(&weights[i], G) &&
             !encode_maps(&weights[i], G, reinterpret_cast<CUtensorMap*>(out[i].maps))) {
             set_error("expert_table_build: cuTensorMapEncodeTiled failed for weight %d (%dx%d, %d bit)", i, weights[i].N,
                       weights[i].K, weights[i].nbits);

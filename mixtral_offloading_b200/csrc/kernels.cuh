@@ -81,6 +81,10 @@ int launch_gemv_tma(float* partial, const uint16_t* x, const int32_t* x_idx, int
 int launch_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx, const uint16_t* x,
                        const uint16_t* gate_w, int64_t M, int64_t K, int32_t E, cudaStream_t st);
 
+// Per-expert row lists of routed tokens; entry_of (may be null): the list entries of token t at [2t], [2t + 1].
+int launch_router_lists(int32_t* counts, int32_t* offsets, int32_t* token_idx, float* token_w, int32_t* entry_of,
+                        const float* topk_w, const int32_t* topk_idx, int64_t M, int32_t E, cudaStream_t st);
+
 // gemv_stream3.cu — the weight-streaming path for 3-bit layers.
 struct Stream3Plan {
     int P3;      // storage-row classes (rows R and R + P3 hold the same residues in the same slots)
@@ -94,24 +98,13 @@ int launch_gemv_stream3(uint16_t* y, float* partial, const uint16_t* x, const in
                         const hqm_weight* w, const uint16_t* bias, int G, int C, const Stream3Plan& plan,
                         cudaStream_t st);
 
-// gemm_tc.cu — tcgen05 / TMEM path for many rows of x.
-bool gemm_tc_supported(const hqm_weight* w, int G, int C, int64_t M);
-int launch_gemm_tc(float* sums, const uint16_t* x, const int32_t* x_idx, int64_t M, const hqm_weight* w0,
-                   const hqm_weight* w1, int G, int C, cudaStream_t st);
+int* tc_error_ptr();                  // device flag the bounded waits set when they give up (device_state.cu)
+void* tma_encode_entry();             // cuTensorMapEncodeTiled of the installed driver, or null
+// y (M, N) = bf16(sums + bias)
 int launch_rows_from_sums(uint16_t* y, const float* sums, const uint16_t* bias, int64_t M, int N, cudaStream_t st);
-int launch_silu_mul_from_sums(uint16_t* h, const float* sums, int64_t M, int F, cudaStream_t st);
-int launch_scatter_from_sums(uint16_t* out, const float* sums, const int32_t* token_idx, const float* route_w,
-                             int accumulate, int64_t M, int H, cudaStream_t st);
-int* tc_error_ptr();                  // device flag the bounded waits set when they give up
-// gemm_tma.cu — the same GEMM with every operand staged by TMA, persistent stream-K CTAs (contiguous rows of x).
-void* tma_encode_entry();
-bool gemm_tma_supported(const hqm_weight* w, int G, int C, int64_t M);
-int launch_gemm_tma(float* sums, const uint16_t* x, int64_t M, const hqm_weight* w0, const hqm_weight* w1, int G, int C,
-                    cudaStream_t st);
-int launch_gather_rows(uint16_t* dst, const uint16_t* x, const int32_t* idx, int64_t M, int K, cudaStream_t st);
-constexpr int64_t TC_MIN_ROWS = 17;   // fewer rows go to the streaming kernels
+constexpr int64_t GG_MIN_ROWS = 5;    // rows from which 2- and 4-bit layers go to gemm_grouped.cu
 
-// gemm_tc3.cu — the same for 3-bit layers (row counts >= 5).
+// gemm_tc3.cu — tcgen05 / TMEM path for 3-bit layers (row counts >= 5).
 bool gemm_tc3_supported(const hqm_weight* w, int G, int C, int64_t M);
 size_t gemm_tc3_scratch_bytes(const hqm_weight* w, int G, int64_t M);
 int launch_gemm_tc3(uint16_t* y, void* scratch, const uint16_t* x, const int32_t* x_idx, int64_t M,
@@ -130,7 +123,8 @@ bool moe_decode_plan_slots(int E, int slots, const hqm_weight* w1, const hqm_wei
 // Dispatcher used by hqm_linear and by the expert FFN: picks the streaming
 // kernel when the layer's shape allows it, the generic one otherwise.
 // (scratch excludes the header; counters points at it)
-size_t linear_scratch_bytes(int64_t M, const hqm_weight* w);
+// `preferred`: what the fastest launch wants instead of the least that works.
+size_t linear_scratch_bytes(int64_t M, const hqm_weight* w, bool preferred = false);
 int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t M, const hqm_weight* w,
                   const uint16_t* bias, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st);
 

@@ -6,6 +6,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "kernels.cuh"
 
 namespace hqm {
 
@@ -122,8 +123,8 @@ router_logits_top2_kernel(uint16_t* __restrict__ logits_out, float* __restrict__
 // ascending) list of the rows routed to each expert with their weights.
 __global__ void router_lists_kernel(int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
                                     int32_t* __restrict__ token_idx, float* __restrict__ token_w,
-                                    const float* __restrict__ topk_w, const int32_t* __restrict__ topk_idx, int M,
-                                    int E) {
+                                    int32_t* __restrict__ entry_of, const float* __restrict__ topk_w,
+                                    const int32_t* __restrict__ topk_idx, int M, int E) {
     __shared__ int s_count[32];
     __shared__ int s_off[33];
     grid_launch_dependents();
@@ -162,6 +163,7 @@ __global__ void router_lists_kernel(int32_t* __restrict__ counts, int32_t* __res
             const int pos = base + __popc(ballot & ((1u << lane) - 1u));
             token_idx[pos] = t;
             token_w[pos] = topk_w[2 * t + slot];
+            if (entry_of) entry_of[2 * t + slot] = pos;
         }
         base += __popc(ballot);
     }
@@ -182,6 +184,14 @@ int launch_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx
     HQM_LAUNCH_CHECK();
     return HQM_OK;
 }
+
+int launch_router_lists(int32_t* counts, int32_t* offsets, int32_t* token_idx, float* token_w, int32_t* entry_of,
+                        const float* topk_w, const int32_t* topk_idx, int64_t M, int32_t E, cudaStream_t st) {
+    launch_overlapped(router_lists_kernel, 1, 32 * E, 0, st, counts, offsets, token_idx, token_w, entry_of, topk_w, topk_idx,
+                      (int)M, (int)E);
+    HQM_LAUNCH_CHECK();
+    return HQM_OK;
+}
 }  // namespace hqm
 
 extern "C" int hqm_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx, int32_t* counts,
@@ -199,8 +209,5 @@ extern "C" int hqm_router_top2(uint16_t* router_logits, float* topk_w, int32_t* 
         const int rc = launch_router_top2(router_logits, topk_w, topk_idx, x, gate_w, M, K, E, st);
         if (rc != HQM_OK) return rc;
     }
-    launch_overlapped(router_lists_kernel, 1, 32 * E, 0, st, counts, offsets, token_idx, token_w, (const float*)topk_w,
-                      (const int32_t*)topk_idx, (int)M, (int)E);
-    HQM_LAUNCH_CHECK();
-    return HQM_OK;
+    return launch_router_lists(counts, offsets, token_idx, token_w, nullptr, topk_w, topk_idx, M, E, st);
 }

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import copy
 import ctypes as C
+from functools import partial
 from typing import Any, Dict, Optional
 
 import torch
@@ -173,7 +174,7 @@ class HQQLinearTritonSavable(nn.Module):
         y = torch.empty((M, N), dtype=torch.bfloat16, device=x2.device)
         d = self.descriptor()
         lib = _cabi.lib()
-        need = lib.hqm_linear_scratch_bytes(M, C.byref(d))
+        need = lib.hqm_linear_scratch_preferred(M, C.byref(d))
         ws = _scratch(x2.device, need) if need else None
         _cabi.check(lib.hqm_linear(_cabi.ptr(y), _cabi.ptr(x2), M, C.byref(d), _cabi.ptr(self.bias),
                                    _cabi.ptr(ws), need, _cabi.stream_ptr(x2.device)))
@@ -351,9 +352,9 @@ class SparseMoeWrapper(nn.Module):
 class ResidentMoe(nn.Module):
     """SparseMoeWrapper.forward for a layer whose experts ALL live on the device (no ExpertCache).
 
-    With nothing to swap, the host does not need to know the routing: for a single token the whole block —
-    router, the two chosen experts, weighted sum — runs as one chain of launches that pick the experts on
-    the device (hqm_moe_decode), so it can be captured in a CUDA graph.  More tokens take the same
+    With nothing to swap, the host does not need to know the routing: the whole block — router, the chosen experts,
+    weighted sum — runs as one chain of launches that pick the experts on the device (hqm_moe_decode for one token,
+    hqm_moe_forward for more), so it can be captured in a CUDA graph.  Shapes without such a path take the same
     per-expert loop as SparseMoeWrapper (one read-back of the row counts).
     `experts` is a list of MixtralBLockSparseTop2MLP_HQQ / MixtralExpertWrapper, index = expert id.
     """
@@ -400,29 +401,41 @@ class ResidentMoe(nn.Module):
             self._table = self._build_table(self._experts, device)
         return self._table
 
+    def _descriptors(self):
+        f0 = self._ffn(self._experts[0])
+        return tuple(C.byref(lyr.descriptor()) for lyr in (f0.w1, f0.w2, f0.w3))
+
+    def scratch_bytes(self, tokens: int) -> int:
+        """Workspace of forward_on_device(); 0 where the shapes have no path without a read-back."""
+        size = _cabi.lib().hqm_moe_decode_scratch_bytes if tokens == 1 else \
+            partial(_cabi.lib().hqm_moe_forward_scratch_bytes, tokens)
+        return size(self.num_experts, *self._descriptors())
+
+    def forward_on_device(self, x2: torch.Tensor):
+        """The block on rows x2 (tokens, hidden) bf16 with nothing read back; returns (out, router logits)."""
+        T, E, dev, lib = x2.shape[0], self.num_experts, x2.device, _cabi.lib()
+        gate_w = self.gate.weight if self.gate.weight.dtype == torch.bfloat16 else self.gate.weight.to(torch.bfloat16)
+        out = torch.empty_like(x2)
+        logits = torch.empty((T, E), dtype=torch.bfloat16, device=dev)
+        ws = _scratch(dev, self.scratch_bytes(T))
+        head = (_cabi.ptr(out), _cabi.ptr(logits), _cabi.ptr(x2), _cabi.ptr(gate_w))
+        tail = (_cabi.ptr(self._descriptor_table(dev)), *self._descriptors(), _cabi.ptr(ws), ws.numel(),
+                _cabi.stream_ptr(dev))
+        _cabi.check(lib.hqm_moe_decode(*head, E, *tail) if T == 1 else lib.hqm_moe_forward(*head, T, E, *tail))
+        return out, logits
+
     @torch.inference_mode()
     def forward(self, hidden_states: torch.Tensor):
         batch, seq, hidden = hidden_states.shape
         x2 = _as_bf16_2d(hidden_states, hidden)
         T, E = x2.shape[0], self.num_experts
         dev = x2.device
-        if T == 1:
-            f0 = self._ffn(self._experts[0])
-            d1, d2, d3 = f0.w1.descriptor(), f0.w2.descriptor(), f0.w3.descriptor()
-            lib = _cabi.lib()
-            need = lib.hqm_moe_decode_scratch_bytes(E, C.byref(d1), C.byref(d2), C.byref(d3))
-            if need:
-                gate_w = self.gate.weight if self.gate.weight.dtype == torch.bfloat16 else self.gate.weight.to(torch.bfloat16)
-                out = torch.empty((1, hidden), dtype=torch.bfloat16, device=dev)
-                logits = torch.empty((1, E), dtype=torch.bfloat16, device=dev)
-                ws = _scratch(dev, need)
-                _cabi.check(lib.hqm_moe_decode(_cabi.ptr(out), _cabi.ptr(logits), _cabi.ptr(x2), _cabi.ptr(gate_w), E,
-                                               _cabi.ptr(self._descriptor_table(dev)), C.byref(d1), C.byref(d2),
-                                               C.byref(d3), _cabi.ptr(ws), ws.numel(), _cabi.stream_ptr(dev)))
-                out = out.reshape(batch, seq, hidden)
-                if hidden_states.dtype != torch.bfloat16:
-                    out, logits = out.to(hidden_states.dtype), logits.to(hidden_states.dtype)
-                return out, logits
+        if self.scratch_bytes(T):
+            out, logits = self.forward_on_device(x2)
+            out = out.reshape(batch, seq, hidden)
+            if hidden_states.dtype != torch.bfloat16:
+                out, logits = out.to(hidden_states.dtype), logits.to(hidden_states.dtype)
+            return out, logits
         logits, _, _, meta, token_idx, token_w = self._router.route(x2)
         if self._host_counts is None:
             with torch.inference_mode(False):

@@ -9,7 +9,9 @@ their many-row path, torch's attention over the prompt).
 """
 from __future__ import annotations
 
-from typing import List, Sequence
+import itertools
+from functools import partial
+from typing import List, Optional, Sequence
 
 import torch
 from torch import nn
@@ -146,13 +148,11 @@ class BatchDecode:
     """B independent sequences advanced one token per step through the layers of a MixtralDecodeModel (the same
     weights), each sequence with its own key/value cache; all of them at the same position.
 
-    The quantized projections and the experts run once per step on all B rows (the few-row streaming kernels read
-    the weights once for the batch); norms, RoPE and attention over the caches are torch ops; the MoE block groups the
-    rows per expert as SparseMoeWrapper.forward does (custom_layers.py:272-314), which needs the row counts on the
-    host once per layer.  A step is therefore a chain of segments, one per layer: [add the previous block's output,
-    attention half, post-attention norm, router] - read the counts back - [the active experts].  capture() records
-    every segment in a CUDA graph (the position is device data: hqm_rope_append_rows reads it, and attention runs
-    over the whole cache under a mask), so that the host issues one replay and the experts per layer."""
+    The quantized projections and the MoE block run once per step on all B rows; norms, RoPE and attention over the
+    caches are torch ops.  capture() records the step in CUDA graphs (the position is device data:
+    hqm_rope_append_rows reads it, and attention runs over the whole cache under a mask).  Where every layer's MoE block
+    chooses its experts on the device that is one graph; a block whose shapes need the row counts on the host
+    (custom_layers.py:272-314) ends a graph, and its experts are issued between two."""
 
     def __init__(self, model: MixtralDecodeModel, batch: int, max_len: int):
         self.model, self.batch, self.max_len = model, batch, max_len
@@ -165,13 +165,15 @@ class BatchDecode:
         self.tokens = torch.zeros((batch,), dtype=torch.int64, device=dev)
         self.position = torch.zeros((1,), dtype=torch.int64, device=dev)
         self.h = torch.zeros((batch, hidden), dtype=torch.bfloat16, device=dev)     # residual streams
-        self.y = torch.zeros((batch, hidden), dtype=torch.bfloat16, device=dev)     # the last MoE block's output
+        self.y: Optional[torch.Tensor] = None                                       # the last MoE block's output
         self._slots = torch.arange(max_len, device=dev)
         E = model.layers[0].moe.num_experts
         self._host_counts = torch.empty((2 * E + 1,), dtype=torch.int32).pin_memory()
-        self.router_logits: List[torch.Tensor] = []
-        self._graphs = None
+        self._on_device = [layer.moe.scratch_bytes(batch) > 0 for layer in model.layers]
+        self.router_logits: List[torch.Tensor] = [None] * len(model.layers)
+        self._plan = None
         self._routes = [None] * len(model.layers)
+        self._y_host = [None] * len(model.layers)
         self._x_moe = [None] * len(model.layers)
         self._mask = None
         self._logits = None
@@ -181,15 +183,15 @@ class BatchDecode:
         """The streams of the fed tokens and the mask of filled cache rows."""
         self._mask = (self._slots <= self.position)[None, None, None, :]
         self.h.copy_(self.model.embed[self.tokens])
-        self.y.zero_()
+        self.y = None
 
     def _attention_segment(self, l: int):
         layer = self.model.layers[l]
         a, B, h = layer.attention, self.batch, self.h
         hidden = h.shape[-1]
         mask = self._mask
-        h.add_(self.y)
-        self.y.zero_()
+        if self.y is not None:
+            h.add_(self.y)
         ln_in = self.model.first_ln if l == 0 else self.model.layers[l - 1].next_ln     # the weights step() applies
         x = rms_norm_rows(h, ln_in, a.rms_eps)
         q = a.q_proj(x)
@@ -200,18 +202,23 @@ class BatchDecode:
                                                                attn_mask=mask, enable_gqa=True)   # (B, heads, 1, head_dim)
         h.add_(a.o_proj(ctx.reshape(B, hidden)))
         self._x_moe[l] = rms_norm_rows(h, a.ln_post, a.rms_eps)
-        self._routes[l] = layer.moe._router.route(self._x_moe[l])
+        if not self._on_device[l]:
+            self._routes[l] = layer.moe._router.route(self._x_moe[l])
+            self.y = self._y_host[l] = torch.zeros_like(h)
 
     def _head_segment(self):
         self.h.add_(self.y)
         x = rms_norm_rows(self.h, self.model.layers[-1].next_ln, self.model.rms_eps)
         self._logits = torch.matmul(x, self.model.lm_head.t())
 
-    def _experts(self, l: int):
+    def _moe_segment(self, l: int):
+        self.y, self.router_logits[l] = self.model.layers[l].moe.forward_on_device(self._x_moe[l])
+
+    def _moe_from_host(self, l: int):
         """The per-expert loop of SparseMoeWrapper.forward (custom_layers.py:295-312) into self.y."""
         moe = self.model.layers[l].moe
         E = moe.num_experts
-        logits, _, _, meta, token_idx, token_w = self._routes[l]
+        self.router_logits[l], _, _, meta, token_idx, token_w = self._routes[l]
         self._host_counts.copy_(meta, non_blocking=True)
         torch.cuda.current_stream(self.h.device).synchronize()
         host = self._host_counts.tolist()
@@ -219,13 +226,20 @@ class BatchDecode:
         for e in range(E):
             if counts[e] > 0:
                 lo, hi = offsets[e], offsets[e + 1]
-                moe._experts[e].forward_routed(self._x_moe[l], token_idx[lo:hi], token_w[lo:hi], self.y, accumulate=True)
-        return logits
+                moe._experts[e].forward_routed(self._x_moe[l], token_idx[lo:hi], token_w[lo:hi], self._y_host[l], accumulate=True)
 
     # ---- a step -----------------------------------------------------------------------------------------------
+    def _segments(self):
+        """The step in order, as (does it stay on the device, function)."""
+        yield True, self._prologue
+        for l in range(len(self.model.layers)):
+            yield True, partial(self._attention_segment, l)
+            yield (True, partial(self._moe_segment, l)) if self._on_device[l] else (False, partial(self._moe_from_host, l))
+        yield True, self._head_segment
+
     @torch.inference_mode()
     def capture(self) -> None:
-        """Records the segments (call after at least one plain step at this batch size, so that the library's
+        """Records the step (call after at least one plain step at this batch size, so that the library's
         workspace has its size)."""
         dev = self.h.device
         tokens, pos = self.tokens.clone(), self.position.clone()
@@ -235,37 +249,26 @@ class BatchDecode:
         with torch.cuda.stream(side):
             self._run_eager()                                              # settles allocations on the capture stream
         torch.cuda.current_stream(dev).wait_stream(side)
-        graphs, pool = [], None
-        segments = [self._prologue] + [lambda l=l: self._attention_segment(l) for l in range(len(self.model.layers))] \
-            + [self._head_segment]
-        for seg in segments:
+        plan, pool = [], None
+        for on_device, group in itertools.groupby(self._segments(), key=lambda seg: seg[0]):
+            if not on_device:
+                plan += [fn for _, fn in group]
+                continue
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, pool=pool):
-                seg()
+                for _, fn in group:
+                    fn()
             pool = g.pool()
-            graphs.append(g)
-        self._graphs = graphs
+            plan.append(g.replay)
+        self._plan = plan
         self.tokens.copy_(tokens)
         self.position.copy_(pos)
         for (k0, v0), k, v in zip(caches, self.k_caches, self.v_caches):   # the settling step wrote this row
             k[:, :, int(pos)], v[:, :, int(pos)] = k0, v0
 
     def _run_eager(self):
-        self._prologue()
-        self.router_logits = []
-        for l in range(len(self.model.layers)):
-            self._attention_segment(l)
-            self.router_logits.append(self._experts(l))
-        self._head_segment()
-
-    def _run_graphs(self):
-        g = self._graphs
-        g[0].replay()
-        self.router_logits = []
-        for l in range(len(self.model.layers)):
-            g[1 + l].replay()
-            self.router_logits.append(self._experts(l))
-        g[-1].replay()
+        for _, fn in self._segments():
+            fn()
 
     @torch.inference_mode()
     def step(self, tokens: torch.Tensor, pos: int) -> torch.Tensor:
@@ -275,8 +278,9 @@ class BatchDecode:
             raise ValueError(f"step wants {self.batch} tokens and a position below {self.max_len}")
         self.tokens.copy_(tokens)
         self.position.fill_(pos)
-        if self._graphs is not None:
-            self._run_graphs()
-        else:
+        if self._plan is None:
             self._run_eager()
+        else:
+            for fn in self._plan:
+                fn()
         return self._logits
