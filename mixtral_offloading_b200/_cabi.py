@@ -135,6 +135,24 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The Python extension over the library (native/host.cpp): the host path of the small calls."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError(f"_host.so cannot be loaded ({e}); python -m mixtral_offloading_b200.build") from e
+        from . import custom_layers
+        module.setup(custom_layers._SCRATCH, custom_layers._scratch)
+        _host = module
+    return _host
+
+
 def last_error() -> str:
     return (lib().hqm_last_error() or b"").decode()
 

@@ -158,7 +158,8 @@ class HQQLinearTritonSavable(nn.Module):
         return self._desc[1]
 
     def forward(self, x):
-        return self.forward_triton(x)
+        y = _cabi.host().linear(self, x)             # contiguous bf16 rows on the device; None for everything else
+        return self.forward_triton(x) if y is None else y
 
     def set_backend(self, backend):
         pass                                                                   # custom_layers.py:52-53
@@ -260,8 +261,12 @@ class MixtralBLockSparseTop2MLP_HQQ(nn.Module):
                                        _cabi.ptr(ws), ws.numel(), _cabi.stream_ptr(x2d.device)))
         return out
 
-    @torch.inference_mode()
     def forward(self, hidden_states):
+        out = _cabi.host().expert(self, hidden_states)
+        return self._forward_general(hidden_states) if out is None else out
+
+    @torch.inference_mode()
+    def _forward_general(self, hidden_states):
         K = self.w1.meta["shape"][1]
         x2 = _as_bf16_2d(hidden_states, K)
         out = torch.empty((x2.shape[0], self.w2.meta["shape"][0]), dtype=torch.bfloat16, device=x2.device)

@@ -1,0 +1,260 @@
+// The host side of the small calls: a quantized linear or an expert on tensors, from the Python call to the library's
+// launches.  What a call of one row costs is this path (the kernels run 5-20 us): through ctypes it was 20-33 us -- struct
+// and pointer objects for some twenty arguments, seven data_ptr() calls, three tensor methods -- and here it is the
+// allocation of the result and the launches (4-bit 1024 x 4096, one row: 21.7 us per call before, 6.5 now, which is the
+// kernel's own time).
+//
+// Every function returns None where it does not cover the arguments (another device, dtype conversions, a layer that has to
+// be validated first, an error from the library); the Python code around it then takes the general way and raises what
+// there is to raise.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <cstring>
+
+#include <ATen/Functions.h>
+#include <ATen/core/Tensor.h>
+#include <c10/core/InferenceMode.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/hqq_moe.h"
+
+namespace {
+
+struct Names {
+    PyObject *dict, *W_q, *meta, *bias, *plan, *ready, *scale_q, *zero_q, *meta_scale, *meta_zero, *scale, *zero, *modules, *w1, *w2, *w3, *axis;
+} N;
+
+PyObject* g_scratch = nullptr;        // custom_layers._SCRATCH: {("cuda", index): uint8 tensor}
+PyObject* g_grow = nullptr;           // custom_layers._scratch(device, bytes)
+PyObject* g_keys[64];                 // ("cuda", index)
+
+// A layer's descriptor (and with it the addresses it was made from) and the workspace of its last row count, as linear
+// layer and as w1 of an expert; kept in the layer's __dict__.  A copied or pickled layer gets None and makes its own.
+struct Plan {
+    PyObject_HEAD
+    hqm_weight w;
+    int64_t linear_rows, expert_rows;
+    size_t linear_bytes, expert_bytes;
+};
+PyObject* plan_copy(PyObject*, PyObject*) { Py_RETURN_NONE; }
+PyObject* plan_reduce(PyObject*, PyObject*) { return Py_BuildValue("(O())", (PyObject*)Py_TYPE(Py_None)); }
+PyMethodDef plan_methods[] = {{"__deepcopy__", plan_copy, METH_O, nullptr},
+                              {"__copy__", plan_copy, METH_NOARGS, nullptr},
+                              {"__reduce__", plan_reduce, METH_NOARGS, nullptr},
+                              {nullptr, nullptr, 0, nullptr}};
+PyTypeObject PlanType = {PyVarObject_HEAD_INIT(nullptr, 0) "mixtral_offloading_b200._host.Plan", sizeof(Plan)};
+
+// borrowed reference out of a dict, null if absent (no error set)
+PyObject* item(PyObject* dict, PyObject* key) {
+    if (dict == nullptr || !PyDict_CheckExact(dict)) return nullptr;
+    PyObject* v = PyDict_GetItemWithError(dict, key);
+    if (v == nullptr) PyErr_Clear();
+    return v;
+}
+const void* address(PyObject* t) { return t != nullptr && THPVariable_Check(t) ? THPVariable_Unpack(t).const_data_ptr() : nullptr; }
+
+// The plan of a layer whose tensors are where they were when its descriptor was made; null: not to be had here.
+Plan* plan_of(PyObject* layer, PyObject* dict) {
+    PyObject* meta = item(dict, N.meta);
+    PyObject *ms = item(meta, N.meta_scale), *mz = item(meta, N.meta_zero);
+    if (item(dict, N.ready) != Py_True || ms == nullptr || mz == nullptr) return nullptr;
+    const void* at[7] = {address(item(dict, N.W_q)),    address(item(meta, N.scale_q)), address(item(meta, N.zero_q)), address(item(ms, N.scale)),
+                         address(item(ms, N.zero)), address(item(mz, N.scale)),     address(item(mz, N.zero))};
+    PyObject* kept = item(dict, N.plan);
+    if (kept != nullptr && Py_TYPE(kept) == &PlanType) {
+        Plan* p = reinterpret_cast<Plan*>(kept);
+        if (p->w.W_q == at[0] && p->w.scale_q == at[1] && p->w.zero_q == at[2] && p->w.ms_scale == at[3] && p->w.mz_scale == at[4] &&
+            p->w.ms_zero == at[5] && p->w.mz_zero == at[6])
+            return p;
+    }
+    PyObject* axis = item(meta, N.axis);
+    if (axis == nullptr || !PyLong_Check(axis) || PyLong_AsLong(axis) != 0) return nullptr;
+    PyObject* d = PyObject_CallMethod(layer, "descriptor", nullptr);      // validates; a ctypes structure
+    if (d == nullptr) {
+        PyErr_Clear();
+        return nullptr;
+    }
+    Plan* p = nullptr;
+    Py_buffer view;
+    if (PyObject_GetBuffer(d, &view, PyBUF_SIMPLE) == 0) {
+        if (view.len == (Py_ssize_t)sizeof(hqm_weight) && (p = PyObject_New(Plan, &PlanType)) != nullptr) {
+            memcpy(&p->w, view.buf, sizeof(hqm_weight));
+            p->linear_rows = p->expert_rows = -1;
+            p->linear_bytes = p->expert_bytes = 0;
+            if (PyDict_SetItem(dict, N.plan, reinterpret_cast<PyObject*>(p)) != 0) p = nullptr;
+            else Py_DECREF(p);                             // the layer's __dict__ holds it
+        }
+        PyBuffer_Release(&view);
+    }
+    Py_DECREF(d);
+    PyErr_Clear();
+    return p;
+}
+
+PyObject* dict_of(PyObject* module) {        // new reference
+    PyObject* d = PyObject_GetAttr(module, N.dict);
+    if (d == nullptr) PyErr_Clear();
+    return d;
+}
+
+// x as the library takes it: bf16, contiguous, on the current device, last dimension K, at least one row; else null.
+const at::Tensor* rows_of(PyObject* obj, int64_t K, int64_t* rows) {
+    if (!THPVariable_CheckExact(obj)) return nullptr;
+    const at::Tensor& x = THPVariable_Unpack(obj);
+    if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() < 1 || x.size(-1) != K || x.numel() == 0 || !x.is_contiguous() ||
+        x.device().index() != c10::cuda::current_device())
+        return nullptr;
+    *rows = x.numel() / K;
+    return &x;
+}
+
+// Workspace of the device (the Python module's, grown through it); its address, null on failure.
+void* scratch(const at::Tensor& on, size_t bytes, size_t* have) {
+    const int dev = on.device().index();
+    if (dev < 0 || dev >= 64) return nullptr;
+    if (g_keys[dev] == nullptr && (g_keys[dev] = Py_BuildValue("(si)", "cuda", dev)) == nullptr) return nullptr;
+    PyObject* t = item(g_scratch, g_keys[dev]);
+    if (t != nullptr && THPVariable_Check(t) && (size_t)THPVariable_Unpack(t).numel() >= bytes) {
+        *have = (size_t)THPVariable_Unpack(t).numel();
+        return THPVariable_Unpack(t).data_ptr();
+    }
+    PyObject* device = THPDevice_New(on.device());
+    t = device == nullptr ? nullptr : PyObject_CallFunction(g_grow, "On", device, (Py_ssize_t)bytes);
+    Py_XDECREF(device);
+    if (t == nullptr) {
+        PyErr_Clear();
+        return nullptr;
+    }
+    void* p = THPVariable_Unpack(t).data_ptr();           // (the module keeps it)
+    *have = (size_t)THPVariable_Unpack(t).numel();
+    Py_DECREF(t);
+    return p;
+}
+
+at::Tensor result(const at::Tensor& x, int64_t n) {
+    c10::SmallVector<int64_t, 8> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = n;
+    return at::empty(shape, x.options());
+}
+
+// linear(layer, x)
+PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2) return PyErr_Format(PyExc_TypeError, "linear(layer, x)");
+    try {
+        PyObject* dict = dict_of(args[0]);
+        Plan* p = dict == nullptr ? nullptr : plan_of(args[0], dict);
+        PyObject* bias = item(dict, N.bias);
+        Py_XDECREF(dict);                                  // (the layer holds it, and it the plan)
+        int64_t rows = 0;
+        const at::Tensor* x = p == nullptr ? nullptr : rows_of(args[1], p->w.K, &rows);
+        if (x == nullptr) Py_RETURN_NONE;
+        c10::InferenceMode guard;
+        if (p->linear_rows != rows) {
+            p->linear_bytes = hqm_linear_scratch_preferred(rows, &p->w);
+            p->linear_rows = rows;
+        }
+        size_t have = 0;
+        void* ws = nullptr;
+        if (p->linear_bytes && (ws = scratch(*x, p->linear_bytes, &have)) == nullptr) Py_RETURN_NONE;
+        at::Tensor y = result(*x, p->w.N);
+        const hqm_weight w = p->w;                         // (without the lock another thread may replace the plan)
+        const size_t bytes = p->linear_bytes;
+        const uint16_t* b = static_cast<const uint16_t*>(address(bias));
+        int rc;
+        Py_BEGIN_ALLOW_THREADS
+        rc = hqm_linear(static_cast<uint16_t*>(y.data_ptr()), static_cast<const uint16_t*>(x->const_data_ptr()), rows, &w, b, ws, bytes,
+                        c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
+        Py_END_ALLOW_THREADS
+        if (rc < 0) Py_RETURN_NONE;
+        return THPVariable_Wrap(std::move(y));
+    } catch (const std::exception& e) {
+        return PyErr_Format(PyExc_RuntimeError, "%s", e.what());
+    }
+}
+
+// The three plans of an expert module.
+bool expert_plans(PyObject* module, Plan* (&p)[3]) {
+    PyObject* dict = dict_of(module);
+    PyObject* modules = item(dict, N.modules);
+    Py_XDECREF(dict);
+    PyObject* names[3] = {N.w1, N.w2, N.w3};
+    for (int i = 0; i < 3; ++i) {
+        PyObject* layer = item(modules, names[i]);
+        PyObject* d = layer == nullptr ? nullptr : dict_of(layer);
+        p[i] = d == nullptr ? nullptr : plan_of(layer, d);
+        Py_XDECREF(d);
+        if (p[i] == nullptr) return false;
+    }
+    return true;
+}
+
+int run_expert(Plan* (&p)[3], const at::Tensor& x, int64_t rows, const int32_t* idx, const float* w, uint16_t* out, int accumulate) {
+    if (p[0]->expert_rows != rows) {
+        p[0]->expert_bytes = hqm_expert_ffn_scratch_bytes(rows, &p[0]->w, &p[1]->w, &p[2]->w);
+        p[0]->expert_rows = rows;
+    }
+    size_t have = 0;
+    void* ws = scratch(x, p[0]->expert_bytes, &have);
+    if (ws == nullptr) return -1;
+    const hqm_weight w1 = p[0]->w, w2 = p[1]->w, w3 = p[2]->w;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = hqm_expert_ffn(out, static_cast<const uint16_t*>(x.const_data_ptr()), rows, idx, w, accumulate, &w1, &w2, &w3, ws, have,
+                        c10::cuda::getCurrentCUDAStream(x.device().index()).stream());
+    Py_END_ALLOW_THREADS
+    return rc;
+}
+
+// expert(module, x): all rows of x
+PyObject* expert(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2) return PyErr_Format(PyExc_TypeError, "expert(module, x)");
+    try {
+        Plan* p[3];
+        if (!expert_plans(args[0], p)) Py_RETURN_NONE;
+        int64_t rows = 0;
+        const at::Tensor* x = rows_of(args[1], p[0]->w.K, &rows);
+        if (x == nullptr) Py_RETURN_NONE;
+        c10::InferenceMode guard;
+        at::Tensor out = result(*x, p[1]->w.N);
+        if (run_expert(p, *x, rows, nullptr, nullptr, static_cast<uint16_t*>(out.data_ptr()), 0) < 0) Py_RETURN_NONE;
+        return THPVariable_Wrap(std::move(out));
+    } catch (const std::exception& e) {
+        return PyErr_Format(PyExc_RuntimeError, "%s", e.what());
+    }
+}
+
+PyObject* setup(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2) return PyErr_Format(PyExc_TypeError, "setup(scratch, grow)");
+    Py_INCREF(args[0]);
+    Py_INCREF(args[1]);
+    Py_XSETREF(g_scratch, args[0]);
+    Py_XSETREF(g_grow, args[1]);
+    Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"setup", (PyCFunction)(void (*)(void))setup, METH_FASTCALL, "setup(scratch_dict, grow)"},
+    {"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, "linear(layer, x) -> tensor or None"},
+    {"expert", (PyCFunction)(void (*)(void))expert, METH_FASTCALL, "expert(module, x) -> tensor or None"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Host path of the quantized layers.", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) {
+    struct {
+        PyObject** to;
+        const char* name;
+    } all[] = {{&N.dict, "__dict__"}, {&N.W_q, "W_q"},     {&N.meta, "meta"},           {&N.bias, "bias"},           {&N.plan, "_plan"}, {&N.ready, "ready"},
+               {&N.scale_q, "scale_q"}, {&N.zero_q, "zero_q"}, {&N.meta_scale, "meta_scale"}, {&N.meta_zero, "meta_zero"}, {&N.scale, "scale"}, {&N.zero, "zero"},
+               {&N.modules, "_modules"}, {&N.w1, "w1"},    {&N.w2, "w2"},               {&N.w3, "w3"}, {&N.axis, "axis"}};
+    for (auto& a : all)
+        if ((*a.to = PyUnicode_InternFromString(a.name)) == nullptr) return nullptr;
+    PlanType.tp_flags = Py_TPFLAGS_DEFAULT;
+    PlanType.tp_methods = plan_methods;
+    if (PyType_Ready(&PlanType) != 0) return nullptr;
+    return PyModule_Create(&module);
+}
