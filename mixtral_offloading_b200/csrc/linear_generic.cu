@@ -127,8 +127,123 @@ __global__ void dequantize_kernel(T* __restrict__ out, hqm_weight w, int G, int 
     }
 }
 
+// The same for K a multiple of 4 and aligned tensors.  A scale and a zero belong to every G-th row: a thread takes RES
+// neighbouring residues and 4 columns, decodes their scales and zeros once and goes through `members` rows of each.  RES is
+// the number of codes in a byte where G is a multiple of it (a byte then holds the same residues in every member), else 1.
+// Bound by the writes.  Per element it is the code's shift, mask and conversion (an OR into 2^23 and an exact subtraction),
+// one subtraction, one product; decoding per element with a 64-bit remainder each took 238 us for
+// 14336 x 4096 in 2 bits, this takes 33 (floor 21), and 11 for 4096 x 4096 in 4 bits.
+template <typename T> struct Four;
+template <> struct Four<float> {
+    __device__ static void store(float* p, const float* v) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+};
+template <> struct Four<__half> {
+    __device__ static void store(__half* p, const float* v) {
+        __half2 h[2] = {__floats2half2_rn(v[0], v[1]), __floats2half2_rn(v[2], v[3])};
+        *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(h);
+    }
+};
+template <> struct Four<__nv_bfloat16> {
+    __device__ static void store(__nv_bfloat16* p, const float* v) {
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+        *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(h);
+    }
+};
+constexpr int DEQ_THREADS = 128;
+// Four neighbouring columns of a meta vector of C columns, from column c on.
+__device__ __forceinline__ void meta4(const uint16_t* p, int c, int C, bool vec, float* f) {
+    if (vec) {                                // 8-byte aligned and C a multiple of 4
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + c));
+        f[0] = f16_bits_to_float((uint16_t)v.x); f[1] = f16_bits_to_float((uint16_t)(v.x >> 16));
+        f[2] = f16_bits_to_float((uint16_t)v.y); f[3] = f16_bits_to_float((uint16_t)(v.y >> 16));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            f[j] = f16_bits_to_float(p[c]);
+            c = c + 1 == C ? 0 : c + 1;
+        }
+    }
+}
+template <int NBITS, int RES, typename T>
+__global__ void __launch_bounds__(DEQ_THREADS) dequantize_members_kernel(T* __restrict__ out, hqm_weight w, int G, int C, int members, bool meta_vec) {
+    constexpr int PER = codes_per_word(NBITS);
+    constexpr uint32_t MASK = (1u << NBITS) - 1u;
+    const int K4 = w.K / 4;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= (int64_t)(G / RES) * K4) return;
+    const int g0 = (int)(i / K4) * RES, k = (int)(i % K4) * 4;
+    const int Cz = (int)zero_meta_cols(w, G);
+    float sc[RES][4], zr[RES][4];
+#pragma unroll
+    for (int r = 0; r < RES; ++r) {
+        const int64_t idx = (int64_t)(g0 + r) * w.K + k;
+        const uint32_t sq = *reinterpret_cast<const uint32_t*>(w.scale_q + idx), zq = *reinterpret_cast<const uint32_t*>(w.zero_q + idx);
+        const int c = (int)(idx % C), cz = Cz == C ? c : (int)(idx % Cz);
+        float ms[4], mz[4], zs[4], zz[4];
+        meta4(w.ms_scale, c, C, meta_vec, ms);
+        meta4(w.mz_scale, c, C, meta_vec, mz);
+        meta4(w.ms_zero, cz, Cz, meta_vec, zs);
+        meta4(w.mz_zero, cz, Cz, meta_vec, zz);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            sc[r][j] = __fmul_rn(__fsub_rn((float)((sq >> (8 * j)) & 255u), mz[j]), ms[j]);
+            zr[r][j] = __fmul_rn(__fsub_rn((float)((zq >> (8 * j)) & 255u), zz[j]), zs[j]);
+        }
+    }
+    const int m0 = blockIdx.y * members, m1 = min(m0 + members, w.group_size);
+#pragma unroll 4
+    for (int m = m0; m < m1; ++m) {
+        const uint32_t n0 = (uint32_t)(m * G + g0);           // < N
+        const uint32_t R = n0 / PER;
+        const int s0 = RES > 1 ? 0 : (int)(n0 - R * PER);
+        uint32_t v[4];                                        // NBITS == 3: a word per column, else one for the four
+        if (NBITS == 3) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const int32_t*>(w.W_q) + (int64_t)R * w.K + k));
+            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        } else {
+            v[0] = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(w.W_q) + (int64_t)R * w.K + k));
+        }
+#pragma unroll
+        for (int r = 0; r < RES; ++r) {
+            const int shift = NBITS * (PER - 1 - s0 - r);
+            float o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t code = (NBITS == 3 ? v[j] >> shift : v[0] >> (8 * j + shift)) & MASK;
+                const float c = __fsub_rn(__uint_as_float(0x4B000000u | code), 8388608.f);
+                o[j] = __fmul_rn(__fsub_rn(c, zr[r][j]), sc[r][j]);
+            }
+            Four<T>::store(out + (int64_t)(n0 + r) * w.K + k, o);
+        }
+    }
+}
+
+template <int NBITS, int RES, typename T>
+static void dequantize_members(T* out, const hqm_weight* w, int G, int C, cudaStream_t st) {
+    const int64_t threads = (int64_t)(G / RES) * (w->K / 4);
+    // Rows per residue of a thread: all of a group, halved down to 4 while that leaves the SMs half empty (a quarter
+    // empty or full instead: 35 and 41 us for the 33 above, as every thread decodes the same scales again).
+    int members = w->group_size;
+    while (members > 4 && threads * ((w->group_size + members - 1) / members) < 148 * 1024) members = (members + 1) / 2;
+    auto a8 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; };
+    const bool meta_vec = C % 4 == 0 && zero_meta_cols(*w, G) % 4 == 0 && a8(w->ms_scale) && a8(w->mz_scale) && a8(w->ms_zero) && a8(w->mz_zero);
+    const dim3 grid((unsigned)((threads + DEQ_THREADS - 1) / DEQ_THREADS), (unsigned)((w->group_size + members - 1) / members));
+    dequantize_members_kernel<NBITS, RES, T><<<grid, DEQ_THREADS, 0, st>>>(out, *w, G, C, members, meta_vec);
+}
+
 template <typename T>
 static int launch_dequantize(void* out, const hqm_weight* w, int G, int C, cudaStream_t st) {
+    auto aligned = [](const void* p, size_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; };
+    const int64_t Cz = zero_meta_cols(*w, G);
+    if (w->K % 4 == 0 && aligned(out, 4 * sizeof(T)) && aligned(w->W_q, w->nbits == 3 ? 16 : 4) && aligned(w->scale_q, 4) &&
+        aligned(w->zero_q, 4) && Cz <= INT32_MAX && w->group_size <= 65535) {
+        T* o = (T*)out;
+        if (w->nbits == 3) dequantize_members<3, 1>(o, w, G, C, st);
+        else if (w->nbits == 2) G % 4 == 0 ? dequantize_members<2, 4>(o, w, G, C, st) : dequantize_members<2, 1>(o, w, G, C, st);
+        else G % 2 == 0 ? dequantize_members<4, 2>(o, w, G, C, st) : dequantize_members<4, 1>(o, w, G, C, st);
+        HQM_LAUNCH_CHECK();
+        return HQM_OK;
+    }
     const int64_t total = storage_rows(w->N, w->nbits) * w->K;
     int64_t blocks = (total + 255) / 256;
     if (blocks > 148 * 32) blocks = 148 * 32;

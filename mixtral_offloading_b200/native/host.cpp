@@ -175,6 +175,35 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
 }
 
+// dequantize(layer, code): the weight in bf16 (0), fp16 (1) or fp32 (2)
+PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2) return PyErr_Format(PyExc_TypeError, "dequantize(layer, code)");
+    try {
+        const long code = PyLong_AsLong(args[1]);
+        PyObject* dict = dict_of(args[0]);
+        Plan* p = dict == nullptr ? nullptr : plan_of(args[0], dict);
+        PyObject* wq = item(dict, N.W_q);
+        Py_XDECREF(dict);
+        if (p == nullptr || code < 0 || code > 2) {
+            PyErr_Clear();
+            Py_RETURN_NONE;
+        }
+        const at::Tensor& like = THPVariable_Unpack(wq);
+        if (like.device().index() != c10::cuda::current_device()) Py_RETURN_NONE;
+        c10::InferenceMode guard;
+        at::Tensor out = at::empty({p->w.N, p->w.K}, like.options().dtype(code == 0 ? at::kBFloat16 : code == 1 ? at::kHalf : at::kFloat));
+        const hqm_weight w = p->w;
+        int rc;
+        Py_BEGIN_ALLOW_THREADS
+        rc = hqm_dequantize(out.data_ptr(), (int)code, &w, c10::cuda::getCurrentCUDAStream(like.device().index()).stream());
+        Py_END_ALLOW_THREADS
+        if (rc < 0) Py_RETURN_NONE;
+        return THPVariable_Wrap(std::move(out));
+    } catch (const std::exception& e) {
+        return PyErr_Format(PyExc_RuntimeError, "%s", e.what());
+    }
+}
+
 // The three plans of an expert module.
 bool expert_plans(PyObject* module, Plan* (&p)[3]) {
     PyObject* dict = dict_of(module);
@@ -238,6 +267,7 @@ PyObject* setup(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef methods[] = {
     {"setup", (PyCFunction)(void (*)(void))setup, METH_FASTCALL, "setup(scratch_dict, grow)"},
     {"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, "linear(layer, x) -> tensor or None"},
+    {"dequantize", (PyCFunction)(void (*)(void))dequantize, METH_FASTCALL, "dequantize(layer, dtype code) -> tensor or None"},
     {"expert", (PyCFunction)(void (*)(void))expert, METH_FASTCALL, "expert(module, x) -> tensor or None"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Host path of the quantized layers.", -1, methods, nullptr, nullptr, nullptr, nullptr};
