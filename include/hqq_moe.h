@@ -129,6 +129,12 @@ size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w);
  * bias may be NULL.  scratch may be NULL when hqm_linear_scratch_bytes() is 0.
  * Rows 1..4 take the weight-streaming kernels, 5 and more the tcgen05 kernels; HQM_FORCE_GENERIC=1 in the environment
  * at load time routes everything through the shape-agnostic kernel. */
+/* Up to four layers of one K, bit width and group size over the same rows (q, k and v of a decoder layer) in one launch:
+ * y[i] = x . W_est[i]^T (+ bias[i]); bias may be NULL.  Five or more rows of 2- or 4-bit layers; the scratch size is 0 for
+ * everything else. */
+size_t hqm_linear_group_scratch_bytes(int64_t M, const hqm_weight* const* w, int32_t count);
+int hqm_linear_group(uint16_t* const* y, const uint16_t* x, int64_t M, const hqm_weight* const* w, const uint16_t* const* bias,
+                     int32_t count, void* scratch, size_t scratch_bytes, void* stream);
 int hqm_linear(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias,
                void* scratch, size_t scratch_bytes, void* stream);
 

@@ -82,8 +82,8 @@ size_t linear_scratch_bytes(int64_t M, const hqm_weight* w, bool preferred) {
     if (M <= 0 || check_weight(w, &G, &C) != HQM_OK) return 0;
     if (force_generic()) return 0;
     if (use_gg(w, G, C, M)) {
-        const GgRows rows = gg_linear_layout(M, w).rows;
-        return gg_stage_bytes(rows.padded(), w->K, true) + (preferred ? gg_scratch_bytes(rows.n) : gg_scratch_least(rows.n, w));
+        const GgRows rows = gg_linear_layout(M, &w, 1).rows;
+        return gg_stage_bytes(rows.padded(), w->K, true) + (preferred ? gg_scratch_bytes(rows.n) : gg_scratch_least(rows.n, &w, 1));
     }
     if (gemm_tc3_supported(w, G, C, M)) return gemm_tc3_scratch_bytes(w, G, M);
     Stream3Plan plan3;
@@ -102,6 +102,32 @@ static int need_scratch(void* scratch, size_t have, size_t need) {
     return HQM_OK;
 }
 
+// Layers of one K and format over the same rows: the rows staged once, one launch over all tiles.
+static int linear_gg(uint16_t* const* y, const hqm_weight* const* ws, const uint16_t* const* bias, int count, const uint16_t* x,
+                     const int32_t* x_idx, int64_t M, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st) {
+    const GgLayout layout = gg_linear_layout(M, ws, count);
+    const int K = ws[0]->K;
+    const int64_t xt_rows = layout.rows.padded();
+    const size_t staged = gg_stage_bytes(xt_rows, K, true);
+    int rc = need_scratch(scratch, scratch_bytes, staged + gg_scratch_least(layout.rows.n, ws, count));
+    if (rc != HQM_OK) return rc;
+    const GgStaged xs = gg_staged(scratch, xt_rows, K, true);
+    rc = launch_gg_stage(xs, x, 0, x_idx, nullptr, 1, M, K, st);
+    if (rc != HQM_OK) return rc;
+    GgJob job{};
+    job.problems = count;
+    job.rows = (int)M;
+    job.layout = layout;
+    job.x = xs;
+    job.mode = GG_LINEAR;
+    for (int i = 0; i < count; ++i) {
+        job.w0[i] = ws[i];
+        job.y[i] = y[i];
+        job.bias[i] = bias ? bias[i] : nullptr;
+    }
+    return launch_gg(job, counters, (uint8_t*)scratch + staged, scratch_bytes - staged, st);
+}
+
 int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t M, const hqm_weight* w,
                   const uint16_t* bias, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st) {
     int G, C;
@@ -112,24 +138,7 @@ int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t 
     const bool x_ok = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     if (!x_ok || force_generic()) return launch_linear_generic(y, x, x_idx, M, w, G, C, bias, st);
     if (use_gg(w, G, C, M)) {
-        const GgLayout layout = gg_linear_layout(M, w);
-        const int64_t xt_rows = layout.rows.padded();
-        const size_t staged = gg_stage_bytes(xt_rows, w->K, true);
-        rc = need_scratch(scratch, scratch_bytes, staged + gg_scratch_least(layout.rows.n, w));
-        if (rc != HQM_OK) return rc;
-        const GgStaged xs = gg_staged(scratch, xt_rows, w->K, true);
-        rc = launch_gg_stage(xs, x, 0, x_idx, nullptr, 1, M, w->K, st);
-        if (rc != HQM_OK) return rc;
-        GgJob job{};
-        job.problems = 1;
-        job.w0[0] = w;
-        job.rows = (int)M;
-        job.layout = layout;
-        job.x = xs;
-        job.mode = GG_LINEAR;
-        job.y[0] = y;
-        job.bias[0] = bias;
-        return launch_gg(job, counters, (uint8_t*)scratch + staged, scratch_bytes - staged, st);
+        return linear_gg(&y, &w, &bias, 1, x, x_idx, M, counters, scratch, scratch_bytes, st);
     }
     if (gemm_tc3_supported(w, G, C, M)) {
         rc = need_scratch(scratch, scratch_bytes, gemm_tc3_scratch_bytes(w, G, M));
@@ -185,6 +194,34 @@ size_t hqm_linear_scratch_bytes(int64_t M, const hqm_weight* w) {
 size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w) {
     const size_t inner = hqm::linear_scratch_bytes(M, w, /*preferred=*/true);
     return inner ? inner + hqm::SCRATCH_HEADER : 0;
+}
+
+size_t hqm_linear_group_scratch_bytes(int64_t M, const hqm_weight* const* w, int32_t count) {
+    using namespace hqm;
+    if (M <= 0 || count < 1 || count > 4 || w == nullptr || force_generic()) return 0;
+    for (int i = 0; i < count; ++i) {
+        int G, C;
+        if (check_weight(w[i], &G, &C) != HQM_OK || !use_gg(w[i], G, C, M)) return 0;
+        if (w[i]->K != w[0]->K || w[i]->nbits != w[0]->nbits || w[i]->group_size != w[0]->group_size) return 0;
+    }
+    const GgRows rows = gg_linear_layout(M, w, count).rows;
+    return SCRATCH_HEADER + gg_stage_bytes(rows.padded(), w[0]->K, true) + gg_scratch_bytes(rows.n);
+}
+
+int hqm_linear_group(uint16_t* const* y, const uint16_t* x, int64_t M, const hqm_weight* const* w, const uint16_t* const* bias,
+                     int32_t count, void* scratch, size_t scratch_bytes, void* stream) {
+    using namespace hqm;
+    const size_t need = hqm_linear_group_scratch_bytes(M, w, count);
+    HQM_CHECK_ARG(need != 0, "linear_group: layers of one K and format and five or more rows are needed");
+    HQM_CHECK_ARG(y && x && (reinterpret_cast<uintptr_t>(x) & 15u) == 0, "linear_group: null or unaligned activation pointer");
+    for (int i = 0; i < count; ++i) HQM_CHECK_ARG(y[i] != nullptr, "linear_group: null output %d", i);
+    if (scratch == nullptr || scratch_bytes < need) {
+        set_error("linear_group: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
+        return HQM_ERR_SCRATCH;
+    }
+    HQM_CHECK_ARG((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "linear_group: scratch must be 256-byte aligned");
+    return linear_gg(y, w, bias, count, x, nullptr, M, (uint32_t*)scratch, (uint8_t*)scratch + SCRATCH_HEADER,
+                     scratch_bytes - SCRATCH_HEADER, (cudaStream_t)stream);
 }
 
 int hqm_linear(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias, void* scratch,

@@ -91,6 +91,7 @@ struct Problem {
     int cnt, n, chunks, cost;              // rows; rows per chunk (padded); chunks; cost of a unit
     int row0, list0;                       // first row in the staged x, first entry in the row list
     int tiles, G, P, C;
+    int N, blocks;                         // output rows; blocks of 16 members
     int f16;
 };
 
@@ -120,7 +121,7 @@ struct TmemMap {
 struct HostProblem {
     CUtensorMap maps[2][3];
     const uint16_t* meta[2][4];
-    int G, P, C, tiles;
+    int G, P, C, tiles, N, blocks;
     void* y;
     const uint16_t* bias;
 };
@@ -162,19 +163,22 @@ struct Shared {
     volatile int failed;
 };
 
-template <int NBITS_, int GS_>
+// A tile is 8 neighbouring residues (the codes of PARTS neighbouring bytes) of 16 members of their groups; GG_UP: 4 of w1
+// and the same 4 of w3.  Larger groups are several blocks of 16 members, each a tile that decodes the scales again: eight
+// neighbouring output rows make one 16-byte store.  (4-bit layers with whole groups of 64 in a tile wrote two rows, 4
+// bytes, at a time: 3000 cycles per 16 rows of x, more than the tile's own time from 128 rows on.)
+template <int NBITS_>
 struct Fmt {
-    static constexpr int NBITS = NBITS_, GS = GS_;
+    static constexpr int NBITS = NBITS_, MEMBERS = 16;
     static constexpr int PER = codes_per_word(NBITS);
-    static constexpr int PARTS = 128 / (PER * GS);         // storage-row residues of a tile (GG_UP: one of w1, one of w3)
-    static_assert(PARTS * PER * GS == 128, "a tile holds whole groups");
+    static constexpr int PARTS = 8 / PER;                  // storage-row residues of a tile
     // Columns of a unit.  What a warp does once per unit (waits, decoding, hand-over) takes about as long as the weights of
     // 128 columns of a 2-bit tile, and those layers are large; 4-bit layers decode little and may be small.
     static constexpr int UK = 128;
     static constexpr int HALVES = UK / 128;                // A slots of a unit
     static constexpr int BLOCKS = UK / 64;
-    static constexpr int SLW = (GS == 16) ? 2 : 1;         // rows of scales a warp needs (GS = 16: one of either part)
-    static constexpr int CODE_PART = GS * 128;             // packed bytes of a part of 128 columns
+    static constexpr int SLW = 2;                          // rows of scales a warp needs: its slot of two parts
+    static constexpr int CODE_PART = MEMBERS * 128;             // packed bytes of a part of 128 columns
     static constexpr int CODE_HALF = PARTS * CODE_PART;
     static constexpr int SZ_PART = PER * 128;
     static constexpr int SQ_OFF = HALVES * CODE_HALF, ZQ_OFF = SQ_OFF + HALVES * PARTS * SZ_PART;
@@ -185,7 +189,7 @@ struct Fmt {
     static constexpr int ST_BLOCK = 2 * SLW * 64, ST_T = BLOCKS * ST_BLOCK;
     // Launches of up to 64 rows per chunk need few staged rows in flight and many packed bytes, others the reverse.
     __host__ __device__ static constexpr int b_ring(int n_max) { return n_max <= 64 ? 64 * 1024 : 128 * 1024; }
-    __host__ __device__ static constexpr int n_raw(int n_max) { return 2 * GROUPS; }
+    __host__ __device__ static constexpr int n_raw(int n_max) { return PARTS == 4 && n_max > 64 ? 6 : 8; }
     static constexpr int ST_OFF = 0, EPI_OFF = ST_OFF + 4 * GROUPS * ST_WARP, BAR_OFF = EPI_OFF + EPI_BYTES, RING_OFF = BAR_OFF + 1024;
     __host__ __device__ static constexpr int smem(int n_max) {
         return (RING_OFF + 1023) / 1024 * 1024 + b_ring(n_max) + n_raw(n_max) * RAW_BYTES + 1024;
@@ -193,15 +197,10 @@ struct Fmt {
     static_assert(smem(64) + (int)sizeof(Shared) <= 227 * 1024 && smem(256) + (int)sizeof(Shared) <= 227 * 1024, "shared memory");
     // Which row of the tile TMEM lane 32 q + 8 j + g holds (q: warp of a group, j = 0..3): part, slot of the byte, member.
     // A thread of the 16x256b store shape holds j = 0..3 at one g: four members of one quantisation group.
-    __device__ __forceinline__ static int part_of(int q, int g) { return GS == 16 ? (g & 1) : (PARTS == 2 ? q >> 1 : 0); }
+    __device__ __forceinline__ static int part_of(int q, int g) { return (NBITS == 2 ? 0 : 2 * (q >> 1)) + (g & 1); }
     __device__ __forceinline__ static int slot_of(int q) { return NBITS == 2 ? q : q & 1; }
-    __device__ __forceinline__ static int member_of(int q, int g, int j) {
-        if (GS == 16) return (g >> 1) + 4 * j;
-        const int low = (g >> 1) | ((g & 1) << 2);         // neighbouring g: rows 4 apart, on other banks after the swizzle
-        return low + 8 * j + (GS == 64 ? 32 * (q >> 1) : 0);
-    }
+    __device__ __forceinline__ static int member_of(int g, int j) { return (g >> 1) + 4 * j; }
 };
-
 // Position of column k of a 64-column block in the staged order (and in the A tile).
 __host__ __device__ constexpr int tile_pos(int k) {
     const int c = k >> 4, i = (k >> 2) & 3, e = k & 3;                  // thread column, word, byte
@@ -398,9 +397,9 @@ __device__ __forceinline__ bool next_seg(const Shared& sh, int ubegin, int uend,
     return true;
 }
 
-template <int NBITS, int GS, int MODE>
+template <int NBITS, int MODE>
 __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__ Params prm) {
-    using F = Fmt<NBITS, GS>;
+    using F = Fmt<NBITS>;
     constexpr int PER = F::PER, PARTS = F::PARTS, SLW = F::SLW, UK = F::UK, HALVES = F::HALVES, BLOCKS = F::BLOCKS, DC = F::DC;
     extern __shared__ unsigned char smem_raw[];
     __shared__ Shared sh;
@@ -466,6 +465,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             p.P = h.P;
             p.C = h.C;
             p.tiles = h.tiles;
+            p.N = h.N;
+            p.blocks = h.blocks;
             p.cnt = cnt;
             const GgRows r = counted ? GgRows::of(cnt) : GgRows{prm.chunks, prm.n_max};
             p.n = r.n;
@@ -525,7 +526,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
         const int group = warp >> 2, q = warp & 3, g = lane >> 2, c = lane & 3;
         const int part = F::part_of(q, g), slot = F::slot_of(q);
         // the row of scales / zeros this lane decodes: DC columns of it
-        const int dpart = (SLW == 2) ? lane >> 4 : part;
+        const int dlocal = lane >> 4, dpart = F::part_of(q, dlocal);
         const int dcol = DC * (lane & (UK / DC - 1));
         const int dhalf = dcol >> 7;
         // The field of the warp's slot inside a byte.  2 bit: slots 0, 1 at bits 7-6, 5-4, slots 2, 3 at 3-2, 1-0; 4 bit: 7-4 or
@@ -538,15 +539,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
         // s / t of the warp: [block][half][part][thread column][8 values], s first; 16-byte pieces, so that the eight lanes of
         // a load phase touch 128 contiguous bytes
         const uint32_t st_area = sbase + F::ST_OFF + warp * F::ST_WARP;
-        const uint32_t st_read = st_area + ((SLW == 2) ? (g & 1) * 64 : 0) + c * 16;
+        const uint32_t st_read = st_area + (g & 1) * 64 + c * 16;
         // this thread's bytes of a staged row: 16 of a 64-column block, members j = 0, 1 (the 128-byte swizzle)
         uint32_t code_off[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            const int m = F::member_of(q, g, j);
+            const int m = F::member_of(g, j);
             code_off[j] = (uint32_t)(part * F::CODE_PART + m * 128 + ((c ^ (m & 7)) << 4));
         }
-        constexpr int J2 = (GS == 16 ? 8 : 16) * 128;                      // from members j = 0, 1 to j = 2, 3
+        constexpr int J2 = 8 * 128;                      // from members j = 0, 1 to j = 2, 3
 
         Seg s;
         s.p = 0;
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             const Problem& pr = sh.pr[s.p];
             const bool f16 = pr.f16 != 0;
             const int wsel = (MODE == GG_UP) ? dpart : 0;
-            const int rho = (MODE == GG_UP) ? s.tile : s.tile * PARTS + dpart;
+            const int rho = (MODE == GG_UP) ? s.tile : s.tile / pr.blocks * PARTS + dpart;
             const int res = min(PER * rho + slot, pr.G - 1);  // (a tile's second part may lie past the last residue)
             mC = pr.C;
 #pragma unroll
@@ -691,7 +692,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
 #pragma unroll
                     for (int h = 0; h < (DC + 7) / 8; ++h) {
                         const int w64 = (dcol + 8 * h) & 63, blk = (dcol + 8 * h) >> 6;
-                        const uint32_t dst = st_area + blk * F::ST_BLOCK + ((w64 >> 3) & 1) * (SLW * 64) + ((SLW == 2) ? dpart * 64 : 0) +
+                        const uint32_t dst = st_area + blk * F::ST_BLOCK + ((w64 >> 3) & 1) * (SLW * 64) + dlocal * 64 +
                                              (w64 >> 4) * 16 + (w64 & 7) * 2;
                         if constexpr (DC >= 8) {
                             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(S[4 * h]), "r"(S[4 * h + 1]), "r"(S[4 * h + 2]), "r"(S[4 * h + 3]) : "memory");
@@ -812,7 +813,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 at += s.k1 - s.k0;
                 const Problem& pr = sh.pr[s.p];
                 const CUtensorMap* maps[2] = {pr.w[0].maps, pr.w[MODE == GG_UP ? 1 : 0].maps};
-                const int rho0 = (MODE == GG_UP) ? s.tile : s.tile * PARTS;
+                const int quad = (MODE == GG_UP) ? s.tile : s.tile / pr.blocks, rho0 = (MODE == GG_UP) ? quad : quad * PARTS;
+                const int m0 = (MODE == GG_UP) ? 0 : 16 * (s.tile - quad * pr.blocks);
                 if (prm.table && fenced != s.p) {             // tensor maps in global memory
                     fenced = s.p;
 #pragma unroll
@@ -820,8 +822,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(maps[i / 3] + i % 3) : "memory");
                 }
                 for (int k = s.k0 + ((s.u0 ^ turn) & 1); k < s.k1; k += 2) {
-                    const int u = s.u0 + (k - s.k0), r = u & (n_raw - 1);         // n_raw is 4 or 8
-                    wait_limited(raw_empty + 8 * r, ((n_raw == 8 ? u >> 3 : u >> 2) & 1) ^ 1, limit);
+                    const int u = s.u0 + (k - s.k0), lap = n_raw == 8 ? u >> 3 : u / 6, r = u - lap * n_raw;
+                    wait_limited(raw_empty + 8 * r, (lap & 1) ^ 1, limit);
                     const uint32_t bar = raw_full + 8 * r, dst = raw_ring + r * F::RAW_BYTES;
                     if (leader) {
                         expect_tx(bar, F::RAW_TX);
@@ -830,11 +832,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
 #pragma unroll
                             for (int p = 0; p < PARTS; ++p) {
                                 const int rho = (MODE == GG_UP) ? rho0 : rho0 + p, col = k * UK + 128 * h;
-#pragma unroll
-                                for (int b = 0; b < GS / 16; ++b)
-                                    tma_3d(dst + h * F::CODE_HALF + p * F::CODE_PART + b * 2048, maps[p], col, rho, 16 * b, bar);
-                                tma_3d(dst + F::SQ_OFF + (h * PARTS + p) * F::SZ_PART, maps[p] + 1, col, PER * rho, 0, bar);
-                                tma_3d(dst + F::ZQ_OFF + (h * PARTS + p) * F::SZ_PART, maps[p] + 2, col, PER * rho, 0, bar);
+                                const CUtensorMap* map = maps[MODE == GG_UP ? p : 0];
+                                tma_3d(dst + h * F::CODE_HALF + p * F::CODE_PART, map, col, rho, m0, bar);
+                                tma_3d(dst + F::SQ_OFF + (h * PARTS + p) * F::SZ_PART, map + 1, col, PER * rho, 0, bar);
+                                tma_3d(dst + F::ZQ_OFF + (h * PARTS + p) * F::SZ_PART, map + 2, col, PER * rho, 0, bar);
                             }
                     }
                 }
@@ -960,7 +961,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
         if (!counted) grid_dependency_wait();
         const int q = warp & 3, g = lane & 7, j4 = lane >> 3;         // TMEM lane 32 q + 8 j4 + g
         const int et = threadIdx.x - WARP_EPI * 32;                   // thread of the epilogue
-        const int part = F::part_of(q, g), slot = F::slot_of(q), member = F::member_of(q, g, j4);
+        const int part = F::part_of(q, g), slot = F::slot_of(q), member = F::member_of(g, j4);
         constexpr int RUN = PARTS * PER;                              // neighbouring output rows of a member in a tile
         unsigned char* epi = base + F::EPI_OFF;
         float* s_scale = reinterpret_cast<float*>(epi + 2 * TILE_BYTES);      // per row of the chunk: factor of the sums,
@@ -980,7 +981,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             const bool whole = s.k0 == 0 && s.k1 == units_k;
             const int rows_here = min(n, cnt - s.chunk * n);          // rows of this chunk that exist
             const int list = pr.list0 + s.chunk * n;                  // list entry of the chunk's first row
-            const int rho0 = (MODE == GG_UP) ? s.tile : s.tile * PARTS;
+            const int quad = (MODE == GG_UP) ? s.tile : s.tile / pr.blocks, rho0 = (MODE == GG_UP) ? quad : quad * PARTS;
+            const int m0 = (MODE == GG_UP) ? 0 : 16 * (s.tile - quad * pr.blocks);
             const int rho = (MODE == GG_UP) ? s.tile : rho0 + part;
             // what the rows need is fetched while the sums are still being formed
             for (int i = et; i < rows_here; i += 128) {
@@ -993,7 +995,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             float bias = 0.f;
             if (MODE == GG_LINEAR) {
                 const uint16_t* bp = prm.hp[s.p].bias;
-                if (bp && rho < pr.P) bias = bf16_bits_to_float(bp[member * pr.G + PER * rho + slot]);
+                if (bp && rho < pr.P) bias = bf16_bits_to_float(bp[(m0 + member) * pr.G + PER * rho + slot]);
             }
             if (!wait(acc_full + 8 * (seg & 1), (seg >> 1) & 1)) ok = false;
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
@@ -1138,9 +1140,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                             tb[i * 128 + idx] = o;
                         }
                         epi_sync();
-                        constexpr int MEMBERS = 128 / RUN;
+                        constexpr int MEMBERS = F::MEMBERS;
                         const int valid = min(PARTS, pr.P - rho0) * PER;      // neighbouring rows that exist
-                        const int64_t ld = (MODE == GG_LINEAR) ? pr.G * GS : prm.N;
+                        const int64_t ld = (MODE == GG_LINEAR) ? pr.N : prm.N;
                         uint16_t* out = reinterpret_cast<uint16_t*>(MODE == GG_LINEAR ? prm.hp[s.p].y : prm.out);
 #pragma unroll 2
                         for (int j = et; j < 16 * MEMBERS; j += 128) {
@@ -1148,7 +1150,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                             if (c0 + t >= rows_here) continue;
                             const uint16_t* src = tb + t * 128 + m * RUN;
                             const int64_t row = MODE == GG_DOWN ? s_row[c0 + t] : list + c0 + t;
-                            uint16_t* dst = out + row * ld + (int64_t)m * pr.G + PER * rho0;
+                            uint16_t* dst = out + row * ld + (int64_t)(m0 + m) * pr.G + PER * rho0;
                             if (MODE == GG_DOWN && (prm.accumulate || prm.out_f16)) {
                                 for (int x = 0; x < valid; ++x) {
                                     float val = bf16_bits_to_float(src[x]);
@@ -1277,8 +1279,7 @@ static constexpr int UK_MIN = 128;
 bool gg_supported(const hqm_weight* w, int G, int C) {
     if ((w->nbits != 2 && w->nbits != 4) || !meta_uniform(w) || tma_encode_entry() == nullptr) return false;
     const int per = codes_per_word(w->nbits), g = w->group_size;
-    if (!((w->nbits == 2 && (g == 16 || g == 32)) || (w->nbits == 4 && (g == 32 || g == 64)))) return false;
-    if (G % per != 0 || w->K % 64 != 0 || w->K < UK_MIN || C < 1) return false;
+    if (g % 16 != 0 || G % per != 0 || w->K % 64 != 0 || w->K < UK_MIN || C < 1) return false;
     if ((int64_t)G * w->K >= ((int64_t)1 << 31)) return false;
     auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     return a16(w->W_q) && a16(w->scale_q) && a16(w->zero_q) && a16(w->ms_scale) && a16(w->mz_scale) && a16(w->ms_zero) &&
@@ -1292,43 +1293,48 @@ static int gg_n_max(int64_t rows) {
 static size_t gg_piece_bytes(int n) { return (size_t)2 * n * 128 * sizeof(float); }      // of one CTA
 size_t gg_scratch_bytes(int n) { return (size_t)gg_sm_count() * gg_piece_bytes(n); }
 static int64_t gg_tiles(const hqm_weight* w) {
-    const int per = codes_per_word(w->nbits), parts = 128 / (per * w->group_size);
-    return (w->N / w->group_size / per + parts - 1) / parts;
+    return (w->N / w->group_size + 7) / 8 * (w->group_size / 16);
 }
 // (a layer with a tile for every SM is not worth running on a third of them)
-size_t gg_scratch_least(int n, const hqm_weight* w) {
-    return (size_t)(gg_tiles(w) >= gg_sm_count() ? gg_sm_count() : GG_LEAST_CTAS) * gg_piece_bytes(n);
+static int64_t gg_tiles(const hqm_weight* const* ws, int count) {
+    int64_t tiles = 0;
+    for (int i = 0; i < count; ++i) tiles += gg_tiles(ws[i]);
+    return tiles;
+}
+size_t gg_scratch_least(int n, const hqm_weight* const* ws, int count) {
+    return (size_t)(gg_tiles(ws, count) >= gg_sm_count() ? gg_sm_count() : GG_LEAST_CTAS) * gg_piece_bytes(n);
 }
 
 GgLayout gg_expert_layout(int64_t M) { return GgLayout{GgRows::of((int)M), gg_sm_count()}; }
-// Rows per chunk and CTAs of a linear layer, by what a launch costs in cycles of its longest CTA:
-//   its units of 128 columns:  unit_cycles
-//   a finished tile, per 16 rows:  ~250, or 1500 + 400 p where the last CTA to arrive reads p pieces back
-// Wide chunks dequantise the weights less often; narrow ones give every SM work without cutting a tile into many pieces.
-// (4-bit 1024 x 4096, 500 rows: 51 us as four chunks of 125 rows over 148 SMs, 27 us as sixteen of 32.)
-GgLayout gg_linear_layout(int64_t M, const hqm_weight* w) {
-    const int64_t tiles = gg_tiles(w), units_k = (w->K + 127) / 128, sms = gg_sm_count();
+// Rows per chunk and CTAs of linear layers over the same rows, by what a launch costs in cycles of its longest CTA (fitted to
+// 2- and 4-bit layers of 1024 to 14336 outputs with 16 to 500 rows):
+//   its units of 128 columns:  850 + 4 n with n rows; beyond 128 rows it is the staged x in every SM, 10 n
+//   a finished tile:           400 for every 16 rows
+//   a tile cut into p pieces:  5000 until the last CTA has seen that it is the last, and 3000 + 400 (p - 2) for every 16 rows;
+//                              twice where shares and tiles are not aligned, as a CTA then holds pieces of two tiles
+// Wide chunks dequantise the weights less often; narrow ones give every SM whole tiles.
+GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count) {
+    const int64_t tiles = gg_tiles(ws, count), units_k = (ws[0]->K + 127) / 128, sms = gg_sm_count();
     GgLayout best{};
     int64_t best_cost = INT64_MAX;
-    for (int cap = 16; cap <= GG_MAX_ROWS; cap *= 2) {
+    int chunks = 0;
+    for (int cap = 16; cap <= GG_MAX_ROWS; cap += 16) {
         const GgRows r = GgRows::of((int)M, cap);
-        const int64_t units = tiles * r.chunks * units_k, unit = gg::unit_cycles(true, r.n);
-        for (int64_t share = (units + sms - 1) / sms, step = 0; step < 3 && share <= units_k; ++step, share *= 2) {
-            const int64_t pieces = share >= units_k ? 1 : (units_k + share - 1) / share + 1;
-            const int64_t cost = share * unit + r.n / 16 * (pieces > 1 ? 1500 + 400 * pieces : 250);
+        if (r.chunks == chunks) continue;    // the same cut
+        chunks = r.chunks;
+        const int64_t units = tiles * r.chunks * units_k, n16 = r.n / 16, s0 = (units + sms - 1) / sms;
+        const int64_t unit = std::max<int64_t>(850 + 4 * r.n, r.n > 128 ? 10 * r.n : 0);
+        auto consider = [&](int64_t share, int64_t pieces, int cuts) {
+            const int64_t cost = share * unit + (share + units_k - 1) / units_k * n16 * 400 + cuts * (5000 + n16 * (3000 + 400 * (pieces - 2)));
             if (cost < best_cost) {
                 best_cost = cost;
                 best = GgLayout{r, (int)std::min<int64_t>(sms, (units + share - 1) / share)};
             }
-        }
-        const int64_t share = (units + sms - 1) / sms;
-        if (share > units_k) {               // a tile and more per CTA: cut in two at most
-            const int64_t cost = share * unit + (share + units_k - 1) / units_k * (r.n / 16) * 250 + r.n / 16 * 2300;
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = GgLayout{r, (int)sms};
-            }
-        }
+        };
+        consider((s0 + units_k - 1) / units_k * units_k, 2, 0);                                  // whole tiles
+        for (int64_t d = 2; d <= 8; d *= 2)
+            if (units_k % d == 0 && units_k / d >= s0) consider(units_k / d, d, 1);              // tiles in d equal parts
+        if (s0 % units_k != 0) consider(s0, s0 > units_k ? 2 : (units_k + s0 - 1) / s0 + 1, 2);  // equal shares of all SMs
         if (r.chunks == 1) break;
     }
     return best;
@@ -1342,10 +1348,10 @@ int launch_gg_stage(const GgStaged& to, const void* x, int x_f16, const int32_t*
     return HQM_OK;
 }
 
-template <int NBITS, int GS, int MODE>
+template <int NBITS, int MODE>
 static int gg_launch_one(const gg::Params& p, int grid, cudaStream_t st) {
-    using F = gg::Fmt<NBITS, GS>;
-    auto kern = gg::gg_kernel<NBITS, GS, MODE>;
+    using F = gg::Fmt<NBITS>;
+    auto kern = gg::gg_kernel<NBITS, MODE>;
     static bool attr_done[MAX_DEVICES];
     bool& done = attr_done[current_device_slot()];
     if (!done) {
@@ -1362,9 +1368,9 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
     const int host_problems = job.table ? 1 : job.problems;
     const hqm_weight* first = job.table ? job.shape : job.w0[0];
     const int nbits = first->nbits, gs = first->group_size, per = codes_per_word(nbits);
-    const int parts = 128 / (per * gs);
+    const int parts = 8 / per;
     HQM_CHECK_ARG(job.problems >= 1 && job.problems <= GG_MAX_PROBLEMS && host_problems <= 4, "gemm: %d problems in a launch", job.problems);
-    HQM_CHECK_ARG(job.mode != GG_UP || parts == 2, "gemm: the fused gate needs tiles of two parts");
+    HQM_CHECK_ARG(job.mode != GG_UP || (parts == 2 && gs == 16), "gemm: the fused gate needs 2-bit layers with groups of 16");
     int64_t tiles_all = 0;
     for (int i = 0; i < host_problems; ++i) {
         gg::HostProblem& h = p.hp[i];
@@ -1376,7 +1382,9 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
             h.G = G;
             h.C = C;
             h.P = G / per;
-            h.tiles = job.mode == GG_UP ? h.P : (h.P + parts - 1) / parts;
+            h.N = w->N;
+            h.blocks = gs / 16;
+            h.tiles = job.mode == GG_UP ? h.P : (h.P + parts - 1) / parts * h.blocks;
             if (!job.table) {
                 h.meta[l][0] = w->ms_scale;
                 h.meta[l][1] = w->mz_scale;
@@ -1420,18 +1428,15 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
     p.counters = counters;
     p.error_flag = tc_error_ptr();
     int64_t grid = job.counts ? gg_sm_count() : job.layout.grid;
-    const size_t least_bytes = job.counts ? gg_scratch_bytes(p.n_max) : std::min((size_t)grid * gg_piece_bytes(p.n_max), gg_scratch_least(p.n_max, first));
+    const size_t least_bytes = job.counts ? gg_scratch_bytes(p.n_max) : std::min((size_t)grid * gg_piece_bytes(p.n_max), gg_scratch_least(p.n_max, job.w0, job.problems));
     if (scratch == nullptr || counters == nullptr || scratch_bytes < least_bytes) {
         set_error("gemm: scratch of %zu bytes given, %zu needed", scratch_bytes, least_bytes);
         return HQM_ERR_SCRATCH;
     }
     grid = std::min<int64_t>(grid, (int64_t)(scratch_bytes / gg_piece_bytes(p.n_max)));
-#define HQM_GG(B, S, M) \
-    if (nbits == B && gs == S && job.mode == M) return gg_launch_one<B, S, M>(p, (int)grid, st);
-    HQM_GG(2, 16, GG_LINEAR) HQM_GG(2, 16, GG_UP) HQM_GG(2, 16, GG_DOWN)
-    HQM_GG(2, 32, GG_LINEAR) HQM_GG(2, 32, GG_DOWN)
-    HQM_GG(4, 32, GG_LINEAR) HQM_GG(4, 32, GG_DOWN)
-    HQM_GG(4, 64, GG_LINEAR) HQM_GG(4, 64, GG_DOWN)
+#define HQM_GG(B, M) \
+    if (nbits == B && job.mode == M) return gg_launch_one<B, M>(p, (int)grid, st);
+    HQM_GG(2, GG_LINEAR) HQM_GG(2, GG_UP) HQM_GG(2, GG_DOWN) HQM_GG(4, GG_LINEAR) HQM_GG(4, GG_DOWN)
 #undef HQM_GG
     set_error("gemm: no kernel for nbits=%d group_size=%d mode=%d", nbits, gs, (int)job.mode);
     return HQM_ERR_ARG;

@@ -79,12 +79,12 @@ struct GgJob {
 };
 
 bool gg_supported(const hqm_weight* w, int G, int C);
-GgLayout gg_linear_layout(int64_t M, const hqm_weight* w);
+GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count);      // layers of one K and format
 GgLayout gg_expert_layout(int64_t M);
 // Bytes of scratch (partial tiles) of a launch with up to n rows per chunk: with a CTA on every SM, and the least a launch
 // without `counts` works with (it then uses fewer CTAs).
 size_t gg_scratch_bytes(int n);
-size_t gg_scratch_least(int n, const hqm_weight* w);
+size_t gg_scratch_least(int n, const hqm_weight* const* ws, int count);
 int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st);
 
 // Stages rows of x (bf16 or fp16).  counts == null: one list of `rows` rows, else `lists` lists of together at most `rows`;

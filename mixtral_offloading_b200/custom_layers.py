@@ -238,6 +238,22 @@ class HQQLinearTritonSavable(nn.Module):
             self.repack()
 
 
+@torch.inference_mode()
+def linear_group(layers, x: torch.Tensor):
+    """[layer(x) for layer in layers]: one launch where the layers share their format and x has rows enough for it."""
+    x2 = _as_bf16_2d(x, x.shape[-1])
+    M, n, lib = x2.shape[0], len(layers), _cabi.lib()
+    ws = (C.c_void_p * n)(*(C.addressof(lyr.descriptor()) for lyr in layers))
+    need = lib.hqm_linear_group_scratch_bytes(M, ws, n)
+    if need == 0 or x2.dtype != x.dtype or any(lyr.bias is not None for lyr in layers):
+        return [lyr(x) for lyr in layers]
+    out = [torch.empty(x.shape[:-1] + (lyr.meta["shape"][0],), dtype=torch.bfloat16, device=x2.device) for lyr in layers]
+    ys = (C.c_void_p * n)(*(y.data_ptr() for y in out))
+    buf = _scratch(x2.device, need)
+    _cabi.check(lib.hqm_linear_group(ys, _cabi.ptr(x2), M, ws, None, n, _cabi.ptr(buf), buf.numel(), _cabi.stream_ptr(x2.device)))
+    return out
+
+
 class MixtralBLockSparseTop2MLP_HQQ(nn.Module):
     """custom_layers.py:243-256: w2(act(w1 x) * w3 x) — one fused call into the library."""
 

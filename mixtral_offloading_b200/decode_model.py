@@ -16,6 +16,7 @@ from typing import List, Optional, Sequence
 import torch
 from torch import nn
 
+from .custom_layers import linear_group
 from .decoder import DecoderLayerDecode, add_rmsnorm, rms_norm_rows, rope_append_rows
 from .sampling import sample_token
 
@@ -94,11 +95,12 @@ class MixtralDecodeModel(nn.Module):
         self.router_logits = []
         ln_in = self.first_ln                       # the norm weights step() applies: first_ln, then each layer's next_ln
         shared = self.layers[0].tokens_shared(T, pos0, h.device)
+        y = None
         for layer in self.layers:
-            h, logits = layer.forward_tokens(h, pos0, ln_in, shared)
+            h, y, logits = layer._tokens(h, y, pos0, ln_in, shared)
             self.router_logits.append(logits)
             ln_in = layer.next_ln
-        x = rms_norm_rows(h[-1:], self.layers[-1].next_ln, self.rms_eps)
+        x = rms_norm_rows(h[-1:], self.layers[-1].next_ln, self.rms_eps, y[-1:])
         logits = torch.matmul(x, self.lm_head.t())
         self.token.copy_(logits.argmax(-1))
         self.position.fill_(pos0 + T)
@@ -190,25 +192,20 @@ class BatchDecode:
         a, B, h = layer.attention, self.batch, self.h
         hidden = h.shape[-1]
         mask = self._mask
-        if self.y is not None:
-            h.add_(self.y)
         ln_in = self.model.first_ln if l == 0 else self.model.layers[l - 1].next_ln     # the weights step() applies
-        x = rms_norm_rows(h, ln_in, a.rms_eps)
-        q = a.q_proj(x)
-        rope_append_rows(q, a.k_proj(x), a.v_proj(x), self.k_caches[l], self.v_caches[l], a.n_heads, a.n_kv_heads,
+        q, k, v = linear_group((a.q_proj, a.k_proj, a.v_proj), rms_norm_rows(h, ln_in, a.rms_eps, self.y))
+        rope_append_rows(q, k, v, self.k_caches[l], self.v_caches[l], a.n_heads, a.n_kv_heads,
                          a.head_dim, a.rope_theta, self.position, 0)
         q = q.view(B, a.n_heads, a.head_dim)
         ctx = torch.nn.functional.scaled_dot_product_attention(q.unsqueeze(2), self.k_caches[l], self.v_caches[l],
                                                                attn_mask=mask, enable_gqa=True)   # (B, heads, 1, head_dim)
-        h.add_(a.o_proj(ctx.reshape(B, hidden)))
-        self._x_moe[l] = rms_norm_rows(h, a.ln_post, a.rms_eps)
+        self._x_moe[l] = rms_norm_rows(h, a.ln_post, a.rms_eps, a.o_proj(ctx.reshape(B, hidden)))
         if not self._on_device[l]:
             self._routes[l] = layer.moe._router.route(self._x_moe[l])
             self.y = self._y_host[l] = torch.zeros_like(h)
 
     def _head_segment(self):
-        self.h.add_(self.y)
-        x = rms_norm_rows(self.h, self.model.layers[-1].next_ln, self.model.rms_eps)
+        x = rms_norm_rows(self.h, self.model.layers[-1].next_ln, self.model.rms_eps, self.y)
         self._logits = torch.matmul(x, self.model.lm_head.t())
 
     def _moe_segment(self, l: int):

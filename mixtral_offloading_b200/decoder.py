@@ -11,12 +11,13 @@ CUDA graph can replay.
 from __future__ import annotations
 
 import ctypes as C
+from typing import Optional
 
 import torch
 from torch import nn
 
 from . import _cabi
-from .custom_layers import HQQLinearTritonSavable, ResidentMoe, _scratch
+from .custom_layers import HQQLinearTritonSavable, ResidentMoe, _scratch, linear_group
 
 
 def _bf16_vec(t: torch.Tensor, n: int) -> torch.Tensor:
@@ -36,16 +37,19 @@ def add_rmsnorm(h: torch.Tensor, delta, weight: torch.Tensor, eps: float = 1e-5)
     return x
 
 
-def rms_norm_rows(h: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+def rms_norm_rows(h: torch.Tensor, w: torch.Tensor, eps: float, delta: Optional[torch.Tensor] = None) -> torch.Tensor:
     """RMSNorm of every row of h (rows, hidden) bf16 as the decode kernels compute it: fp32 normalisation, one
-    rounding to bf16, times the bf16 weight (the Hugging Face form).  One launch (hqm_add_rmsnorm_rows)."""
+    rounding to bf16, times the bf16 weight (the Hugging Face form); h += delta first, in place, when delta is given.
+    One launch (hqm_add_rmsnorm_rows)."""
     rows, hidden = h.shape
     _cabi.require_cuda(h, w)
-    if h.dtype != torch.bfloat16 or not h.is_contiguous():
+    if delta is not None:
+        assert delta.shape == h.shape and all(t.dtype == torch.bfloat16 and t.is_contiguous() for t in (h, delta))
+    elif h.dtype != torch.bfloat16 or not h.is_contiguous():
         h = h.to(torch.bfloat16).contiguous()
     _bf16_vec(w, hidden)
     x = torch.empty_like(h)
-    _cabi.check(_cabi.lib().hqm_add_rmsnorm_rows(_cabi.ptr(h), None, _cabi.ptr(w), _cabi.ptr(x), rows, hidden, eps,
+    _cabi.check(_cabi.lib().hqm_add_rmsnorm_rows(_cabi.ptr(h), None if delta is None else _cabi.ptr(delta), _cabi.ptr(w), _cabi.ptr(x), rows, hidden, eps,
                                                  _cabi.stream_ptr(h.device)))
     return x
 
@@ -180,23 +184,28 @@ class DecoderLayerDecode(nn.Module):
         norm weight when it is not attention.ln_in (a model hands every layer the weight its predecessor was built
         with as next_ln, which is what the one-token path applies).  shared: what tokens_shared() returned for the
         same (T, pos0), when several layers process the same tokens (the mask is the same for all of them)."""
+        h, y, logits = self._tokens(h, None, pos0, ln_in, shared)
+        return h + y, logits
+
+    def _tokens(self, h, delta, pos0: int, ln_in, shared):
+        """forward_tokens with the residual adds left to the norms behind them: the stream is h + delta on entry (h is
+        written when delta is given) and h + y of the returned (h, y, router logits)."""
         a = self.attention
         ln_in = a.ln_in if ln_in is None else ln_in
         T, hidden = h.shape
         if pos0 < 0 or pos0 + T > a.max_len:
             raise ValueError(f"{T} tokens at position {pos0} do not fit a cache of {a.max_len}")
         mask = shared if shared is not None else self.tokens_shared(T, pos0, h.device)
-        x = rms_norm_rows(h, ln_in, a.rms_eps)
-        q = a.q_proj(x)
-        rope_append_rows(q, a.k_proj(x), a.v_proj(x), a.k_cache, a.v_cache, a.n_heads, a.n_kv_heads, a.head_dim,
+        q, k, v = linear_group((a.q_proj, a.k_proj, a.v_proj), rms_norm_rows(h, ln_in, a.rms_eps, delta))
+        rope_append_rows(q, k, v, a.k_cache, a.v_cache, a.n_heads, a.n_kv_heads, a.head_dim,
                          a.rope_theta, pos0, 1)
         q = q.view(T, a.n_heads, a.head_dim)
         keys, vals = a.k_cache[:, :pos0 + T].unsqueeze(0), a.v_cache[:, :pos0 + T].unsqueeze(0)
         ctx = torch.nn.functional.scaled_dot_product_attention(q.transpose(0, 1).unsqueeze(0), keys, vals, attn_mask=mask,
                                                                enable_gqa=True)          # (1, heads, T, head_dim)
-        h = h + a.o_proj(ctx[0].transpose(0, 1).reshape(T, hidden))
-        y, logits = self.moe(rms_norm_rows(h, a.ln_post, a.rms_eps).view(1, T, hidden))
-        return h + y.view(T, hidden), logits
+        out = a.o_proj(ctx[0].transpose(0, 1).reshape(T, hidden))
+        y, logits = self.moe(rms_norm_rows(out, a.ln_post, a.rms_eps, h).view(1, T, hidden))       # out += h
+        return out, y.view(T, hidden), logits
 
     @torch.inference_mode()
     def forward(self, h: torch.Tensor, x: torch.Tensor, pos: torch.Tensor):
