@@ -118,7 +118,7 @@ int hqm_scratch_init(void* scratch, void* stream);
 /* Bytes of scratch hqm_linear needs for M rows of this layer (0 if none). */
 size_t hqm_linear_scratch_bytes(int64_t M, const hqm_weight* w);
 
-/* The same for the fastest launch: with less, hqm_linear at five or more rows of a 2- or 4-bit layer spreads over fewer
+/* The same for the fastest launch: with less, hqm_linear at five or more rows spreads over fewer
  * SMs.  At least hqm_linear_scratch_bytes(). */
 size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w);
 
@@ -129,8 +129,13 @@ size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w);
  * bias may be NULL.  scratch may be NULL when hqm_linear_scratch_bytes() is 0.
  * Rows 1..4 take the weight-streaming kernels, 5 and more the tcgen05 kernels; HQM_FORCE_GENERIC=1 in the environment
  * at load time routes everything through the shape-agnostic kernel. */
+/* hqm_linear for fp16 x and y (five or more rows; the scratch size is 0 where only hqm_linear takes the layer). */
+size_t hqm_linear_f16_scratch_bytes(int64_t M, const hqm_weight* w);
+int hqm_linear_f16(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias, void* scratch,
+                   size_t scratch_bytes, void* stream);
+
 /* Up to four layers of one K, bit width and group size over the same rows (q, k and v of a decoder layer) in one launch:
- * y[i] = x . W_est[i]^T (+ bias[i]); bias may be NULL.  Five or more rows of 2- or 4-bit layers; the scratch size is 0 for
+ * y[i] = x . W_est[i]^T (+ bias[i]); bias may be NULL.  Five or more rows; the scratch size is 0 for
  * everything else. */
 size_t hqm_linear_group_scratch_bytes(int64_t M, const hqm_weight* const* w, int32_t count);
 int hqm_linear_group(uint16_t* const* y, const uint16_t* x, int64_t M, const hqm_weight* const* w, const uint16_t* const* bias,

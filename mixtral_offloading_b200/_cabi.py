@@ -79,6 +79,8 @@ SIGNATURES = {
     "hqm_linear_scratch_preferred": (C.c_size_t, [_I64, _WP]),
     "hqm_linear": (C.c_int, [_P, _P, _I64, _WP, _P, _P, C.c_size_t, _P]),
     "hqm_static_scratch_capacity": (C.c_size_t, []),
+    "hqm_linear_f16_scratch_bytes": (C.c_size_t, [_I64, _WP]),
+    "hqm_linear_f16": (C.c_int, [_P, _P, _I64, _WP, _P, _P, C.c_size_t, _P]),
     "hqm_linear_group_scratch_bytes": (C.c_size_t, [_I64, _P, _I32]),
     "hqm_linear_group": (C.c_int, [_P, _P, _I64, _P, _P, _I32, _P, C.c_size_t, _P]),
     "hqm_linear_static_scratch": (C.c_int, [_P, _P, _I64, _WP, _P, _P]),

@@ -72,9 +72,10 @@ int set_overlap(int on) {
     return prev;
 }
 
-// Rows from which a 2- or 4-bit layer goes to the tensor-core kernel (gemm_grouped.cu); below, the streaming kernels,
+// Rows from which a layer goes to the tensor-core kernel (gemm_grouped.cu); below, the streaming kernels,
 // whose work per weight grows with the rows, are faster.
-static bool use_gg(const hqm_weight* w, int G, int C, int64_t M) { return M >= GG_MIN_ROWS && M <= (1 << 22) && gg_supported(w, G, C); }
+// (3 bit: from two on, as the streaming kernel takes one row per launch: 14336 x 4096 21 us each, here 29 up to 16 rows.)
+static bool use_gg(const hqm_weight* w, int G, int C, int64_t M) { return M >= (w->nbits == 3 ? 2 : GG_MIN_ROWS) && M <= (1 << 22) && gg_supported(w, G, C); }
 
 size_t linear_scratch_bytes(int64_t M, const hqm_weight* w, bool preferred) {
     int G, C;
@@ -104,7 +105,8 @@ static int need_scratch(void* scratch, size_t have, size_t need) {
 
 // Layers of one K and format over the same rows: the rows staged once, one launch over all tiles.
 static int linear_gg(uint16_t* const* y, const hqm_weight* const* ws, const uint16_t* const* bias, int count, const uint16_t* x,
-                     const int32_t* x_idx, int64_t M, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st) {
+                     const int32_t* x_idx, int64_t M, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st,
+                     int f16 = 0) {
     const GgLayout layout = gg_linear_layout(M, ws, count);
     const int K = ws[0]->K;
     const int64_t xt_rows = layout.rows.padded();
@@ -112,7 +114,7 @@ static int linear_gg(uint16_t* const* y, const hqm_weight* const* ws, const uint
     int rc = need_scratch(scratch, scratch_bytes, staged + gg_scratch_least(layout.rows.n, ws, count));
     if (rc != HQM_OK) return rc;
     const GgStaged xs = gg_staged(scratch, xt_rows, K, true);
-    rc = launch_gg_stage(xs, x, 0, x_idx, nullptr, 1, M, K, st);
+    rc = launch_gg_stage(xs, x, f16, x_idx, nullptr, 1, M, K, ws[0]->nbits, st);
     if (rc != HQM_OK) return rc;
     GgJob job{};
     job.problems = count;
@@ -120,6 +122,7 @@ static int linear_gg(uint16_t* const* y, const hqm_weight* const* ws, const uint
     job.layout = layout;
     job.x = xs;
     job.mode = GG_LINEAR;
+    job.y_f16 = f16;
     for (int i = 0; i < count; ++i) {
         job.w0[i] = ws[i];
         job.y[i] = y[i];
@@ -194,6 +197,23 @@ size_t hqm_linear_scratch_bytes(int64_t M, const hqm_weight* w) {
 size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w) {
     const size_t inner = hqm::linear_scratch_bytes(M, w, /*preferred=*/true);
     return inner ? inner + hqm::SCRATCH_HEADER : 0;
+}
+
+size_t hqm_linear_f16_scratch_bytes(int64_t M, const hqm_weight* w) { return hqm_linear_group_scratch_bytes(M, &w, 1); }
+
+int hqm_linear_f16(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias, void* scratch,
+                   size_t scratch_bytes, void* stream) {
+    using namespace hqm;
+    const size_t need = hqm_linear_f16_scratch_bytes(M, w);
+    HQM_CHECK_ARG(need != 0, "linear_f16: five or more rows of a layer that the tensor-core kernel takes are needed");
+    HQM_CHECK_ARG(y && x && (reinterpret_cast<uintptr_t>(x) & 15u) == 0, "linear_f16: null or unaligned activation pointer");
+    if (scratch == nullptr || scratch_bytes < need) {
+        set_error("linear_f16: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
+        return HQM_ERR_SCRATCH;
+    }
+    HQM_CHECK_ARG((reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "linear_f16: scratch must be 256-byte aligned");
+    return linear_gg(&y, &w, &bias, 1, x, nullptr, M, (uint32_t*)scratch, (uint8_t*)scratch + SCRATCH_HEADER,
+                     scratch_bytes - SCRATCH_HEADER, (cudaStream_t)stream, 1);
 }
 
 size_t hqm_linear_group_scratch_bytes(int64_t M, const hqm_weight* const* w, int32_t count) {

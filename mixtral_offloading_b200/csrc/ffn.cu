@@ -132,7 +132,7 @@ int hqm_expert_ffn(uint16_t* out, const uint16_t* x, int64_t M, const int32_t* t
         // 3 launches: x staged -> h = silu(w1 x) * w3 x, staged -> w2 h, weighted, into out
         uint8_t *xt = p, *ht = p + gp.x_bytes, *parts = ht + gp.h_bytes;
         const GgStaged xs = gg_staged(xt, gp.xt_rows, w1->K, true), hs = gg_staged(ht, gp.xt_rows, w1->N, false);
-        int rc = launch_gg_stage(xs, x, 0, token_idx, nullptr, 1, M, w1->K, st);
+        int rc = launch_gg_stage(xs, x, 0, token_idx, nullptr, 1, M, w1->K, w1->nbits, st);
         if (rc != HQM_OK) return rc;
         GgJob up{}, down{};
         up.problems = down.problems = 1;
@@ -279,7 +279,7 @@ int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, c
     rc = launch_router_lists(counts, offsets, token_idx, token_w, entry_of, topk_w, topk_idx, T, E, st);
     if (rc != HQM_OK) return rc;
     const GgStaged xs = gg_staged(xt, mp.gg.xt_rows, w1->K, true), hs = gg_staged(ht, mp.gg.xt_rows, w1->N, false);
-    rc = launch_gg_stage(xs, x, 0, token_idx, counts, E, 2 * T, w1->K, st);
+    rc = launch_gg_stage(xs, x, 0, token_idx, counts, E, 2 * T, w1->K, w1->nbits, st);
     if (rc != HQM_OK) return rc;
     GgJob up{}, down{};
     up.problems = down.problems = E;

@@ -46,6 +46,12 @@
 // and zeros, the weights' arithmetic and the MMAs the same pipeline runs at ~430.  At 256 rows it is the staged x that
 // bounds it (64 KB per unit into every SM).
 //
+// 3-bit layers (ten codes of one column in 32 bits; 10 does not divide the number of groups): storage rows rho + i * P3 hold
+// the same residues in the same slots, so a tile is again 8 neighbouring residues x 16 members, from one or two rho.  The
+// two bytes that hold a thread's field are picked out of two columns' words by one PRMT and multiplied up to bit 4; the rest
+// is as above.  14336 x 4096, 100 rows: 112 us before (decoded tables of scales in memory, dequantisation bound by the
+// latency of loads that nothing ran ahead of, A in shared memory), 41 now.
+//
 // Every wait is bounded; a wait that runs out sets the error flag, all roles leave, TMEM is freed.
 #include <cuda.h>
 #include <type_traits>
@@ -92,16 +98,17 @@ struct Problem {
     int row0, list0;                       // first row in the staged x, first entry in the row list
     int tiles, G, P, C;
     int N, blocks;                         // output rows; blocks of 16 members
+    int R, full, left;                     // 3 bit: residues (G is then the rows from member to member); Members3
     int f16;
 };
 
 // How a list's rows share the ring of staged x: a stage holds 256 columns of all rows of a chunk (128 beyond 64 rows, 64
-// beyond 128), as a wait, an expectation and a copy together cost the copying warp about 340 cycles.
+// beyond 128 or in a small ring), as a wait, an expectation and a copy together cost the copying warp about 340 cycles.
 struct BClass {
     int bytes, stages, blocks;             // bytes reserved per stage, stages in the ring, 64-column blocks in a stage
     __device__ __forceinline__ static BClass of(int n, int ring) {
         BClass c;
-        c.blocks = n > 128 ? 1 : (n > 64 ? 2 : 4);
+        c.blocks = n > 128 || (n > 64 && ring < 128 * 1024) ? 1 : (n > 64 ? 2 : 4);
         const int rows = n <= 16 ? 16 : (n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : 256)));
         c.bytes = rows * 128 * c.blocks;
         c.stages = min(MAX_B_STAGES, ring / c.bytes);
@@ -121,7 +128,7 @@ struct TmemMap {
 struct HostProblem {
     CUtensorMap maps[2][3];
     const uint16_t* meta[2][4];
-    int G, P, C, tiles, N, blocks;
+    int G, P, C, tiles, N, blocks, R, full, left;
     void* y;
     const uint16_t* bias;
 };
@@ -170,7 +177,9 @@ struct Shared {
 template <int NBITS_>
 struct Fmt {
     static constexpr int NBITS = NBITS_, MEMBERS = 16;
-    static constexpr int PER = codes_per_word(NBITS);
+    static constexpr bool WORDS = NBITS == 3;              // ten codes of one column in 32 bits
+    // Residues in a byte.  (3 bit: 8 neighbouring ones as two parts of four; they lie in one or two storage rows.)
+    static constexpr int PER = WORDS ? 4 : codes_per_word(NBITS);
     static constexpr int PARTS = 8 / PER;                  // storage-row residues of a tile
     // Columns of a unit.  What a warp does once per unit (waits, decoding, hand-over) takes about as long as the weights of
     // 128 columns of a 2-bit tile, and those layers are large; 4-bit layers decode little and may be small.
@@ -178,7 +187,7 @@ struct Fmt {
     static constexpr int HALVES = UK / 128;                // A slots of a unit
     static constexpr int BLOCKS = UK / 64;
     static constexpr int SLW = 2;                          // rows of scales a warp needs: its slot of two parts
-    static constexpr int CODE_PART = MEMBERS * 128;             // packed bytes of a part of 128 columns
+    static constexpr int CODE_PART = MEMBERS * 128 * (WORDS ? 4 : 1);             // packed bytes of a part of 128 columns
     static constexpr int CODE_HALF = PARTS * CODE_PART;
     static constexpr int SZ_PART = PER * 128;
     static constexpr int SQ_OFF = HALVES * CODE_HALF, ZQ_OFF = SQ_OFF + HALVES * PARTS * SZ_PART;
@@ -188,8 +197,9 @@ struct Fmt {
     static constexpr int ST_WARP = SLW * UK * 4;           // s and t of a warp's rows
     static constexpr int ST_BLOCK = 2 * SLW * 64, ST_T = BLOCKS * ST_BLOCK;
     // Launches of up to 64 rows per chunk need few staged rows in flight and many packed bytes, others the reverse.
-    __host__ __device__ static constexpr int b_ring(int n_max) { return n_max <= 64 ? 64 * 1024 : 128 * 1024; }
-    __host__ __device__ static constexpr int n_raw(int n_max) { return PARTS == 4 && n_max > 64 ? 6 : 8; }
+    __host__ __device__ static constexpr int b_ring(int n_max) { return WORDS ? 80 * 1024 : (n_max <= 64 ? 64 * 1024 : 128 * 1024); }
+    // (Even: a slot is filled by one of the two copying warps then, and its phases are waited for in order.)
+    __host__ __device__ static constexpr int n_raw(int n_max) { return WORDS ? 6 : (PARTS == 4 && n_max > 64 ? 6 : 8); }
     static constexpr int ST_OFF = 0, EPI_OFF = ST_OFF + 4 * GROUPS * ST_WARP, BAR_OFF = EPI_OFF + EPI_BYTES, RING_OFF = BAR_OFF + 1024;
     __host__ __device__ static constexpr int smem(int n_max) {
         return (RING_OFF + 1023) / 1024 * 1024 + b_ring(n_max) + n_raw(n_max) * RAW_BYTES + 1024;
@@ -197,11 +207,12 @@ struct Fmt {
     static_assert(smem(64) + (int)sizeof(Shared) <= 227 * 1024 && smem(256) + (int)sizeof(Shared) <= 227 * 1024, "shared memory");
     // Which row of the tile TMEM lane 32 q + 8 j + g holds (q: warp of a group, j = 0..3): part, slot of the byte, member.
     // A thread of the 16x256b store shape holds j = 0..3 at one g: four members of one quantisation group.
-    __device__ __forceinline__ static int part_of(int q, int g) { return (NBITS == 2 ? 0 : 2 * (q >> 1)) + (g & 1); }
-    __device__ __forceinline__ static int slot_of(int q) { return NBITS == 2 ? q : q & 1; }
+    __device__ __forceinline__ static int part_of(int q, int g) { return (NBITS == 4 ? 2 * (q >> 1) : 0) + (g & 1); }
+    __device__ __forceinline__ static int slot_of(int q) { return NBITS == 4 ? q & 1 : q; }
     __device__ __forceinline__ static int member_of(int g, int j) { return (g >> 1) + 4 * j; }
 };
-// Position of column k of a 64-column block in the staged order (and in the A tile).
+// Position of column k of a 64-column block in the staged order (and in the A tile).  (3 bit: a thread column takes words
+// 16 i + 4 c .. + 3 instead, so that four neighbouring lanes read 64 contiguous bytes: bits 2-3 and 4-5 of k change places.)
 __host__ __device__ constexpr int tile_pos(int k) {
     const int c = k >> 4, i = (k >> 2) & 3, e = k & 3;                  // thread column, word, byte
     return 16 * i + 4 * c + ((e & 1) << 1 | (e >> 1));                  // bytes in the order 0, 2, 1, 3
@@ -375,6 +386,29 @@ __device__ __forceinline__ uint32_t bf2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// 16 rows x 32 columns of A from a warp's registers.
+__device__ __forceinline__ void store_a(uint32_t at, const uint32_t (&o)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(at), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]),
+        "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15])
+        : "memory");
+}
+// The field of slot s (0..9, bits 27 .. 0) of a 3-bit word.
+struct Field3 {
+    uint32_t sel, up, mask;                // PRMT selector for two words, factor, mask
+    int fpos;                              // first bit of the field, less 4
+    __device__ __forceinline__ static Field3 of(int s) {
+        const uint32_t bit = 3u * (9u - (uint32_t)s), b0 = bit >> 3, b1 = min(b0 + 1, 3u), p = bit & 7;
+        Field3 f;
+        f.sel = b0 | (b1 << 4) | ((4 + b0) << 8) | ((4 + b1) << 12);
+        f.up = p < 4 ? 16u : 1u;
+        f.fpos = (int)(p < 4 ? p : p - 4);
+        f.mask = (7u << (4 + f.fpos)) * 0x00010001u;
+        return f;
+    }
+};
+
 // A run of this CTA's units inside one tile.
 struct Seg {
     int p, tile, chunk, k0, k1;            // problem, tile, row chunk, 128-column units [k0, k1)
@@ -467,6 +501,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             p.tiles = h.tiles;
             p.N = h.N;
             p.blocks = h.blocks;
+            p.R = h.R;
+            p.full = h.full;
+            p.left = h.left;
             p.cnt = cnt;
             const GgRows r = counted ? GgRows::of(cnt) : GgRows{prm.chunks, prm.n_max};
             p.n = r.n;
@@ -532,7 +569,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
         // The field of the warp's slot inside a byte.  2 bit: slots 0, 1 at bits 7-6, 5-4, slots 2, 3 at 3-2, 1-0; 4 bit: 7-4 or
         // 3-0.  `upper`: it lies in the upper half of the byte; fpos: its first bit inside that half.
         const bool upper = (NBITS == 2) ? q < 2 : (q & 1) == 0;
-        const int fpos = (NBITS == 2) ? ((q & 1) ? 0 : 2) : 0;
+        const int fpos = (NBITS == 2) ? ((q & 1) ? 0 : 2) : 0;              // (3 bit: set for every tile)
         const uint32_t field = (NBITS == 2) ? 3u : 15u;
         const uint32_t mask_hi = (field << (4 + fpos)) * 0x00010001u;      // field in bits 7-4 of each half
         const uint32_t mask_lo = (field << fpos) * 0x00010001u;            // field in bits 3-0 of each half
@@ -600,7 +637,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             const bool f16 = pr.f16 != 0;
             const int wsel = (MODE == GG_UP) ? dpart : 0;
             const int rho = (MODE == GG_UP) ? s.tile : s.tile / pr.blocks * PARTS + dpart;
-            const int res = min(PER * rho + slot, pr.G - 1);  // (a tile's second part may lie past the last residue)
+            // 3 bit: the words of this thread's residue and, in them, its field: two bytes that hold it at bit 0 .. 7, moved up to
+            // bit 4 + fpos; the same of the residue whose scales this lane decodes
+            Field3 mine{}, decoded{};
+            uint32_t words3 = 0;
+            if constexpr (F::WORDS) {
+                const int q0 = s.tile / pr.blocks * 8, r0 = q0 / 10, e = q0 + PER * part + slot;
+                mine = Field3::of(e % 10);
+                decoded = Field3::of((PER * rho + slot) % 10);
+                words3 = (uint32_t)((e / 10 - r0) * F::CODE_PART + (g >> 1) * 512 + c * 16);
+            }
+            const int res = F::WORDS ? (PER * rho + slot) % pr.R : min(PER * rho + slot, pr.G - 1);  // (a tile's last parts may lie past the last residue)
             mC = pr.C;
 #pragma unroll
             for (int a = 0; a < 4; ++a) mp[a] = pr.w[wsel].meta[a];
@@ -613,6 +660,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 const uint32_t rw = raw_ring + r * F::RAW_BYTES;
                 uint4 wv[4];
                 auto load_codes = [&](int sub) {
+                    if constexpr (F::WORDS) return;
                     const uint32_t at0 = rw + (sub >> 1) * F::CODE_HALF;
                     const uint32_t c0 = at0 + (code_off[0] ^ (64u * (sub & 1))), c1 = at0 + (code_off[1] ^ (64u * (sub & 1)));
                     wv[0] = lds128(c0);
@@ -665,7 +713,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                         big = __any_sync(0xffffffffu, (mx & 0xffffu) > 0x33FFu || (mx >> 16) > 0x33FFu);           // 1/4 and more
                         // * 2^(18 - fpos), exact; big: the field will be read as c * 2^(4 + fpos), so s / 4 / 2^(4 + fpos)
                         const uint32_t f1 = big ? 0x3C003C00u : 0x64006400u;
-                        const uint32_t f2 = big ? (fpos ? 0x1C001C00u : 0x24002400u) : (fpos ? 0x54005400u : 0x5C005C00u);
+                        const uint32_t f2 = (big ? 0x24002400u : 0x5C005C00u) - (uint32_t)(F::WORDS ? decoded.fpos : fpos) * 0x04000400u;
 #pragma unroll
                         for (int j = 0; j < DC / 2; ++j) S[j] = h2mul(h2mul(S[j], f1), f2);
                     } else {
@@ -689,6 +737,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                         }
                     }
                     // publish to the warp
+                    if constexpr (F::WORDS) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int w64 = (dcol + 4 * h) & 63, blk = (dcol + 4 * h) >> 6, i = w64 >> 4;
+                            const uint32_t dst = st_area + blk * F::ST_BLOCK + (i >> 1) * (SLW * 64) + dlocal * 64 + ((w64 >> 2) & 3) * 16 + (i & 1) * 8;
+                            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst), "r"(S[2 * h]), "r"(S[2 * h + 1]) : "memory");
+                            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst + F::ST_T), "r"(T[2 * h]), "r"(T[2 * h + 1]) : "memory");
+                        }
+                    } else
 #pragma unroll
                     for (int h = 0; h < (DC + 7) / 8; ++h) {
                         const int w64 = (dcol + 8 * h) & 63, blk = (dcol + 8 * h) >> 6;
@@ -731,6 +788,28 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                             if (sub) load_codes(sub);
                             const uint32_t SS[8] = {S0.x, S0.y, S0.z, S0.w, S1.x, S1.y, S1.z, S1.w};
                             const uint32_t TT[8] = {T0.x, T0.y, T0.z, T0.w, T1.x, T1.y, T1.z, T1.w};
+                            if constexpr (F::WORDS) {
+                                const uint32_t at0 = rw + words3 + 256u * sub;
+                                auto all3 = [&](auto&& weight) {
+#pragma unroll
+                                    for (int h = 0; h < 2; ++h) {
+                                        uint32_t o[16];
+#pragma unroll
+                                        for (int b = 0; b < 2; ++b)
+#pragma unroll
+                                            for (int i = 0; i < 4; ++i) {
+                                                const uint4 v = lds128(at0 + (2 * h + b) * 2048 + 64 * i);
+                                                o[4 * i + 2 * b] = weight(perm(v.x, v.z, mine.sel) * mine.up, SS[2 * i], TT[2 * i]);
+                                                o[4 * i + 2 * b + 1] = weight(perm(v.y, v.w, mine.sel) * mine.up, SS[2 * i + 1], TT[2 * i + 1]);
+                                            }
+                                        store_a(ta + 32 * sub2 + ((uint32_t)(16 * h) << 16), o);
+                                    }
+                                };
+                                const uint32_t magic = 0x64006400u;                                                     // 1024
+                                if (!big) all3([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(x & mine.mask, S, T); });
+                                else all3([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x, mine.mask, magic), magic), S, T); });
+                                continue;
+                            }
                             // one pair of weights per (member, word i, e): fields of bytes (0, 2) and (1, 3) of the word
                             auto all = [&](auto&& pair_lo, auto&& pair_hi) {
 #pragma unroll
@@ -746,12 +825,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                                             o[4 * i + 2 * b + 1] = pair_hi(w[i], SS[2 * i + 1], TT[2 * i + 1]);
                                         }
                                     }
-                                    asm volatile(
-                                        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                                        ::"r"(ta + 32 * sub2 + ((uint32_t)(16 * h) << 16)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]),
-                                        "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]),
-                                        "r"(o[14]), "r"(o[15])
-                                        : "memory");
+                                    store_a(ta + 32 * sub2 + ((uint32_t)(16 * h) << 16), o);
                                 }
                             };
                             // (the shift to the left is written as a product: it then runs beside the ANDs, on the other pipe)
@@ -822,9 +896,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(maps[i / 3] + i % 3) : "memory");
                 }
                 for (int k = s.k0 + ((s.u0 ^ turn) & 1); k < s.k1; k += 2) {
-                    const int u = s.u0 + (k - s.k0), lap = n_raw == 8 ? u >> 3 : u / 6, r = u - lap * n_raw;
+                    const int u = s.u0 + (k - s.k0), lap = u / n_raw, r = u - lap * n_raw;
                     wait_limited(raw_empty + 8 * r, (lap & 1) ^ 1, limit);
                     const uint32_t bar = raw_full + 8 * r, dst = raw_ring + r * F::RAW_BYTES;
+                    if constexpr (F::WORDS) {
+                        const int r0 = 8 * quad / 10, two = 8 * quad - 10 * r0 > 2 ? 2 : 1;           // storage rows of a member
+                        if (leader) {
+                            expect_tx(bar, (uint32_t)(two * 512 * (min(pr.full, 16) + (pr.left ? 1 : 0)) + 2 * 1024));
+                            for (int p = 0; p < two; ++p) {
+                                tma_3d(dst + p * F::CODE_PART, maps[0], k * UK, r0 + p, m0, bar);
+                                if (pr.left) tma_3d(dst + p * F::CODE_PART + pr.full * 512, maps[0] + 3, k * UK, r0 + p, 0, bar);
+                            }
+                            tma_3d(dst + F::SQ_OFF, maps[0] + 1, k * UK, 8 * quad % pr.R, 0, bar);
+                            tma_3d(dst + F::ZQ_OFF, maps[0] + 2, k * UK, 8 * quad % pr.R, 0, bar);
+                        }
+                        continue;
+                    }
                     if (leader) {
                         expect_tx(bar, F::RAW_TX);
 #pragma unroll
@@ -917,7 +1004,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                     }
                     ready = peek(a_bar, a_par);               // of the next unit, while this one's MMAs are issued
                     const bool two = 2 * k + 1 < prm.subs_k;  // (K may be an odd number of blocks)
-                    if (!wide) {
+                    if (bc.blocks > 1) {
                         if (left == 0) {
                             wait_limited(b_full + 8 * st, (par >> st) & 1, limit);
                             par ^= 1u << st;
@@ -995,7 +1082,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             float bias = 0.f;
             if (MODE == GG_LINEAR) {
                 const uint16_t* bp = prm.hp[s.p].bias;
-                if (bp && rho < pr.P) bias = bf16_bits_to_float(bp[(m0 + member) * pr.G + PER * rho + slot]);
+                if (bp && rho < pr.P && (!F::WORDS || (m0 + member) * pr.G + PER * rho + slot < pr.N)) bias = bf16_bits_to_float(bp[(m0 + member) * pr.G + PER * rho + slot]);
             }
             if (!wait(acc_full + 8 * (seg & 1), (seg >> 1) & 1)) ok = false;
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
@@ -1147,7 +1234,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
 #pragma unroll 2
                         for (int j = et; j < 16 * MEMBERS; j += 128) {
                             const int t = j / MEMBERS, m = j % MEMBERS;
-                            if (c0 + t >= rows_here) continue;
+                            if (c0 + t >= rows_here || (F::WORDS && (m0 + m) * pr.G + PER * rho0 >= pr.N)) continue;
                             const uint16_t* src = tb + t * 128 + m * RUN;
                             const int64_t row = MODE == GG_DOWN ? s_row[c0 + t] : list + c0 + t;
                             uint16_t* dst = out + row * ld + (int64_t)(m0 + m) * pr.G + PER * rho0;
@@ -1192,7 +1279,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
 template <bool X_F16>
 __global__ void __launch_bounds__(256) gg_stage_kernel(unsigned char* __restrict__ xt, float* __restrict__ row_scale, int64_t xt_rows,
                                                        const uint16_t* __restrict__ x, const int32_t* __restrict__ idx,
-                                                       const int32_t* __restrict__ counts, int lists, int K) {
+                                                       const int32_t* __restrict__ counts, int lists, int K, bool words) {
     __shared__ float s_max[8];
     grid_launch_dependents();
     grid_dependency_wait();
@@ -1244,8 +1331,8 @@ __global__ void __launch_bounds__(256) gg_stage_kernel(unsigned char* __restrict
     for (int i = threadIdx.x; i < K / 8; i += 256) {
         const int b = i >> 3, ch = i & 7;
         // piece ch of the staged block: words (thread column 2 (ch & 1), word ch >> 1) and the next thread column
-        const int k0 = b * 64 + 32 * (ch & 1) + 4 * (ch >> 1);
-        const uint2 a = *reinterpret_cast<const uint2*>(src + k0), d = *reinterpret_cast<const uint2*>(src + k0 + 16);
+        const int k0 = b * 64 + (words ? 8 * (ch & 1) + 16 * (ch >> 1) : 32 * (ch & 1) + 4 * (ch >> 1));
+        const uint2 a = *reinterpret_cast<const uint2*>(src + k0), d = *reinterpret_cast<const uint2*>(src + k0 + (words ? 4 : 16));
         const uint32_t o[4] = {perm(a.x, a.y, 0x5410u), perm(a.x, a.y, 0x7632u), perm(d.x, d.y, 0x5410u), perm(d.x, d.y, 0x7632u)};
         uint32_t h[4];
 #pragma unroll
@@ -1277,8 +1364,12 @@ static int gg_sm_count() {
 
 static constexpr int UK_MIN = 128;
 bool gg_supported(const hqm_weight* w, int G, int C) {
-    if ((w->nbits != 2 && w->nbits != 4) || !meta_uniform(w) || tma_encode_entry() == nullptr) return false;
-    const int per = codes_per_word(w->nbits), g = w->group_size;
+    if (!meta_uniform(w) || tma_encode_entry() == nullptr) return false;
+    const int per = w->nbits == 3 ? 8 : codes_per_word(w->nbits), g = w->group_size;
+    if (w->nbits == 3) {                     // members in whole blocks of 16, or all of them (and the last rows) in one
+        const Members3 m = Members3::of(w, G);
+        if (m.full < 1 || m.full + (m.left ? 1 : 0) > 16 ? m.full < 1 || m.left != 0 || m.full % 16 != 0 : false) return false;
+    }
     if (g % 16 != 0 || G % per != 0 || w->K % 64 != 0 || w->K < UK_MIN || C < 1) return false;
     if ((int64_t)G * w->K >= ((int64_t)1 << 31)) return false;
     auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
@@ -1293,6 +1384,10 @@ static int gg_n_max(int64_t rows) {
 static size_t gg_piece_bytes(int n) { return (size_t)2 * n * 128 * sizeof(float); }      // of one CTA
 size_t gg_scratch_bytes(int n) { return (size_t)gg_sm_count() * gg_piece_bytes(n); }
 static int64_t gg_tiles(const hqm_weight* w) {
+    if (w->nbits == 3) {
+        const Members3 m = Members3::of(w, w->N / w->group_size);
+        return (int64_t)m.P3 * 10 / 8 * ((m.full + 15) / 16);
+    }
     return (w->N / w->group_size + 7) / 8 * (w->group_size / 16);
 }
 // (a layer with a tile for every SM is not worth running on a third of them)
@@ -1318,7 +1413,8 @@ GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count) {
     GgLayout best{};
     int64_t best_cost = INT64_MAX;
     int chunks = 0;
-    for (int cap = 16; cap <= GG_MAX_ROWS; cap += 16) {
+    const int most = ws[0]->nbits == 3 ? 128 : GG_MAX_ROWS;       // (the small ring of a 3-bit launch)
+    for (int cap = 16; cap <= most; cap += 16) {
         const GgRows r = GgRows::of((int)M, cap);
         if (r.chunks == chunks) continue;    // the same cut
         chunks = r.chunks;
@@ -1341,9 +1437,9 @@ GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count) {
 }
 
 int launch_gg_stage(const GgStaged& to, const void* x, int x_f16, const int32_t* idx, const int32_t* counts, int lists, int64_t rows,
-                    int K, cudaStream_t st) {
+                    int K, int nbits, cudaStream_t st) {
     auto kern = x_f16 ? gg::gg_stage_kernel<true> : gg::gg_stage_kernel<false>;
-    launch_overlapped(kern, (int)rows, 256, 0, st, (unsigned char*)to.data, to.scale, to.rows, (const uint16_t*)x, idx, counts, lists, K);
+    launch_overlapped(kern, (int)rows, 256, 0, st, (unsigned char*)to.data, to.scale, to.rows, (const uint16_t*)x, idx, counts, lists, K, nbits == 3);
     HQM_LAUNCH_CHECK();
     return HQM_OK;
 }
@@ -1367,7 +1463,7 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
     gg::Params p{};
     const int host_problems = job.table ? 1 : job.problems;
     const hqm_weight* first = job.table ? job.shape : job.w0[0];
-    const int nbits = first->nbits, gs = first->group_size, per = codes_per_word(nbits);
+    const int nbits = first->nbits, gs = first->group_size, per = nbits == 3 ? 4 : codes_per_word(nbits);
     const int parts = 8 / per;
     HQM_CHECK_ARG(job.problems >= 1 && job.problems <= GG_MAX_PROBLEMS && host_problems <= 4, "gemm: %d problems in a launch", job.problems);
     HQM_CHECK_ARG(job.mode != GG_UP || (parts == 2 && gs == 16), "gemm: the fused gate needs 2-bit layers with groups of 16");
@@ -1385,12 +1481,26 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
             h.N = w->N;
             h.blocks = gs / 16;
             h.tiles = job.mode == GG_UP ? h.P : (h.P + parts - 1) / parts * h.blocks;
+            if (nbits == 3) {
+                const Members3 m = Members3::of(w, G);
+                h.R = G;
+                h.G = 10 * m.P3;
+                h.P = h.G / per;
+                h.full = m.full;
+                h.left = m.left;
+                h.blocks = (m.full + 15) / 16;
+                h.tiles = h.G / 8 * h.blocks;
+                if (l == 0 && !stream_cached_maps3(w, G, m, h.maps[0])) {
+                    set_error("gemm: cuTensorMapEncodeTiled failed for a %dx%d 3-bit layer", w->N, w->K);
+                    return HQM_ERR_CUDA;
+                }
+            }
             if (!job.table) {
                 h.meta[l][0] = w->ms_scale;
                 h.meta[l][1] = w->mz_scale;
                 h.meta[l][2] = w->ms_zero;
                 h.meta[l][3] = w->mz_zero;
-                if ((l == 0 || job.mode == GG_UP) && !stream_cached_maps(w, G, h.maps[l])) {
+                if (nbits != 3 && (l == 0 || job.mode == GG_UP) && !stream_cached_maps(w, G, h.maps[l])) {
                     set_error("gemm: cuTensorMapEncodeTiled failed for a %dx%d %d-bit layer", w->N, w->K, w->nbits);
                     return HQM_ERR_CUDA;
                 }
@@ -1437,6 +1547,7 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
 #define HQM_GG(B, M) \
     if (nbits == B && job.mode == M) return gg_launch_one<B, M>(p, (int)grid, st);
     HQM_GG(2, GG_LINEAR) HQM_GG(2, GG_UP) HQM_GG(2, GG_DOWN) HQM_GG(4, GG_LINEAR) HQM_GG(4, GG_DOWN)
+    HQM_GG(3, GG_LINEAR)
 #undef HQM_GG
     set_error("gemm: no kernel for nbits=%d group_size=%d mode=%d", nbits, gs, (int)job.mode);
     return HQM_ERR_ARG;

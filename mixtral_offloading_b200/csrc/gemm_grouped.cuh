@@ -87,9 +87,9 @@ size_t gg_scratch_bytes(int n);
 size_t gg_scratch_least(int n, const hqm_weight* const* ws, int count);
 int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st);
 
-// Stages rows of x (bf16 or fp16).  counts == null: one list of `rows` rows, else `lists` lists of together at most `rows`;
+// Stages rows of x (bf16 or fp16) for layers of `nbits`.  counts == null: one list of `rows` rows, else `lists` lists of together at most `rows`;
 // idx: row of x of list entry i (null: i).
 int launch_gg_stage(const GgStaged& to, const void* x, int x_f16, const int32_t* idx, const int32_t* counts, int lists, int64_t rows,
-                    int K, cudaStream_t st);
+                    int K, int nbits, cudaStream_t st);
 
 }  // namespace hqm

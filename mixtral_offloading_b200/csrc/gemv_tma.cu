@@ -672,25 +672,29 @@ struct MapKeyHash {
         return h;
     }
 };
-struct MapTriple {
-    CUtensorMap m[3];
+struct MapSet {
+    CUtensorMap m[4];
 };
 
 // Tensor maps of a layer, encoded once per (pointers, shape) and kept (encoding is host-only work, but not free).
-bool cached_maps(const hqm_weight* w, int G, CUtensorMap* out) {
+template <typename Encode>
+bool cached_maps(const hqm_weight* w, int G, CUtensorMap* out, int count, const Encode& encode) {
     static std::mutex mu;
-    static std::unordered_map<MapKey, MapTriple, MapKeyHash> cache;
+    static std::unordered_map<MapKey, MapSet, MapKeyHash> cache;
     const MapKey key{w->W_q, w->scale_q, w->zero_q, w->N, w->K, w->nbits, w->group_size};
     std::lock_guard<std::mutex> lock(mu);
     auto itr = cache.find(key);
     if (itr == cache.end()) {
-        MapTriple tr;
-        if (!encode_maps(w, G, tr.m)) return false;
+        MapSet tr;
+        if (!encode(tr.m)) return false;
         if (cache.size() > 16384) cache.clear();
         itr = cache.emplace(key, tr).first;
     }
-    for (int i = 0; i < 3; ++i) out[i] = itr->second.m[i];
+    for (int i = 0; i < count; ++i) out[i] = itr->second.m[i];
     return true;
+}
+bool cached_maps(const hqm_weight* w, int G, CUtensorMap* out) {
+    return cached_maps(w, G, out, 3, [&](CUtensorMap* to) { return encode_maps(w, G, to); });
 }
 
 size_t tma_smem_bytes(int depth, int nx, int K) {
@@ -761,6 +765,37 @@ bool prepare_kernel(size_t smem) {
 // The tensor maps of a layer for the other TMA users (three CUtensorMaps; the codes' box is 128 columns x 16 members).
 bool stream_cached_maps(const hqm_weight* w, int G, void* out3) {
     return maps_ok(w, G) && cached_maps(w, G, static_cast<CUtensorMap*>(out3));
+}
+
+// The maps of a 3-bit layer: words as (K, P3, members) with box (128, 1, up to 16), scale and zero bytes as (K, G) with box
+// (128, 8), and, where the last storage rows do not fill a member, those rows as (K, left).
+static bool encode_maps3(const hqm_weight* w, int G, const Members3& m, CUtensorMap* out) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return false;
+    const cuuint64_t K = (cuuint64_t)w->K;
+    const cuuint32_t ones[3] = {1, 1, 1};
+    auto words = [&](CUtensorMap* to, const void* at, int rows, int members, int box_members) {
+        const cuuint64_t dims[3] = {K, (cuuint64_t)rows, (cuuint64_t)members}, strides[2] = {K * 4, (cuuint64_t)rows * K * 4};
+        const cuuint32_t box[3] = {128, 1, (cuuint32_t)box_members};
+        return enc(to, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, const_cast<void*>(at), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!words(&out[0], w->W_q, m.P3, m.full, m.full < 16 ? m.full : 16)) return false;
+    if (!words(&out[3], static_cast<const uint8_t*>(w->W_q) + (m.left ? (size_t)m.full * m.P3 * K * 4 : 0), m.left ? m.left : 1, 1, 1))
+        return false;
+    const void* bytes[2] = {w->scale_q, w->zero_q};
+    for (int i = 0; i < 2; ++i) {
+        const cuuint64_t dims[3] = {K, (cuuint64_t)G, 1}, strides[2] = {K, (cuuint64_t)G * K};
+        const cuuint32_t box[3] = {128, 8, 1};
+        if (enc(&out[1 + i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(bytes[i]), dims, strides, box, ones,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    }
+    return true;
+}
+bool stream_cached_maps3(const hqm_weight* w, int G, const Members3& m, void* out4) {
+    return cached_maps(w, G, static_cast<CUtensorMap*>(out4), 4, [&](CUtensorMap* to) { return encode_maps3(w, G, m, to); });
 }
 
 // cuTensorMapEncodeTiled of the installed driver (null when it cannot be had), for the other TMA users.

@@ -85,6 +85,18 @@ int launch_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx
 int launch_router_lists(int32_t* counts, int32_t* offsets, int32_t* token_idx, float* token_w, int32_t* entry_of,
                         const float* topk_w, const int32_t* topk_idx, int64_t M, int32_t E, cudaStream_t st);
 
+// How the storage rows of a 3-bit layer repeat: row rho + i * P3 holds the same ten residues in the same slots for every
+// member i; `full` whole members and `left` rows of one more.
+struct Members3 {
+    int P3, full, left;
+    static Members3 of(const hqm_weight* w, int G) {
+        int a = G, b = 10;
+        while (b) { const int t = a % b; a = b; b = t; }
+        const int rows = (w->N + 9) / 10, P3 = G / a;
+        return Members3{P3, rows / P3, rows % P3};
+    }
+};
+bool stream_cached_maps3(const hqm_weight* w, int G, const Members3& m, void* out4);      // words, scales, zeros, left-over words
 // gemv_stream3.cu — the weight-streaming path for 3-bit layers.
 struct Stream3Plan {
     int P3;      // storage-row classes (rows R and R + P3 hold the same residues in the same slots)

@@ -158,7 +158,7 @@ class HQQLinearTritonSavable(nn.Module):
         return self._desc[1]
 
     def forward(self, x):
-        y = _cabi.host().linear(self, x)             # contiguous bf16 rows on the device; None for everything else
+        y = _cabi.host().linear(self, x)             # contiguous rows on the device; None for everything else
         return self.forward_triton(x) if y is None else y
 
     def set_backend(self, backend):

@@ -37,7 +37,7 @@ struct Plan {
     PyObject_HEAD
     hqm_weight w;
     int64_t linear_rows, expert_rows;
-    size_t linear_bytes, expert_bytes;
+    size_t linear_bytes, f16_bytes, expert_bytes;
 };
 PyObject* plan_copy(PyObject*, PyObject*) { Py_RETURN_NONE; }
 PyObject* plan_reduce(PyObject*, PyObject*) { return Py_BuildValue("(O())", (PyObject*)Py_TYPE(Py_None)); }
@@ -83,7 +83,7 @@ Plan* plan_of(PyObject* layer, PyObject* dict) {
         if (view.len == (Py_ssize_t)sizeof(hqm_weight) && (p = PyObject_New(Plan, &PlanType)) != nullptr) {
             memcpy(&p->w, view.buf, sizeof(hqm_weight));
             p->linear_rows = p->expert_rows = -1;
-            p->linear_bytes = p->expert_bytes = 0;
+            p->linear_bytes = p->f16_bytes = p->expert_bytes = 0;
             if (PyDict_SetItem(dict, N.plan, reinterpret_cast<PyObject*>(p)) != 0) p = nullptr;
             else Py_DECREF(p);                             // the layer's __dict__ holds it
         }
@@ -100,11 +100,12 @@ PyObject* dict_of(PyObject* module) {        // new reference
     return d;
 }
 
-// x as the library takes it: bf16, contiguous, on the current device, last dimension K, at least one row; else null.
+// x if it is bf16, fp16 or fp32, contiguous, on the current device, last dimension K, at least one row; else null.
 const at::Tensor* rows_of(PyObject* obj, int64_t K, int64_t* rows) {
     if (!THPVariable_CheckExact(obj)) return nullptr;
     const at::Tensor& x = THPVariable_Unpack(obj);
-    if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() < 1 || x.size(-1) != K || x.numel() == 0 || !x.is_contiguous() ||
+    const auto type = x.scalar_type();
+    if (!x.is_cuda() || (type != at::kBFloat16 && type != at::kHalf && type != at::kFloat) || x.dim() < 1 || x.size(-1) != K || x.numel() == 0 || !x.is_contiguous() ||
         x.device().index() != c10::cuda::current_device())
         return nullptr;
     *rows = x.numel() / K;
@@ -152,23 +153,32 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         const at::Tensor* x = p == nullptr ? nullptr : rows_of(args[1], p->w.K, &rows);
         if (x == nullptr) Py_RETURN_NONE;
         c10::InferenceMode guard;
+        const auto type = x->scalar_type();
         if (p->linear_rows != rows) {
             p->linear_bytes = hqm_linear_scratch_preferred(rows, &p->w);
+            p->f16_bytes = hqm_linear_f16_scratch_bytes(rows, &p->w);
             p->linear_rows = rows;
         }
+        const bool f16 = type == at::kHalf && p->f16_bytes != 0;
+        at::Tensor converted;
+        if (type != at::kBFloat16 && !f16) {
+            converted = x->to(at::kBFloat16);
+            x = &converted;
+        }
+        const size_t bytes = f16 ? p->f16_bytes : p->linear_bytes;
         size_t have = 0;
         void* ws = nullptr;
-        if (p->linear_bytes && (ws = scratch(*x, p->linear_bytes, &have)) == nullptr) Py_RETURN_NONE;
+        if (bytes && (ws = scratch(*x, bytes, &have)) == nullptr) Py_RETURN_NONE;
         at::Tensor y = result(*x, p->w.N);
         const hqm_weight w = p->w;                         // (without the lock another thread may replace the plan)
-        const size_t bytes = p->linear_bytes;
         const uint16_t* b = static_cast<const uint16_t*>(address(bias));
         int rc;
         Py_BEGIN_ALLOW_THREADS
-        rc = hqm_linear(static_cast<uint16_t*>(y.data_ptr()), static_cast<const uint16_t*>(x->const_data_ptr()), rows, &w, b, ws, bytes,
-                        c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
+        rc = (f16 ? hqm_linear_f16 : hqm_linear)(static_cast<uint16_t*>(y.data_ptr()), static_cast<const uint16_t*>(x->const_data_ptr()), rows,
+                                                 &w, b, ws, bytes, c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
         Py_END_ALLOW_THREADS
         if (rc < 0) Py_RETURN_NONE;
+        if (y.scalar_type() != type) y = y.to(type);
         return THPVariable_Wrap(std::move(y));
     } catch (const std::exception& e) {
         return PyErr_Format(PyExc_RuntimeError, "%s", e.what());
@@ -247,8 +257,15 @@ PyObject* expert(PyObject*, PyObject* const* args, Py_ssize_t n) {
         const at::Tensor* x = rows_of(args[1], p[0]->w.K, &rows);
         if (x == nullptr) Py_RETURN_NONE;
         c10::InferenceMode guard;
+        const auto type = x->scalar_type();
+        at::Tensor converted;
+        if (type != at::kBFloat16) {
+            converted = x->to(at::kBFloat16);
+            x = &converted;
+        }
         at::Tensor out = result(*x, p[1]->w.N);
         if (run_expert(p, *x, rows, nullptr, nullptr, static_cast<uint16_t*>(out.data_ptr()), 0) < 0) Py_RETURN_NONE;
+        if (type != at::kBFloat16) out = out.to(type);
         return THPVariable_Wrap(std::move(out));
     } catch (const std::exception& e) {
         return PyErr_Format(PyExc_RuntimeError, "%s", e.what());

@@ -17,18 +17,28 @@ TOL = 4e-3          # bf16 results of 16-bit factors with fp32 sums
     (2, 16, 512, 512, 0.02), (2, 16, 192, 192, 0.02),        # an odd number of tile parts and of column blocks
     (2, 16, 320, 704, 2.0),                                  # scales beyond the range of the denormal fields
     (2, 32, 256, 320, 0.02), (4, 32, 256, 512, 0.02),
-    (4, 64, 256, 320, 0.02), (4, 64, 1024, 1024, 30.0)])
+    (4, 64, 256, 320, 0.02), (4, 64, 1024, 1024, 30.0),
+    (3, 64, 512, 128, 0.02), (3, 64, 1024, 320, 0.02), (3, 64, 2560, 192, 0.02), (3, 64, 5120, 256, 30.0)])
 def test_linear_edges(nbits, group, N, K, std):
     od = random_layer(N, K, nbits, group, seed=nbits + group, std=std)
     layer = layer_from_oracle(od, DEV)
     W = layer.dequantize(torch.float32).double()
-    for M in (5, 16, 17, 64, 65, 128, 129, 256, 257, 530):
+    for M in (2, 5, 16, 17, 64, 65, 128, 129, 256, 257, 530):
         x = (torch.randn(M, K, generator=torch.Generator().manual_seed(M)) * 10.0 ** (M % 7 - 3)).to(torch.bfloat16).to(DEV)
         y = layer(x)
         want = x.double() @ W.t()
         assert ((y.double() - want).norm() / want.norm()).item() < TOL, M
         assert torch.equal(y, layer(x)), M                   # pieces of a tile are added in a fixed order
     assert _cabi.lib().hqm_device_error() == 0
+
+
+@pytest.mark.parametrize("nbits,group", [(2, 16), (3, 64), (4, 64)])
+def test_fp16_rows_stay_fp16(nbits, group):
+    layer = layer_from_oracle(random_layer(1024, 512, nbits, group, seed=nbits), DEV)
+    x = torch.randn(33, 512, generator=torch.Generator().manual_seed(1)).to(torch.float16).to(DEV)
+    want = x.double() @ layer.dequantize(torch.float32).double().t()
+    y = layer(x)
+    assert y.dtype == torch.float16 and ((y.double() - want).norm() / want.norm()).item() < 1e-3
 
 
 @pytest.mark.parametrize("tokens", [2, 3, 17, 70, 300])
