@@ -94,10 +94,9 @@ class MixtralDecodeModel(nn.Module):
         h = self.embed[ids]                                                # (T, hidden)
         self.router_logits = []
         ln_in = self.first_ln                       # the norm weights step() applies: first_ln, then each layer's next_ln
-        shared = self.layers[0].tokens_shared(T, pos0, h.device)
         y = None
         for layer in self.layers:
-            h, y, logits = layer._tokens(h, y, pos0, ln_in, shared)
+            h, y, logits = layer._tokens(h, y, pos0, ln_in, None)
             self.router_logits.append(logits)
             ln_in = layer.next_ln
         x = rms_norm_rows(h[-1:], self.layers[-1].next_ln, self.rms_eps, y[-1:])

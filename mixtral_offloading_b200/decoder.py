@@ -15,6 +15,7 @@ from typing import Optional
 
 import torch
 from torch import nn
+from torch.nn.attention.bias import causal_lower_right
 
 from . import _cabi
 from .custom_layers import HQQLinearTritonSavable, ResidentMoe, _scratch, linear_group
@@ -170,9 +171,10 @@ class DecoderLayerDecode(nn.Module):
 
     @staticmethod
     def tokens_shared(T: int, pos0: int, device):
-        """The attention mask of T tokens at positions pos0 .. pos0 + T - 1: token i sees positions 0 .. pos0 + i."""
-        positions = torch.arange(pos0, pos0 + T, device=device)
-        return torch.arange(pos0 + T, device=device)[None, :] <= positions[:, None]
+        """The attention mask of T tokens at positions pos0 .. pos0 + T - 1: token i sees positions 0 .. pos0 + i.  (Not as a
+        tensor: the attention kernels leave out the blocks that a causal mask hides.  500 tokens: 62 us with a mask, 17
+        without; 500 behind 1000: 156 and 52.)"""
+        return causal_lower_right(T, pos0 + T)
 
     @torch.inference_mode()
     def forward_tokens(self, h: torch.Tensor, pos0: int, ln_in=None, shared=None):
@@ -201,8 +203,9 @@ class DecoderLayerDecode(nn.Module):
                          a.rope_theta, pos0, 1)
         q = q.view(T, a.n_heads, a.head_dim)
         keys, vals = a.k_cache[:, :pos0 + T].unsqueeze(0), a.v_cache[:, :pos0 + T].unsqueeze(0)
-        ctx = torch.nn.functional.scaled_dot_product_attention(q.transpose(0, 1).unsqueeze(0), keys, vals, attn_mask=mask,
-                                                               enable_gqa=True)          # (1, heads, T, head_dim)
+        ctx = torch.nn.functional.scaled_dot_product_attention(
+            q.transpose(0, 1).unsqueeze(0), keys, vals, attn_mask=None if pos0 == 0 and shared is None else mask,
+            is_causal=pos0 == 0 and shared is None, enable_gqa=True)                     # (1, heads, T, head_dim)
         out = a.o_proj(ctx[0].transpose(0, 1).reshape(T, hidden))
         y, logits = self.moe(rms_norm_rows(out, a.ln_post, a.rms_eps, h).view(1, T, hidden))       # out += h
         return out, y.view(T, hidden), logits

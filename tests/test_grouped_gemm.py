@@ -38,7 +38,7 @@ def test_fp16_rows_stay_fp16(nbits, group):
     x = torch.randn(33, 512, generator=torch.Generator().manual_seed(1)).to(torch.float16).to(DEV)
     want = x.double() @ layer.dequantize(torch.float32).double().t()
     y = layer(x)
-    assert y.dtype == torch.float16 and ((y.double() - want).norm() / want.norm()).item() < 1e-3
+    assert y.dtype == torch.float16 and ((y.double() - want).norm() / want.norm()).item() < 2e-3
 
 
 @pytest.mark.parametrize("tokens", [2, 3, 17, 70, 300])
