@@ -589,7 +589,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
         Seg s;
         s.p = 0;
         int at = 0;
-        bool ok = true;
         // meta values (fp16 scale / zero of the 8-bit scale and zero bytes), requested a unit ahead
         uint32_t mt[4][DC / 2];
         int mcol = 0, mC = 1, mstep = 0;
@@ -621,13 +620,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                     }
             }
         };
-        int r = group, v = group * HALVES;                    // slots of this group's next unit: packed bytes; A, and its phase
-        uint32_t r_par = 0, v_round = 0;
-        while (v >= slots) {
-            v -= slots;
-            ++v_round;
-        }
-        while (ok && next_seg(sh, ub, ue, at, units_k, s)) {
+        static_assert(HALVES == 1, "an A slot holds a unit");
+        int r = group, v = group;                             // slots of this group's next unit: packed bytes; A, and its phase
+        uint32_t r_par = 0, v_round = 0, limit = WAIT_LIMIT, raw_ready = 0, a_ready = 0;
+        // The A slot that has been written and not yet handed to the MMAs: the stores are waited for when the next unit's loads
+        // are on their way (or before a wait for them).
+        uint32_t pending = 0;
+        auto hand_over = [&] {
+            if (pending) {
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                if (lane == 0) arrive(pending);
+                pending = 0;
+            }
+        };
+        while (next_seg(sh, ub, ue, at, units_k, s)) {
             const int n_seg = s.k1 - s.k0;
             at += n_seg;
             int first = group - s.u0 % GROUPS;                // first unit of the run that is this group's
@@ -655,8 +662,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             mstep = (GROUPS * UK) % mC;
             load_meta();
             for (int k = s.k0 + first; k < s.k1; k += GROUPS) {
-                if (!wait(raw_full + 8 * r, r_par)) ok = false;
-                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                if (!raw_ready) hand_over();
+                wait_peeked(raw_full + 8 * r, r_par, raw_ready, limit);
                 const uint32_t rw = raw_ring + r * F::RAW_BYTES;
                 uint4 wv[4];
                 auto load_codes = [&](int sub) {
@@ -686,6 +693,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                         zq[0] = lds32(sqa + ZS);
                     }
                     load_codes(0);                            // on their way while the scales are decoded
+                    hand_over();
+                    a_ready = v_round > 0 ? peek(a_empty + 8 * (v + ((v_round & 1) ? 0 : NA)), ((v_round - 1) >> 1) & 1) : 1u;
                     uint32_t S[DC / 2], T[DC / 2];            // per four columns: pair (0, 2), pair (1, 3)
                     if (f16) {
                         // s * 2^(22 - p) and -z * s / 4, p = 4 + fpos the field's first bit
@@ -770,15 +779,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 const int subs = min(BLOCKS, prm.subs_k - BLOCKS * k);
 #pragma unroll
                 for (int half = 0; half < HALVES; ++half) {
-                    const int av = v + half, aslot = av >= slots ? av - slots : av;
-                    const uint32_t round = v_round + (av >= slots ? 1u : 0u);
                     // The A slot's tile of the round before has been read by its MMAs.  (A parity only tells the last phase from
-                    // the one before it, and with two slots to a unit a group may be two rounds behind when it comes to wait:
-                    // even and odd rounds have barriers of their own.)
-                    if (round > 0 && !wait(a_empty + 8 * (aslot + ((round & 1) ? 0 : NA)), ((round - 1) >> 1) & 1)) ok = false;
-                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                    // the one before it: even and odd rounds have barriers of their own.)
+                    if (v_round > 0) wait_peeked(a_empty + 8 * (v + ((v_round & 1) ? 0 : NA)), ((v_round - 1) >> 1) & 1, a_ready, limit);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t ta = tmem + tmap.a_base + 64 * aslot + ((uint32_t)(32 * q) << 16);
+                    const uint32_t ta = tmem + tmap.a_base + 64 * v + ((uint32_t)(32 * q) << 16);
 #pragma unroll
                     for (int sub2 = 0; sub2 < 2; ++sub2) {
                         const int sub = 2 * half + sub2;
@@ -847,29 +852,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                             }
                         }
                     }
-                    if (half == HALVES - 1) {
-                        // The staged bytes have been read.  (Only here: what was loaded has been used by every lane.)
-                        __syncwarp();
-                        if (lane == 0) arrive(raw_empty + 8 * r);
-                    }
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    if (lane == 0) arrive(a_full + 8 * aslot);
+                    // The staged bytes have been read.  (Only here: what was loaded has been used by every lane.)
+                    __syncwarp();
+                    if (lane == 0) arrive(raw_empty + 8 * r);
+                    pending = a_full + 8 * v;
                 }
-                if (!ok) break;
                 r += GROUPS;
                 if (r >= n_raw) {
                     r -= n_raw;
                     r_par ^= 1u;
                 }
-                v += GROUPS * HALVES;
-                while (v >= slots) {
+                v += GROUPS;
+                if (v >= slots) {
                     v -= slots;
                     ++v_round;
                 }
+                raw_ready = peek(raw_full + 8 * r, r_par);
             }
         }
-        if (!ok) sh.failed = 1;
+        hand_over();
+        if (limit == 0) sh.failed = 1;
     } else if (warp >= WARP_RAW) {
         regs_down<REGS_ISSUE>();
         // The copying and the MMA-issuing warps: all lanes run the same code on the same values and an elected one issues, so
