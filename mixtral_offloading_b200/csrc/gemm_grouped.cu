@@ -386,6 +386,11 @@ __device__ __forceinline__ uint32_t bf2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+__device__ __forceinline__ uint32_t bf2_mul(uint32_t a, uint32_t b) {      // one rounding, as of the fp32 product
+    uint32_t d;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
 // 16 rows x 32 columns of A from a warp's registers.
 __device__ __forceinline__ void store_a(uint32_t at, const uint32_t (&o)[16]) {
     asm volatile(
@@ -784,7 +789,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                     if (v_round > 0) wait_peeked(a_empty + 8 * (v + ((v_round & 1) ? 0 : NA)), ((v_round - 1) >> 1) & 1, a_ready, limit);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t ta = tmem + tmap.a_base + 64 * v + ((uint32_t)(32 * q) << 16);
-#pragma unroll
+#pragma unroll 1                                  // (unrolled it is 3 % slower: the code of 16 warps at different places)
                     for (int sub2 = 0; sub2 < 2; ++sub2) {
                         const int sub = 2 * half + sub2;
                         if (sub < subs) {
@@ -1191,12 +1196,27 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                         const bool up = (lane & 1) != 0;
                         uint16_t hv[8];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const float give = up ? v[i] : v[i + 8];
-                            const float other = __shfl_xor_sync(0xffffffffu, give, 1);
-                            const float a = round_bf16(up ? other : v[i]), b = round_bf16(up ? v[i + 8] : other);
-                            const float hh = round_bf16(round_bf16(__fdividef(a, 1.f + __expf(-a))) * b);
-                            hv[i] = cnt <= GG_F16_ROWS ? __half_as_ushort(__float2half_rn(hh)) : float_to_bf16_bits(hh);
+                        for (int i = 0; i < 8; i += 2) {                  // two rows at a time: packed roundings and products
+                            uint32_t a2, b2;
+                            float a[2], b[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const float give = up ? v[i + e] : v[i + e + 8];
+                                const float other = __shfl_xor_sync(0xffffffffu, give, 1);
+                                a[e] = up ? other : v[i + e];
+                                b[e] = up ? v[i + e + 8] : other;
+                            }
+                            a2 = bf2(a[0], a[1]);
+                            b2 = bf2(b[0], b[1]);
+                            const float a0 = __uint_as_float(a2 << 16), a1 = __uint_as_float(a2 & 0xffff0000u);
+                            const uint32_t g2 = bf2(__fdividef(a0, 1.f + __expf(-a0)), __fdividef(a1, 1.f + __expf(-a1)));
+                            uint32_t h2 = bf2_mul(g2, b2);
+                            if (cnt <= GG_F16_ROWS) {
+                                const __half2 f = __floats2half2_rn(__uint_as_float(h2 << 16), __uint_as_float(h2 & 0xffff0000u));
+                                h2 = *reinterpret_cast<const uint32_t*>(&f);
+                            }
+                            hv[i] = (uint16_t)h2;
+                            hv[i + 1] = (uint16_t)(h2 >> 16);
                         }
                         // [row][member][slot in the order 0, 2, 1, 3]
                         const int so = ((slot & 1) << 1) | (slot >> 1);
