@@ -612,14 +612,20 @@ struct QkvSource {                 // FUSED only: where q, k, v of this token co
 };
 
 // rotate-half RoPE of the pair (a, b) = (t[d], t[d + 64]) at position pos, bf16 arithmetic as Hugging Face does it
-__device__ __forceinline__ void rope_pair(float a, float b, int d, int pos, float theta, float& o0, float& o1) {
+__device__ __forceinline__ void rope_angle(int d, int pos, float theta, float& sn, float& cs) {
     const float inv_freq = powf(theta, -(float)(2 * d) / (float)HEAD_DIM);
-    float sn, cs;
     sincosf((float)pos * inv_freq, &sn, &cs);
     sn = round_bf16(sn);
     cs = round_bf16(cs);
+}
+__device__ __forceinline__ void rope_rotate(float a, float b, float sn, float cs, float& o0, float& o1) {
     o0 = round_bf16(round_bf16(a * cs) + round_bf16(-b * sn));
     o1 = round_bf16(round_bf16(b * cs) + round_bf16(a * sn));
+}
+__device__ __forceinline__ void rope_pair(float a, float b, int d, int pos, float theta, float& o0, float& o1) {
+    float sn, cs;
+    rope_angle(d, pos, theta, sn, cs);
+    rope_rotate(a, b, sn, cs, o0, o1);
 }
 
 // RoPE and cache append for many tokens at once (a prompt: token t at position pos0 + t in ONE cache; a batch of
@@ -640,11 +646,15 @@ __global__ void __launch_bounds__(256) rope_append_rows_kernel(uint16_t* __restr
     }
     constexpr int HALF = HEAD_DIM / 2;
     uint16_t* qt = q + (int64_t)t * n_heads * HEAD_DIM;
+    static_assert(256 % HALF == 0, "a thread keeps its column: one angle (500 tokens: 8 us with one for every pair, 4 so)");
+    float sn, cs;
+    rope_angle(threadIdx.x % HALF, pos, theta, sn, cs);
+#pragma unroll 4
     for (int i = threadIdx.x; i < n_heads * HALF; i += 256) {
         const int head = i / HALF, d = i % HALF;
         uint16_t* p = qt + head * HEAD_DIM + d;
         float o0, o1;
-        rope_pair(bf16_bits_to_float(p[0]), bf16_bits_to_float(p[HALF]), d, pos, theta, o0, o1);
+        rope_rotate(bf16_bits_to_float(p[0]), bf16_bits_to_float(p[HALF]), sn, cs, o0, o1);
         p[0] = float_to_bf16_bits(o0);
         p[HALF] = float_to_bf16_bits(o1);
     }
@@ -654,8 +664,7 @@ __global__ void __launch_bounds__(256) rope_append_rows_kernel(uint16_t* __restr
         const int head = i / HALF, d = i % HALF;
         const int64_t row = (int64_t)t * batch_stride + ((int64_t)head * max_len + pos) * HEAD_DIM + d;
         float o0, o1;
-        rope_pair(bf16_bits_to_float(kt[head * HEAD_DIM + d]), bf16_bits_to_float(kt[head * HEAD_DIM + d + HALF]), d, pos, theta,
-                  o0, o1);
+        rope_rotate(bf16_bits_to_float(kt[head * HEAD_DIM + d]), bf16_bits_to_float(kt[head * HEAD_DIM + d + HALF]), sn, cs, o0, o1);
         k_cache[row] = float_to_bf16_bits(o0);
         k_cache[row + HALF] = float_to_bf16_bits(o1);
         v_cache[row] = vt[head * HEAD_DIM + d];

@@ -19,6 +19,85 @@ namespace cg = cooperative_groups;
 // experts held in registers.
 constexpr int ROUTER_CTAS = 8;
 
+// Softmax, top-2 and renormalisation of one token from its rounded logits (mx: their maximum).
+template <int EMAX>
+__device__ __forceinline__ void finish_token(const float (&acc)[EMAX], float mx, int t, int E, uint16_t* __restrict__ logits_out,
+                                             float* __restrict__ topk_w, int32_t* __restrict__ topk_idx) {
+    float p[EMAX], sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < EMAX; ++e) {
+        p[e] = (e < E) ? expf(acc[e] - mx) : 0.f;
+        sum += p[e];
+    }
+    int i0 = 0, i1 = -1;
+    float p0 = -1.f, p1 = -1.f;
+#pragma unroll
+    for (int e = 0; e < EMAX; ++e) {
+        if (e < E) {
+            const float pe = p[e] / sum;
+            logits_out[(int64_t)t * E + e] = float_to_bf16_bits(acc[e]);
+            if (pe > p0) { p1 = p0; i1 = i0; p0 = pe; i0 = e; }
+            else if (pe > p1) { p1 = pe; i1 = e; }
+        }
+    }
+    if (i1 < 0) { i1 = i0; p1 = 0.f; }   // E == 1
+    const float norm = p0 + p1;
+    topk_w[2 * t] = round_bf16(p0 / norm);
+    topk_w[2 * t + 1] = round_bf16(p1 / norm);
+    topk_idx[2 * t] = i0;
+    topk_idx[2 * t + 1] = i1;
+}
+
+// Up to 8 experts and 4096 columns: a CTA per token, a thread per 8 columns; the sums are formed in the order of the kernel
+// below (whose cluster has work for two of its eight CTAs here, and costs two cluster barriers).  500 tokens: 28 us with
+// the cluster, 5 without.
+__global__ void __launch_bounds__(512)
+router_short_rows_kernel(uint16_t* __restrict__ logits_out, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
+                         const uint16_t* __restrict__ x, const uint16_t* __restrict__ gate_w, int K, int E) {
+    __shared__ float s_part[16][8];
+    grid_launch_dependents();
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, t = blockIdx.x, k = 8 * threadIdx.x;
+    uint4 gv[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e)                               // (weights: no kernel in front writes them)
+        gv[e] = e < E && k < K ? __ldg(reinterpret_cast<const uint4*>(gate_w + (int64_t)e * K + k)) : make_uint4(0u, 0u, 0u, 0u);
+    grid_dependency_wait();
+    const uint4 xv = k < K ? *reinterpret_cast<const uint4*>(x + (int64_t)t * K + k) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const uint32_t gw[4] = {gv[e].x, gv[e].y, gv[e].z, gv[e].w};
+        float a = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            a = fmaf(__uint_as_float(xw[j] << 16), __uint_as_float(gw[j] << 16), a);
+            a = fmaf(__uint_as_float(xw[j] & 0xffff0000u), __uint_as_float(gw[j] & 0xffff0000u), a);
+        }
+        a = warp_sum(a);
+        if (lane == 0) s_part[wi][e] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        float v = 0.f;                                        // lane e: expert e
+        if (lane < 8) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float c = 0.f;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) c += s_part[8 * h + w][lane];
+                v += c;
+            }
+        }
+        float acc[8], mx = -INFINITY;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            acc[e] = round_bf16(__shfl_sync(0xffffffffu, v, e));
+            if (e < E) mx = fmaxf(mx, acc[e]);
+        }
+        if (lane == 0) finish_token<8>(acc, mx, t, E, logits_out, topk_w, topk_idx);
+    }
+}
+
 template <int EMAX>
 __global__ void __launch_bounds__(256)
 router_logits_top2_kernel(uint16_t* __restrict__ logits_out, float* __restrict__ topk_w, int32_t* __restrict__ topk_idx,
@@ -92,33 +171,12 @@ router_logits_top2_kernel(uint16_t* __restrict__ logits_out, float* __restrict__
             acc[e] = round_bf16(v);
             if (e < E) mx = fmaxf(mx, acc[e]);
         }
-        float p[EMAX], sum = 0.f;
-#pragma unroll
-        for (int e = 0; e < EMAX; ++e) {
-            p[e] = (e < E) ? expf(acc[e] - mx) : 0.f;
-            sum += p[e];
-        }
-        int i0 = 0, i1 = -1;
-        float p0 = -1.f, p1 = -1.f;
-#pragma unroll
-        for (int e = 0; e < EMAX; ++e) {
-            if (e < E) {
-                const float pe = p[e] / sum;
-                logits_out[(int64_t)t * E + e] = float_to_bf16_bits(acc[e]);
-                if (pe > p0) { p1 = p0; i1 = i0; p0 = pe; i0 = e; }
-                else if (pe > p1) { p1 = pe; i1 = e; }
-            }
-        }
-        if (i1 < 0) { i1 = i0; p1 = 0.f; }   // E == 1
-        const float norm = p0 + p1;
-        topk_w[2 * t] = round_bf16(p0 / norm);
-        topk_w[2 * t + 1] = round_bf16(p1 / norm);
-        topk_idx[2 * t] = i0;
-        topk_idx[2 * t + 1] = i1;
+        finish_token<EMAX>(acc, mx, t, E, logits_out, topk_w, topk_idx);
     }
     cluster.sync();                                     // nobody leaves while its shared memory may still be read
 }
 
+constexpr int LISTS_SMEM = 2048;
 // One CTA, one warp per expert: count, exclusive scan, then a stable (token
 // ascending) list of the rows routed to each expert with their weights.
 __global__ void router_lists_kernel(int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
@@ -127,14 +185,23 @@ __global__ void router_lists_kernel(int32_t* __restrict__ counts, int32_t* __res
                                     const int32_t* __restrict__ topk_idx, int M, int E) {
     __shared__ int s_count[32];
     __shared__ int s_off[33];
+    // The choices of up to LISTS_SMEM tokens are fetched once, all at a time; the two passes over them then run on shared
+    // memory (500 tokens: 11 us with a dependent round trip for every 32 tokens of either pass, 4 without).
+    __shared__ int2 s_idx[LISTS_SMEM];
     grid_launch_dependents();
     grid_dependency_wait();
     const int lane = threadIdx.x & 31, e = threadIdx.x >> 5;
+    const bool fetched = M <= LISTS_SMEM;
+    if (fetched) {
+        for (int t = threadIdx.x; t < M; t += blockDim.x) s_idx[t] = make_int2(topk_idx[2 * t], topk_idx[2 * t + 1]);
+        __syncthreads();
+    }
+    auto choice = [&](int t) { return fetched ? s_idx[t] : make_int2(topk_idx[2 * t], topk_idx[2 * t + 1]); };
     int cnt = 0;
     for (int t0 = 0; t0 < M; t0 += 32) {
         const int t = t0 + lane;
-        const bool hit = t < M && (topk_idx[2 * t] == e || topk_idx[2 * t + 1] == e);
-        cnt += __popc(__ballot_sync(0xffffffffu, hit));
+        const int2 c = t < M ? choice(t) : make_int2(-1, -1);
+        cnt += __popc(__ballot_sync(0xffffffffu, c.x == e || c.y == e));
     }
     if (lane == 0) s_count[e] = cnt;
     __syncthreads();
@@ -155,8 +222,9 @@ __global__ void router_lists_kernel(int32_t* __restrict__ counts, int32_t* __res
         const int t = t0 + lane;
         int slot = -1;
         if (t < M) {
-            if (topk_idx[2 * t] == e) slot = 0;
-            else if (topk_idx[2 * t + 1] == e) slot = 1;
+            const int2 c = choice(t);
+            if (c.x == e) slot = 0;
+            else if (c.y == e) slot = 1;
         }
         const unsigned ballot = __ballot_sync(0xffffffffu, slot >= 0);
         if (slot >= 0) {
@@ -175,7 +243,10 @@ namespace hqm {
 // Logits, top-2 indices and weights only (no per-expert lists): what the single-token MoE block needs.
 int launch_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx, const uint16_t* x,
                        const uint16_t* gate_w, int64_t M, int64_t K, int32_t E, cudaStream_t st) {
-    if (E <= 8)
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate_w)) & 15u) == 0;
+    if (E <= 8 && K <= 4096 && K % 8 == 0 && aligned)
+        launch_overlapped(router_short_rows_kernel, (int)M, 512, 0, st, router_logits, topk_w, topk_idx, x, gate_w, (int)K, (int)E);
+    else if (E <= 8)
         launch_overlapped_cluster(router_logits_top2_kernel<8>, (int)M * ROUTER_CTAS, 256, 0, ROUTER_CTAS, st,
                                   router_logits, topk_w, topk_idx, x, gate_w, (int)M, (int)K, (int)E);
     else
