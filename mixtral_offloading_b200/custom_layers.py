@@ -393,6 +393,7 @@ class ResidentMoe(nn.Module):
         self._experts = list(experts)              # kept out of the module registry like the wrapper does
         self._router = SparseMoeWrapper(config, layer_id, gate, expert_cache=None)
         self._table = None
+        self._shapes, self._bytes = None, {}       # references to the descriptors that give the shapes; bytes per token count
         self._host_counts = None
 
     @staticmethod
@@ -401,7 +402,8 @@ class ResidentMoe(nn.Module):
 
     def invalidate(self):
         """Forget the device-side descriptor table (call after the experts' tensors were replaced or moved)."""
-        self._table = None
+        self._table = self._shapes = None
+        self._bytes.clear()
 
     @staticmethod
     def _build_table(experts, device):
@@ -426,14 +428,20 @@ class ResidentMoe(nn.Module):
         return self._table
 
     def _descriptors(self):
-        f0 = self._ffn(self._experts[0])
-        return tuple(C.byref(lyr.descriptor()) for lyr in (f0.w1, f0.w2, f0.w3))
+        if self._shapes is None:
+            f0 = self._ffn(self._experts[0])
+            self._shapes = tuple(C.byref(lyr.descriptor()) for lyr in (f0.w1, f0.w2, f0.w3))
+        return self._shapes
 
     def scratch_bytes(self, tokens: int) -> int:
         """Workspace of forward_on_device(); 0 where the shapes have no path without a read-back."""
-        size = _cabi.lib().hqm_moe_decode_scratch_bytes if tokens == 1 else \
-            partial(_cabi.lib().hqm_moe_forward_scratch_bytes, tokens)
-        return size(self.num_experts, *self._descriptors())
+        if tokens not in self._bytes:
+            if len(self._bytes) >= 1024:
+                self._bytes.clear()
+            size = _cabi.lib().hqm_moe_decode_scratch_bytes if tokens == 1 else \
+                partial(_cabi.lib().hqm_moe_forward_scratch_bytes, tokens)
+            self._bytes[tokens] = size(self.num_experts, *self._descriptors())
+        return self._bytes[tokens]
 
     def forward_on_device(self, x2: torch.Tensor):
         """The block on rows x2 (tokens, hidden) bf16 with nothing read back; returns (out, router logits)."""
