@@ -357,10 +357,10 @@ class SparseMoeWrapper(nn.Module):
             guess = nxt.route(x2)[2][:, :self.speculate_width].reshape(-1)
             n_guess = guess.numel()
             self._host_counts[2 * E + 1:2 * E + 1 + n_guess].copy_(guess, non_blocking=True)
-        torch.cuda.current_stream(x2.device).synchronize()
+        final = torch.zeros((x2.shape[0], hidden_dim), dtype=torch.bfloat16, device=x2.device)
+        torch.cuda.current_stream(x2.device).synchronize()      # (what follows delays the copies: nothing that can go before)
         host = self._host_counts.tolist()
         counts, offsets = host[:E], host[E:2 * E + 1]
-        final = torch.zeros((x2.shape[0], hidden_dim), dtype=torch.bfloat16, device=x2.device)
         active = [e for e in range(E) if counts[e] > 0]
         for (_layer, e), expert in self.experts.load_experts(*((self.layer_id, e) for e in active), unordered=True):
             lo, hi = offsets[e], offsets[e + 1]
