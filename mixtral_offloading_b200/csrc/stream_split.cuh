@@ -56,7 +56,7 @@ __device__ __forceinline__ int partial_count(const Split& sp, const ColMap& cm, 
 
 // Sum of the partial row-sets of element (m, col), added in a fixed order; `row` is the row length,
 // MR = rows * row.  BATCHED = false is a plain loop (the compiler groups its loads): best when a residue has
-// few row-sets (the kernels behind hqm_linear / hqm_expert_ffn).  BATCHED = true keeps eight loads in flight at
+// few row-sets (the kernels behind hqm_linear / hqm_expert_ffn).  BATCHED = true keeps 24 loads in flight at
 // a time: best for the decode step's small layers, whose K dimension is cut into about twenty pieces.  (Each
 // measured a few percent slower in the other's place.)
 template <bool BATCHED>
@@ -68,11 +68,13 @@ __device__ __forceinline__ float partial_sum(const float* __restrict__ partial, 
     if constexpr (!BATCHED) {
         for (int s = 0; s < cnt; ++s) v += p[(int64_t)s * MR];
     } else {
-        for (int s = 0; s < cnt; s += 8) {
-            float a[8];
+        for (int s = 0; s < cnt; s += 24) {
+            float a[24];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) a[j] = (s + j < cnt) ? p[(int64_t)(s + j) * MR] : 0.f;
-            v += ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+            for (int j = 0; j < 24; ++j) a[j] = (s + j < cnt) ? p[(int64_t)(s + j) * MR] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 24; j += 8)
+                v += ((a[j] + a[j + 1]) + (a[j + 2] + a[j + 3])) + ((a[j + 4] + a[j + 5]) + (a[j + 6] + a[j + 7]));
         }
     }
     return v;
@@ -98,15 +100,18 @@ __device__ __forceinline__ void partial_sum_pair(const float* __restrict__ parti
         for (int s = both; s < cnt_b; ++s) vb += pb[(int64_t)s * MR];
     } else {
         const int cnt = cnt_a > cnt_b ? cnt_a : cnt_b;
-        for (int s = 0; s < cnt; s += 8) {
-            float a[8], b[8];
+        for (int s = 0; s < cnt; s += 24) {
+            float a[24], b[24];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < 24; ++j) {
                 a[j] = (s + j < cnt_a) ? pa[(int64_t)(s + j) * MR] : 0.f;
                 b[j] = (s + j < cnt_b) ? pb[(int64_t)(s + j) * MR] : 0.f;
             }
-            va += ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-            vb += ((b[0] + b[1]) + (b[2] + b[3])) + ((b[4] + b[5]) + (b[6] + b[7]));
+#pragma unroll
+            for (int j = 0; j < 24; j += 8) {
+                va += ((a[j] + a[j + 1]) + (a[j + 2] + a[j + 3])) + ((a[j + 4] + a[j + 5]) + (a[j + 6] + a[j + 7]));
+                vb += ((b[j] + b[j + 1]) + (b[j + 2] + b[j + 3])) + ((b[j + 4] + b[j + 5]) + (b[j + 6] + b[j + 7]));
+            }
         }
     }
     out_a = va;
