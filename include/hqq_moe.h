@@ -309,6 +309,9 @@ int hqm_add_rmsnorm(uint16_t* h, const uint16_t* delta, const uint16_t* weight, 
  * (rows, hidden) bf16; delta may be NULL (then h is only read). */
 int hqm_add_rmsnorm_rows(uint16_t* h, const uint16_t* delta, const uint16_t* weight, uint16_t* x_out, int64_t rows,
                          int32_t hidden, float eps, void* stream);
+/* The end of a greedy decoding step on the device: *token = index of the largest logit (bf16; the first of equal ones),
+ * *position += 1 (position may be NULL). */
+int hqm_greedy_advance(int64_t* token, int32_t* position, const uint16_t* logits, int32_t vocab, void* stream);
 /* Rotary embedding and cache append for `tokens` tokens at once (modeling_mixtral.py apply_rotary_pos_emb and the
  * cache update of MixtralAttention.forward, with the arithmetic of hqm_attn_decode): q (tokens, n_heads, 128) bf16 is
  * rotated in place; k (tokens, n_kv_heads, 128) is rotated and, with v, written to row `pos` of the caches

@@ -104,6 +104,7 @@ SIGNATURES = {
     "hqm_ep_combine_add_rmsnorm": (C.c_int, [_P, C.POINTER(HqmEpComm), _P, _P, _I32, C.c_float, _P]),
     "hqm_add_f32_rmsnorm": (C.c_int, [_P, _P, _P, _P, _I32, C.c_float, _P]),
     "hqm_add_rmsnorm": (C.c_int, [_P, _P, _P, _P, _I32, C.c_float, _P]),
+    "hqm_greedy_advance": (C.c_int, [_P, _P, _P, _I32, _P]),
     "hqm_add_rmsnorm_rows": (C.c_int, [_P, _P, _P, _P, C.c_int64, _I32, C.c_float, _P]),
     "hqm_rope_append_rows": (C.c_int, [_P, _P, _P, _P, _P, C.c_int64, _I32, _I32, _I32, _I32, C.c_int64, _P, _I32, _I32,
                                        C.c_float, _P]),

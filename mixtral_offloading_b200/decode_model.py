@@ -17,7 +17,7 @@ import torch
 from torch import nn
 
 from .custom_layers import linear_group
-from .decoder import DecoderLayerDecode, add_rmsnorm, rms_norm_rows, rope_append_rows
+from .decoder import DecoderLayerDecode, add_rmsnorm, greedy_advance, rms_norm_rows, rope_append_rows
 from .sampling import sample_token
 
 
@@ -46,12 +46,11 @@ class MixtralDecodeModel(nn.Module):
     def step(self) -> torch.Tensor:
         """Feeds self.token at self.position through the model; afterwards self.token is the greedy next token
         and self.position has advanced.  Returns the logits (1, vocab)."""
-        h = self.embed[self.token]                                         # (1, hidden), a fresh tensor
+        h = torch.nn.functional.embedding(self.token, self.embed)   # (1, hidden), a fresh tensor
         x = add_rmsnorm(h, None, self.first_ln, self.rms_eps)
         self.router_logits = [layer(h, x, self.position) for layer in self.layers]
         logits = torch.matmul(x, self.lm_head.t())     # x is the final norm of h after the last layer
-        self.token.copy_(logits.argmax(-1))
-        self.position.add_(1)
+        greedy_advance(logits, self.token, self.position)
         return logits
 
     @torch.inference_mode()

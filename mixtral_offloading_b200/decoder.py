@@ -38,6 +38,17 @@ def add_rmsnorm(h: torch.Tensor, delta, weight: torch.Tensor, eps: float = 1e-5)
     return x
 
 
+def greedy_advance(logits: torch.Tensor, token: torch.Tensor, position: torch.Tensor) -> None:
+    """token = argmax of logits (1, vocab) bf16, position += 1, in one launch (hqm_greedy_advance)."""
+    if logits.dtype != torch.bfloat16 or token.dtype != torch.int64 or position.dtype != torch.int32:
+        token.copy_(logits.argmax(-1))
+        position.add_(1)
+        return
+    logits = logits.contiguous()
+    _cabi.check(_cabi.lib().hqm_greedy_advance(_cabi.ptr(token), _cabi.ptr(position), _cabi.ptr(logits), logits.shape[-1],
+                                               _cabi.stream_ptr(logits.device)))
+
+
 def rms_norm_rows(h: torch.Tensor, w: torch.Tensor, eps: float, delta: Optional[torch.Tensor] = None) -> torch.Tensor:
     """RMSNorm of every row of h (rows, hidden) bf16 as the decode kernels compute it: fp32 normalisation, one
     rounding to bf16, times the bf16 weight (the Hugging Face form); h += delta first, in place, when delta is given.

@@ -17,7 +17,7 @@ import torch
 from torch import nn
 
 from .custom_layers import SparseMoeWrapper
-from .decoder import AttentionDecode, add_rmsnorm
+from .decoder import AttentionDecode, add_rmsnorm, greedy_advance
 
 
 class MixtralOffloadModel(nn.Module):
@@ -51,7 +51,7 @@ class MixtralOffloadModel(nn.Module):
     def step(self) -> torch.Tensor:
         """Feeds self.token at self.position; afterwards self.token is the greedy next token and self.position has
         advanced.  Returns the logits (1, vocab)."""
-        h = self.embed[self.token]                       # (1, hidden), a fresh tensor; the residual stream
+        h = torch.nn.functional.embedding(self.token, self.embed)   # (1, hidden), a fresh tensor; the residual stream
         delta, logits_per_layer = None, []
         for attn, blk in zip(self.attentions, self.blocks):
             x = attn(h, self.position, delta)            # h += previous block's output; attention; x = norm(h) * ln_post
@@ -61,8 +61,7 @@ class MixtralOffloadModel(nn.Module):
         x = add_rmsnorm(h, delta, self.final_norm, self.rms_eps)
         logits = torch.matmul(x, self.lm_head.t())
         self.router_logits = logits_per_layer
-        self.token.copy_(logits.argmax(-1))
-        self.position.add_(1)
+        greedy_advance(logits, self.token, self.position)
         return logits
 
     @torch.inference_mode()
