@@ -239,13 +239,16 @@ __global__ void __launch_bounds__(NORM_THREADS) finalize_add_rmsnorm_router_kern
     // the norm weight and the gate rows of this thread's columns are weights: they are fetched while the launch in
     // front is still finishing
     uint16_t wv[NORM_PER_THREAD], gv[NORM_PER_THREAD][ROUTER_EMAX];
+    int cnt[NORM_PER_THREAD];
 #pragma unroll
     for (int j = 0; j < NORM_PER_THREAD; ++j) {
         const int i = first + j * stride;
         wv[j] = 0;
+        cnt[j] = 0;
 #pragma unroll
         for (int e = 0; e < ROUTER_EMAX; ++e) gv[j][e] = 0;
         if (i < H) {
+            cnt[j] = partial_count(sp, cm, i);
             wv[j] = w[i];
 #pragma unroll
             for (int e = 0; e < ROUTER_EMAX; ++e)
@@ -260,7 +263,7 @@ __global__ void __launch_bounds__(NORM_THREADS) finalize_add_rmsnorm_router_kern
         const int i = first + j * stride;
         v[j] = 0.f;
         if (i < H) {
-            const float y = round_bf16(partial_sum<true>(partial, sp, cm, 0, i, H, H));
+            const float y = round_bf16(partial_sum<true>(partial, cnt[j], 0, i, H, H));
             v[j] = round_bf16(bf16_bits_to_float(h[i]) + y);
             h[i] = float_to_bf16_bits(v[j]);
         }
@@ -369,10 +372,13 @@ __global__ void __launch_bounds__(NORM_THREADS) finalize_scatter_add_rmsnorm_ker
     grid_launch_dependents();
     const int stride = NORM_CTAS * NORM_THREADS, first = blockIdx.x * NORM_THREADS + threadIdx.x;
     uint16_t wv[NORM_PER_THREAD];                 // the norm weight is fetched while the launch in front finishes
+    int cnt0[NORM_PER_THREAD], cnt1[NORM_PER_THREAD];
 #pragma unroll
     for (int j = 0; j < NORM_PER_THREAD; ++j) {
         const int i = first + j * stride;
         wv[j] = i < H ? w[i] : (uint16_t)0;
+        cnt0[j] = i < H ? partial_count(sp, cm, cm.col0[0] + i) : 0;
+        cnt1[j] = i < H ? partial_count(sp, cm, cm.col0[1] + i) : 0;
     }
     grid_dependency_wait();
     float v[NORM_PER_THREAD];
@@ -384,7 +390,7 @@ __global__ void __launch_bounds__(NORM_THREADS) finalize_scatter_add_rmsnorm_ker
         if (i < H) {
             // the launch holds the token's two experts: both sums are requested together
             float s0, s1;
-            partial_sum_pair<true>(partial, sp, cm, 0, cm.col0[0] + i, cm.col0[1] + i, row, row, s0, s1);
+            partial_sum_pair<true>(partial, cnt0[j], cnt1[j], 0, cm.col0[0] + i, cm.col0[1] + i, row, row, s0, s1);
             const float y = round_bf16(round_bf16(round_bf16(s0) * route_w[0]) + round_bf16(round_bf16(s1) * route_w[1]));
             v[j] = round_bf16(bf16_bits_to_float(h[i]) + y);
             h[i] = float_to_bf16_bits(v[j]);
@@ -742,6 +748,18 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(uint16_t* __restrict__
             asm volatile("prefetch.global.L2 [%0];" ::"l"(vb + off));
         }
     }
+    // what does not need the projections: the columns, their pieces and the angle of this thread's pair
+    int col = 0, cnt_a = 0, cnt_b = 0;
+    float sn = 0.f, cs = 1.f;
+    if constexpr (FUSED) {
+        const int which = threadIdx.x >> 6, d = threadIdx.x & 63;     // 0: q, 1: k, 2: v;  pair (d, d + 64)
+        if (which < 3) {
+            col = (which == 0 ? head : (which == 1 ? src.n_heads + kvh : src.n_heads + src.n_kv + kvh)) * HEAD_DIM + d;
+            cnt_a = partial_count(src.sp, src.cm, col);
+            cnt_b = partial_count(src.sp, src.cm, col + HEAD_DIM / 2);
+            if (which < 2) rope_angle(d, pos, src.theta, sn, cs);
+        }
+    }
     grid_dependency_wait();
     int len;                                            // positions read from the cache
     bool fresh = false;                                 // the new position is attended to from shared memory
@@ -749,15 +767,14 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(uint16_t* __restrict__
     if constexpr (FUSED) {
         const bool pos_ok = pos >= 0 && pos < max_len;
         if (!pos_ok && blockIdx.x == 0 && threadIdx.x == 0 && src.error_flag) atomicExch(src.error_flag, 2);
-        const int which = threadIdx.x >> 6, d = threadIdx.x & 63;     // 0: q, 1: k, 2: v;  pair (d, d + 64)
+        const int which = threadIdx.x >> 6, d = threadIdx.x & 63;
         if (which < 3) {
-            const int col = (which == 0 ? head : (which == 1 ? src.n_heads + kvh : src.n_heads + src.n_kv + kvh)) * HEAD_DIM + d;
             float a, b;
-            partial_sum_pair<true>(src.partial, src.sp, src.cm, 0, col, col + HEAD_DIM / 2, src.row, src.row, a, b);
+            partial_sum_pair<true>(src.partial, cnt_a, cnt_b, 0, col, col + HEAD_DIM / 2, src.row, src.row, a, b);
             a = round_bf16(a);
             b = round_bf16(b);
             float o0 = a, o1 = b;
-            if (which < 2) rope_pair(a, b, d, pos, src.theta, o0, o1);
+            if (which < 2) rope_rotate(a, b, sn, cs, o0, o1);
             float* dst = which == 0 ? s_q : (which == 1 ? s_kn : s_vn);
             dst[d] = o0;
             dst[d + HEAD_DIM / 2] = o1;

@@ -603,15 +603,25 @@ __global__ void finalize_linear_kernel(uint16_t* __restrict__ y, const float* __
 __global__ void finalize_silu_mul_kernel(uint16_t* __restrict__ h, const float* __restrict__ partial, int64_t M,
                                          int F, int pairs, int row, int late_trigger, Split sp, ColMap cm) {
     if (!late_trigger) grid_launch_dependents();
+    const int64_t MF = M * F, total = MF * pairs, MR = M * row;
+    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, m = 0;
+    int ca = 0, cb = 0, na = 0, nb = 0;        // columns of the gate and the up sum, and how many pieces each has
+    auto locate = [&] {
+        if (i >= total) return;
+        const int p = (int)(i / MF);
+        m = (i - p * MF) / F;
+        const int f = (int)(i - p * MF - m * F);
+        ca = layer_col0(cm, 2 * p) + f;
+        cb = layer_col0(cm, 2 * p + 1) + f;
+        na = partial_count(sp, cm, ca);
+        nb = partial_count(sp, cm, cb);
+    };
+    locate();                                  // (the first element's while the launch in front is still running)
     grid_dependency_wait();
     if (late_trigger) grid_launch_dependents();
-    const int64_t MF = M * F, total = MF * pairs, MR = M * row;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int p = (int)(i / MF);
-        const int64_t m = (i - p * MF) / F;
-        const int f = (int)(i - p * MF - m * F);
+    for (; i < total; i += (int64_t)gridDim.x * blockDim.x, locate()) {
         float a, b;
-        partial_sum_pair<false>(partial, sp, cm, m, layer_col0(cm, 2 * p) + f, layer_col0(cm, 2 * p + 1) + f, row, MR, a, b);
+        partial_sum_pair<false>(partial, na, nb, m, ca, cb, row, MR, a, b);
         a = round_bf16(a);
         b = round_bf16(b);
         const float act = round_bf16(a / (1.f + __expf(-a)));

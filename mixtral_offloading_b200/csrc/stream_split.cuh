@@ -59,10 +59,9 @@ __device__ __forceinline__ int partial_count(const Split& sp, const ColMap& cm, 
 // few row-sets (the kernels behind hqm_linear / hqm_expert_ffn).  BATCHED = true keeps 24 loads in flight at
 // a time: best for the decode step's small layers, whose K dimension is cut into about twenty pieces.  (Each
 // measured a few percent slower in the other's place.)
+// cnt = partial_count() of the element: some ten divisions, which a kernel does while it waits for the launch in front.
 template <bool BATCHED>
-__device__ __forceinline__ float partial_sum(const float* __restrict__ partial, const Split& sp, const ColMap& cm,
-                                             int64_t m, int col, int row, int64_t MR) {
-    const int cnt = partial_count(sp, cm, col);
+__device__ __forceinline__ float partial_sum(const float* __restrict__ partial, int cnt, int64_t m, int col, int row, int64_t MR) {
     const float* p = partial + m * row + col;
     float v = 0.f;
     if constexpr (!BATCHED) {
@@ -83,10 +82,8 @@ __device__ __forceinline__ float partial_sum(const float* __restrict__ partial, 
 // Two elements of the same row at once (a rotation pair, the gate and up halves of an FFN, the two experts of a
 // token): the row-sets of both are requested together, so the pair costs the round trips of one.
 template <bool BATCHED>
-__device__ __forceinline__ void partial_sum_pair(const float* __restrict__ partial, const Split& sp, const ColMap& cm,
-                                                 int64_t m, int col_a, int col_b, int row, int64_t MR, float& out_a,
-                                                 float& out_b) {
-    const int cnt_a = partial_count(sp, cm, col_a), cnt_b = partial_count(sp, cm, col_b);
+__device__ __forceinline__ void partial_sum_pair(const float* __restrict__ partial, int cnt_a, int cnt_b, int64_t m, int col_a,
+                                                 int col_b, int row, int64_t MR, float& out_a, float& out_b) {
     const float* pa = partial + m * row + col_a;
     const float* pb = partial + m * row + col_b;
     float va = 0.f, vb = 0.f;
@@ -116,6 +113,18 @@ __device__ __forceinline__ void partial_sum_pair(const float* __restrict__ parti
     }
     out_a = va;
     out_b = vb;
+}
+
+template <bool BATCHED>
+__device__ __forceinline__ float partial_sum(const float* __restrict__ partial, const Split& sp, const ColMap& cm,
+                                             int64_t m, int col, int row, int64_t MR) {
+    return partial_sum<BATCHED>(partial, partial_count(sp, cm, col), m, col, row, MR);
+}
+template <bool BATCHED>
+__device__ __forceinline__ void partial_sum_pair(const float* __restrict__ partial, const Split& sp, const ColMap& cm,
+                                                 int64_t m, int col_a, int col_b, int row, int64_t MR, float& out_a,
+                                                 float& out_b) {
+    partial_sum_pair<BATCHED>(partial, partial_count(sp, cm, col_a), partial_count(sp, cm, col_b), m, col_a, col_b, row, MR, out_a, out_b);
 }
 
 // The split the CONSUMERS of a launch's sums see.  A TMA-staged launch finishes its sums itself (one fp32 row-set,
