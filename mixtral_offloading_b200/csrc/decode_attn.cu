@@ -196,8 +196,11 @@ __global__ void __launch_bounds__(NORM_THREADS) finalize_add_rmsnorm_kernel(uint
     __shared__ float red[32];
     __shared__ float mine;
     grid_launch_dependents();
-    grid_dependency_wait();
     const int stride = NORM_CTAS * NORM_THREADS, first = blockIdx.x * NORM_THREADS + threadIdx.x;
+    int cnt[NORM_PER_THREAD];                    // (while the launch in front finishes)
+#pragma unroll
+    for (int j = 0; j < NORM_PER_THREAD; ++j) cnt[j] = first + j * stride < H ? partial_count(sp, cm, first + j * stride) : 0;
+    grid_dependency_wait();
     float v[NORM_PER_THREAD];
     float ss = 0.f;
 #pragma unroll
@@ -205,7 +208,7 @@ __global__ void __launch_bounds__(NORM_THREADS) finalize_add_rmsnorm_kernel(uint
         const int i = first + j * stride;
         v[j] = 0.f;
         if (i < H) {
-            const float y = round_bf16(partial_sum<true>(partial, sp, cm, 0, i, H, H));
+            const float y = round_bf16(partial_sum<true>(partial, cnt[j], 0, i, H, H));
             v[j] = round_bf16(bf16_bits_to_float(h[i]) + y);
             h[i] = float_to_bf16_bits(v[j]);
         }
@@ -557,6 +560,22 @@ __global__ void __launch_bounds__(NORM_THREADS) add_f32_rmsnorm_kernel(uint16_t*
     }
 }
 
+__device__ __forceinline__ void rope_angle(int d, int pos, float theta, float& sn, float& cs) {
+    const float inv_freq = powf(theta, -(float)(2 * d) / (float)HEAD_DIM);
+    sincosf((float)pos * inv_freq, &sn, &cs);
+    sn = round_bf16(sn);
+    cs = round_bf16(cs);
+}
+__device__ __forceinline__ void rope_rotate(float a, float b, float sn, float cs, float& o0, float& o1) {
+    o0 = round_bf16(round_bf16(a * cs) + round_bf16(-b * sn));
+    o1 = round_bf16(round_bf16(b * cs) + round_bf16(a * sn));
+}
+__device__ __forceinline__ void rope_pair(float a, float b, int d, int pos, float theta, float& o0, float& o1) {
+    float sn, cs;
+    rope_angle(d, pos, theta, sn, cs);
+    rope_rotate(a, b, sn, cs, o0, o1);
+}
+
 // One CTA of 64 threads per head of the [q | k | v] partial row: sums the partials, rounds to bf16 (the
 // projection's output), rotates q and k by the position's angles and writes q to `qbuf`, k and v to the
 // caches at `pos`.  A position outside the cache sets the error flag and writes nothing.
@@ -567,27 +586,22 @@ __global__ void __launch_bounds__(64) finalize_qkv_rope_kernel(uint16_t* __restr
                                                                int n_kv, int max_len, float theta, int row, Split sp,
                                                                ColMap cm, int* __restrict__ error_flag) {
     grid_launch_dependents();
-    grid_dependency_wait();
     const int head = blockIdx.x, d = threadIdx.x;        // d in [0, 64): pairs (d, d + 64)
+    const int col = head * HEAD_DIM + d;                 // q heads, then k heads, then v heads: the row's order
+    const int cnt_a = partial_count(sp, cm, col), cnt_b = partial_count(sp, cm, col + HEAD_DIM / 2);
+    grid_dependency_wait();
     const int pos = pos_ptr[0];
     if (pos < 0 || pos >= max_len) {
         if (d == 0 && head == 0 && error_flag) atomicExch(error_flag, 2);
         return;
     }
-    const int col = head * HEAD_DIM + d;                 // q heads, then k heads, then v heads: the row's order
     float a, b;
-    partial_sum_pair<true>(partial, sp, cm, 0, col, col + HEAD_DIM / 2, row, row, a, b);
+    partial_sum_pair<true>(partial, cnt_a, cnt_b, 0, col, col + HEAD_DIM / 2, row, row, a, b);
     a = round_bf16(a);
     b = round_bf16(b);
     float o0 = a, o1 = b;
     if (head < n_heads + n_kv) {
-        const float inv_freq = powf(theta, -(float)(2 * d) / (float)HEAD_DIM);
-        float sn, cs;
-        sincosf((float)pos * inv_freq, &sn, &cs);
-        sn = round_bf16(sn);
-        cs = round_bf16(cs);
-        o0 = round_bf16(round_bf16(a * cs) + round_bf16(-b * sn));
-        o1 = round_bf16(round_bf16(b * cs) + round_bf16(a * sn));
+        rope_pair(a, b, d, pos, theta, o0, o1);
     }
     uint16_t* dst;
     if (head < n_heads) dst = qbuf + head * HEAD_DIM;
@@ -618,22 +632,6 @@ struct QkvSource {                 // FUSED only: where q, k, v of this token co
 };
 
 // rotate-half RoPE of the pair (a, b) = (t[d], t[d + 64]) at position pos, bf16 arithmetic as Hugging Face does it
-__device__ __forceinline__ void rope_angle(int d, int pos, float theta, float& sn, float& cs) {
-    const float inv_freq = powf(theta, -(float)(2 * d) / (float)HEAD_DIM);
-    sincosf((float)pos * inv_freq, &sn, &cs);
-    sn = round_bf16(sn);
-    cs = round_bf16(cs);
-}
-__device__ __forceinline__ void rope_rotate(float a, float b, float sn, float cs, float& o0, float& o1) {
-    o0 = round_bf16(round_bf16(a * cs) + round_bf16(-b * sn));
-    o1 = round_bf16(round_bf16(b * cs) + round_bf16(a * sn));
-}
-__device__ __forceinline__ void rope_pair(float a, float b, int d, int pos, float theta, float& o0, float& o1) {
-    float sn, cs;
-    rope_angle(d, pos, theta, sn, cs);
-    rope_rotate(a, b, sn, cs, o0, o1);
-}
-
 // The end of a greedy step: token = index of the largest of `vocab` bf16 logits (the first of equal ones; a NaN is larger
 // than everything), position += 1.  One CTA: 64 KB of logits that the launch in front has just written are one round trip
 // to L2 for 1024 threads.  (A reduction over the whole chip, a copy and an addition before: 15 us, 6 now.)
@@ -691,7 +689,7 @@ __global__ void __launch_bounds__(256) rope_append_rows_kernel(uint16_t* __restr
     }
     constexpr int HALF = HEAD_DIM / 2;
     uint16_t* qt = q + (int64_t)t * n_heads * HEAD_DIM;
-    static_assert(256 % HALF == 0, "a thread keeps its column: one angle (500 tokens: 8 us with one for every pair, 4 so)");
+    static_assert(256 % HALF == 0, "a thread keeps its column: one angle (500 tokens: 8.2 us with one for every pair, 6.5 so)");
     float sn, cs;
     rope_angle(threadIdx.x % HALF, pos, theta, sn, cs);
 #pragma unroll 4

@@ -586,12 +586,19 @@ gemv_stream_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, 
 __global__ void finalize_linear_kernel(uint16_t* __restrict__ y, const float* __restrict__ partial,
                                        const uint16_t* __restrict__ bias, int64_t M, int row, Split sp, ColMap cm) {
     grid_launch_dependents();
-    grid_dependency_wait();
     const int64_t MR = M * row;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < MR; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t m = i / row;
-        const int n = (int)(i - m * row);
-        float v = partial_sum<false>(partial, sp, cm, m, n, row, MR);
+    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, m = 0;
+    int n = 0, cnt = 0;
+    auto locate = [&] {
+        if (i >= MR) return;
+        m = i / row;
+        n = (int)(i - m * row);
+        cnt = partial_count(sp, cm, n);
+    };
+    locate();                                  // (the first element's while the launch in front is still running)
+    grid_dependency_wait();
+    for (; i < MR; i += (int64_t)gridDim.x * blockDim.x, locate()) {
+        float v = partial_sum<false>(partial, cnt, m, n, row, MR);
         if (bias) v += bf16_bits_to_float(bias[n]);
         y[i] = float_to_bf16_bits(v);
     }
@@ -636,11 +643,19 @@ __global__ void finalize_scatter_kernel(uint16_t* __restrict__ out, const float*
                                         const int32_t* __restrict__ token_idx, const float* __restrict__ route_w,
                                         int64_t M, int H, int row, int accumulate, Split sp, ColMap cm) {
     grid_launch_dependents();
-    grid_dependency_wait();
     const int64_t MH = M * H, MR = M * row;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < MH; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t m = i / H;
-        const int n = (int)(i - m * H);
+    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, m = 0;
+    int n = 0, cnt[STREAM_MAX_LAYERS];
+    auto locate = [&] {
+        if (i >= MH) return;
+        m = i / H;
+        n = (int)(i - m * H);
+#pragma unroll
+        for (int l = 0; l < STREAM_MAX_LAYERS; ++l) cnt[l] = l < cm.count ? partial_count(sp, cm, cm.col0[l] + n) : 0;
+    };
+    locate();                                  // (the first element's while the launch in front is still running)
+    grid_dependency_wait();
+    for (; i < MH; i += (int64_t)gridDim.x * blockDim.x, locate()) {
         const int64_t tk = token_idx ? token_idx[m] : m;
         uint16_t* dst = out + tk * H + n;
         float acc = accumulate ? bf16_bits_to_float(*dst) : 0.f;
@@ -648,7 +663,7 @@ __global__ void finalize_scatter_kernel(uint16_t* __restrict__ out, const float*
         for (int l = 0; l < STREAM_MAX_LAYERS; ++l) {
             if (l < cm.count) {
                 const float wgt = route_w ? route_w[l * M + m] : 1.f;
-                const float v = round_bf16(round_bf16(partial_sum<false>(partial, sp, cm, m, cm.col0[l] + n, row, MR)) * wgt);
+                const float v = round_bf16(round_bf16(partial_sum<false>(partial, cnt[l], m, cm.col0[l] + n, row, MR)) * wgt);
                 acc = (l == 0 && !accumulate) ? v : round_bf16(acc + v);
             }
         }

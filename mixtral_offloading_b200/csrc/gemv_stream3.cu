@@ -238,13 +238,24 @@ gemv_stream3_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x,
 __global__ void finalize3_kernel(uint16_t* __restrict__ y, const float* __restrict__ partial,
                                  const uint16_t* __restrict__ bias, int64_t MN, int N, Split3 sp) {
     grid_launch_dependents();
-    grid_dependency_wait();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < MN; i += (int64_t)gridDim.x * blockDim.x) {
-        const int n = (int)(i % N);
+    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int n = 0, cnt = 0;
+    auto locate = [&] {
+        n = (int)(i % N);
         const uint32_t rho = (uint32_t)((n / 10) % sp.P3);
-        const int cnt = sp.owner(rho * sp.PT + sp.PT - 1) - sp.owner(rho * sp.PT) + 1;
+        cnt = sp.owner(rho * sp.PT + sp.PT - 1) - sp.owner(rho * sp.PT) + 1;
+    };
+    locate();                                  // (the first element's while the launch in front is still running)
+    grid_dependency_wait();
+    for (; i < MN; i += (int64_t)gridDim.x * blockDim.x, locate()) {
         float v = 0.f;
-        for (int s = 0; s < cnt; ++s) v += partial[s * MN + i];
+        for (int s = 0; s < cnt; s += 8) {     // eight pieces on their way at a time
+            float a[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[j] = s + j < cnt ? partial[(s + j) * MN + i] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v += a[j];
+        }
         if (bias) v += bf16_bits_to_float(bias[n]);
         y[i] = float_to_bf16_bits(v);
     }
