@@ -1384,16 +1384,13 @@ static int gg_sm_count() {
     return c;
 }
 
-static constexpr int UK_MIN = 128;
 bool gg_supported(const hqm_weight* w, int G, int C) {
-    if (!meta_uniform(w) || tma_encode_entry() == nullptr) return false;
-    const int per = w->nbits == 3 ? 8 : codes_per_word(w->nbits), g = w->group_size;
-    if (w->nbits == 3) {                     // members in whole blocks of 16, or all of them (and the last rows) in one
-        const Members3 m = Members3::of(w, G);
-        if (m.full < 1 || m.full + (m.left ? 1 : 0) > 16 ? m.full < 1 || m.left != 0 || m.full % 16 != 0 : false) return false;
-    }
-    if (g % 16 != 0 || G % per != 0 || w->K % 64 != 0 || w->K < UK_MIN || C < 1) return false;
-    if ((int64_t)G * w->K >= ((int64_t)1 << 31)) return false;
+    if (tma_encode_entry() == nullptr || C < 1 || w->K % 64 != 0 || w->K < 128) return false;
+    if (w->nbits != 3) return tensor_maps_ok(w, G);
+    if (!meta_uniform(w) || w->group_size % 16 != 0 || G % 8 != 0 || (int64_t)G * w->K >= ((int64_t)1 << 31)) return false;
+    // members in whole blocks of 16, or all of them (and the last rows) in one
+    const Members3 m = Members3::of(w, G);
+    if (m.full < 1 || (m.full + (m.left ? 1 : 0) > 16 && (m.left != 0 || m.full % 16 != 0))) return false;
     auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     return a16(w->W_q) && a16(w->scale_q) && a16(w->zero_q) && a16(w->ms_scale) && a16(w->mz_scale) && a16(w->ms_zero) &&
            a16(w->mz_zero);

@@ -612,8 +612,9 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// Layers whose tensor maps can be encoded.
-bool maps_ok(const hqm_weight* w, int G) {
+}  // namespace
+
+bool tensor_maps_ok(const hqm_weight* w, int G) {
     if ((w->nbits != 2 && w->nbits != 4) || !meta_uniform(w)) return false;
     const int per = codes_per_word(w->nbits);
     if (w->group_size % 16 != 0 || w->K % 16 != 0 || w->K < KC || G % per != 0) return false;
@@ -622,8 +623,10 @@ bool maps_ok(const hqm_weight* w, int G) {
     return a16(w->W_q) && a16(w->scale_q) && a16(w->zero_q) && a16(w->ms_scale) && a16(w->mz_scale) && a16(w->ms_zero) &&
            a16(w->mz_zero);
 }
+
+namespace {
 // Layers this file's kernel takes: whole passes whose meta columns do not wrap.
-bool tma_shape_ok(const hqm_weight* w, int G, int C) { return maps_ok(w, G) && w->K % KC == 0 && C % KC == 0; }
+bool tma_shape_ok(const hqm_weight* w, int G, int C) { return tensor_maps_ok(w, G) && w->K % KC == 0 && C % KC == 0; }
 
 // The three tensor maps of a layer: codes as (K, P, group_size) bytes with box (128, 1, 16) and the 128-byte
 // swizzle; scale_q and zero_q as (K, G, 1) bytes with box (128, PER, 1).
@@ -764,7 +767,7 @@ bool prepare_kernel(size_t smem) {
 
 // The tensor maps of a layer for the other TMA users (three CUtensorMaps; the codes' box is 128 columns x 16 members).
 bool stream_cached_maps(const hqm_weight* w, int G, void* out3) {
-    return maps_ok(w, G) && cached_maps(w, G, static_cast<CUtensorMap*>(out3));
+    return tensor_maps_ok(w, G) && cached_maps(w, G, static_cast<CUtensorMap*>(out3));
 }
 
 // The maps of a 3-bit layer: words as (K, P3, members) with box (128, 1, up to 16), scale and zero bytes as (K, G) with box
@@ -968,7 +971,7 @@ int hqm_expert_table_build(void* host_out, const hqm_weight* weights, int32_t n_
         int G, C;
         const int rc = check_weight(&weights[i], &G, &C);
         if (rc != HQM_OK) return rc;
-        if (encode_fn() != nullptr && maps_ok(&weights[i], G) &&
+        if (encode_fn() != nullptr && tensor_maps_ok(&weights[i], G) &&
             !encode_maps(&weights[i], G, reinterpret_cast<CUtensorMap*>(out[i].maps))) {
             set_error("expert_table_build: cuTensorMapEncodeTiled failed for weight %d (%dx%d, %d bit)", i, weights[i].N,
                       weights[i].K, weights[i].nbits);

@@ -96,6 +96,8 @@ struct Members3 {
         return Members3{P3, rows / P3, rows % P3};
     }
 };
+// gemv_tma.cu — 2- and 4-bit layers whose tensor maps can be encoded: what every kernel that copies tiles of them has to ask.
+bool tensor_maps_ok(const hqm_weight* w, int G);
 bool stream_cached_maps3(const hqm_weight* w, int G, const Members3& m, void* out4);      // words, scales, zeros, left-over words
 // gemv_stream3.cu — the weight-streaming path for 3-bit layers.
 struct Stream3Plan {
