@@ -106,6 +106,10 @@ __device__ __forceinline__ uint32_t ld_stream_4(const void* p) {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Asks for the line of p in L2, the point where all SMs' writes meet: unlike a load it may stand in front of
+// grid_dependency_wait() for memory that a kernel in front may still write (the load behind the wait is ld.global.cg).
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // HQM_NO_OVERLAP=1 in the environment turns launch_overlapped() into a plain launch.
 bool overlap_enabled();
 

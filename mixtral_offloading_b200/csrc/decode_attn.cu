@@ -133,13 +133,14 @@ __global__ void __launch_bounds__(256) add_rmsnorm_rows_vec_kernel(uint16_t* __r
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         const int i = 8 * (threadIdx.x + 256 * c);
-        if (i < H) wv[c] = __ldg(reinterpret_cast<const uint4*>(w + i));
+        if (i < H && (threadIdx.x & 7) == 0) prefetch_l2(w + i);
     }
     grid_dependency_wait();
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         const int i = 8 * (threadIdx.x + 256 * c);
         if (i < H) {
+            wv[c] = __ldcg(reinterpret_cast<const uint4*>(w + i));
             hv[c] = *reinterpret_cast<const uint4*>(h + row + i);
             if (delta) dv[c] = *reinterpret_cast<const uint4*>(delta + row + i);
         }

@@ -57,11 +57,15 @@ router_short_rows_kernel(uint16_t* __restrict__ logits_out, float* __restrict__ 
     __shared__ float s_part[16][8];
     grid_launch_dependents();
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, t = blockIdx.x, k = 8 * threadIdx.x;
+    // The gate may be the output of the kernel in front (a conversion to bf16): what can be done before the wait is to ask
+    // for its rows in L2, where the kernel in front writes them too.
+    if (k < K && (lane & 7) == 0)
+        for (int e = 0; e < E; ++e) prefetch_l2(gate_w + (int64_t)e * K + k);
+    grid_dependency_wait();
     uint4 gv[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e)                               // (weights: no kernel in front writes them)
-        gv[e] = e < E && k < K ? __ldg(reinterpret_cast<const uint4*>(gate_w + (int64_t)e * K + k)) : make_uint4(0u, 0u, 0u, 0u);
-    grid_dependency_wait();
+    for (int e = 0; e < 8; ++e)
+        gv[e] = e < E && k < K ? __ldcg(reinterpret_cast<const uint4*>(gate_w + (int64_t)e * K + k)) : make_uint4(0u, 0u, 0u, 0u);
     const uint4 xv = k < K ? *reinterpret_cast<const uint4*>(x + (int64_t)t * K + k) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll
