@@ -74,7 +74,10 @@ int hqm_device_error(void);
  * scratch are touched only after everything in front has completed.  The consequence for the caller: the
  * weight tensors of a call (W_q, scale_q, zero_q and the fp16 meta) must not be written by the work that
  * immediately precedes the call on the same stream; order such writes with an event, a copy or a
- * synchronisation, as a cache swap does.  hqm_set_overlap(0) switches to plain launches (so does
+ * synchronisation, as a cache swap does.  hqm_attn_decode, hqm_decode_layer and hqm_decode_layer_ep read three
+ * more tensors that early: the gate, the norm weights and the position.  (A decode step that advances the position
+ * at its end and looks its token up at the start of the next has that order.)  The gate of the other calls and the
+ * norm weight of hqm_add_rmsnorm* may come from the work right in front.  hqm_set_overlap(0) switches to plain launches (so does
  * HQM_NO_OVERLAP=1 in the environment at load time), hqm_set_overlap(1) switches back; returns the previous
  * setting.  Process wide. */
 int hqm_set_overlap(int on);
