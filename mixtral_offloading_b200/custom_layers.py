@@ -100,7 +100,7 @@ class HQQLinearTritonSavable(nn.Module):
             mm["scale"], mm["zero"] = ms.to(torch.float16).contiguous(), mz.to(torch.float16).contiguous()
         self.meta = meta
         self.ready = True
-        self._desc = None
+        self._drop_descriptor()
 
     def repack(self):
         """custom_layers.py:41-47: bring a tensor packed over the (group_size, G*K) code matrix
@@ -112,13 +112,18 @@ class HQQLinearTritonSavable(nn.Module):
         codes = packing.UNPACK[self.meta["packing"]](self.W_q)
         codes = codes.reshape((-1, K))[:N]
         self.W_q = packing.PACK[self.meta["packing"]](codes)
-        self._desc = None
+        self._drop_descriptor()
 
     @classmethod
     def get_hqq_meta(cls, linear_shape, quant_config):
         """custom_layers.py:118-134.  linear_shape is (in_features, out_features) as passed to
         nn.Linear; the reference quantises a throw-away layer to harvest this dictionary."""
         return meta_template((linear_shape[1], linear_shape[0]), quant_config)
+
+    def _drop_descriptor(self):
+        """Forget what was derived from the tensors (they were replaced): the descriptor and native/host.cpp's plan."""
+        self._desc = None
+        self.__dict__.pop("_plan", None)
 
     # ---------------------------------------------------------------- compute
     def descriptor(self) -> _cabi.HqmWeight:
@@ -233,7 +238,7 @@ class HQQLinearTritonSavable(nn.Module):
             node[path[-1]] = state_dict.pop(prefix + key)
         self.meta["quant_scale"] = self.meta["quant_zero"] = True
         self.ready = True
-        self._desc = None
+        self._drop_descriptor()
         if self.W_q.is_cuda:
             self.repack()
 

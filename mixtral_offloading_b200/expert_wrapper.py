@@ -87,5 +87,5 @@ class MixtralExpertWrapper(nn.Module):
             patched.W_q = views[id(states["W_q"])]
             patched.meta = repoint(states["meta"])
             patched.bias = None if states["bias"] is None else views[id(states["bias"])]
-            patched._desc = None
+            patched._drop_descriptor()
         return layer, storage

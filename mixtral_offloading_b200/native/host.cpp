@@ -24,7 +24,7 @@
 namespace {
 
 struct Names {
-    PyObject *dict, *W_q, *meta, *bias, *plan, *ready, *scale_q, *zero_q, *meta_scale, *meta_zero, *scale, *zero, *modules, *w1, *w2, *w3, *axis;
+    PyObject *dict, *W_q, *meta, *bias, *plan, *desc, *ready, *scale_q, *zero_q, *meta_scale, *meta_zero, *scale, *zero, *modules, *w1, *w2, *w3, *axis;
 } N;
 
 PyObject* g_scratch = nullptr;        // custom_layers._SCRATCH: {("cuda", index): uint8 tensor}
@@ -32,7 +32,9 @@ PyObject* g_grow = nullptr;           // custom_layers._scratch(device, bytes)
 PyObject* g_keys[64];                 // ("cuda", index)
 
 // A layer's descriptor (and with it the addresses it was made from) and the workspace of its last row count, as linear
-// layer and as w1 of an expert; kept in the layer's __dict__.  A copied or pickled layer gets None and makes its own.
+// layer and as w1 of an expert; kept in the layer's __dict__ for as long as the layer keeps its own descriptor (_desc): the
+// addresses alone do not tell a layer that was quantized again, in another format, into recycled memory.  A copied or pickled
+// layer gets None and makes its own.
 struct Plan {
     PyObject_HEAD
     hqm_weight w;
@@ -63,8 +65,8 @@ Plan* plan_of(PyObject* layer, PyObject* dict) {
     if (item(dict, N.ready) != Py_True || ms == nullptr || mz == nullptr) return nullptr;
     const void* at[7] = {address(item(dict, N.W_q)),    address(item(meta, N.scale_q)), address(item(meta, N.zero_q)), address(item(ms, N.scale)),
                          address(item(ms, N.zero)), address(item(mz, N.scale)),     address(item(mz, N.zero))};
-    PyObject* kept = item(dict, N.plan);
-    if (kept != nullptr && Py_TYPE(kept) == &PlanType) {
+    PyObject *kept = item(dict, N.plan), *desc = item(dict, N.desc);
+    if (kept != nullptr && Py_TYPE(kept) == &PlanType && desc != nullptr && desc != Py_None) {
         Plan* p = reinterpret_cast<Plan*>(kept);
         if (p->w.W_q == at[0] && p->w.scale_q == at[1] && p->w.zero_q == at[2] && p->w.ms_scale == at[3] && p->w.mz_scale == at[4] &&
             p->w.ms_zero == at[5] && p->w.mz_zero == at[6])
@@ -295,7 +297,7 @@ PyMODINIT_FUNC PyInit__host(void) {
     struct {
         PyObject** to;
         const char* name;
-    } all[] = {{&N.dict, "__dict__"}, {&N.W_q, "W_q"},     {&N.meta, "meta"},           {&N.bias, "bias"},           {&N.plan, "_plan"}, {&N.ready, "ready"},
+    } all[] = {{&N.dict, "__dict__"}, {&N.W_q, "W_q"},     {&N.meta, "meta"},           {&N.bias, "bias"},           {&N.plan, "_plan"}, {&N.desc, "_desc"}, {&N.ready, "ready"},
                {&N.scale_q, "scale_q"}, {&N.zero_q, "zero_q"}, {&N.meta_scale, "meta_scale"}, {&N.meta_zero, "meta_zero"}, {&N.scale, "scale"}, {&N.zero, "zero"},
                {&N.modules, "_modules"}, {&N.w1, "w1"},    {&N.w2, "w2"},               {&N.w3, "w3"}, {&N.axis, "axis"}};
     for (auto& a : all)
