@@ -34,7 +34,7 @@ PyObject* g_keys[64];                 // ("cuda", index)
 // A layer's descriptor (and with it the addresses it was made from) and the workspace of its last row count, as linear
 // layer and as w1 of an expert; kept in the layer's __dict__ for as long as the layer keeps its own descriptor (_desc): the
 // addresses alone do not tell a layer that was quantized again, in another format, into recycled memory.  A copied or pickled
-// layer gets None and makes its own.
+// layer gets None and makes its own.  The descriptor is never changed once it is made.
 struct Plan {
     PyObject_HEAD
     hqm_weight w;
@@ -56,9 +56,29 @@ PyObject* item(PyObject* dict, PyObject* key) {
     if (v == nullptr) PyErr_Clear();
     return v;
 }
+// An owned reference.  A layer's dictionary may drop what it holds while a call is under way (another thread runs wherever
+// Python code does: a workspace that grows, a descriptor that is made), so the call holds what it uses.
+template <typename T>
+struct Held {
+    T* p;
+    explicit Held(T* owned = nullptr) : p(owned) {}
+    Held(const Held&) = delete;
+    Held& operator=(const Held&) = delete;
+    ~Held() { Py_XDECREF(reinterpret_cast<PyObject*>(p)); }
+    T* operator->() const { return p; }
+    explicit operator bool() const { return p != nullptr; }
+    void take(T* owned) {
+        Py_XDECREF(reinterpret_cast<PyObject*>(p));
+        p = owned;
+    }
+};
+PyObject* own(PyObject* borrowed) {
+    Py_XINCREF(borrowed);
+    return borrowed;
+}
 const void* address(PyObject* t) { return t != nullptr && THPVariable_Check(t) ? THPVariable_Unpack(t).const_data_ptr() : nullptr; }
 
-// The plan of a layer whose tensors are where they were when its descriptor was made; null: not to be had here.
+// The plan of a layer whose tensors are where they were when its descriptor was made (new reference); null: not to be had here.
 Plan* plan_of(PyObject* layer, PyObject* dict) {
     PyObject* meta = item(dict, N.meta);
     PyObject *ms = item(meta, N.meta_scale), *mz = item(meta, N.meta_zero);
@@ -70,7 +90,7 @@ Plan* plan_of(PyObject* layer, PyObject* dict) {
         Plan* p = reinterpret_cast<Plan*>(kept);
         if (p->w.W_q == at[0] && p->w.scale_q == at[1] && p->w.zero_q == at[2] && p->w.ms_scale == at[3] && p->w.mz_scale == at[4] &&
             p->w.ms_zero == at[5] && p->w.mz_zero == at[6])
-            return p;
+            return reinterpret_cast<Plan*>(own(kept));
     }
     PyObject* axis = item(meta, N.axis);
     if (axis == nullptr || !PyLong_Check(axis) || PyLong_AsLong(axis) != 0) return nullptr;
@@ -86,8 +106,10 @@ Plan* plan_of(PyObject* layer, PyObject* dict) {
             memcpy(&p->w, view.buf, sizeof(hqm_weight));
             p->linear_rows = p->expert_rows = -1;
             p->linear_bytes = p->f16_bytes = p->expert_bytes = 0;
-            if (PyDict_SetItem(dict, N.plan, reinterpret_cast<PyObject*>(p)) != 0) p = nullptr;
-            else Py_DECREF(p);                             // the layer's __dict__ holds it
+            if (PyDict_SetItem(dict, N.plan, reinterpret_cast<PyObject*>(p)) != 0) {
+                Py_DECREF(p);
+                p = nullptr;
+            }
         }
         PyBuffer_Release(&view);
     }
@@ -147,12 +169,11 @@ at::Tensor result(const at::Tensor& x, int64_t n) {
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 2) return PyErr_Format(PyExc_TypeError, "linear(layer, x)");
     try {
-        PyObject* dict = dict_of(args[0]);
-        Plan* p = dict == nullptr ? nullptr : plan_of(args[0], dict);
-        PyObject* bias = item(dict, N.bias);
-        Py_XDECREF(dict);                                  // (the layer holds it, and it the plan)
+        Held<PyObject> dict(dict_of(args[0]));
+        Held<Plan> p(dict ? plan_of(args[0], dict.p) : nullptr);
+        Held<PyObject> bias(own(item(dict.p, N.bias)));
         int64_t rows = 0;
-        const at::Tensor* x = p == nullptr ? nullptr : rows_of(args[1], p->w.K, &rows);
+        const at::Tensor* x = p ? rows_of(args[1], p->w.K, &rows) : nullptr;
         if (x == nullptr) Py_RETURN_NONE;
         c10::InferenceMode guard;
         const auto type = x->scalar_type();
@@ -172,12 +193,11 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         void* ws = nullptr;
         if (bytes && (ws = scratch(*x, bytes, &have)) == nullptr) Py_RETURN_NONE;
         at::Tensor y = result(*x, p->w.N);
-        const hqm_weight w = p->w;                         // (without the lock another thread may replace the plan)
-        const uint16_t* b = static_cast<const uint16_t*>(address(bias));
+        const uint16_t* b = static_cast<const uint16_t*>(address(bias.p));
         int rc;
         Py_BEGIN_ALLOW_THREADS
         rc = (f16 ? hqm_linear_f16 : hqm_linear)(static_cast<uint16_t*>(y.data_ptr()), static_cast<const uint16_t*>(x->const_data_ptr()), rows,
-                                                 &w, b, ws, bytes, c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
+                                                 &p->w, b, ws, bytes, c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
         Py_END_ALLOW_THREADS
         if (rc < 0) Py_RETURN_NONE;
         if (y.scalar_type() != type) y = y.to(type);
@@ -192,22 +212,20 @@ PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 2) return PyErr_Format(PyExc_TypeError, "dequantize(layer, code)");
     try {
         const long code = PyLong_AsLong(args[1]);
-        PyObject* dict = dict_of(args[0]);
-        Plan* p = dict == nullptr ? nullptr : plan_of(args[0], dict);
-        PyObject* wq = item(dict, N.W_q);
-        Py_XDECREF(dict);
-        if (p == nullptr || code < 0 || code > 2) {
+        Held<PyObject> dict(dict_of(args[0]));
+        Held<Plan> p(dict ? plan_of(args[0], dict.p) : nullptr);
+        Held<PyObject> wq(own(item(dict.p, N.W_q)));
+        if (!p || address(wq.p) != p->w.W_q || code < 0 || code > 2) {
             PyErr_Clear();
             Py_RETURN_NONE;
         }
-        const at::Tensor& like = THPVariable_Unpack(wq);
+        const at::Tensor& like = THPVariable_Unpack(wq.p);
         if (like.device().index() != c10::cuda::current_device()) Py_RETURN_NONE;
         c10::InferenceMode guard;
         at::Tensor out = at::empty({p->w.N, p->w.K}, like.options().dtype(code == 0 ? at::kBFloat16 : code == 1 ? at::kHalf : at::kFloat));
-        const hqm_weight w = p->w;
         int rc;
         Py_BEGIN_ALLOW_THREADS
-        rc = hqm_dequantize(out.data_ptr(), (int)code, &w, c10::cuda::getCurrentCUDAStream(like.device().index()).stream());
+        rc = hqm_dequantize(out.data_ptr(), (int)code, &p->w, c10::cuda::getCurrentCUDAStream(like.device().index()).stream());
         Py_END_ALLOW_THREADS
         if (rc < 0) Py_RETURN_NONE;
         return THPVariable_Wrap(std::move(out));
@@ -217,22 +235,20 @@ PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // The three plans of an expert module.
-bool expert_plans(PyObject* module, Plan* (&p)[3]) {
-    PyObject* dict = dict_of(module);
-    PyObject* modules = item(dict, N.modules);
-    Py_XDECREF(dict);
+bool expert_plans(PyObject* module, Held<Plan> (&p)[3]) {
+    Held<PyObject> dict(dict_of(module));
+    Held<PyObject> modules(own(item(dict.p, N.modules)));
     PyObject* names[3] = {N.w1, N.w2, N.w3};
     for (int i = 0; i < 3; ++i) {
-        PyObject* layer = item(modules, names[i]);
-        PyObject* d = layer == nullptr ? nullptr : dict_of(layer);
-        p[i] = d == nullptr ? nullptr : plan_of(layer, d);
-        Py_XDECREF(d);
-        if (p[i] == nullptr) return false;
+        Held<PyObject> layer(own(item(modules.p, names[i])));
+        Held<PyObject> d(layer ? dict_of(layer.p) : nullptr);
+        p[i].take(d ? plan_of(layer.p, d.p) : nullptr);
+        if (!p[i]) return false;
     }
     return true;
 }
 
-int run_expert(Plan* (&p)[3], const at::Tensor& x, int64_t rows, const int32_t* idx, const float* w, uint16_t* out, int accumulate) {
+int run_expert(const Held<Plan> (&p)[3], const at::Tensor& x, int64_t rows, const int32_t* idx, const float* w, uint16_t* out, int accumulate) {
     if (p[0]->expert_rows != rows) {
         p[0]->expert_bytes = hqm_expert_ffn_scratch_bytes(rows, &p[0]->w, &p[1]->w, &p[2]->w);
         p[0]->expert_rows = rows;
@@ -240,10 +256,9 @@ int run_expert(Plan* (&p)[3], const at::Tensor& x, int64_t rows, const int32_t* 
     size_t have = 0;
     void* ws = scratch(x, p[0]->expert_bytes, &have);
     if (ws == nullptr) return -1;
-    const hqm_weight w1 = p[0]->w, w2 = p[1]->w, w3 = p[2]->w;
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = hqm_expert_ffn(out, static_cast<const uint16_t*>(x.const_data_ptr()), rows, idx, w, accumulate, &w1, &w2, &w3, ws, have,
+    rc = hqm_expert_ffn(out, static_cast<const uint16_t*>(x.const_data_ptr()), rows, idx, w, accumulate, &p[0]->w, &p[1]->w, &p[2]->w, ws, have,
                         c10::cuda::getCurrentCUDAStream(x.device().index()).stream());
     Py_END_ALLOW_THREADS
     return rc;
@@ -253,7 +268,7 @@ int run_expert(Plan* (&p)[3], const at::Tensor& x, int64_t rows, const int32_t* 
 PyObject* expert(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 2) return PyErr_Format(PyExc_TypeError, "expert(module, x)");
     try {
-        Plan* p[3];
+        Held<Plan> p[3];
         if (!expert_plans(args[0], p)) Py_RETURN_NONE;
         int64_t rows = 0;
         const at::Tensor* x = rows_of(args[1], p[0]->w.K, &rows);

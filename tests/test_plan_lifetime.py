@@ -1,10 +1,11 @@
-"""The native plan of a layer (native/host.cpp) lives as long as the layer's own descriptor."""
+"""The native plan of a layer (native/host.cpp) lives as long as the layer's own descriptor, and a call holds the plans it uses."""
 import pytest
 import torch
 
-from mixtral_offloading_b200 import HQQLinearTritonSavable
+from mixtral_offloading_b200 import HQQLinearTritonSavable, _cabi, custom_layers
 from oracle import hqq_oracle as O
 from tests.helpers import layer_from_oracle, quant_config, random_layer
+from tests.test_gpu_parity import make_expert
 
 DEV = torch.device("cuda:0")
 
@@ -68,3 +69,35 @@ def test_plan_is_not_used_without_the_descriptor():
     la.W_q, la.meta, la._desc = into(la.W_q, lb.W_q), meta, None
     y = la(x.to(DEV))
     assert y.shape == (3, 1024) and O.rel_err(y.cpu(), O.linear(x, b)) < 1e-2
+
+
+@pytest.mark.gpu
+def test_layer_replaced_while_its_workspace_grows(monkeypatch):
+    """The workspace grows through Python code, which may drop the plan that the call works with."""
+    od = random_layer(512, 256, 4, 64, seed=1)
+    ods = tuple(random_layer(n, k, 2, 16, seed=3 + i) for i, (n, k) in enumerate(((512, 256), (256, 512), (512, 256))))
+    layer, expert = layer_from_oracle(od, DEV), make_expert(256, 512, ods)
+    x = torch.randn(40, 256, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16)
+    layer(x[:1].to(DEV)), expert(x[:1].to(DEV))
+    grow, calls = custom_layers._scratch, []
+
+    def dropping(device, nbytes):
+        for lyr in (layer, expert.w1, expert.w2, expert.w3):
+            lyr._drop_descriptor()
+        calls.append([bytes(4096) for _ in range(64)])       # whatever was freed is written over
+        return grow(device, nbytes)
+
+    host = _cabi.host()
+    old = dict(custom_layers._SCRATCH)
+    try:
+        host.setup(custom_layers._SCRATCH, dropping)
+        custom_layers._SCRATCH.clear()
+        y = layer(x.to(DEV))
+        custom_layers._SCRATCH.clear()
+        z = expert(x.to(DEV))
+    finally:
+        host.setup(custom_layers._SCRATCH, grow)
+        custom_layers._SCRATCH.update(old)
+    assert len(calls) == 2
+    assert O.rel_err(y.cpu(), O.linear(x, od)) < 1e-2
+    assert O.rel_err(z.cpu(), O.expert_ffn(x, *ods)) < 1e-2
