@@ -2,6 +2,8 @@
 // front and the routing-weight scale + accumulate into the MoE output behind
 // (MixtralBLockSparseTop2MLP_HQQ.forward and the per-expert body of
 // SparseMoeWrapper.forward in the reference's custom_layers.py).
+#include <algorithm>
+
 #include "common.cuh"
 #include "gemm_grouped.cuh"
 #include "kernels.cuh"
@@ -86,24 +88,30 @@ static bool fused_plan(int64_t M, const hqm_weight* w1, const hqm_weight* w2, co
     return true;
 }
 
+// The three layers one after the other: their outputs, and what a single layer's launch needs.
+static size_t separate_bytes(int64_t M, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3) {
+    size_t lin = 0, rows = 0;
+    for (const hqm_weight* w : {w1, w3, w2}) {
+        lin = std::max(lin, linear_scratch_bytes(M, w));
+        rows += align_up((size_t)M * (size_t)w->N * 2, 256);
+    }
+    return rows + lin;
+}
+
 }  // namespace hqm
 
 extern "C" {
 
 size_t hqm_expert_ffn_scratch_bytes(int64_t M, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3) {
+    using namespace hqm;
     if (!w1 || !w2 || !w3 || M <= 0) return 0;
-    const size_t H = hqm::SCRATCH_HEADER;
-    hqm::GgPlan gp;
-    if (M >= hqm::GG_MIN_ROWS && hqm::gg_plan(M, 1, M, w1, w2, w3, &gp)) return H + gp.total();
-    hqm::FusedPlan fp;
-    if (hqm::fused_plan(M, w1, w2, w3, nullptr, &fp)) return H + fp.up_bytes + fp.h_bytes + fp.down_bytes;
-    const size_t a = hqm::align_up((size_t)M * (size_t)w1->N * 2, 256);
-    const size_t b = hqm::align_up((size_t)M * (size_t)w3->N * 2, 256);
-    const size_t c = hqm::align_up((size_t)M * (size_t)w2->N * 2, 256);
-    size_t lin = hqm::linear_scratch_bytes(M, w1);
-    lin = lin > hqm::linear_scratch_bytes(M, w3) ? lin : hqm::linear_scratch_bytes(M, w3);
-    lin = lin > hqm::linear_scratch_bytes(M, w2) ? lin : hqm::linear_scratch_bytes(M, w2);
-    return H + a + b + c + lin;
+    // (whatever the shapes allow, rows of x that are not 16-byte aligned take the layers one after the other)
+    size_t bytes = separate_bytes(M, w1, w2, w3);
+    GgPlan gp;
+    FusedPlan fp;
+    if (M >= GG_MIN_ROWS && gg_plan(M, 1, M, w1, w2, w3, &gp)) bytes = std::max(bytes, gp.total());
+    else if (fused_plan(M, w1, w2, w3, nullptr, &fp)) bytes = std::max(bytes, fp.up_bytes + fp.h_bytes + fp.down_bytes);
+    return SCRATCH_HEADER + bytes;
 }
 
 int hqm_expert_ffn(uint16_t* out, const uint16_t* x, int64_t M, const int32_t* token_idx, const float* route_w,

@@ -250,7 +250,7 @@ def linear_group(layers, x: torch.Tensor):
     M, n, lib = x2.shape[0], len(layers), _cabi.lib()
     ws = (C.c_void_p * n)(*(C.addressof(lyr.descriptor()) for lyr in layers))
     need = lib.hqm_linear_group_scratch_bytes(M, ws, n)
-    if need == 0 or x2.dtype != x.dtype or any(lyr.bias is not None for lyr in layers):
+    if need == 0 or x2.dtype != x.dtype or x2.data_ptr() % 16 or any(lyr.bias is not None or lyr.meta["shape"][1] != x2.shape[1] for lyr in layers):
         return [lyr(x) for lyr in layers]
     out = [torch.empty(x.shape[:-1] + (lyr.meta["shape"][0],), dtype=torch.bfloat16, device=x2.device) for lyr in layers]
     ys = (C.c_void_p * n)(*(y.data_ptr() for y in out))
@@ -467,7 +467,7 @@ class ResidentMoe(nn.Module):
         x2 = _as_bf16_2d(hidden_states, hidden)
         T, E = x2.shape[0], self.num_experts
         dev = x2.device
-        if self.scratch_bytes(T):
+        if self.scratch_bytes(T) and (T == 1 or x2.data_ptr() % 16 == 0):
             out, logits = self.forward_on_device(x2)
             out = out.reshape(batch, seq, hidden)
             if hidden_states.dtype != torch.bfloat16:
