@@ -2,6 +2,7 @@
 #include <stdarg.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
@@ -77,21 +78,29 @@ int set_overlap(int on) {
 // (3 bit: from two on, as the streaming kernel takes one row per launch: 14336 x 4096 21 us each, here 29 up to 16 rows.)
 static bool use_gg(const hqm_weight* w, int G, int C, int64_t M) { return M >= (w->nbits == 3 ? 2 : GG_MIN_ROWS) && M <= (1 << 22) && gg_supported(w, G, C); }
 
-size_t linear_scratch_bytes(int64_t M, const hqm_weight* w, bool preferred) {
-    int G, C;
-    StreamPlan plan;
-    if (M <= 0 || check_weight(w, &G, &C) != HQM_OK) return 0;
-    if (force_generic()) return 0;
-    if (use_gg(w, G, C, M)) {
-        const GgRows rows = gg_linear_layout(M, &w, 1).rows;
-        return gg_stage_bytes(rows.padded(), w->K, true) + (preferred ? gg_scratch_bytes(rows.n) : gg_scratch_least(rows.n, &w, 1));
-    }
+// The kernels beside gemm_grouped.cu: what the one that takes the call needs.
+static size_t other_scratch_bytes(int64_t M, const hqm_weight* w, int G, int C) {
     if (gemm_tc3_supported(w, G, C, M)) return gemm_tc3_scratch_bytes(w, G, M);
     Stream3Plan plan3;
     if (gemv_stream3_plan(w, G, C, M, &plan3)) return gemv_stream3_scratch_bytes(plan3, M, w->N);
+    StreamPlan plan;
     const hqm_weight* one[1] = {w};
     if (!gemv_stream_plan(one, 1, M, &plan, /*chained=*/false)) return 0;
     return (gemv_stream_scratch_bytes(plan, M) + 255) / 256 * 256;
+}
+
+// The least is a contract with callers whose memory plan is fixed: the fp32 sums of the call, or what the streaming and
+// 3-bit kernels leave behind for as few rows as they take.  The tensor-core kernel makes do with that (linear_gg); it only
+// wants room for 16 rows at a time on a third of the SMs.
+size_t linear_scratch_bytes(int64_t M, const hqm_weight* w, bool preferred) {
+    int G, C;
+    if (M <= 0 || check_weight(w, &G, &C) != HQM_OK || force_generic()) return 0;
+    if (!use_gg(w, G, C, M)) return other_scratch_bytes(M, w, G, C);
+    const size_t sums = w->nbits != 3 && M > STREAM_MAX_ROWS ? (size_t)M * w->N * sizeof(float) : other_scratch_bytes(M, w, G, C);
+    const size_t least = std::max(gg_least_bytes(w->K), (sums + 255) / 256 * 256);
+    if (!preferred) return least;
+    const GgRows rows = gg_linear_layout(M, &w, 1).rows;
+    return std::max(least, gg_stage_bytes(rows.padded(), w->K, true) + gg_scratch_bytes(rows.n));
 }
 
 static int need_scratch(void* scratch, size_t have, size_t need) {
@@ -103,32 +112,56 @@ static int need_scratch(void* scratch, size_t have, size_t need) {
     return HQM_OK;
 }
 
-// Layers of one K and format over the same rows: the rows staged once, one launch over all tiles.
+// Layers of one K and format over the same rows: the rows staged once, one launch over all tiles.  With less scratch than
+// that wants, narrower chunks and fewer CTAs, or the rows in several passes, by the cost that gg_linear_layout gives.
 static int linear_gg(uint16_t* const* y, const hqm_weight* const* ws, const uint16_t* const* bias, int count, const uint16_t* x,
                      const int32_t* x_idx, int64_t M, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st,
                      int f16 = 0) {
-    const GgLayout layout = gg_linear_layout(M, ws, count);
     const int K = ws[0]->K;
-    const int64_t xt_rows = layout.rows.padded();
-    const size_t staged = gg_stage_bytes(xt_rows, K, true);
-    int rc = need_scratch(scratch, scratch_bytes, staged + gg_scratch_least(layout.rows.n, ws, count));
+    int rc = need_scratch(scratch, scratch_bytes, gg_least_bytes(K));
     if (rc != HQM_OK) return rc;
-    const GgStaged xs = gg_staged(scratch, xt_rows, K, true);
-    rc = launch_gg_stage(xs, x, f16, x_idx, nullptr, 1, M, K, ws[0]->nbits, st);
-    if (rc != HQM_OK) return rc;
-    GgJob job{};
-    job.problems = count;
-    job.rows = (int)M;
-    job.layout = layout;
-    job.x = xs;
-    job.mode = GG_LINEAR;
-    job.y_f16 = f16;
-    for (int i = 0; i < count; ++i) {
-        job.w0[i] = ws[i];
-        job.y[i] = y[i];
-        job.bias[i] = bias ? bias[i] : nullptr;
+    GgLayout layout = gg_linear_layout(M, ws, count, scratch_bytes);
+    int64_t rows = M;
+    if (layout.grid == 0 || gg_stage_bytes(layout.rows.padded(), K, true) + gg_scratch_bytes(layout.rows.n) > scratch_bytes) {
+        rc = need_scratch(scratch, scratch_bytes, linear_scratch_bytes(M, ws[0]));
+        if (rc != HQM_OK) return rc;
+        constexpr int64_t PASS = 10000;          // cycles of two more launches
+        int64_t best = layout.grid ? layout.cost : INT64_MAX;
+        const int64_t most = (M + 15) / 16;
+        for (int64_t passes = 2; passes <= most; passes = passes == most ? most + 1 : std::min(most, passes + 1 + passes / 4)) {
+            const int64_t r = ((M + passes - 1) / passes + 15) / 16 * 16;
+            const GgLayout l = gg_linear_layout(r, ws, count, scratch_bytes);
+            if (l.grid && passes * (l.cost + PASS) < best) {
+                best = passes * (l.cost + PASS);
+                layout = l;
+                rows = r;
+            }
+        }
     }
-    return launch_gg(job, counters, (uint8_t*)scratch + staged, scratch_bytes - staged, st);
+    for (int64_t r0 = 0; r0 < M; r0 += rows) {
+        const int64_t m = std::min(rows, M - r0);
+        if (r0 > 0 && m < rows) layout = gg_linear_layout(m, ws, count, scratch_bytes);
+        const int64_t xt_rows = layout.rows.padded();
+        const size_t staged = gg_stage_bytes(xt_rows, K, true);
+        const GgStaged xs = gg_staged(scratch, xt_rows, K, true);
+        rc = launch_gg_stage(xs, x_idx ? x : x + r0 * K, f16, x_idx ? x_idx + r0 : nullptr, nullptr, 1, m, K, ws[0]->nbits, st);
+        if (rc != HQM_OK) return rc;
+        GgJob job{};
+        job.problems = count;
+        job.rows = (int)m;
+        job.layout = layout;
+        job.x = xs;
+        job.mode = GG_LINEAR;
+        job.y_f16 = f16;
+        for (int i = 0; i < count; ++i) {
+            job.w0[i] = ws[i];
+            job.y[i] = y[i] + r0 * ws[i]->N;
+            job.bias[i] = bias ? bias[i] : nullptr;
+        }
+        rc = launch_gg(job, counters, (uint8_t*)scratch + staged, scratch_bytes - staged, st);
+        if (rc != HQM_OK) return rc;
+    }
+    return HQM_OK;
 }
 
 int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t M, const hqm_weight* w,

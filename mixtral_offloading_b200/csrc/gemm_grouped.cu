@@ -1409,26 +1409,21 @@ static int64_t gg_tiles(const hqm_weight* w) {
     }
     return (w->N / w->group_size + 7) / 8 * (w->group_size / 16);
 }
-// (a layer with a tile for every SM is not worth running on a third of them)
 static int64_t gg_tiles(const hqm_weight* const* ws, int count) {
     int64_t tiles = 0;
     for (int i = 0; i < count; ++i) tiles += gg_tiles(ws[i]);
     return tiles;
 }
-size_t gg_scratch_least(int n, const hqm_weight* const* ws, int count) {
-    return (size_t)(gg_tiles(ws, count) >= gg_sm_count() ? gg_sm_count() : GG_LEAST_CTAS) * gg_piece_bytes(n);
-}
-
-GgLayout gg_expert_layout(int64_t M) { return GgLayout{GgRows::of((int)M), gg_sm_count()}; }
+GgLayout gg_expert_layout(int64_t M) { return GgLayout{GgRows::of((int)M), gg_sm_count(), 0}; }
 // Rows per chunk and CTAs of linear layers over the same rows, by what a launch costs in cycles of its longest CTA (fitted to
 // 2- and 4-bit layers of 1024 to 14336 outputs with 16 to 500 rows):
 //   its units of 128 columns:  850 + 4 n with n rows; beyond 128 rows it is the staged x in every SM, 10 n
 //   a finished tile:           400 for every 16 rows
 //   a tile cut into p pieces:  5000 until the last CTA has seen that it is the last, and 3000 + 400 (p - 2) for every 16 rows;
 //                              twice where shares and tiles are not aligned, as a CTA then holds pieces of two tiles
-// Wide chunks dequantise the weights less often; narrow ones give every SM whole tiles.
-GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count) {
-    const int64_t tiles = gg_tiles(ws, count), units_k = (ws[0]->K + 127) / 128, sms = gg_sm_count();
+// Wide chunks dequantise the weights less often; narrow ones give every SM whole tiles, and need less scratch.
+GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count, size_t bytes) {
+    const int64_t tiles = gg_tiles(ws, count), units_k = (ws[0]->K + 127) / 128;
     GgLayout best{};
     int64_t best_cost = INT64_MAX;
     int chunks = 0;
@@ -1437,13 +1432,19 @@ GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count) {
         const GgRows r = GgRows::of((int)M, cap);
         if (r.chunks == chunks) continue;    // the same cut
         chunks = r.chunks;
+        const size_t staged = gg_stage_bytes(r.padded(), ws[0]->K, true);
+        const int64_t sms = bytes > staged ? std::min<int64_t>(gg_sm_count(), (int64_t)((bytes - staged) / gg_piece_bytes(r.n))) : 0;
+        if (sms == 0) {
+            if (r.chunks == 1) break;
+            continue;
+        }
         const int64_t units = tiles * r.chunks * units_k, n16 = r.n / 16, s0 = (units + sms - 1) / sms;
         const int64_t unit = std::max<int64_t>(850 + 4 * r.n, r.n > 128 ? 10 * r.n : 0);
         auto consider = [&](int64_t share, int64_t pieces, int cuts) {
             const int64_t cost = share * unit + (share + units_k - 1) / units_k * n16 * 400 + cuts * (5000 + n16 * (3000 + 400 * (pieces - 2)));
             if (cost < best_cost) {
                 best_cost = cost;
-                best = GgLayout{r, (int)std::min<int64_t>(sms, (units + share - 1) / share)};
+                best = GgLayout{r, (int)std::min<int64_t>(sms, (units + share - 1) / share), cost};
             }
         };
         consider((s0 + units_k - 1) / units_k * units_k, 2, 0);                                  // whole tiles
@@ -1556,15 +1557,14 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
     p.chunks = job.layout.rows.chunks;
     p.counters = counters;
     p.error_flag = tc_error_ptr();
-    int64_t grid = job.counts ? gg_sm_count() : job.layout.grid;
-    const size_t least_bytes = job.counts ? gg_scratch_bytes(p.n_max) : std::min((size_t)grid * gg_piece_bytes(p.n_max), gg_scratch_least(p.n_max, job.w0, job.problems));
-    if (scratch == nullptr || counters == nullptr || scratch_bytes < least_bytes) {
-        set_error("gemm: scratch of %zu bytes given, %zu needed", scratch_bytes, least_bytes);
+    const int grid = job.counts ? gg_sm_count() : job.layout.grid;
+    const size_t need = (size_t)grid * gg_piece_bytes(p.n_max);
+    if (scratch == nullptr || counters == nullptr || scratch_bytes < need) {
+        set_error("gemm: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
         return HQM_ERR_SCRATCH;
     }
-    grid = std::min<int64_t>(grid, (int64_t)(scratch_bytes / gg_piece_bytes(p.n_max)));
 #define HQM_GG(B, M) \
-    if (nbits == B && job.mode == M) return gg_launch_one<B, M>(p, (int)grid, st);
+    if (nbits == B && job.mode == M) return gg_launch_one<B, M>(p, grid, st);
     HQM_GG(2, GG_LINEAR) HQM_GG(2, GG_UP) HQM_GG(2, GG_DOWN) HQM_GG(4, GG_LINEAR) HQM_GG(4, GG_DOWN)
     HQM_GG(3, GG_LINEAR)
 #undef HQM_GG

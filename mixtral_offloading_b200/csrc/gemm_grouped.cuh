@@ -7,7 +7,7 @@ namespace hqm {
 
 constexpr int GG_MAX_PROBLEMS = 32;
 constexpr int GG_MAX_ROWS = 256;          // rows of x per pass over a weight (the MMA's N)
-constexpr int GG_LEAST_CTAS = 48;
+constexpr int GG_LEAST_CTAS = 48;         // a third of the SMs: what a call may ask scratch for at the least
 constexpr int GG_F16_ROWS = 16;           // up to here h of an expert is staged as fp16, beyond it as bf16
 
 // How a launch's rows are laid out in the staged copy of x ("tiles": [K / 64][row][64], see gemm_grouped.cu): a row
@@ -25,6 +25,7 @@ struct GgRows {
 struct GgLayout {                         // of a launch whose row count the host knows
     GgRows rows;
     int grid;
+    int64_t cost;                         // cycles, by the rule of gg_linear_layout
 };
 // Upper bound of the padded rows of `rows` rows spread over `lists` lists.
 inline int64_t gg_padded_rows(int64_t rows, int lists) {
@@ -79,12 +80,12 @@ struct GgJob {
 };
 
 bool gg_supported(const hqm_weight* w, int G, int C);
-GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count);      // layers of one K and format
+// Layers of one K and format over M rows, with `bytes` of scratch for the staged rows and the partial tiles (grid 0: too few).
+GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count, size_t bytes = SIZE_MAX);
 GgLayout gg_expert_layout(int64_t M);
-// Bytes of scratch (partial tiles) of a launch with up to n rows per chunk: with a CTA on every SM, and the least a launch
-// without `counts` works with (it then uses fewer CTAs).
-size_t gg_scratch_bytes(int n);
-size_t gg_scratch_least(int n, const hqm_weight* const* ws, int count);
+size_t gg_scratch_bytes(int n);           // partial tiles of a launch with up to n rows per chunk and a CTA on every SM
+// Scratch with which 16 rows at a time can be multiplied on GG_LEAST_CTAS SMs, whatever the layer's size.
+inline size_t gg_least_bytes(int K) { return gg_stage_bytes(16, K, true) + (size_t)GG_LEAST_CTAS * 2 * 16 * 128 * sizeof(float); }
 int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st);
 
 // Stages rows of x (bf16 or fp16) for layers of `nbits`.  counts == null: one list of `rows` rows, else `lists` lists of together at most `rows`;

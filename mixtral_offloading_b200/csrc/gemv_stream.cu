@@ -738,7 +738,7 @@ bool gemv_stream_plan(const hqm_weight* const* ws, int count, int64_t M, StreamP
     const int nb = g / 16;
     const int pw = nb == 1 ? 128 : 64;
     if (!group_ok || w->K % pw != 0) return false;
-    if (M < 1 || M > 16) return false;
+    if (M < 1 || M > STREAM_MAX_ROWS) return false;
     plan->count = count;
     plan->rho0[0] = 0;
     plan->col0[0] = 0;

@@ -10,6 +10,7 @@ int launch_linear_generic(uint16_t* y, const uint16_t* x, const int32_t* x_idx, 
 
 // gemv_stream.cu — the weight-streaming path for small row counts.
 constexpr int STREAM_MAX_LAYERS = 4;
+constexpr int STREAM_MAX_ROWS = 16;
 // What one launch multiplies: up to four layers of the same K, bit width and group size (N may differ).
 // Layer l reads rows x_idx?[m] + xrow[l] of x.  With `table` set, layer l's descriptor is read on the
 // device: table[3 * *sel[l] + which[l]] (3 entries per expert: w1, w2, w3), and w[l] only gives the shape.

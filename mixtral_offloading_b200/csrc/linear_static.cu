@@ -17,12 +17,13 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "gemm_grouped.cuh"
 #include "kernels.cuh"
 
 namespace hqm {
 
-// 2 MiB: enough for the decode-sized calls this entry point is meant for (a Mixtral
-// expert projection, 14336 x 4096, needs ~172 KB per row of x).
+// 2 MiB: enough for the decode-sized calls this entry point is meant for, and for a few dozen
+// rows of most layers (fp32 sums: 57 KB per row of a 14336 x 4096 projection).
 constexpr size_t STATIC_SCRATCH_BYTES = 2u << 20;
 static __device__ __align__(256) unsigned char g_static_scratch[STATIC_SCRATCH_BYTES];
 
@@ -59,6 +60,10 @@ int hqm_linear_static_scratch(uint16_t* y, const uint16_t* x, int64_t M, const h
     const size_t inner = linear_scratch_bytes(M, w);
     const size_t need = inner ? inner + SCRATCH_HEADER : 0;
     if (need > STATIC_SCRATCH_BYTES) {
+        int G, C;
+        // (a layer so wide that not even 16 of its rows can be staged, but with few enough sums)
+        if (inner == gg_least_bytes(w->K) && check_weight(w, &G, &C) == HQM_OK)
+            return launch_linear_generic(y, x, nullptr, M, w, G, C, bias, (cudaStream_t)stream);
         set_error("linear_static_scratch: this call needs %zu bytes of workspace but the built-in one holds %zu; "
                   "use hqm_linear with a caller-provided buffer", need, (size_t)STATIC_SCRATCH_BYTES);
         return HQM_ERR_SCRATCH;
@@ -73,8 +78,8 @@ int hqm_linear_static_scratch(uint16_t* y, const uint16_t* x, int64_t M, const h
     // zero is the header (arrival counters); the array is zero when the library is loaded and every call
     // leaves the header zero again.
     if (ws == nullptr) return launch_linear(y, x, nullptr, M, w, bias, nullptr, nullptr, 0, (cudaStream_t)stream);
-    return launch_linear(y, x, nullptr, M, w, bias, (uint32_t*)ws, (uint8_t*)ws + SCRATCH_HEADER, inner,
-                         (cudaStream_t)stream);
+    return launch_linear(y, x, nullptr, M, w, bias, (uint32_t*)ws, (uint8_t*)ws + SCRATCH_HEADER,
+                         STATIC_SCRATCH_BYTES - SCRATCH_HEADER, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -8,11 +8,11 @@ import torch
 from mixtral_offloading_b200 import ResidentMoe, _cabi
 from mixtral_offloading_b200.custom_layers import linear_group
 from oracle import hqq_oracle as O
-from tests.helpers import layer_from_oracle, random_layer
+from tests.helpers import layer_from_oracle, random_layer, random_layer_fast
 from tests.test_gpu_parity import Cfg, make_expert
 
 DEV = torch.device("cuda:0")
-# bf16 results: 2^-9 / sqrt(3) for a rounding that is uniform in the last place, and the kernels' 16-bit factors under it
+# of the largest result: half a unit in the last place of bf16 (2^-9), and as much again for the kernels' 16-bit factors
 TOL = 4e-3
 
 
@@ -26,6 +26,58 @@ def test_groups_of_more_than_256_rows(nbits, group, N, K, M):
     y = layer_from_oracle(od, DEV)(x.to(DEV))
     assert O.rel_err(y.cpu(), O.linear(x, od)) < TOL
     assert _cabi.lib().hqm_device_error() == 0
+
+
+def _in_scratch(d, x, size, y):
+    """hqm_linear with exactly `size` bytes of scratch; the bytes behind them stay as they are."""
+    lib, guard = _cabi.lib(), 1 << 16
+    ws = torch.full((size + guard,), 7, dtype=torch.uint8, device=DEV)
+    _cabi.check(lib.hqm_scratch_init(_cabi.ptr(ws), _cabi.stream_ptr(DEV)))
+    rc = lib.hqm_linear(_cabi.ptr(y), _cabi.ptr(x), x.shape[0], C.byref(d), None, _cabi.ptr(ws), size, _cabi.stream_ptr(DEV))
+    assert bool((ws[size:] == 7).all()) and int(ws[:lib.hqm_scratch_header_bytes()].max()) == 0
+    return rc
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nbits,group,N,K,Ms", [
+    (2, 16, 4096, 14336, (17, 32, 100)), (2, 16, 14336, 4096, (5, 17, 34)), (4, 64, 4096, 4096, (64, 100)),
+    (4, 64, 1024, 4096, (5, 100, 400)), (3, 64, 1024, 4096, (5, 100))])
+def test_little_scratch(nbits, group, N, K, Ms):
+    """Calls whose fp32 sums fit a fixed workspace work in it: the built-in one of 2 MiB, and one of the size that
+    hqm_linear_scratch_bytes names (narrow chunks, few CTAs, several passes); with a byte less they are refused."""
+    lib = _cabi.lib()
+    layer = layer_from_oracle(random_layer_fast(N, K, nbits, group, seed=nbits), DEV)
+    d, W = layer.descriptor(), layer.dequantize(torch.float32).double()
+    for M in Ms:
+        x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(DEV)
+        want, y = x.double() @ W.t(), torch.empty((M, N), dtype=torch.bfloat16, device=DEV)
+
+        def right():
+            return ((y.double() - want).abs().max() / want.abs().max()).item() < TOL
+
+        need = lib.hqm_linear_scratch_bytes(M, C.byref(d))
+        if nbits != 3:
+            assert need <= lib.hqm_static_scratch_capacity()
+            assert lib.hqm_linear_static_scratch(_cabi.ptr(y.fill_(7.0)), _cabi.ptr(x), M, C.byref(d), None, _cabi.stream_ptr(DEV)) == 0
+            assert right(), M
+        for size in (need, (need + lib.hqm_linear_scratch_preferred(M, C.byref(d))) // 512 * 256):
+            y.fill_(7.0)
+            assert _in_scratch(d, x, size, y) == 0 and right(), (M, size)
+        assert _in_scratch(d, x, need - 1, y) == _cabi.HQM_ERR_SCRATCH
+    assert lib.hqm_device_error() == 0
+
+
+@pytest.mark.gpu
+def test_builtin_scratch_takes_a_layer_too_wide_for_it():
+    """16 staged rows of 65536 columns are more than 2 MiB; the sums of 20 rows are not."""
+    N, K, M = 128, 65536, 20
+    layer = layer_from_oracle(random_layer_fast(N, K, 4, 64, seed=1), DEV)
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    y = torch.empty((M, N), dtype=torch.bfloat16, device=DEV)
+    assert _cabi.lib().hqm_linear_static_scratch(_cabi.ptr(y), _cabi.ptr(x), M, C.byref(layer.descriptor()), None,
+                                                 _cabi.stream_ptr(DEV)) == 0
+    want = x.double() @ layer.dequantize(torch.float32).double().t()
+    assert ((y.double() - want).abs().max() / want.abs().max()).item() < TOL
 
 
 def _at_odd_address(t):
