@@ -18,7 +18,8 @@
 //     in the matching order (tile_pos below).
 //   * fp16: a field of a byte, left where it is, IS an fp16 denormal c * 2^(p-24); one fused multiply-add with
 //     s * 2^(24-p-2) and -z*s * 2^-2 gives a quarter of the weight.  One AND and one FMA per two weights; the sums are
-//     multiplied by 4 at the end.  Where s * 2^(22-p) leaves the fp16 range (s >= 1/4), the warp takes the longer way
+//     multiplied by 4 at the end.  -z*s is formed from an fp32 z: with z in fp16 the two roundings of z are the largest
+//     errors of all (4 bit: 1.07e-3 of the result against 5.5e-4; the streaming kernels' fp16 x * s give 9.8e-4).  Where s * 2^(22-p) leaves the fp16 range (s >= 1/4), the warp takes the longer way
 //     for that unit: OR into 1024, exact subtract, FMA.  x is staged as fp16 with a power-of-two factor per row.
 //   * bf16 (down projections of more than 16 rows: h has no factor per row and may exceed fp16): OR into 128, exact
 //     subtract, FMA.
@@ -381,6 +382,31 @@ __device__ __forceinline__ float half_at(uint32_t pair, int hi) { return f16_bit
 __device__ __forceinline__ float byte_at(uint32_t v, int i) {           // 2^23 + b is exact
     return __uint_as_float(perm(v, 0x4B000000u, 0x7650u + (uint32_t)i)) - 8388608.f;
 }
+__device__ __forceinline__ uint32_t h2_of(float lo, float hi) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// half `hi` of a times the same of b, plus c in fp32
+__device__ __forceinline__ float fma_half(uint32_t a, uint32_t b, float c, int hi) {
+    float d;
+    if (hi) asm("{\n\t.reg .b16 l, x, y;\n\tmov.b32 {l, x}, %1;\n\tmov.b32 {l, y}, %2;\n\tfma.rn.f32.f16 %0, x, y, %3;\n\t}" : "=f"(d) : "r"(a), "r"(b), "f"(c));
+    else asm("{\n\t.reg .b16 h, x, y;\n\tmov.b32 {x, h}, %1;\n\tmov.b32 {y, h}, %2;\n\tfma.rn.f32.f16 %0, x, y, %3;\n\t}" : "=f"(d) : "r"(a), "r"(b), "f"(c));
+    return d;
+}
+// -z * s / 4 of two columns, z = (byte - zz) * zs in fp32 from bytes i and i + 1 of q and halves zz, zs; s as halves
+__device__ __forceinline__ void neg_quarter_zs(uint32_t q, int i, uint32_t zz, uint32_t zs, uint32_t s, float& lo, float& hi) {
+    // 2^23 + byte, then -byte / 4, exact
+    uint64_t b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "r"(perm(q, 0x4B000000u, 0x7650u + (uint32_t)i)), "r"(perm(q, 0x4B000000u, 0x7651u + (uint32_t)i)));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(b) : "l"(0xBE800000BE800000ull), "l"(0x4A0000004A000000ull));
+    float b0, b1;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(b0), "=f"(b1) : "l"(b));
+    uint64_t t, u;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(t) : "f"(fma_half(zz, 0x34003400u, b0, 0)), "f"(fma_half(zz, 0x34003400u, b1, 1)));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(u) : "f"(fma_half(zs, s, 0.f, 0)), "f"(fma_half(zs, s, 0.f, 1)));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(t) : "l"(u));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(t));
+}
 __device__ __forceinline__ uint32_t bf2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -702,23 +728,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                     a_ready = v_round > 0 ? peek(a_empty + 8 * (v + ((v_round & 1) ? 0 : NA)), ((v_round - 1) >> 1) & 1) : 1u;
                     uint32_t S[DC / 2], T[DC / 2];            // per four columns: pair (0, 2), pair (1, 3)
                     if (f16) {
-                        // s * 2^(22 - p) and -z * s / 4, p = 4 + fpos the field's first bit
+                        // s * 2^(22 - p) and -z * s / 4, p = 4 + fpos the field's first bit.  The second is formed from the rounded s
+                        // and an unrounded z: what s is off then scales the whole (c - z) s, and T adds one rounding of its own.
 #pragma unroll
                         for (int j = 0; j < DC / 4; ++j) {
-                            uint32_t s2[2], z2[2];
+                            uint32_t s2[2];
+                            float tt[4];
 #pragma unroll
                             for (int e = 0; e < 2; ++e) {
-                                const uint32_t sel = e ? 0x4342u : 0x4140u;
-                                const uint32_t qs = h2sub(perm(sq[j], 0x64646464u, sel), 0x64006400u);
-                                const uint32_t qz = h2sub(perm(zq[j], 0x64646464u, sel), 0x64006400u);
+                                const uint32_t qs = h2sub(perm(sq[j], 0x64646464u, e ? 0x4342u : 0x4140u), 0x64006400u);
                                 s2[e] = h2mul(h2sub(qs, mt[1][2 * j + e]), mt[0][2 * j + e]);
-                                z2[e] = h2mul(h2sub(qz, mt[3][2 * j + e]), mt[2][2 * j + e]);
+                                neg_quarter_zs(zq[j], 2 * e, mt[3][2 * j + e], mt[2][2 * j + e], s2[e], tt[2 * e], tt[2 * e + 1]);
                             }
                             // to the order (0, 2), (1, 3)
                             S[2 * j] = perm(s2[0], s2[1], 0x5410u);
                             S[2 * j + 1] = perm(s2[0], s2[1], 0x7632u);
-                            T[2 * j] = h2mul(perm(z2[0], z2[1], 0x5410u), h2mul(S[2 * j], 0xB400B400u));          // -z * (s / 4)
-                            T[2 * j + 1] = h2mul(perm(z2[0], z2[1], 0x7632u), h2mul(S[2 * j + 1], 0xB400B400u));
+                            T[2 * j] = h2_of(tt[0], tt[2]);
+                            T[2 * j + 1] = h2_of(tt[1], tt[3]);
                         }
                         // |s| * 2^(18 - fpos) must stay finite: |s| < 1/4 (fpos = 2: < 1)
                         uint32_t mx = 0;
