@@ -76,7 +76,9 @@ int set_overlap(int on) {
 // Rows from which a layer goes to the tensor-core kernel (gemm_grouped.cu); below, the streaming kernels,
 // whose work per weight grows with the rows, are faster.
 // (3 bit: from two on, as the streaming kernel takes one row per launch: 14336 x 4096 21 us each, here 29 up to 16 rows.)
-static bool use_gg(const hqm_weight* w, int G, int C, int64_t M) { return M >= (w->nbits == 3 ? 2 : GG_MIN_ROWS) && M <= (1 << 22) && gg_supported(w, G, C); }
+static bool use_gg(const hqm_weight* w, int G, int C, int64_t M) {
+    return M >= (w->nbits == 3 ? 2 : GG_MIN_ROWS) && M <= (1 << 22) && gg_takes(w, G, C, M);
+}
 
 // The kernels beside gemm_grouped.cu: what the one that takes the call needs.
 static size_t other_scratch_bytes(int64_t M, const hqm_weight* w, int G, int C) {

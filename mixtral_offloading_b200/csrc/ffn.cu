@@ -57,7 +57,8 @@ static bool gg_plan(int64_t entries, int lists, int64_t most, const hqm_weight* 
     if (force_generic() || !same_format(w1, w3) || entries > (1 << 22)) return false;
     if (check_weight(w1, &G1, &C1) != HQM_OK || check_weight(w3, &G1, &C1) != HQM_OK || check_weight(w2, &G2, &C2) != HQM_OK)
         return false;
-    if (!gg_supported(w1, G1, C1) || !gg_supported(w3, G1, C1) || !gg_supported(w2, G2, C2)) return false;
+    for (int64_t rows : {most, lists > 1 ? (int64_t)1 : most})       // (lists of any length up to the most)
+        if (!gg_takes(w1, G1, C1, rows) || !gg_takes(w3, G1, C1, rows) || !gg_takes(w2, G2, C2, rows)) return false;
     if (w1->nbits != 2 || w1->group_size != 16 || w2->nbits != 2 || w2->group_size != 16) return false;   // tiles of two parts
     gp->xt_rows = gg_padded_rows(entries, lists);
     gp->x_bytes = gg_stage_bytes(gp->xt_rows, w1->K, true);

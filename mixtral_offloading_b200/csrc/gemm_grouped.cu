@@ -1422,6 +1422,22 @@ bool gg_supported(const hqm_weight* w, int G, int C) {
            a16(w->mz_zero);
 }
 
+// The kernel multiplies with fp16 weights.  That is no loss where the alternative has 16-bit factors too: the streaming
+// kernels up to their row limit, and beyond it the formats whose groups make whole tiles of 128 rows; 3 bit from five
+// rows on.  Everything else belongs to the shape-agnostic kernel, which computes in fp32: its results are as exact as bf16
+// holds them (1.66e-3 from 64 bits; 1.75e-3 here).
+bool gg_takes(const hqm_weight* w, int G, int C, int64_t M) {
+    if (!gg_supported(w, G, C)) return false;
+    if (w->nbits == 3) {
+        Stream3Plan plan;
+        return M > STREAM3_ROWS || gemv_stream3_plan(w, G, C, M, &plan);
+    }
+    if (M <= STREAM_MAX_ROWS) return gemv_stream_shape_ok(w, G, C);
+    const int per = codes_per_word(w->nbits), g = w->group_size;
+    const bool format = w->nbits == 2 ? g == 16 || g == 32 : g == 32 || g == 64;
+    return format && G / per % (128 / (g * per)) == 0 && C % 4 == 0;
+}
+
 static int gg_n_max(int64_t rows) {
     const int64_t n = (rows + 15) / 16 * 16;
     return (int)(n < 16 ? 16 : (n > GG_MAX_ROWS ? GG_MAX_ROWS : n));

@@ -80,6 +80,8 @@ struct GgJob {
 };
 
 bool gg_supported(const hqm_weight* w, int G, int C);
+// Is M rows of the layer a call for 16-bit factors?  (gemm_grouped.cu)
+bool gg_takes(const hqm_weight* w, int G, int C, int64_t M);
 // Layers of one K and format over M rows, with `bytes` of scratch for the staged rows and the partial tiles (grid 0: too few).
 GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count, size_t bytes = SIZE_MAX);
 GgLayout gg_expert_layout(int64_t M);

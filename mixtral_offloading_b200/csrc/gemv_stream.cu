@@ -724,34 +724,33 @@ static int dispatch(int nbits, int nb, int toks, Fn&& fn) {
     return -1;
 }
 
+bool gemv_stream_shape_ok(const hqm_weight* w, int G, int C) {
+    if ((w->nbits != 2 && w->nbits != 4) || !meta_uniform(w)) return false;
+    const int per = codes_per_word(w->nbits), g = w->group_size, pw = g == 16 ? 128 : 64;
+    if (w->nbits == 2 ? g != 16 && g != 32 : g != 32 && g != 64) return false;
+    if (w->K % pw != 0 || G % per != 0 || C % (w->nbits == 2 ? 8 : 4) != 0) return false;
+    if ((int64_t)(G / per) * (w->K / pw) < 8) return false;                 // a pass for every warp of a CTA
+    if ((int64_t)G * w->K >= (int64_t)1 << 31 || (int64_t)(w->N / per) * w->K >= (int64_t)1 << 31) return false;
+    return aligned16(w->W_q) && aligned16(w->scale_q) && aligned16(w->zero_q) && aligned16(w->ms_scale) && aligned16(w->mz_scale) &&
+           aligned16(w->ms_zero) && aligned16(w->mz_zero);
+}
+
 bool gemv_stream_plan(const hqm_weight* const* ws, int count, int64_t M, StreamPlan* plan, bool chained) {
     if (count < 1 || count > STREAM_MAX_LAYERS || force_generic()) return false;
     plan->tma = 0;
     if (M == 1 && gemv_tma_plan(ws, count, chained, plan)) return true;
     plan->tma = 0;
     const hqm_weight* w = ws[0];
-    if (w->nbits != 2 && w->nbits != 4) return false;
-    const int per = codes_per_word(w->nbits);
-    const int dk = w->nbits == 2 ? 8 : 4;
-    const int g = w->group_size;
-    const bool group_ok = (w->nbits == 2) ? (g == 16 || g == 32) : (g == 32 || g == 64);
-    const int nb = g / 16;
-    const int pw = nb == 1 ? 128 : 64;
-    if (!group_ok || w->K % pw != 0) return false;
-    if (M < 1 || M > STREAM_MAX_ROWS) return false;
+    if ((w->nbits != 2 && w->nbits != 4) || M < 1 || M > STREAM_MAX_ROWS) return false;
+    const int per = codes_per_word(w->nbits), nb = w->group_size / 16, pw = nb == 1 ? 128 : 64;
     plan->count = count;
     plan->rho0[0] = 0;
     plan->col0[0] = 0;
     for (int l = 0; l < count; ++l) {
         const hqm_weight* v = ws[l];
         int G, C;
-        if (check_weight(v, &G, &C) != HQM_OK || !meta_uniform(v)) return false;
-        if (v->nbits != w->nbits || v->group_size != g || v->K != w->K || v->meta_group != w->meta_group) return false;
-        if (G % per != 0 || C % dk != 0) return false;
-        if ((int64_t)G * v->K >= (int64_t)1 << 31 || (int64_t)(v->N / per) * v->K >= (int64_t)1 << 31) return false;
-        if (!aligned16(v->W_q) || !aligned16(v->scale_q) || !aligned16(v->zero_q) || !aligned16(v->ms_scale) ||
-            !aligned16(v->mz_scale) || !aligned16(v->ms_zero) || !aligned16(v->mz_zero))
-            return false;
+        if (check_weight(v, &G, &C) != HQM_OK || !gemv_stream_shape_ok(v, G, C)) return false;
+        if (v->nbits != w->nbits || v->group_size != w->group_size || v->K != w->K || v->meta_group != w->meta_group) return false;
         plan->G[l] = G;
         plan->C[l] = C;
         plan->rho0[l + 1] = plan->rho0[l] + G / per;

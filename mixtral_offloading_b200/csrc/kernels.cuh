@@ -57,6 +57,8 @@ struct StreamPlan {
     int tma;     // 1: the TMA-staged single-row kernel (gemv_tma.cu): units are (residue, block of 16 members),
                  // rho0 counts those units, and `warps` counts CTAs
 };
+// 2- and 4-bit layers of the streaming kernels' formats and shapes.
+bool gemv_stream_shape_ok(const hqm_weight* w, int G, int C);
 // False when the layers / row count are outside what the streaming kernels cover.  `chained`: the launch is a
 // link of the decode step's launch chain (its consumers read the sums); false for a linear that stands alone.
 bool gemv_stream_plan(const hqm_weight* const* ws, int count, int64_t M, StreamPlan* plan, bool chained = true);
@@ -101,6 +103,7 @@ struct Members3 {
 bool tensor_maps_ok(const hqm_weight* w, int G);
 bool stream_cached_maps3(const hqm_weight* w, int G, const Members3& m, void* out4);      // words, scales, zeros, left-over words
 // gemv_stream3.cu — the weight-streaming path for 3-bit layers.
+constexpr int STREAM3_ROWS = 4;      // beyond it the tensor-core kernels
 struct Stream3Plan {
     int P3;      // storage-row classes (rows R and R + P3 hold the same residues in the same slots)
     int PT;      // 64-column passes per class

@@ -37,3 +37,28 @@ def test_factors_of_16_bits(nbits, group, bound, M):
     x = torch.randn(M, 2048, generator=torch.Generator().manual_seed(M)).to(torch.float16).to(DEV)
     err, rounding = errors(layer(x), x.double() @ weight64(layer).t())
     assert (err ** 2 - rounding ** 2) ** 0.5 < bound
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nbits,group,N,K,Ms", [
+    (3, 64, 5120, 256, (2, 4)),                              # more members than the 3-bit streaming kernel takes
+    (2, 64, 512, 256, (5, 17)), (2, 48, 384, 256, (5, 17)), (4, 128, 1024, 256, (5, 64)), (4, 16, 256, 256, (5, 64)),
+    (2, 16, 192, 192, (5, 17)), (2, 16, 320, 704, (17,)), (4, 32, 192, 256, (17,))])
+def test_formats_that_only_the_fp32_kernel_takes(nbits, group, N, K, Ms):
+    """Weights, products and sums in fp32: what is left is the rounding of the result (and 2^-24 sqrt(K) of the sums)."""
+    layer = layer_from_oracle(random_layer(N, K, nbits, group, seed=group), DEV)
+    for M in Ms:
+        x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(DEV)
+        err, rounding = errors(layer(x), x.double() @ weight64(layer).t())
+        assert err < 1.002 * rounding, M
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nbits,group,N,K", [(2, 16, 256, 320), (4, 64, 256, 320), (4, 64, 1024, 192)])
+def test_odd_column_blocks_and_tile_parts(nbits, group, N, K):
+    """From 17 rows on: K an odd number of 64-column blocks, some of a tile's parts beyond the last residue."""
+    layer = layer_from_oracle(random_layer(N, K, nbits, group, seed=N), DEV)
+    for M in (17, 130, 257):
+        x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(DEV)
+        err, rounding = errors(layer(x), x.double() @ weight64(layer).t())
+        assert rounding < err < 1.25 * rounding, M           # (and not the fp32 kernel's)
