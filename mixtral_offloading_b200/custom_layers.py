@@ -398,6 +398,7 @@ class ResidentMoe(nn.Module):
         self._experts = list(experts)              # kept out of the module registry like the wrapper does
         self._router = SparseMoeWrapper(config, layer_id, gate, expert_cache=None)
         self._table = None
+        self._key = self._descs = self._held = None        # _expert_key() of the tensors in use, and all their descriptors
         self._shapes, self._bytes = None, {}       # references to the descriptors that give the shapes; bytes per token count
         self._host_counts = None
 
@@ -406,55 +407,85 @@ class ResidentMoe(nn.Module):
         return expert._expert if hasattr(expert, "_expert") else expert
 
     def invalidate(self):
-        """Forget the device-side descriptor table (call after the experts' tensors were replaced or moved)."""
+        """Forget the device-side descriptor table (call after the experts' tensors were replaced or moved: a DecoderLayerDecode
+        and a captured graph keep using what they have; the block's own calls notice it by themselves)."""
         self._table = self._shapes = None
         self._bytes.clear()
 
+    def _expert_key(self):
+        key = _cabi.host().expert_addresses(self._experts)
+        if key is None:                            # a layer without a descriptor, or of another build
+            key = tuple(bytes(lyr.descriptor()) for e in self._experts for lyr in self._layers(e))
+        return key
+
+    def _refresh(self):
+        """Drops the table when an expert's tensors are not those it was built from."""
+        if self._key is None or self._expert_key() != self._key:
+            self.invalidate()
+            layers = [lyr for e in self._experts for lyr in self._layers(e)]
+            self._descs = (_cabi.HqmWeight * len(layers))(*(lyr.descriptor() for lyr in layers))
+            self._held = [getattr(lyr, "_desc", None) for lyr in layers]        # (the key names them by address)
+            self._key = self._expert_key()
+
     @staticmethod
-    def _build_table(experts, device):
-        """The device-side expert table (hqm_expert_table_build): (w1, w2, w3) of experts[0], experts[1], ..."""
-        lib = _cabi.lib()
-        n = 3 * len(experts)
-        descs = (_cabi.HqmWeight * n)()
-        for e, ex in enumerate(experts):
-            f = ResidentMoe._ffn(ex)
-            for i, lyr in enumerate((f.w1, f.w2, f.w3)):
-                descs[3 * e + i] = lyr.descriptor()
+    def _layers(expert):
+        f = ResidentMoe._ffn(expert)
+        return f.w1, f.w2, f.w3
+
+    @staticmethod
+    def _build_table(descriptors, device):
+        """The device-side expert table (hqm_expert_table_build) of an array of descriptors: w1, w2, w3 of one expert after another."""
+        lib, n = _cabi.lib(), len(descriptors)
         nbytes = lib.hqm_expert_table_bytes(n)
         with torch.inference_mode(False):
             host = torch.empty(nbytes + 64, dtype=torch.uint8)
             off = (-host.data_ptr()) % 64
-            _cabi.check(lib.hqm_expert_table_build(C.c_void_p(host.data_ptr() + off), descs, n))
+            _cabi.check(lib.hqm_expert_table_build(C.c_void_p(host.data_ptr() + off), descriptors, n))
             return host[off:off + nbytes].to(device)
 
     def _descriptor_table(self, device):
         if self._table is None:
-            self._table = self._build_table(self._experts, device)
+            self._refresh()
+            self._table = self._build_table(self._descs, device)
         return self._table
 
     def _descriptors(self):
+        """References to expert 0's descriptors; () where the experts are not all alike (the launches over a table take the
+        shapes, the format and the alignment of one for those of all)."""
         if self._shapes is None:
-            f0 = self._ffn(self._experts[0])
-            self._shapes = tuple(C.byref(lyr.descriptor()) for lyr in (f0.w1, f0.w2, f0.w3))
+            self._refresh()
+            words, n = memoryview(bytes(self._descs)).cast("Q").tolist(), C.sizeof(_cabi.HqmWeight) // 8
+            alike = all(words[i:i + 3] == words[i % (3 * n):][:3] for i in range(0, len(words), n)) and \
+                not any(word & 15 for i in range(0, len(words), n) for word in words[i + 3:i + n])     # six int32 of the form, seven addresses
+            self._shapes = tuple(C.byref(self._descs[i]) for i in range(3)) if alike else ()
         return self._shapes
 
     def scratch_bytes(self, tokens: int) -> int:
-        """Workspace of forward_on_device(); 0 where the shapes have no path without a read-back."""
+        """Workspace of forward_on_device(); 0 where the experts have no path without a read-back."""
+        self._refresh()
+        return self._scratch_bytes(tokens)
+
+    def _scratch_bytes(self, tokens: int) -> int:
         if tokens not in self._bytes:
             if len(self._bytes) >= 1024:
                 self._bytes.clear()
             size = _cabi.lib().hqm_moe_decode_scratch_bytes if tokens == 1 else \
                 partial(_cabi.lib().hqm_moe_forward_scratch_bytes, tokens)
-            self._bytes[tokens] = size(self.num_experts, *self._descriptors())
+            self._bytes[tokens] = size(self.num_experts, *self._descriptors()) if self._descriptors() else 0
         return self._bytes[tokens]
 
     def forward_on_device(self, x2: torch.Tensor):
         """The block on rows x2 (tokens, hidden) bf16 with nothing read back; returns (out, router logits)."""
+        if not self.scratch_bytes(x2.shape[0]):
+            raise ValueError("these experts have no path without a read-back")
+        return self._on_device(x2)
+
+    def _on_device(self, x2: torch.Tensor):
         T, E, dev, lib = x2.shape[0], self.num_experts, x2.device, _cabi.lib()
         gate_w = self.gate.weight if self.gate.weight.dtype == torch.bfloat16 else self.gate.weight.to(torch.bfloat16)
         out = torch.empty_like(x2)
         logits = torch.empty((T, E), dtype=torch.bfloat16, device=dev)
-        ws = _scratch(dev, self.scratch_bytes(T))
+        ws = _scratch(dev, self._scratch_bytes(T))
         head = (_cabi.ptr(out), _cabi.ptr(logits), _cabi.ptr(x2), _cabi.ptr(gate_w))
         tail = (_cabi.ptr(self._descriptor_table(dev)), *self._descriptors(), _cabi.ptr(ws), ws.numel(),
                 _cabi.stream_ptr(dev))
@@ -468,7 +499,7 @@ class ResidentMoe(nn.Module):
         T, E = x2.shape[0], self.num_experts
         dev = x2.device
         if self.scratch_bytes(T) and (T == 1 or x2.data_ptr() % 16 == 0):
-            out, logits = self.forward_on_device(x2)
+            out, logits = self._on_device(x2)
             out = out.reshape(batch, seq, hidden)
             if hidden_states.dtype != torch.bfloat16:
                 out, logits = out.to(hidden_states.dtype), logits.to(hidden_states.dtype)

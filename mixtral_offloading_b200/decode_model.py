@@ -239,7 +239,7 @@ class BatchDecode:
     @torch.inference_mode()
     def capture(self) -> None:
         """Records the step (call after at least one plain step at this batch size, so that the library's
-        workspace has its size)."""
+        workspace has its size).  The graphs hold the addresses of the weights: after one is replaced, capture again."""
         dev = self.h.device
         tokens, pos = self.tokens.clone(), self.position.clone()
         caches = [(k[:, :, int(pos)].clone(), v[:, :, int(pos)].clone()) for k, v in zip(self.k_caches, self.v_caches)]

@@ -301,7 +301,8 @@ class ExpertParallelDecoderLayer(nn.Module):
     def _descriptor(self, device) -> _cabi.HqmDecoderLayer:
         attn_desc = self.attention._descriptor()
         if self._table is None:
-            self._table = ResidentMoe._build_table(self._experts, device)
+            layers = [lyr for e in self._experts for lyr in ResidentMoe._layers(e)]
+            self._table = ResidentMoe._build_table((_cabi.HqmWeight * len(layers))(*(lyr.descriptor() for lyr in layers)), device)
         key = (self.attention._layer_key, self.gate.weight.data_ptr(), self.next_ln.data_ptr(), self._table.data_ptr())
         if self._layer is None or self._layer_key != key:
             self._layer_key = key

@@ -24,7 +24,7 @@
 namespace {
 
 struct Names {
-    PyObject *dict, *W_q, *meta, *bias, *plan, *desc, *ready, *scale_q, *zero_q, *meta_scale, *meta_zero, *scale, *zero, *modules, *w1, *w2, *w3, *axis;
+    PyObject *dict, *W_q, *meta, *bias, *plan, *desc, *ready, *expert, *scale_q, *zero_q, *meta_scale, *meta_zero, *scale, *zero, *modules, *w1, *w2, *w3, *axis;
 } N;
 
 PyObject* g_scratch = nullptr;        // custom_layers._SCRATCH: {("cuda", index): uint8 tensor}
@@ -32,15 +32,21 @@ PyObject* g_grow = nullptr;           // custom_layers._scratch(device, bytes)
 PyObject* g_keys[64];                 // ("cuda", index)
 
 // A layer's descriptor (and with it the addresses it was made from) and the workspace of its last row count, as linear
-// layer and as w1 of an expert; kept in the layer's __dict__ for as long as the layer keeps its own descriptor (_desc): the
-// addresses alone do not tell a layer that was quantized again, in another format, into recycled memory.  A copied or pickled
-// layer gets None and makes its own.  The descriptor is never changed once it is made.
+// layer and as w1 of an expert; kept in the layer's __dict__.  It is good for as long as the layer keeps the descriptor it was
+// made from (`of`, the layer's _desc, held here so that its address is not given to another) and its tensors stay where they
+// are: the addresses alone do not tell a layer that was quantized again, in another format, into recycled memory.  A copied or
+// pickled layer gets None and makes its own.  The descriptor is never changed once it is made.
 struct Plan {
     PyObject_HEAD
+    PyObject* of;
     hqm_weight w;
     int64_t linear_rows, expert_rows;
     size_t linear_bytes, f16_bytes, expert_bytes;
 };
+void plan_dealloc(PyObject* self) {
+    Py_XDECREF(reinterpret_cast<Plan*>(self)->of);
+    PyObject_Free(self);
+}
 PyObject* plan_copy(PyObject*, PyObject*) { Py_RETURN_NONE; }
 PyObject* plan_reduce(PyObject*, PyObject*) { return Py_BuildValue("(O())", (PyObject*)Py_TYPE(Py_None)); }
 PyMethodDef plan_methods[] = {{"__deepcopy__", plan_copy, METH_O, nullptr},
@@ -78,21 +84,28 @@ PyObject* own(PyObject* borrowed) {
 }
 const void* address(PyObject* t) { return t != nullptr && THPVariable_Check(t) ? THPVariable_Unpack(t).const_data_ptr() : nullptr; }
 
-// The plan of a layer whose tensors are where they were when its descriptor was made (new reference); null: not to be had here.
-Plan* plan_of(PyObject* layer, PyObject* dict) {
+// The addresses of a layer's seven tensors; false where it is not ready or has another form.
+bool addresses_of(PyObject* dict, const void* (&at)[7]) {
     PyObject* meta = item(dict, N.meta);
     PyObject *ms = item(meta, N.meta_scale), *mz = item(meta, N.meta_zero);
-    if (item(dict, N.ready) != Py_True || ms == nullptr || mz == nullptr) return nullptr;
-    const void* at[7] = {address(item(dict, N.W_q)),    address(item(meta, N.scale_q)), address(item(meta, N.zero_q)), address(item(ms, N.scale)),
-                         address(item(ms, N.zero)), address(item(mz, N.scale)),     address(item(mz, N.zero))};
-    PyObject *kept = item(dict, N.plan), *desc = item(dict, N.desc);
-    if (kept != nullptr && Py_TYPE(kept) == &PlanType && desc != nullptr && desc != Py_None) {
+    if (item(dict, N.ready) != Py_True || ms == nullptr || mz == nullptr) return false;
+    PyObject* t[7] = {item(dict, N.W_q), item(meta, N.scale_q), item(meta, N.zero_q), item(ms, N.scale), item(ms, N.zero), item(mz, N.scale), item(mz, N.zero)};
+    for (int i = 0; i < 7; ++i) at[i] = address(t[i]);
+    return true;
+}
+
+// The plan of a layer whose tensors are where they were when its descriptor was made (new reference); null: not to be had here.
+Plan* plan_of(PyObject* layer, PyObject* dict) {
+    const void* at[7];
+    if (!addresses_of(dict, at)) return nullptr;
+    PyObject* kept = item(dict, N.plan);
+    if (kept != nullptr && Py_TYPE(kept) == &PlanType) {
         Plan* p = reinterpret_cast<Plan*>(kept);
-        if (p->w.W_q == at[0] && p->w.scale_q == at[1] && p->w.zero_q == at[2] && p->w.ms_scale == at[3] && p->w.mz_scale == at[4] &&
+        if (p->of == item(dict, N.desc) && p->w.W_q == at[0] && p->w.scale_q == at[1] && p->w.zero_q == at[2] && p->w.ms_scale == at[3] && p->w.mz_scale == at[4] &&
             p->w.ms_zero == at[5] && p->w.mz_zero == at[6])
             return reinterpret_cast<Plan*>(own(kept));
     }
-    PyObject* axis = item(meta, N.axis);
+    PyObject* axis = item(item(dict, N.meta), N.axis);
     if (axis == nullptr || !PyLong_Check(axis) || PyLong_AsLong(axis) != 0) return nullptr;
     PyObject* d = PyObject_CallMethod(layer, "descriptor", nullptr);      // validates; a ctypes structure
     if (d == nullptr) {
@@ -104,6 +117,7 @@ Plan* plan_of(PyObject* layer, PyObject* dict) {
     if (PyObject_GetBuffer(d, &view, PyBUF_SIMPLE) == 0) {
         if (view.len == (Py_ssize_t)sizeof(hqm_weight) && (p = PyObject_New(Plan, &PlanType)) != nullptr) {
             memcpy(&p->w, view.buf, sizeof(hqm_weight));
+            p->of = own(item(dict, N.desc));
             p->linear_rows = p->expert_rows = -1;
             p->linear_bytes = p->f16_bytes = p->expert_bytes = 0;
             if (PyDict_SetItem(dict, N.plan, reinterpret_cast<PyObject*>(p)) != 0) {
@@ -289,6 +303,37 @@ PyObject* expert(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
 }
 
+// expert_addresses(experts): the addresses of all layers' descriptors and tensors as bytes; None where a layer has no descriptor
+// (its tensors were replaced) or another form.  For as long as the caller holds the descriptors, what it made from them is good
+// while this does not change.
+PyObject* expert_addresses(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 1 || !PyList_CheckExact(args[0])) return PyErr_Format(PyExc_TypeError, "expert_addresses(list)");
+    const Py_ssize_t experts = PyList_GET_SIZE(args[0]);
+    Held<PyObject> out(PyBytes_FromStringAndSize(nullptr, experts * 3 * 8 * (Py_ssize_t)sizeof(void*)));
+    if (!out) return nullptr;
+    char* to = PyBytes_AS_STRING(out.p);
+    PyObject* names[3] = {N.w1, N.w2, N.w3};
+    for (Py_ssize_t e = 0; e < experts; ++e) {
+        if (e >= PyList_GET_SIZE(args[0])) Py_RETURN_NONE;
+        Held<PyObject> module(own(PyList_GET_ITEM(args[0], e)));
+        Held<PyObject> outer(dict_of(module.p));
+        if (PyObject* inner = item(outer.p, N.expert)) module.take(own(inner));       // a wrapper around the expert
+        Held<PyObject> dict(dict_of(module.p));
+        Held<PyObject> modules(own(item(dict.p, N.modules)));
+        for (PyObject* name : names) {
+            Held<PyObject> layer(own(item(modules.p, name)));
+            Held<PyObject> d(layer ? dict_of(layer.p) : nullptr);
+            PyObject* desc = item(d.p, N.desc);
+            const void* at[7];
+            if (desc == nullptr || desc == Py_None || !addresses_of(d.p, at)) Py_RETURN_NONE;
+            memcpy(to, &desc, sizeof(desc));
+            memcpy(to + sizeof(desc), at, sizeof(at));
+            to += sizeof(desc) + sizeof(at);
+        }
+    }
+    return own(out.p);
+}
+
 PyObject* setup(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 2) return PyErr_Format(PyExc_TypeError, "setup(scratch, grow)");
     Py_INCREF(args[0]);
@@ -303,6 +348,7 @@ PyMethodDef methods[] = {
     {"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, "linear(layer, x) -> tensor or None"},
     {"dequantize", (PyCFunction)(void (*)(void))dequantize, METH_FASTCALL, "dequantize(layer, dtype code) -> tensor or None"},
     {"expert", (PyCFunction)(void (*)(void))expert, METH_FASTCALL, "expert(module, x) -> tensor or None"},
+    {"expert_addresses", (PyCFunction)(void (*)(void))expert_addresses, METH_FASTCALL, "expert_addresses(experts) -> bytes or None"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Host path of the quantized layers.", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
@@ -312,13 +358,14 @@ PyMODINIT_FUNC PyInit__host(void) {
     struct {
         PyObject** to;
         const char* name;
-    } all[] = {{&N.dict, "__dict__"}, {&N.W_q, "W_q"},     {&N.meta, "meta"},           {&N.bias, "bias"},           {&N.plan, "_plan"}, {&N.desc, "_desc"}, {&N.ready, "ready"},
+    } all[] = {{&N.dict, "__dict__"}, {&N.W_q, "W_q"},     {&N.meta, "meta"},           {&N.bias, "bias"},           {&N.plan, "_plan"}, {&N.desc, "_desc"}, {&N.ready, "ready"}, {&N.expert, "_expert"},
                {&N.scale_q, "scale_q"}, {&N.zero_q, "zero_q"}, {&N.meta_scale, "meta_scale"}, {&N.meta_zero, "meta_zero"}, {&N.scale, "scale"}, {&N.zero, "zero"},
                {&N.modules, "_modules"}, {&N.w1, "w1"},    {&N.w2, "w2"},               {&N.w3, "w3"}, {&N.axis, "axis"}};
     for (auto& a : all)
         if ((*a.to = PyUnicode_InternFromString(a.name)) == nullptr) return nullptr;
     PlanType.tp_flags = Py_TPFLAGS_DEFAULT;
     PlanType.tp_methods = plan_methods;
+    PlanType.tp_dealloc = plan_dealloc;
     if (PyType_Ready(&PlanType) != 0) return nullptr;
     return PyModule_Create(&module);
 }
