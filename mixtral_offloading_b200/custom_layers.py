@@ -482,7 +482,9 @@ class ResidentMoe(nn.Module):
 
     def _on_device(self, x2: torch.Tensor):
         T, E, dev, lib = x2.shape[0], self.num_experts, x2.device, _cabi.lib()
-        gate_w = self.gate.weight if self.gate.weight.dtype == torch.bfloat16 else self.gate.weight.to(torch.bfloat16)
+        gate_w = self.gate.weight
+        if gate_w.dtype != torch.bfloat16 or not gate_w.is_contiguous():
+            gate_w = gate_w.to(torch.bfloat16).contiguous()
         out = torch.empty_like(x2)
         logits = torch.empty((T, E), dtype=torch.bfloat16, device=dev)
         ws = _scratch(dev, self._scratch_bytes(T))

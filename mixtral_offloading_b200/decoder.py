@@ -171,7 +171,7 @@ class DecoderLayerDecode(nn.Module):
             self._layer_key = key
             hidden = self.attention.n_heads * self.attention.head_dim
             gate = self.moe.gate.weight
-            self._gate_w = gate if gate.dtype == torch.bfloat16 else gate.to(torch.bfloat16)
+            self._gate_w = gate.to(torch.bfloat16).contiguous()
             f0 = self.moe._ffn(self.moe._experts[0])
             self._layer = _cabi.HqmDecoderLayer(
                 attn=attn_desc, gate_w=self._gate_w.data_ptr(),
@@ -308,7 +308,7 @@ class ExpertParallelDecoderLayer(nn.Module):
             self._layer_key = key
             hidden = self.attention.n_heads * self.attention.head_dim
             gate = self.gate.weight
-            self._gate_w = gate if gate.dtype == torch.bfloat16 else gate.to(torch.bfloat16)
+            self._gate_w = gate.to(torch.bfloat16).contiguous()
             f0 = ResidentMoe._ffn(self._experts[0])
             self._layer = _cabi.HqmDecoderLayer(
                 attn=attn_desc, gate_w=self._gate_w.data_ptr(), table=self._table.data_ptr(), w1=f0.w1.descriptor(),

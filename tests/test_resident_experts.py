@@ -1,5 +1,5 @@
-"""ResidentMoe computes with the experts as they are at the call: replaced, of different formats, at odd
-addresses."""
+"""ResidentMoe computes with the experts as they are at the call: replaced, of different formats, at odd addresses; and with a
+gate of any strides."""
 import pytest
 import torch
 
@@ -99,4 +99,13 @@ def test_expert_at_an_odd_address():
     room = torch.empty(layer.W_q.numel() + 4, dtype=torch.uint8, device=DEV)
     layer.W_q = room[4:].copy_(layer.W_q.view(-1)).view(layer.W_q.shape)
     assert block.moe.scratch_bytes(1) == block.moe.scratch_bytes(40) == 0
+    block.check()
+
+
+def test_gate_with_other_strides():
+    block = _Block()
+    wide = torch.zeros(HIDDEN, EXPERTS + 3, dtype=torch.bfloat16, device=DEV)
+    wide[:, :EXPERTS] = block.gate.weight.data.t()
+    block.gate.weight.data = wide[:, :EXPERTS].t()
+    assert not block.gate.weight.is_contiguous()
     block.check()
