@@ -146,11 +146,9 @@ struct Params {
     const unsigned char* xt;
     int64_t xt_rows;
     const float* row_scale;                // of the staged rows (null: 1)
-    int mode;
     int y_f16;
     unsigned char* ht;
     void* out;
-    int out_f16;
     const int32_t* out_idx;
     const float* row_w;
     int accumulate;
@@ -185,16 +183,15 @@ struct Fmt {
     // Columns of a unit.  What a warp does once per unit (waits, decoding, hand-over) takes about as long as the weights of
     // 128 columns of a 2-bit tile, and those layers are large; 4-bit layers decode little and may be small.
     static constexpr int UK = 128;
-    static constexpr int HALVES = UK / 128;                // A slots of a unit
     static constexpr int BLOCKS = UK / 64;
     static constexpr int SLW = 2;                          // rows of scales a warp needs: its slot of two parts
     static constexpr int CODE_PART = MEMBERS * 128 * (WORDS ? 4 : 1);             // packed bytes of a part of 128 columns
-    static constexpr int CODE_HALF = PARTS * CODE_PART;
     static constexpr int SZ_PART = PER * 128;
-    static constexpr int SQ_OFF = HALVES * CODE_HALF, ZQ_OFF = SQ_OFF + HALVES * PARTS * SZ_PART;
-    static constexpr int RAW_TX = ZQ_OFF + HALVES * PARTS * SZ_PART;
+    static constexpr int SQ_OFF = PARTS * CODE_PART, ZQ_OFF = SQ_OFF + PARTS * SZ_PART;
+    static constexpr int RAW_TX = ZQ_OFF + PARTS * SZ_PART;
     static constexpr int RAW_BYTES = (RAW_TX + 1023) / 1024 * 1024;
     static constexpr int DC = UK * SLW / 32;               // columns a lane decodes
+    static_assert(UK == 128 && DC == 8, "an A slot holds a unit; a lane's columns are one 16-byte load of fp16");
     static constexpr int ST_WARP = SLW * UK * 4;           // s and t of a warp's rows
     static constexpr int ST_BLOCK = 2 * SLW * 64, ST_T = BLOCKS * ST_BLOCK;
     // Launches of up to 64 rows per chunk need few staged rows in flight and many packed bytes, others the reverse.
@@ -348,11 +345,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
 __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
@@ -465,7 +457,7 @@ __device__ __forceinline__ bool next_seg(const Shared& sh, int ubegin, int uend,
 template <int NBITS, int MODE>
 __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__ Params prm) {
     using F = Fmt<NBITS>;
-    constexpr int PER = F::PER, PARTS = F::PARTS, SLW = F::SLW, UK = F::UK, HALVES = F::HALVES, BLOCKS = F::BLOCKS, DC = F::DC;
+    constexpr int PER = F::PER, PARTS = F::PARTS, SLW = F::SLW, UK = F::UK, BLOCKS = F::BLOCKS, DC = F::DC;
     extern __shared__ unsigned char smem_raw[];
     __shared__ Shared sh;
     const uint32_t raw0 = smem_u32(smem_raw);
@@ -596,7 +588,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
         // the row of scales / zeros this lane decodes: DC columns of it
         const int dlocal = lane >> 4, dpart = F::part_of(q, dlocal);
         const int dcol = DC * (lane & (UK / DC - 1));
-        const int dhalf = dcol >> 7;
         // The field of the warp's slot inside a byte.  2 bit: slots 0, 1 at bits 7-6, 5-4, slots 2, 3 at 3-2, 1-0; 4 bit: 7-4 or
         // 3-0.  `upper`: it lies in the upper half of the byte; fpos: its first bit inside that half.
         const bool upper = (NBITS == 2) ? q < 2 : (q & 1) == 0;
@@ -627,19 +618,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
         auto load_meta = [&]() {
             if ((mC & 7) == 0) {
 #pragma unroll
-                for (int h = 0; h < (DC + 7) / 8; ++h) {
-                    int col = mcol + 8 * h;
-                    if (col >= mC) col -= mC;
-#pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-                        if constexpr (DC >= 8) {
-                            const uint4 v = __ldg(reinterpret_cast<const uint4*>(mp[a] + col));
-                            mt[a][4 * h] = v.x; mt[a][4 * h + 1] = v.y; mt[a][4 * h + 2] = v.z; mt[a][4 * h + 3] = v.w;
-                        } else {
-                            const uint2 v = __ldg(reinterpret_cast<const uint2*>(mp[a] + col));
-                            mt[a][0] = v.x; mt[a][1] = v.y;
-                        }
-                    }
+                for (int a = 0; a < 4; ++a) {
+                    const uint4 v = __ldg(reinterpret_cast<const uint4*>(mp[a] + mcol));
+                    mt[a][0] = v.x; mt[a][1] = v.y; mt[a][2] = v.z; mt[a][3] = v.w;
                 }
             } else {                                          // a run of columns may wrap around anywhere: one by one
 #pragma unroll
@@ -651,7 +632,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                     }
             }
         };
-        static_assert(HALVES == 1, "an A slot holds a unit");
         int r = group, v = group;                             // slots of this group's next unit: packed bytes; A, and its phase
         uint32_t r_par = 0, v_round = 0, limit = WAIT_LIMIT, raw_ready = 0, a_ready = 0;
         // The A slot that has been written and not yet handed to the MMAs: the stores are waited for when the next unit's loads
@@ -699,8 +679,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 uint4 wv[4];
                 auto load_codes = [&](int sub) {
                     if constexpr (F::WORDS) return;
-                    const uint32_t at0 = rw + (sub >> 1) * F::CODE_HALF;
-                    const uint32_t c0 = at0 + (code_off[0] ^ (64u * (sub & 1))), c1 = at0 + (code_off[1] ^ (64u * (sub & 1)));
+                    const uint32_t c0 = rw + (code_off[0] ^ (64u * sub)), c1 = rw + (code_off[1] ^ (64u * sub));
                     wv[0] = lds128(c0);
                     wv[1] = lds128(c1);
                     wv[2] = lds128(c0 + J2);
@@ -709,20 +688,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 // ---- scale and zero of the warp's rows
                 bool big = false;
                 {
-                    const uint32_t sqa = rw + F::SQ_OFF + (dhalf * PARTS + dpart) * F::SZ_PART + slot * 128 + (dcol & 127);
+                    const uint32_t sqa = rw + F::SQ_OFF + dpart * F::SZ_PART + slot * 128 + dcol;
                     constexpr int ZS = F::ZQ_OFF - F::SQ_OFF;
-                    uint32_t sq[DC / 4], zq[DC / 4];
-                    if constexpr (DC == 16) {
-                        const uint4 a = lds128(sqa), b = lds128(sqa + ZS);
-                        sq[0] = a.x; sq[1] = a.y; sq[2] = a.z; sq[3] = a.w;
-                        zq[0] = b.x; zq[1] = b.y; zq[2] = b.z; zq[3] = b.w;
-                    } else if constexpr (DC == 8) {
-                        const uint2 a = lds64(sqa), b = lds64(sqa + ZS);
-                        sq[0] = a.x; sq[1] = a.y; zq[0] = b.x; zq[1] = b.y;
-                    } else {
-                        sq[0] = lds32(sqa);
-                        zq[0] = lds32(sqa + ZS);
-                    }
+                    const uint2 s8 = lds64(sqa), z8 = lds64(sqa + ZS);
+                    const uint32_t sq[DC / 4] = {s8.x, s8.y}, zq[DC / 4] = {z8.x, z8.y};
                     load_codes(0);                            // on their way while the scales are decoded
                     hand_over();
                     a_ready = v_round > 0 ? peek(a_empty + 8 * (v + ((v_round & 1) ? 0 : NA)), ((v_round - 1) >> 1) & 1) : 1u;
@@ -785,19 +754,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                             asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst), "r"(S[2 * h]), "r"(S[2 * h + 1]) : "memory");
                             asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst + F::ST_T), "r"(T[2 * h]), "r"(T[2 * h + 1]) : "memory");
                         }
-                    } else
-#pragma unroll
-                    for (int h = 0; h < (DC + 7) / 8; ++h) {
-                        const int w64 = (dcol + 8 * h) & 63, blk = (dcol + 8 * h) >> 6;
-                        const uint32_t dst = st_area + blk * F::ST_BLOCK + ((w64 >> 3) & 1) * (SLW * 64) + dlocal * 64 +
-                                             (w64 >> 4) * 16 + (w64 & 7) * 2;
-                        if constexpr (DC >= 8) {
-                            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(S[4 * h]), "r"(S[4 * h + 1]), "r"(S[4 * h + 2]), "r"(S[4 * h + 3]) : "memory");
-                            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + F::ST_T), "r"(T[4 * h]), "r"(T[4 * h + 1]), "r"(T[4 * h + 2]), "r"(T[4 * h + 3]) : "memory");
-                        } else {
-                            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst), "r"(S[0]), "r"(S[1]) : "memory");
-                            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(dst + F::ST_T), "r"(T[0]), "r"(T[1]) : "memory");
-                        }
+                    } else {
+                        const int w64 = dcol & 63, blk = dcol >> 6;
+                        const uint32_t dst = st_area + blk * F::ST_BLOCK + ((w64 >> 3) & 1) * (SLW * 64) + dlocal * 64 + (w64 >> 4) * 16;
+                        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(S[0]), "r"(S[1]), "r"(S[2]), "r"(S[3]) : "memory");
+                        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + F::ST_T), "r"(T[0]), "r"(T[1]), "r"(T[2]), "r"(T[3]) : "memory");
                     }
                 }
                 if (k + GROUPS < s.k1) {                      // the next unit's meta values
@@ -808,86 +769,82 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 __syncwarp();
                 // ---- the weights, 64 columns at a time
                 const int subs = min(BLOCKS, prm.subs_k - BLOCKS * k);
-#pragma unroll
-                for (int half = 0; half < HALVES; ++half) {
-                    // The A slot's tile of the round before has been read by its MMAs.  (A parity only tells the last phase from
-                    // the one before it: even and odd rounds have barriers of their own.)
-                    if (v_round > 0) wait_peeked(a_empty + 8 * (v + ((v_round & 1) ? 0 : NA)), ((v_round - 1) >> 1) & 1, a_ready, limit);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t ta = tmem + tmap.a_base + 64 * v + ((uint32_t)(32 * q) << 16);
+                // The A slot's tile of the round before has been read by its MMAs.  (A parity only tells the last phase from
+                // the one before it: even and odd rounds have barriers of their own.)
+                if (v_round > 0) wait_peeked(a_empty + 8 * (v + ((v_round & 1) ? 0 : NA)), ((v_round - 1) >> 1) & 1, a_ready, limit);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ta = tmem + tmap.a_base + 64 * v + ((uint32_t)(32 * q) << 16);
 #pragma unroll 1                                  // (unrolled it is 3 % slower: the code of 16 warps at different places)
-                    for (int sub2 = 0; sub2 < 2; ++sub2) {
-                        const int sub = 2 * half + sub2;
-                        if (sub < subs) {
-                            const uint32_t sa = st_read + sub * F::ST_BLOCK;
-                            const uint4 S0 = lds128(sa), S1 = lds128(sa + SLW * 64), T0 = lds128(sa + F::ST_T), T1 = lds128(sa + F::ST_T + SLW * 64);
-                            if (sub) load_codes(sub);
-                            const uint32_t SS[8] = {S0.x, S0.y, S0.z, S0.w, S1.x, S1.y, S1.z, S1.w};
-                            const uint32_t TT[8] = {T0.x, T0.y, T0.z, T0.w, T1.x, T1.y, T1.z, T1.w};
-                            if constexpr (F::WORDS) {
-                                const uint32_t at0 = rw + words3 + 256u * sub;
-                                auto all3 = [&](auto&& weight) {
-#pragma unroll
-                                    for (int h = 0; h < 2; ++h) {
-                                        uint32_t o[16];
-#pragma unroll
-                                        for (int b = 0; b < 2; ++b)
-#pragma unroll
-                                            for (int i = 0; i < 4; ++i) {
-                                                const uint4 v = lds128(at0 + (2 * h + b) * 2048 + 64 * i);
-                                                o[4 * i + 2 * b] = weight(perm(v.x, v.z, mine.sel) * mine.up, SS[2 * i], TT[2 * i]);
-                                                o[4 * i + 2 * b + 1] = weight(perm(v.y, v.w, mine.sel) * mine.up, SS[2 * i + 1], TT[2 * i + 1]);
-                                            }
-                                        store_a(ta + 32 * sub2 + ((uint32_t)(16 * h) << 16), o);
-                                    }
-                                };
-                                const uint32_t magic = 0x64006400u;                                                     // 1024
-                                if (!big) all3([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(x & mine.mask, S, T); });
-                                else all3([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x, mine.mask, magic), magic), S, T); });
-                                continue;
-                            }
-                            // one pair of weights per (member, word i, e): fields of bytes (0, 2) and (1, 3) of the word
-                            auto all = [&](auto&& pair_lo, auto&& pair_hi) {
+                for (int sub = 0; sub < 2; ++sub) {
+                    if (sub < subs) {
+                        const uint32_t sa = st_read + sub * F::ST_BLOCK;
+                        const uint4 S0 = lds128(sa), S1 = lds128(sa + SLW * 64), T0 = lds128(sa + F::ST_T), T1 = lds128(sa + F::ST_T + SLW * 64);
+                        if (sub) load_codes(sub);
+                        const uint32_t SS[8] = {S0.x, S0.y, S0.z, S0.w, S1.x, S1.y, S1.z, S1.w};
+                        const uint32_t TT[8] = {T0.x, T0.y, T0.z, T0.w, T1.x, T1.y, T1.z, T1.w};
+                        if constexpr (F::WORDS) {
+                            const uint32_t at0 = rw + words3 + 256u * sub;
+                            auto all3 = [&](auto&& weight) {
 #pragma unroll
                                 for (int h = 0; h < 2; ++h) {
                                     uint32_t o[16];
 #pragma unroll
-                                    for (int b = 0; b < 2; ++b) {
-                                        const uint4 vv = wv[2 * h + b];
-                                        const uint32_t w[4] = {vv.x, vv.y, vv.z, vv.w};
+                                    for (int b = 0; b < 2; ++b)
 #pragma unroll
                                         for (int i = 0; i < 4; ++i) {
-                                            o[4 * i + 2 * b] = pair_lo(w[i], SS[2 * i], TT[2 * i]);
-                                            o[4 * i + 2 * b + 1] = pair_hi(w[i], SS[2 * i + 1], TT[2 * i + 1]);
+                                            const uint4 v = lds128(at0 + (2 * h + b) * 2048 + 64 * i);
+                                            o[4 * i + 2 * b] = weight(perm(v.x, v.z, mine.sel) * mine.up, SS[2 * i], TT[2 * i]);
+                                            o[4 * i + 2 * b + 1] = weight(perm(v.y, v.w, mine.sel) * mine.up, SS[2 * i + 1], TT[2 * i + 1]);
                                         }
-                                    }
-                                    store_a(ta + 32 * sub2 + ((uint32_t)(16 * h) << 16), o);
+                                    store_a(ta + 32 * sub + ((uint32_t)(16 * h) << 16), o);
                                 }
                             };
-                            // (the shift to the left is written as a product: it then runs beside the ANDs, on the other pipe)
-                            if (f16 && !big) {
-                                if (upper)
-                                    all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(x & mask_hi, S, T); },
-                                        [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x >> 8) & mask_hi, S, T); });
-                                else
-                                    all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x * 16u) & mask_hi, S, T); },
-                                        [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x >> 4) & mask_hi, S, T); });
-                            } else if (f16) {
-                                const uint32_t magic = 0x64006400u, mul = upper ? 1u : 16u, sh = upper ? 8u : 4u;      // 1024
-                                all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x * mul, mask_hi, magic), magic), S, T); },
-                                    [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x >> sh, mask_hi, magic), magic), S, T); });
-                            } else {
-                                const uint32_t magic = 0x43004300u, sl = upper ? 4u : 0u;                               // 128
-                                all([&](uint32_t x, uint32_t S, uint32_t T) { return bf2_fma(bf2_sub(lop_and_or(x >> sl, mask_lo, magic), magic), S, T); },
-                                    [&](uint32_t x, uint32_t S, uint32_t T) { return bf2_fma(bf2_sub(lop_and_or(x >> (sl + 8u), mask_lo, magic), magic), S, T); });
+                            const uint32_t magic = 0x64006400u;                                                     // 1024
+                            if (!big) all3([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(x & mine.mask, S, T); });
+                            else all3([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x, mine.mask, magic), magic), S, T); });
+                            continue;
+                        }
+                        // one pair of weights per (member, word i, e): fields of bytes (0, 2) and (1, 3) of the word
+                        auto all = [&](auto&& pair_lo, auto&& pair_hi) {
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                uint32_t o[16];
+#pragma unroll
+                                for (int b = 0; b < 2; ++b) {
+                                    const uint4 vv = wv[2 * h + b];
+                                    const uint32_t w[4] = {vv.x, vv.y, vv.z, vv.w};
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) {
+                                        o[4 * i + 2 * b] = pair_lo(w[i], SS[2 * i], TT[2 * i]);
+                                        o[4 * i + 2 * b + 1] = pair_hi(w[i], SS[2 * i + 1], TT[2 * i + 1]);
+                                    }
+                                }
+                                store_a(ta + 32 * sub + ((uint32_t)(16 * h) << 16), o);
                             }
+                        };
+                        // (the shift to the left is written as a product: it then runs beside the ANDs, on the other pipe)
+                        if (f16 && !big) {
+                            if (upper)
+                                all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(x & mask_hi, S, T); },
+                                    [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x >> 8) & mask_hi, S, T); });
+                            else
+                                all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x * 16u) & mask_hi, S, T); },
+                                    [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma((x >> 4) & mask_hi, S, T); });
+                        } else if (f16) {
+                            const uint32_t magic = 0x64006400u, mul = upper ? 1u : 16u, sh = upper ? 8u : 4u;      // 1024
+                            all([&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x * mul, mask_hi, magic), magic), S, T); },
+                                [&](uint32_t x, uint32_t S, uint32_t T) { return h2fma(h2sub(lop_and_or(x >> sh, mask_hi, magic), magic), S, T); });
+                        } else {
+                            const uint32_t magic = 0x43004300u, sl = upper ? 4u : 0u;                               // 128
+                            all([&](uint32_t x, uint32_t S, uint32_t T) { return bf2_fma(bf2_sub(lop_and_or(x >> sl, mask_lo, magic), magic), S, T); },
+                                [&](uint32_t x, uint32_t S, uint32_t T) { return bf2_fma(bf2_sub(lop_and_or(x >> (sl + 8u), mask_lo, magic), magic), S, T); });
                         }
                     }
-                    // The staged bytes have been read.  (Only here: what was loaded has been used by every lane.)
-                    __syncwarp();
-                    if (lane == 0) arrive(raw_empty + 8 * r);
-                    pending = a_full + 8 * v;
                 }
+                // The staged bytes have been read.  (Only here: what was loaded has been used by every lane.)
+                __syncwarp();
+                if (lane == 0) arrive(raw_empty + 8 * r);
+                pending = a_full + 8 * v;
                 r += GROUPS;
                 if (r >= n_raw) {
                     r -= n_raw;
@@ -948,15 +905,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                     if (leader) {
                         expect_tx(bar, F::RAW_TX);
 #pragma unroll
-                        for (int h = 0; h < HALVES; ++h)
-#pragma unroll
-                            for (int p = 0; p < PARTS; ++p) {
-                                const int rho = (MODE == GG_UP) ? rho0 : rho0 + p, col = k * UK + 128 * h;
-                                const CUtensorMap* map = maps[MODE == GG_UP ? p : 0];
-                                tma_3d(dst + h * F::CODE_HALF + p * F::CODE_PART, map, col, rho, m0, bar);
-                                tma_3d(dst + F::SQ_OFF + (h * PARTS + p) * F::SZ_PART, map + 1, col, PER * rho, 0, bar);
-                                tma_3d(dst + F::ZQ_OFF + (h * PARTS + p) * F::SZ_PART, map + 2, col, PER * rho, 0, bar);
-                            }
+                        for (int p = 0; p < PARTS; ++p) {
+                            const int rho = (MODE == GG_UP) ? rho0 : rho0 + p;
+                            const CUtensorMap* map = maps[MODE == GG_UP ? p : 0];
+                            tma_3d(dst + p * F::CODE_PART, map, k * UK, rho, m0, bar);
+                            tma_3d(dst + F::SQ_OFF + p * F::SZ_PART, map + 1, k * UK, PER * rho, 0, bar);
+                            tma_3d(dst + F::ZQ_OFF + p * F::SZ_PART, map + 2, k * UK, PER * rho, 0, bar);
+                        }
                     }
                 }
             }
@@ -1286,12 +1241,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                             const uint16_t* src = tb + t * 128 + m * RUN;
                             const int64_t row = MODE == GG_DOWN ? s_row[c0 + t] : list + c0 + t;
                             uint16_t* dst = out + row * ld + (int64_t)(m0 + m) * pr.G + PER * rho0;
-                            if (MODE == GG_DOWN && (prm.accumulate || prm.out_f16)) {
-                                for (int x = 0; x < valid; ++x) {
-                                    float val = bf16_bits_to_float(src[x]);
-                                    if (prm.accumulate) val += bf16_bits_to_float(dst[x]);
-                                    dst[x] = prm.out_f16 ? __half_as_ushort(__float2half_rn(val)) : float_to_bf16_bits(val);
-                                }
+                            if (MODE == GG_DOWN && prm.accumulate) {
+                                for (int x = 0; x < valid; ++x) dst[x] = float_to_bf16_bits(bf16_bits_to_float(src[x]) + bf16_bits_to_float(dst[x]));
                             } else if (valid == RUN && (((uintptr_t)dst) & (RUN * 2 - 1)) == 0) {
                                 if constexpr (RUN == 8) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
                                 else if constexpr (RUN == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
@@ -1586,11 +1537,9 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
     p.xt = (const unsigned char*)job.x.data;
     p.row_scale = job.x.scale;
     p.xt_rows = job.x.rows;
-    p.mode = job.mode;
     p.y_f16 = job.y_f16;
     p.ht = (unsigned char*)job.ht;
     p.out = job.out;
-    p.out_f16 = job.out_f16;
     p.out_idx = job.out_idx;
     p.row_w = job.row_w;
     p.accumulate = job.accumulate;
@@ -1607,7 +1556,7 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
     }
 #define HQM_GG(B, M) \
     if (nbits == B && job.mode == M) return gg_launch_one<B, M>(p, grid, st);
-    HQM_GG(2, GG_LINEAR) HQM_GG(2, GG_UP) HQM_GG(2, GG_DOWN) HQM_GG(4, GG_LINEAR) HQM_GG(4, GG_DOWN)
+    HQM_GG(2, GG_LINEAR) HQM_GG(2, GG_UP) HQM_GG(2, GG_DOWN) HQM_GG(4, GG_LINEAR)
     HQM_GG(3, GG_LINEAR)
 #undef HQM_GG
     set_error("gemm: no kernel for nbits=%d group_size=%d mode=%d", nbits, gs, (int)job.mode);

@@ -73,7 +73,6 @@ struct GgJob {
     void* ht;                             // staged h
     // GG_DOWN
     void* out;                            // (*, H)
-    int out_f16;
     const int32_t* out_idx;               // row of `out` of list entry i (null: i)
     const float* row_w;                   // weight of list entry i (null: 1)
     int accumulate;
