@@ -607,8 +607,8 @@ def run_decode(args):
             torch.cuda.synchronize(dev)
             ms8 = k0.elapsed_time(k1) / (steps8 - 2)
             batch8 = {"tokens_per_s": B8 * 1e3 / (ms8 * 32.0 / L), "ms_per_step": ms8, "steps": steps8 - 2,
-                      "what": f"8 sequences, one token each per step, context {args.context} each; per layer one recorded "
-                              "segment (attention half + router), one read-back of the routing, the active experts"}
+                      "what": f"8 sequences, one token each per step, context {args.context} each; the whole step recorded as "
+                              "one CUDA graph (experts chosen on the device), nothing read back inside it"}
             del bd
         clocks = sampler.stop() if sampler is not None else None
         # prompt processing through the same model: a 512-token prompt in one pass (informative, rank 0 only)

@@ -121,8 +121,8 @@ int hqm_scratch_init(void* scratch, void* stream);
 /* Bytes of scratch hqm_linear needs for M rows of this layer (0 if none). */
 size_t hqm_linear_scratch_bytes(int64_t M, const hqm_weight* w);
 
-/* The same for the fastest launch: with less, hqm_linear at five or more rows spreads over fewer
- * SMs.  At least hqm_linear_scratch_bytes(). */
+/* The same for the fastest launch: with less, the tcgen05 kernel spreads over fewer SMs or takes the rows in several
+ * passes.  At least hqm_linear_scratch_bytes(). */
 size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w);
 
 /* HQQLinearTritonSavable.forward / forward_triton (custom_layers.py:49-92) with the
@@ -130,21 +130,24 @@ size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w);
  * and the per-call 8-bit scale/zero decode fused in:
  *   y[M, N] = x[M, K] . W_est^T (+ bias[N]),  fp32 accumulation, bf16 in/out.
  * bias may be NULL.  scratch may be NULL when hqm_linear_scratch_bytes() is 0.
- * Rows 1..4 take the weight-streaming kernels, 5 and more the tcgen05 kernels; HQM_FORCE_GENERIC=1 in the environment
- * at load time routes everything through the shape-agnostic kernel. */
-/* hqm_linear for fp16 x and y (five or more rows; the scratch size is 0 where only hqm_linear takes the layer). */
+ * 1 to 4 rows (3 bit: one) take the weight-streaming kernels, more the tcgen05 kernels, formats and shapes that neither
+ * covers and unaligned x the shape-agnostic one; HQM_FORCE_GENERIC=1 in the environment at load time routes everything
+ * through that. */
+int hqm_linear(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias,
+               void* scratch, size_t scratch_bytes, void* stream);
+
+/* hqm_linear for fp16 x and y, where the tcgen05 kernel takes the call (five or more rows, 3 bit: two); the scratch size is
+ * 0 where only hqm_linear does. */
 size_t hqm_linear_f16_scratch_bytes(int64_t M, const hqm_weight* w);
 int hqm_linear_f16(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias, void* scratch,
                    size_t scratch_bytes, void* stream);
 
 /* Up to four layers of one K, bit width and group size over the same rows (q, k and v of a decoder layer) in one launch:
- * y[i] = x . W_est[i]^T (+ bias[i]); bias may be NULL.  Five or more rows; the scratch size is 0 for
+ * y[i] = x . W_est[i]^T (+ bias[i]); bias may be NULL.  Row counts as for hqm_linear_f16; the scratch size is 0 for
  * everything else. */
 size_t hqm_linear_group_scratch_bytes(int64_t M, const hqm_weight* const* w, int32_t count);
 int hqm_linear_group(uint16_t* const* y, const uint16_t* x, int64_t M, const hqm_weight* const* w, const uint16_t* const* bias,
                      int32_t count, void* scratch, size_t scratch_bytes, void* stream);
-int hqm_linear(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias,
-               void* scratch, size_t scratch_bytes, void* stream);
 
 /* Same result as hqm_linear, for callers that cannot hand over a scratch buffer: code
  * running under CUDA stream capture (where allocating is not allowed), hosts that pass

@@ -74,7 +74,7 @@ int set_overlap(int on) {
 }
 
 // Rows from which a layer goes to the tensor-core kernel (gemm_grouped.cu); below, the streaming kernels,
-// whose work per weight grows with the rows, are faster.
+// whose work per weight grows with the rows, are faster (figures at GG_MIN_ROWS).
 // (3 bit: from two on, as the streaming kernel takes one row per launch: 14336 x 4096 21 us each, here 29 up to 16 rows.)
 static bool use_gg(const hqm_weight* w, int G, int C, int64_t M) {
     return M >= (w->nbits == 3 ? 2 : GG_MIN_ROWS) && M <= (1 << 22) && gg_takes(w, G, C, M);
@@ -240,7 +240,7 @@ int hqm_linear_f16(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* 
                    size_t scratch_bytes, void* stream) {
     using namespace hqm;
     const size_t need = hqm_linear_f16_scratch_bytes(M, w);
-    HQM_CHECK_ARG(need != 0, "linear_f16: five or more rows of a layer that the tensor-core kernel takes are needed");
+    HQM_CHECK_ARG(need != 0, "linear_f16: rows and a layer that the tensor-core kernel takes are needed");
     HQM_CHECK_ARG(y && x && (reinterpret_cast<uintptr_t>(x) & 15u) == 0, "linear_f16: null or unaligned activation pointer");
     if (scratch == nullptr || scratch_bytes < need) {
         set_error("linear_f16: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
@@ -267,7 +267,7 @@ int hqm_linear_group(uint16_t* const* y, const uint16_t* x, int64_t M, const hqm
                      int32_t count, void* scratch, size_t scratch_bytes, void* stream) {
     using namespace hqm;
     const size_t need = hqm_linear_group_scratch_bytes(M, w, count);
-    HQM_CHECK_ARG(need != 0, "linear_group: layers of one K and format and five or more rows are needed");
+    HQM_CHECK_ARG(need != 0, "linear_group: layers of one K and format, and rows that the tensor-core kernel takes, are needed");
     HQM_CHECK_ARG(y && x && (reinterpret_cast<uintptr_t>(x) & 15u) == 0, "linear_group: null or unaligned activation pointer");
     for (int i = 0; i < count; ++i) HQM_CHECK_ARG(y[i] != nullptr, "linear_group: null output %d", i);
     if (scratch == nullptr || scratch_bytes < need) {

@@ -561,6 +561,8 @@ __global__ void __launch_bounds__(NORM_THREADS) add_f32_rmsnorm_kernel(uint16_t*
     }
 }
 
+// rotate-half RoPE of the pair (a, b) = (t[d], t[d + 64]) at position pos, bf16 arithmetic as Hugging Face does it
+// (rope_pair), as the angle of column d and the rotation by it.
 __device__ __forceinline__ void rope_angle(int d, int pos, float theta, float& sn, float& cs) {
     const float inv_freq = powf(theta, -(float)(2 * d) / (float)HEAD_DIM);
     sincosf((float)pos * inv_freq, &sn, &cs);
@@ -632,7 +634,6 @@ struct QkvSource {                 // FUSED only: where q, k, v of this token co
     int* error_flag;
 };
 
-// rotate-half RoPE of the pair (a, b) = (t[d], t[d + 64]) at position pos, bf16 arithmetic as Hugging Face does it
 // The end of a greedy step: token = index of the largest of `vocab` bf16 logits (the first of equal ones; a NaN is larger
 // than everything), position += 1.  One CTA: 64 KB of logits that the launch in front has just written are one round trip
 // to L2 for 1024 threads.  (A reduction over the whole chip, a copy and an addition before: 15 us, 6 now.)

@@ -21,8 +21,10 @@
 //     multiplied by 4 at the end.  -z*s is formed from an fp32 z: with z in fp16 the two roundings of z are the largest
 //     errors of all (4 bit: 1.07e-3 of the result against 5.5e-4; the streaming kernels' fp16 x * s give 9.8e-4).  Where s * 2^(22-p) leaves the fp16 range (s >= 1/4), the warp takes the longer way
 //     for that unit: OR into 1024, exact subtract, FMA.  x is staged as fp16 with a power-of-two factor per row.
-//   * bf16 (down projections of more than 16 rows: h has no factor per row and may exceed fp16): OR into 128, exact
-//     subtract, FMA.
+//   * bf16 (down projections of more than GG_F16_ROWS rows): OR into 128, exact subtract, FMA.  h has no factor per row, as
+//     a row's largest value is not known until every tile of it is finished.  Up to GG_F16_ROWS rows it is fp16 all the same:
+//     like the streaming kernels, which took those row counts before and have the same limit, such a launch overflows
+//     where |h| exceeds 65504, and one with more rows does not; it keeps three more bits of every h for that.
 //
 // Measured on B200 (148 SMs): LOP3 / SHF / PRMT and HFMA2 both issue every second cycle per scheduler but on two
 // pipes; tcgen05.st of a 128 x 64 tile takes 65 cycles; tcgen05.mma (K = 16, A in TMEM) 15 / 32 / 64 / 128 cycles at
@@ -41,17 +43,20 @@
 // row count, and every CTA takes an equal contiguous share.  A tile cut by a share's boundary is summed from fp32
 // pieces in scratch memory by whichever CTA arrives last, in CTA order (no atomics on results, deterministic).
 //
-// Measured (one launch; before: the same layers through a kernel that staged A in shared memory, expert by expert):
-// up + gate of 8 experts, 4096 -> 14336, 33 tokens: 201 us, down 102 us; the whole block 943 -> 316 us.  One expert with
-// 512 rows 325 -> 238 us.  A unit takes ~930 cycles (2440 warp instructions) at few rows: without the decoding of scales
-// and zeros, the weights' arithmetic and the MMAs the same pipeline runs at ~430.  At 256 rows it is the staged x that
-// bounds it (64 KB per unit into every SM).
+// Measured (before: the same layers through a kernel that staged A in shared memory, expert by expert): up + gate of 8
+// experts, 4096 -> 14336, 33 tokens: 201 us alone, down 103 us; the whole block 943 -> 299 us.  One expert with 512 rows
+// 325 -> 226 us: up 134, down 83.  A unit takes ~930 cycles (2500 warp instructions) at few rows, with 63 % of the issue
+// slots, 6 % of the tensor pipe and 23 % of HBM in use; without the decoding of scales and zeros, the weights' arithmetic
+// and the MMAs the same pipeline runs at ~430.  With 256 rows and whole tiles (14336 x 14336 on 112 SMs) it takes 1350, of
+// which the MMAs are 1024.  Where tiles are cut and all SMs run, the second 256 rows of an expert's up projection cost
+// 2100 per unit, and its down projection takes 79 us with 256 rows and 83 with 512; what the pieces of cut tiles, the
+// staged rows and the single accumulator contribute there has not been told apart.
 //
 // 3-bit layers (ten codes of one column in 32 bits; 10 does not divide the number of groups): storage rows rho + i * P3 hold
 // the same residues in the same slots, so a tile is again 8 neighbouring residues x 16 members, from one or two rho.  The
 // two bytes that hold a thread's field are picked out of two columns' words by one PRMT and multiplied up to bit 4; the rest
 // is as above.  14336 x 4096, 100 rows: 112 us before (decoded tables of scales in memory, dequantisation bound by the
-// latency of loads that nothing ran ahead of, A in shared memory), 41 now.
+// latency of loads that nothing ran ahead of, A in shared memory), 40 now.
 //
 // Every wait is bounded; a wait that runs out sets the error flag, all roles leave, TMEM is freed.
 #include <cuda.h>
@@ -77,8 +82,8 @@ constexpr int REGS_DEQUANT = 96, REGS_EPI = 64, REGS_ISSUE = 32;
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 constexpr int MAX_B_STAGES = 16, MAX_RAW = 2 * GROUPS;
-// Cycles of 128 columns of a tile with n rows (measured: 930 at 16, 1060 at 64, 1400 at 128, 2660 at 256), the weights of
-// the work split.
+// Cycles of 128 columns of a tile with n rows, the weights of the work split (measured in an expert's up projection, the
+// epilogue and cut tiles included: 930 at 16, 1060 at 64, 1400 at 128, 2660 at 256).
 __host__ __device__ constexpr int unit_cycles(bool f16, int n) {
     return n > 128 ? n * 10 + (f16 ? 0 : 200) : (f16 ? 900 : 1170) + 4 * n;
 }
@@ -1410,7 +1415,7 @@ static int64_t gg_tiles(const hqm_weight* const* ws, int count) {
 GgLayout gg_expert_layout(int64_t M) { return GgLayout{GgRows::of((int)M), gg_sm_count(), 0}; }
 // Rows per chunk and CTAs of linear layers over the same rows, by what a launch costs in cycles of its longest CTA (fitted to
 // 2- and 4-bit layers of 1024 to 14336 outputs with 16 to 500 rows):
-//   its units of 128 columns:  850 + 4 n with n rows; beyond 128 rows it is the staged x in every SM, 10 n
+//   its units of 128 columns:  850 + 4 n with n rows; beyond 128 rows, with one accumulator, 10 n
 //   a finished tile:           400 for every 16 rows
 //   a tile cut into p pieces:  5000 until the last CTA has seen that it is the last, and 3000 + 400 (p - 2) for every 16 rows;
 //                              twice where shares and tiles are not aligned, as a CTA then holds pieces of two tiles

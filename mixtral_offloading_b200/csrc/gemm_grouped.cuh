@@ -7,8 +7,10 @@ namespace hqm {
 
 constexpr int GG_MAX_PROBLEMS = 32;
 constexpr int GG_MAX_ROWS = 256;          // rows of x per pass over a weight (the MMA's N)
-constexpr int GG_LEAST_CTAS = 48;         // a third of the SMs: what a call may ask scratch for at the least
-constexpr int GG_F16_ROWS = 16;           // up to here h of an expert is staged as fp16, beyond it as bf16
+// The scratch that a call asks for at the least lets 16 rows at a time run on this many SMs, a third of them.  (4096 x 14336
+// 2-bit, 17 rows: 81 us in that, 53 in 2 MiB, 23 with a CTA on every SM.)
+constexpr int GG_LEAST_CTAS = 48;
+constexpr int GG_F16_ROWS = 16;           // up to here h of an expert is staged as fp16, beyond it as bf16 (gemm_grouped.cu)
 
 // How a launch's rows are laid out in the staged copy of x ("tiles": [K / 64][row][64], see gemm_grouped.cu): a row
 // list of `cnt` rows is cut into equal chunks of at most GG_MAX_ROWS rows, padded to a multiple of 16.

@@ -1,6 +1,7 @@
 // 3-bit quantized GEMM on the tcgen05 tensor cores: the path that replaces the reference's
 // matmul3_kernel_transpose (triton_kernels.py:414-564) and the two Quantizer.dequantize calls in
-// front of it (custom_layers.py:62-66) for five or more rows of x.
+// front of it (custom_layers.py:62-66) for five or more rows of x, where gemm_grouped.cu does not take the layer: its
+// members do not fall into blocks of 16 (other group sizes than 64, mostly).
 //
 // Two launches per call.
 //   1. meta_tables_kernel decodes the 8-bit scale and zero of the whole layer ONCE into two bf16

@@ -120,9 +120,15 @@ int* tc_error_ptr();                  // device flag the bounded waits set when 
 void* tma_encode_entry();             // cuTensorMapEncodeTiled of the installed driver, or null
 // y (M, N) = bf16(sums + bias)
 int launch_rows_from_sums(uint16_t* y, const float* sums, const uint16_t* bias, int64_t M, int N, cudaStream_t st);
-constexpr int64_t GG_MIN_ROWS = 5;    // rows from which 2- and 4-bit layers go to gemm_grouped.cu
+// Rows from which 2- and 4-bit layers go to gemm_grouped.cu.  The streaming kernels decode up to 4 rows in one
+// instantiation, 5 to 8 in the next one up, and more rows in more passes over the weight.  us, streaming / here:
+//   rows                      3            4            5            8           16
+//   2 bit 14336 x 4096   18.0 / 19.2  18.3 / 19.1  27.4 / 19.1  29.1 / 19.1  53.7 / 19.4
+//   4 bit 4096 x 4096    11.3 / 11.1  12.3 / 11.2  14.0 / 11.2  15.5 / 11.3  24.4 / 11.5
+//   expert (three 2-bit) 51.3 / 53.6  51.7 / 53.4  76.3 / 53.5  79.5 / 54.4   145 / 55.0
+constexpr int64_t GG_MIN_ROWS = 5;
 
-// gemm_tc3.cu — tcgen05 / TMEM path for 3-bit layers (row counts >= 5).
+// gemm_tc3.cu — tcgen05 / TMEM path for the 3-bit layers that gemm_grouped.cu does not take, from five rows on.
 bool gemm_tc3_supported(const hqm_weight* w, int G, int C, int64_t M);
 size_t gemm_tc3_scratch_bytes(const hqm_weight* w, int G, int64_t M);
 int launch_gemm_tc3(uint16_t* y, void* scratch, const uint16_t* x, const int32_t* x_idx, int64_t M,

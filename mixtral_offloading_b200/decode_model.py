@@ -152,8 +152,8 @@ class BatchDecode:
     """B independent sequences advanced one token per step through the layers of a MixtralDecodeModel (the same
     weights), each sequence with its own key/value cache; all of them at the same position.
 
-    The quantized projections and the MoE block run once per step on all B rows; norms, RoPE and attention over the
-    caches are torch ops.  capture() records the step in CUDA graphs (the position is device data:
+    The quantized projections and the MoE block run once per step on all B rows, as do the norms and RoPE; attention over
+    the caches is torch's.  capture() records the step in CUDA graphs (the position is device data:
     hqm_rope_append_rows reads it, and attention runs over the whole cache under a mask).  Where every layer's MoE block
     chooses its experts on the device that is one graph; a block whose shapes need the row counts on the host
     (custom_layers.py:272-314) ends a graph, and its experts are issued between two."""

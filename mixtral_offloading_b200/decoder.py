@@ -191,8 +191,8 @@ class DecoderLayerDecode(nn.Module):
     def forward_tokens(self, h: torch.Tensor, pos0: int, ln_in=None, shared=None):
         """T new tokens at once (a prompt, or a chunk of 32 / 256 tokens behind a cache that already holds pos0
         positions): h (T, hidden) bf16 is the residual stream of the tokens at positions pos0 .. pos0 + T - 1.
-        The quantized projections and the experts take their many-row (tensor-core) kernels; norms, RoPE and the
-        attention over the cache are torch ops; the MoE block groups the tokens per expert.  Appends the tokens'
+        The quantized projections and the experts take their many-row (tensor-core) kernels, norms and RoPE with the cache
+        append are one launch each, the attention over the cache is torch's; the MoE block groups the tokens per expert.  Appends the tokens'
         keys and values to the cache; returns (updated h, router logits (T, n_experts)).  ln_in: the layer's input
         norm weight when it is not attention.ln_in (a model hands every layer the weight its predecessor was built
         with as next_ln, which is what the one-token path applies).  shared: what tokens_shared() returned for the

@@ -548,9 +548,8 @@ def test_state_dict_round_trip_of_layer_and_expert_slab():
     assert torch.equal(fresh(x), lay(x))
 
 
-def test_many_row_gemm_without_tma_staging():
-    """HQM_GEMM_TMA=0 at load time keeps the many-row GEMM on its first-generation kernel (operand tiles filled by
-    the producer threads): same oracle, same bound; run in a process of its own because the switch is read once."""
+def test_many_rows_as_the_first_call_of_a_process():
+    """The many-row GEMM where nothing has run before it: function attributes, tensor maps, workspace, host module."""
     import subprocess
     import sys
     code = (
@@ -567,7 +566,6 @@ def test_many_row_gemm_without_tma_staging():
         "    assert err < 1e-2, err\n"
         "assert _cabi.lib().hqm_device_error() == 0\n"
         "print('ok')\n")
-    env = dict(os.environ, HQM_GEMM_TMA="0")
-    res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, timeout=600,
+    res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600,
                          cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert res.returncode == 0 and res.stdout.strip().endswith("ok"), res.stdout + res.stderr
