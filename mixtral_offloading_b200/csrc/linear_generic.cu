@@ -1,9 +1,10 @@
 // Shape-agnostic quantized linear and full dequantisation.
 //
-// linear_generic_kernel is the path for layers whose shape the streaming
-// kernels (gemv_stream.cu) do not cover.  It decodes scale and zero per element
-// from their 8-bit form, so it is instruction bound, not HBM bound; it exists
-// for generality and as an independent check of the fast kernels.
+// linear_members_kernel is the path for formats, shapes and row alignments that the
+// kernels with 16-bit factors do not take: weights, products and sums in fp32.
+// linear_generic_kernel decodes scale and zero per element from their 8-bit form
+// (instruction bound, by far); it takes what is left and is the independent check of
+// all other kernels (HQM_FORCE_GENERIC).
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -84,8 +85,181 @@ linear_generic_kernel(uint16_t* __restrict__ y, const uint16_t* __restrict__ x, 
     }
 }
 
+// Four neighbouring columns of a meta vector of C columns, from column c on.
+__device__ __forceinline__ void meta4(const uint16_t* p, int c, int C, bool vec, float* f) {
+    if (vec) {                                // 8-byte aligned and C a multiple of 4
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + c));
+        f[0] = f16_bits_to_float((uint16_t)v.x); f[1] = f16_bits_to_float((uint16_t)(v.x >> 16));
+        f[2] = f16_bits_to_float((uint16_t)v.y); f[3] = f16_bits_to_float((uint16_t)(v.y >> 16));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            f[j] = f16_bits_to_float(p[c]);
+            c = c + 1 == C ? 0 : c + 1;
+        }
+    }
+}
+// Scales and zeros of residue g at four columns from k on; c and cz are their columns of the meta vectors.
+__device__ __forceinline__ void decode_four(const hqm_weight& w, int g, int k, int c, int cz, int C, int Cz, bool meta_vec, float* sc, float* zr) {
+    const int64_t idx = (int64_t)g * w.K + k;
+    const uint32_t sq = *reinterpret_cast<const uint32_t*>(w.scale_q + idx), zq = *reinterpret_cast<const uint32_t*>(w.zero_q + idx);
+    float ms[4], mz[4], zs[4], zz[4];
+    meta4(w.ms_scale, c, C, meta_vec, ms);
+    meta4(w.mz_scale, c, C, meta_vec, mz);
+    meta4(w.ms_zero, cz, Cz, meta_vec, zs);
+    meta4(w.mz_zero, cz, Cz, meta_vec, zz);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        sc[j] = __fmul_rn(__fsub_rn((float)((sq >> (8 * j)) & 255u), mz[j]), ms[j]);
+        zr[j] = __fmul_rn(__fsub_rn((float)((zq >> (8 * j)) & 255u), zz[j]), zs[j]);
+    }
+}
+// The packed codes of storage row R at four columns from k on (3 bit: a word per column, else one for the four), and code
+// j of them at bit `shift` of its byte or word, as fp32: an OR into 2^23 and an exact subtraction.
+template <int NBITS>
+__device__ __forceinline__ void load_four(const hqm_weight& w, uint32_t R, int k, uint32_t (&v)[4]) {
+    if (NBITS == 3) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const int32_t*>(w.W_q) + (int64_t)R * w.K + k));
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+        v[0] = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(w.W_q) + (int64_t)R * w.K + k));
+    }
+}
+template <int NBITS>
+__device__ __forceinline__ float code_of(const uint32_t (&v)[4], int j, int shift) {
+    const uint32_t code = (NBITS == 3 ? v[j] >> shift : v[0] >> (8 * j + shift)) & ((1u << NBITS) - 1u);
+    return __fsub_rn(__uint_as_float(0x4B000000u | code), 8388608.f);
+}
+
+// A CTA: RES neighbouring residues of MC members (OUT output rows) times MT rows of x; its warps take every eighth block of
+// 128 columns, a lane 4 columns of it, and add up at the end in warp order.  A scale and a zero are decoded once for MC
+// members, a weight once for MT rows: per weight it is the code's shift, mask and conversion, one subtraction, one product
+// and MT fused multiply-adds, which bound it; 3 bit: the words, each read for one of its ten codes only.  RES is the number
+// of codes in a byte where G is a multiple of it, else 1.  us, before (a decode for every element) / now:
+//   3 bit g64 5120 x 4096, 2 to 4 rows     638 / 29       (OUT 8, three CTAs per SM; 16 and two: 41)
+//   4 bit g128 4096 x 4096, 4 / 100 rows   129 / 21, 1587 / 308     (OUT 16 / 8, two CTAs; 8 / 4 and three: 27, 426)
+//   2 bit g64 14336 x 4096, 5 / 100 rows   573 / 114, 5808 / 1333
+__host__ __device__ constexpr int members_out(int nbits, int mt) { return (nbits == 3 ? 32 : 64) / mt; }
+template <int NBITS, int RES, int MT>
+__global__ void __launch_bounds__(256, NBITS == 3 ? 3 : 2)
+linear_members_kernel(uint16_t* __restrict__ y, const uint16_t* __restrict__ x, const int32_t* __restrict__ x_idx, int M, hqm_weight w,
+                      int G, int C, const uint16_t* __restrict__ bias, bool meta_vec, bool x_vec) {
+    constexpr int PER = codes_per_word(NBITS), OUT = members_out(NBITS, MT), MC = OUT / RES, WARPS = 8, STEP = 128 * WARPS;
+    __shared__ float s_sum[WARPS][OUT * MT];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, K = w.K;
+    const int chunks = (w.group_size + MC - 1) / MC;
+    const int g0 = (int)(blockIdx.x / chunks) * RES, m0 = (int)(blockIdx.x % chunks) * MC, t0 = (int)blockIdx.y * MT;
+    const int Cz = (int)zero_meta_cols(w, G);
+    const int k0 = 4 * lane + 128 * wi;
+    int c[RES], cz[RES];
+#pragma unroll
+    for (int r = 0; r < RES; ++r) {
+        const int64_t idx = (int64_t)(g0 + r) * K + k0;
+        c[r] = (int)(idx % C);
+        cz[r] = (int)(idx % Cz);
+    }
+    const int step = STEP % C, stepz = STEP % Cz;
+    const uint16_t* xr[MT];
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+        const int t = min(t0 + i, M - 1);
+        xr[i] = x + (int64_t)(x_idx ? x_idx[t] : t) * K;
+    }
+    float acc[OUT][MT];
+#pragma unroll
+    for (int o = 0; o < OUT; ++o)
+#pragma unroll
+        for (int i = 0; i < MT; ++i) acc[o][i] = 0.f;
+
+    for (int k = k0; k < K; k += STEP) {
+        float sc[RES][4], zr[RES][4], xv[MT][4];
+#pragma unroll
+        for (int r = 0; r < RES; ++r) {
+            decode_four(w, g0 + r, k, c[r], cz[r], C, Cz, meta_vec, sc[r], zr[r]);
+            c[r] += step;
+            cz[r] += stepz;
+            c[r] -= c[r] >= C ? C : 0;
+            cz[r] -= cz[r] >= Cz ? Cz : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+            if (x_vec) {
+                const uint2 v = __ldg(reinterpret_cast<const uint2*>(xr[i] + k));
+                xv[i][0] = __uint_as_float(v.x << 16); xv[i][1] = __uint_as_float(v.x & 0xffff0000u);
+                xv[i][2] = __uint_as_float(v.y << 16); xv[i][3] = __uint_as_float(v.y & 0xffff0000u);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) xv[i][j] = bf16_bits_to_float(xr[i][k + j]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < MC; ++m) {
+            if (m0 + m >= w.group_size) break;
+            const uint32_t n0 = (uint32_t)((m0 + m) * G + g0), R = n0 / PER;          // < N
+            const int s0 = RES > 1 ? 0 : (int)(n0 - R * PER);
+            uint32_t v[4];
+            load_four<NBITS>(w, R, k, v);
+#pragma unroll
+            for (int r = 0; r < RES; ++r)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float wv = __fmul_rn(__fsub_rn(code_of<NBITS>(v, j, NBITS * (PER - 1 - s0 - r)), zr[r][j]), sc[r][j]);
+#pragma unroll
+                    for (int i = 0; i < MT; ++i) acc[m * RES + r][i] = fmaf(wv, xv[i][j], acc[m * RES + r][i]);
+                }
+        }
+    }
+#pragma unroll
+    for (int o = 0; o < OUT; ++o)
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+            const float v = warp_sum(acc[o][i]);
+            if (lane == 0) s_sum[wi][o * MT + i] = v;
+        }
+    __syncthreads();
+    for (int e = threadIdx.x; e < OUT * MT; e += 256) {
+        const int o = e / MT, t = t0 + e % MT, m = m0 + o / RES;
+        if (t >= M || m >= w.group_size) continue;
+        const int64_t n = (int64_t)m * G + g0 + o % RES;
+        float v = 0.f;
+#pragma unroll
+        for (int i = 0; i < WARPS; ++i) v += s_sum[i][e];
+        y[(int64_t)t * w.N + n] = float_to_bf16_bits(v + (bias ? bf16_bits_to_float(bias[n]) : 0.f));
+    }
+}
+
+// K a multiple of 4, packed tensors aligned for four columns at a time.
+static bool four_columns_ok(const hqm_weight* w, int G) {
+    auto aligned = [](const void* p, size_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; };
+    return w->K % 4 == 0 && aligned(w->W_q, w->nbits == 3 ? 16 : 4) && aligned(w->scale_q, 4) && aligned(w->zero_q, 4) &&
+           zero_meta_cols(*w, G) <= INT32_MAX;
+}
+static bool meta_four_ok(const hqm_weight* w, int G, int C) {
+    auto a8 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; };
+    return C % 4 == 0 && zero_meta_cols(*w, G) % 4 == 0 && a8(w->ms_scale) && a8(w->mz_scale) && a8(w->ms_zero) && a8(w->mz_zero);
+}
+
+template <int NBITS, int RES>
+static void linear_members(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t M, const hqm_weight* w, int G, int C,
+                           const uint16_t* bias, cudaStream_t st) {
+    const bool meta_vec = meta_four_ok(w, G, C), x_vec = (reinterpret_cast<uintptr_t>(x) & 7u) == 0;
+    auto go = [&](auto kern, int mt, int mc) {
+        const int64_t blocks = (int64_t)(G / RES) * ((w->group_size + mc - 1) / mc);
+        kern<<<dim3((unsigned)blocks, (unsigned)((M + mt - 1) / mt)), 256, 0, st>>>(y, x, x_idx, (int)M, *w, G, C, bias, meta_vec, x_vec);
+    };
+    if (M <= 4) go(linear_members_kernel<NBITS, RES, 4>, 4, members_out(NBITS, 4) / RES);
+    else go(linear_members_kernel<NBITS, RES, 8>, 8, members_out(NBITS, 8) / RES);
+}
+
 int launch_linear_generic(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t M, const hqm_weight* w, int G,
                           int C, const uint16_t* bias, cudaStream_t st) {
+    if (!force_generic() && four_columns_ok(w, G)) {
+        if (w->nbits == 3) linear_members<3, 1>(y, x, x_idx, M, w, G, C, bias, st);
+        else if (w->nbits == 2) G % 4 == 0 ? linear_members<2, 4>(y, x, x_idx, M, w, G, C, bias, st) : linear_members<2, 1>(y, x, x_idx, M, w, G, C, bias, st);
+        else G % 2 == 0 ? linear_members<4, 2>(y, x, x_idx, M, w, G, C, bias, st) : linear_members<4, 1>(y, x, x_idx, M, w, G, C, bias, st);
+        HQM_LAUNCH_CHECK();
+        return HQM_OK;
+    }
     constexpr int MT = 4;
     const int64_t rows = storage_rows(w->N, w->nbits);
     dim3 grid((unsigned)((rows + 7) / 8), (unsigned)((M + MT - 1) / MT));
@@ -150,24 +324,9 @@ template <> struct Four<__nv_bfloat16> {
     }
 };
 constexpr int DEQ_THREADS = 128;
-// Four neighbouring columns of a meta vector of C columns, from column c on.
-__device__ __forceinline__ void meta4(const uint16_t* p, int c, int C, bool vec, float* f) {
-    if (vec) {                                // 8-byte aligned and C a multiple of 4
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + c));
-        f[0] = f16_bits_to_float((uint16_t)v.x); f[1] = f16_bits_to_float((uint16_t)(v.x >> 16));
-        f[2] = f16_bits_to_float((uint16_t)v.y); f[3] = f16_bits_to_float((uint16_t)(v.y >> 16));
-    } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            f[j] = f16_bits_to_float(p[c]);
-            c = c + 1 == C ? 0 : c + 1;
-        }
-    }
-}
 template <int NBITS, int RES, typename T>
 __global__ void __launch_bounds__(DEQ_THREADS) dequantize_members_kernel(T* __restrict__ out, hqm_weight w, int G, int C, int members, bool meta_vec) {
     constexpr int PER = codes_per_word(NBITS);
-    constexpr uint32_t MASK = (1u << NBITS) - 1u;
     const int K4 = w.K / 4;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= (int64_t)(G / RES) * K4) return;
@@ -177,18 +336,8 @@ __global__ void __launch_bounds__(DEQ_THREADS) dequantize_members_kernel(T* __re
 #pragma unroll
     for (int r = 0; r < RES; ++r) {
         const int64_t idx = (int64_t)(g0 + r) * w.K + k;
-        const uint32_t sq = *reinterpret_cast<const uint32_t*>(w.scale_q + idx), zq = *reinterpret_cast<const uint32_t*>(w.zero_q + idx);
         const int c = (int)(idx % C), cz = Cz == C ? c : (int)(idx % Cz);
-        float ms[4], mz[4], zs[4], zz[4];
-        meta4(w.ms_scale, c, C, meta_vec, ms);
-        meta4(w.mz_scale, c, C, meta_vec, mz);
-        meta4(w.ms_zero, cz, Cz, meta_vec, zs);
-        meta4(w.mz_zero, cz, Cz, meta_vec, zz);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            sc[r][j] = __fmul_rn(__fsub_rn((float)((sq >> (8 * j)) & 255u), mz[j]), ms[j]);
-            zr[r][j] = __fmul_rn(__fsub_rn((float)((zq >> (8 * j)) & 255u), zz[j]), zs[j]);
-        }
+        decode_four(w, g0 + r, k, c, cz, C, Cz, meta_vec, sc[r], zr[r]);
     }
     const int m0 = blockIdx.y * members, m1 = min(m0 + members, w.group_size);
 #pragma unroll 4
@@ -196,23 +345,13 @@ __global__ void __launch_bounds__(DEQ_THREADS) dequantize_members_kernel(T* __re
         const uint32_t n0 = (uint32_t)(m * G + g0);           // < N
         const uint32_t R = n0 / PER;
         const int s0 = RES > 1 ? 0 : (int)(n0 - R * PER);
-        uint32_t v[4];                                        // NBITS == 3: a word per column, else one for the four
-        if (NBITS == 3) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const int32_t*>(w.W_q) + (int64_t)R * w.K + k));
-            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-        } else {
-            v[0] = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(w.W_q) + (int64_t)R * w.K + k));
-        }
+        uint32_t v[4];
+        load_four<NBITS>(w, R, k, v);
 #pragma unroll
         for (int r = 0; r < RES; ++r) {
-            const int shift = NBITS * (PER - 1 - s0 - r);
             float o[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t code = (NBITS == 3 ? v[j] >> shift : v[0] >> (8 * j + shift)) & MASK;
-                const float c = __fsub_rn(__uint_as_float(0x4B000000u | code), 8388608.f);
-                o[j] = __fmul_rn(__fsub_rn(c, zr[r][j]), sc[r][j]);
-            }
+            for (int j = 0; j < 4; ++j) o[j] = __fmul_rn(__fsub_rn(code_of<NBITS>(v, j, NBITS * (PER - 1 - s0 - r)), zr[r][j]), sc[r][j]);
             Four<T>::store(out + (int64_t)(n0 + r) * w.K + k, o);
         }
     }
@@ -225,18 +364,14 @@ static void dequantize_members(T* out, const hqm_weight* w, int G, int C, cudaSt
     // empty or full instead: 35 and 41 us for the 33 above, as every thread decodes the same scales again).
     int members = w->group_size;
     while (members > 4 && threads * ((w->group_size + members - 1) / members) < 148 * 1024) members = (members + 1) / 2;
-    auto a8 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; };
-    const bool meta_vec = C % 4 == 0 && zero_meta_cols(*w, G) % 4 == 0 && a8(w->ms_scale) && a8(w->mz_scale) && a8(w->ms_zero) && a8(w->mz_zero);
+    const bool meta_vec = meta_four_ok(w, G, C);
     const dim3 grid((unsigned)((threads + DEQ_THREADS - 1) / DEQ_THREADS), (unsigned)((w->group_size + members - 1) / members));
     dequantize_members_kernel<NBITS, RES, T><<<grid, DEQ_THREADS, 0, st>>>(out, *w, G, C, members, meta_vec);
 }
 
 template <typename T>
 static int launch_dequantize(void* out, const hqm_weight* w, int G, int C, cudaStream_t st) {
-    auto aligned = [](const void* p, size_t to) { return (reinterpret_cast<uintptr_t>(p) & (to - 1)) == 0; };
-    const int64_t Cz = zero_meta_cols(*w, G);
-    if (w->K % 4 == 0 && aligned(out, 4 * sizeof(T)) && aligned(w->W_q, w->nbits == 3 ? 16 : 4) && aligned(w->scale_q, 4) &&
-        aligned(w->zero_q, 4) && Cz <= INT32_MAX && w->group_size <= 65535) {
+    if (four_columns_ok(w, G) && (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(T) - 1)) == 0 && w->group_size <= 65535) {
         T* o = (T*)out;
         if (w->nbits == 3) dequantize_members<3, 1>(o, w, G, C, st);
         else if (w->nbits == 2) G % 4 == 0 ? dequantize_members<2, 4>(o, w, G, C, st) : dequantize_members<2, 1>(o, w, G, C, st);
