@@ -76,8 +76,10 @@ int set_overlap(int on) {
 // Rows from which a layer goes to the tensor-core kernel (gemm_grouped.cu); below, the streaming kernels,
 // whose work per weight grows with the rows, are faster (figures at GG_MIN_ROWS).
 // (3 bit: from two on, as the streaming kernel takes one row per launch: 14336 x 4096 21 us each, here 29 up to 16 rows.)
-static bool use_gg(const hqm_weight* w, int G, int C, int64_t M) {
-    return M >= (w->nbits == 3 ? 2 : GG_MIN_ROWS) && M <= (1 << 22) && gg_takes(w, G, C, M);
+// fp16 rows go there in every format that it can read: the alternative rounds the rows and the result to bf16 (2.3e-3 from 64
+// bits, 6e-4 there).
+static bool use_gg(const hqm_weight* w, int G, int C, int64_t M, bool f16 = false) {
+    return M >= (w->nbits == 3 ? 2 : GG_MIN_ROWS) && M <= (1 << 22) && (f16 ? gg_supported(w, G, C) : gg_takes(w, G, C, M));
 }
 
 // The kernels beside gemm_grouped.cu: what the one that takes the call needs.
@@ -206,6 +208,18 @@ int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t 
     return launch_linear_generic(y, x, x_idx, M, w, G, C, bias, st);
 }
 
+// Workspace, header included, of a launch over several layers; 0 where the tensor-core kernel does not take them.
+static size_t group_scratch_bytes(int64_t M, const hqm_weight* const* w, int count, bool f16) {
+    if (M <= 0 || count < 1 || count > 4 || w == nullptr || force_generic()) return 0;
+    for (int i = 0; i < count; ++i) {
+        int G, C;
+        if (check_weight(w[i], &G, &C) != HQM_OK || !use_gg(w[i], G, C, M, f16)) return 0;
+        if (w[i]->K != w[0]->K || w[i]->nbits != w[0]->nbits || w[i]->group_size != w[0]->group_size) return 0;
+    }
+    const GgRows rows = gg_linear_layout(M, w, count).rows;
+    return SCRATCH_HEADER + gg_stage_bytes(rows.padded(), w[0]->K, true) + gg_scratch_bytes(rows.n);
+}
+
 }  // namespace hqm
 
 extern "C" {
@@ -234,7 +248,7 @@ size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w) {
     return inner ? inner + hqm::SCRATCH_HEADER : 0;
 }
 
-size_t hqm_linear_f16_scratch_bytes(int64_t M, const hqm_weight* w) { return hqm_linear_group_scratch_bytes(M, &w, 1); }
+size_t hqm_linear_f16_scratch_bytes(int64_t M, const hqm_weight* w) { return hqm::group_scratch_bytes(M, &w, 1, /*f16=*/true); }
 
 int hqm_linear_f16(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias, void* scratch,
                    size_t scratch_bytes, void* stream) {
@@ -252,15 +266,7 @@ int hqm_linear_f16(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* 
 }
 
 size_t hqm_linear_group_scratch_bytes(int64_t M, const hqm_weight* const* w, int32_t count) {
-    using namespace hqm;
-    if (M <= 0 || count < 1 || count > 4 || w == nullptr || force_generic()) return 0;
-    for (int i = 0; i < count; ++i) {
-        int G, C;
-        if (check_weight(w[i], &G, &C) != HQM_OK || !use_gg(w[i], G, C, M)) return 0;
-        if (w[i]->K != w[0]->K || w[i]->nbits != w[0]->nbits || w[i]->group_size != w[0]->group_size) return 0;
-    }
-    const GgRows rows = gg_linear_layout(M, w, count).rows;
-    return SCRATCH_HEADER + gg_stage_bytes(rows.padded(), w[0]->K, true) + gg_scratch_bytes(rows.n);
+    return hqm::group_scratch_bytes(M, w, count, /*f16=*/false);
 }
 
 int hqm_linear_group(uint16_t* const* y, const uint16_t* x, int64_t M, const hqm_weight* const* w, const uint16_t* const* bias,

@@ -51,6 +51,10 @@ def test_formats_that_only_the_fp32_kernel_takes(nbits, group, N, K, Ms):
         x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(DEV)
         err, rounding = errors(layer(x), x.double() @ weight64(layer).t())
         assert err < 1.002 * rounding, M
+        # fp16 rows through bf16 would be 2^-9 / sqrt(3) off twice, 2.3e-3
+        half = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.float16).to(DEV)
+        err, rounding = errors(layer(half), half.double() @ weight64(layer).t())
+        assert M < 5 and nbits != 3 or err < 1e-3, M
 
 
 @pytest.mark.gpu
