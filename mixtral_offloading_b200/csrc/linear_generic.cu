@@ -327,17 +327,29 @@ constexpr int DEQ_THREADS = 128;
 template <int NBITS, int RES, typename T>
 __global__ void __launch_bounds__(DEQ_THREADS) dequantize_members_kernel(T* __restrict__ out, hqm_weight w, int G, int C, int members, bool meta_vec) {
     constexpr int PER = codes_per_word(NBITS);
+    constexpr uint32_t MASK = (1u << NBITS) - 1u;
     const int K4 = w.K / 4;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= (int64_t)(G / RES) * K4) return;
     const int g0 = (int)(i / K4) * RES, k = (int)(i % K4) * 4;
     const int Cz = (int)zero_meta_cols(w, G);
+    // (written out: through decode_four and load_four the 2-bit weight in fp32 takes 2 % longer)
     float sc[RES][4], zr[RES][4];
 #pragma unroll
     for (int r = 0; r < RES; ++r) {
         const int64_t idx = (int64_t)(g0 + r) * w.K + k;
+        const uint32_t sq = *reinterpret_cast<const uint32_t*>(w.scale_q + idx), zq = *reinterpret_cast<const uint32_t*>(w.zero_q + idx);
         const int c = (int)(idx % C), cz = Cz == C ? c : (int)(idx % Cz);
-        decode_four(w, g0 + r, k, c, cz, C, Cz, meta_vec, sc[r], zr[r]);
+        float ms[4], mz[4], zs[4], zz[4];
+        meta4(w.ms_scale, c, C, meta_vec, ms);
+        meta4(w.mz_scale, c, C, meta_vec, mz);
+        meta4(w.ms_zero, cz, Cz, meta_vec, zs);
+        meta4(w.mz_zero, cz, Cz, meta_vec, zz);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            sc[r][j] = __fmul_rn(__fsub_rn((float)((sq >> (8 * j)) & 255u), mz[j]), ms[j]);
+            zr[r][j] = __fmul_rn(__fsub_rn((float)((zq >> (8 * j)) & 255u), zz[j]), zs[j]);
+        }
     }
     const int m0 = blockIdx.y * members, m1 = min(m0 + members, w.group_size);
 #pragma unroll 4
@@ -345,13 +357,23 @@ __global__ void __launch_bounds__(DEQ_THREADS) dequantize_members_kernel(T* __re
         const uint32_t n0 = (uint32_t)(m * G + g0);           // < N
         const uint32_t R = n0 / PER;
         const int s0 = RES > 1 ? 0 : (int)(n0 - R * PER);
-        uint32_t v[4];
-        load_four<NBITS>(w, R, k, v);
+        uint32_t v[4];                                        // NBITS == 3: a word per column, else one for the four
+        if (NBITS == 3) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const int32_t*>(w.W_q) + (int64_t)R * w.K + k));
+            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        } else {
+            v[0] = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(w.W_q) + (int64_t)R * w.K + k));
+        }
 #pragma unroll
         for (int r = 0; r < RES; ++r) {
+            const int shift = NBITS * (PER - 1 - s0 - r);
             float o[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) o[j] = __fmul_rn(__fsub_rn(code_of<NBITS>(v, j, NBITS * (PER - 1 - s0 - r)), zr[r][j]), sc[r][j]);
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t code = (NBITS == 3 ? v[j] >> shift : v[0] >> (8 * j + shift)) & MASK;
+                const float c = __fsub_rn(__uint_as_float(0x4B000000u | code), 8388608.f);
+                o[j] = __fmul_rn(__fsub_rn(c, zr[r][j]), sc[r][j]);
+            }
             Four<T>::store(out + (int64_t)(n0 + r) * w.K + k, o);
         }
     }
