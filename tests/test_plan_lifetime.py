@@ -72,7 +72,7 @@ def test_plan_is_not_used_without_the_descriptor():
 
 
 @pytest.mark.gpu
-def test_layer_replaced_while_its_workspace_grows(monkeypatch):
+def test_layer_replaced_while_its_workspace_grows():
     """The workspace grows through Python code, which may drop the plan that the call works with."""
     od = random_layer(512, 256, 4, 64, seed=1)
     ods = tuple(random_layer(n, k, 2, 16, seed=3 + i) for i, (n, k) in enumerate(((512, 256), (256, 512), (512, 256))))
