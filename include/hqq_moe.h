@@ -194,7 +194,7 @@ int hqm_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx, i
 
 /* No counterpart in the reference (its experts are Python modules picked on the host,
  * custom_layers.py:295-312).  The device-side expert table that hqm_moe_decode / hqm_decode_layer pick the
- * router's experts from: one 512-byte entry per weight, holding the descriptor and the three TMA tensor maps
+ * router's experts from: one 896-byte entry per weight, holding the descriptor and the TMA tensor maps
  * (packed codes, scale bytes, zero bytes) the streaming kernel copies its tiles with.  hqm_expert_table_build
  * fills `host_out` (hqm_expert_table_bytes(n_weights) bytes, 64-byte aligned) on the HOST from n_weights
  * descriptors, ordered expert 0's w1, w2, w3, expert 1's w1, ...; the caller copies the bytes to device memory

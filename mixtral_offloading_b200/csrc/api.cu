@@ -196,7 +196,7 @@ int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t 
         StreamJob job{};
         job.w[0] = w;
         job.counters = counters;
-        if (plan.tma) {                      // the launch finishes the row itself: bf16, bias added
+        if (plan.kind == STREAM_TMA) {                      // the launch finishes the row itself: bf16, bias added
             job.y_out = y;
             job.bias = bias;
             return launch_gemv_stream((float*)scratch, x, x_idx, M, job, plan, st);

@@ -1126,6 +1126,7 @@ static int decode_layer_run(uint16_t* h, uint16_t* x, uint16_t* router_logits, f
     // 5.-7. the slots' experts: [w1; w3] per slot, silu * mul, w2 per slot
     StreamJob gate_up{}, down_proj{};
     gate_up.table = down_proj.table = static_cast<const StreamEntry*>(L->table);
+    gate_up.experts = down_proj.experts = ep_n;
     gate_up.counters = down_proj.counters = counters;
     for (int slot = 0; slot < slots; ++slot) {
         gate_up.w[2 * slot] = &L->w1;

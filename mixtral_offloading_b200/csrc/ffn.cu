@@ -89,6 +89,13 @@ static bool fused_plan(int64_t M, const hqm_weight* w1, const hqm_weight* w2, co
     return true;
 }
 
+// Rows from which an expert goes to the tensor-core kernel: where gemv_rows.cu takes its layers, those that it does not.
+static bool expert_uses_gg(int64_t M, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3, GgPlan* gp) {
+    FusedPlan fp;
+    if (M < GG_MIN_ROWS || !gg_plan(M, 1, M, w1, w2, w3, gp)) return false;
+    return !(fused_plan(M, w1, w2, w3, nullptr, &fp) && fp.up.kind == STREAM_ROWS && fp.down.kind == STREAM_ROWS);
+}
+
 // The three layers one after the other: their outputs, and what a single layer's launch needs.
 static size_t separate_bytes(int64_t M, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3) {
     size_t lin = 0, rows = 0;
@@ -110,7 +117,7 @@ size_t hqm_expert_ffn_scratch_bytes(int64_t M, const hqm_weight* w1, const hqm_w
     size_t bytes = separate_bytes(M, w1, w2, w3);
     GgPlan gp;
     FusedPlan fp;
-    if (M >= GG_MIN_ROWS && gg_plan(M, 1, M, w1, w2, w3, &gp)) bytes = std::max(bytes, gp.total());
+    if (expert_uses_gg(M, w1, w2, w3, &gp)) bytes = std::max(bytes, gp.total());
     else if (fused_plan(M, w1, w2, w3, nullptr, &fp)) bytes = std::max(bytes, fp.up_bytes + fp.h_bytes + fp.down_bytes);
     return SCRATCH_HEADER + bytes;
 }
@@ -137,7 +144,7 @@ int hqm_expert_ffn(uint16_t* out, const uint16_t* x, int64_t M, const int32_t* t
     uint32_t* counters = (uint32_t*)scratch;
     uint8_t* p = (uint8_t*)scratch + SCRATCH_HEADER;
     GgPlan gp;
-    if (M >= GG_MIN_ROWS && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && gg_plan(M, 1, M, w1, w2, w3, &gp)) {
+    if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0 && expert_uses_gg(M, w1, w2, w3, &gp)) {
         // 3 launches: x staged -> h = silu(w1 x) * w3 x, staged -> w2 h, weighted, into out
         uint8_t *xt = p, *ht = p + gp.x_bytes, *parts = ht + gp.h_bytes;
         const GgStaged xs = gg_staged(xt, gp.xt_rows, w1->K, true), hs = gg_staged(ht, gp.xt_rows, w1->N, false);
@@ -382,6 +389,7 @@ int hqm_moe_decode(uint16_t* out, uint16_t* router_logits, const uint16_t* x, co
     // the experts are whatever the router wrote to topk_idx[0..1]; their descriptors come from the table
     StreamJob gate_up{}, down_proj{};
     gate_up.table = down_proj.table = static_cast<const StreamEntry*>(table);
+    gate_up.experts = down_proj.experts = E;
     gate_up.counters = down_proj.counters = counters;
     for (int slot = 0; slot < 2; ++slot) {
         gate_up.w[2 * slot] = w1;

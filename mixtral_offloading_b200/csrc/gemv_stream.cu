@@ -738,9 +738,9 @@ bool gemv_stream_shape_ok(const hqm_weight* w, int G, int C) {
 
 bool gemv_stream_plan(const hqm_weight* const* ws, int count, int64_t M, StreamPlan* plan, bool chained) {
     if (count < 1 || count > STREAM_MAX_LAYERS || force_generic()) return false;
-    plan->tma = 0;
+    if (chained && gemv_rows_plan(ws, count, M, plan)) return true;
     if (M == 1 && gemv_tma_plan(ws, count, chained, plan)) return true;
-    plan->tma = 0;
+    plan->kind = STREAM_WARPS;
     const hqm_weight* w = ws[0];
     if ((w->nbits != 2 && w->nbits != 4) || M < 1 || M > STREAM_MAX_ROWS) return false;
     const int per = codes_per_word(w->nbits), nb = w->group_size / 16, pw = nb == 1 ? 128 : 64;
@@ -793,13 +793,14 @@ bool gemv_stream_plan(const hqm_weight* const* ws, int count, int64_t M, StreamP
 
 size_t gemv_tma_scratch_bytes(const StreamPlan& plan, int64_t M);
 size_t gemv_stream_scratch_bytes(const StreamPlan& plan, int64_t M) {
-    if (plan.tma) return gemv_tma_scratch_bytes(plan, M);
+    if (plan.kind == STREAM_TMA) return gemv_tma_scratch_bytes(plan, M);
     return (size_t)plan.slots * (size_t)M * (size_t)plan.col0[plan.count] * sizeof(float);
 }
 
 int launch_gemv_stream(float* partial, const uint16_t* x, const int32_t* x_idx, int64_t M, const StreamJob& job,
                        const StreamPlan& plan, cudaStream_t st) {
-    if (plan.tma) return launch_gemv_tma(partial, x, x_idx, M, job, plan, st);
+    if (plan.kind == STREAM_ROWS) return launch_gemv_rows(partial, x, x_idx, M, job, plan, st);
+    if (plan.kind == STREAM_TMA) return launch_gemv_tma(partial, x, x_idx, M, job, plan, st);
     Layers ly{};
     ly.count = plan.count;
     for (int l = 0; l < plan.count; ++l) {

@@ -658,6 +658,25 @@ bool encode_maps(const hqm_weight* w, int G, CUtensorMap* out) {
     return true;
 }
 
+// The same for 16 neighbouring storage-row residues at a time (gemv_rows.cu): codes as (K, group_size, P) with box
+// (128, 16, 16), scale_q and zero_q with box (128, 16 PER), all with the 128-byte swizzle.
+bool encode_rows_maps(const hqm_weight* w, int G, CUtensorMap* out) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return false;
+    const int per = codes_per_word(w->nbits);
+    const cuuint64_t K = (cuuint64_t)w->K, P = (cuuint64_t)(G / per);
+    const cuuint32_t ones[3] = {1, 1, 1};
+    auto map = [&](CUtensorMap* to, const void* at, cuuint64_t d1, cuuint64_t d2, cuuint64_t s1, cuuint64_t s2, cuuint32_t b1, cuuint32_t b2) {
+        const cuuint64_t dims[3] = {K, d1, d2}, strides[2] = {s1, s2};
+        const cuuint32_t box[3] = {(cuuint32_t)KC, b1, b2};
+        return enc(to, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(at), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    return map(&out[0], w->W_q, (cuuint64_t)w->group_size, P, P * K, K, 16, 16) &&
+           map(&out[1], w->scale_q, (cuuint64_t)G, 1, K, (cuuint64_t)G * K, (cuuint32_t)(16 * per), 1) &&
+           map(&out[2], w->zero_q, (cuuint64_t)G, 1, K, (cuuint64_t)G * K, (cuuint32_t)(16 * per), 1);
+}
+
 struct MapKey {
     const void* q;
     const void* s;
@@ -770,6 +789,14 @@ bool stream_cached_maps(const hqm_weight* w, int G, void* out3) {
     return tensor_maps_ok(w, G) && cached_maps(w, G, static_cast<CUtensorMap*>(out3));
 }
 
+bool gemv_rows_shape_ok(const hqm_weight* w, int G, int C) {
+    return w->nbits == 2 && w->group_size == 16 && tma_shape_ok(w, G, C);
+}
+bool rows_cached_maps(const hqm_weight* w, int G, void* out3) {
+    return gemv_rows_shape_ok(w, G, w->meta_group > 0 ? (int)((int64_t)G * w->K / w->meta_group) : 0) &&
+           cached_maps(w, G, static_cast<CUtensorMap*>(out3), 3, [&](CUtensorMap* to) { return encode_rows_maps(w, G, to); });
+}
+
 // The maps of a 3-bit layer: words as (K, P3, members) with box (128, 1, up to 16), scale and zero bytes as (K, G) with box
 // (128, 8), and, where the last storage rows do not fill a member, those rows as (K, left).
 static bool encode_maps3(const hqm_weight* w, int G, const Members3& m, CUtensorMap* out) {
@@ -855,7 +882,7 @@ bool gemv_tma_plan(const hqm_weight* const* ws, int count, bool chained, StreamP
     plan->toks = 1;
     const int64_t min_range = total / grid;
     plan->slots = (int)((plan->PT + min_range - 1) / min_range) + 1;
-    plan->tma = 1;
+    plan->kind = STREAM_TMA;
     return true;
 }
 
@@ -975,6 +1002,11 @@ int hqm_expert_table_build(void* host_out, const hqm_weight* weights, int32_t n_
             !encode_maps(&weights[i], G, reinterpret_cast<CUtensorMap*>(out[i].maps))) {
             set_error("expert_table_build: cuTensorMapEncodeTiled failed for weight %d (%dx%d, %d bit)", i, weights[i].N,
                       weights[i].K, weights[i].nbits);
+            return HQM_ERR_CUDA;
+        }
+        if (encode_fn() != nullptr && gemv_rows_shape_ok(&weights[i], G, C) &&
+            !rows_cached_maps(&weights[i], G, out[i].rows_maps)) {
+            set_error("expert_table_build: cuTensorMapEncodeTiled failed for weight %d (%dx%d)", i, weights[i].N, weights[i].K);
             return HQM_ERR_CUDA;
         }
     }

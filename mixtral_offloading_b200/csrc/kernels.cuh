@@ -14,26 +14,28 @@ constexpr int STREAM_MAX_ROWS = 16;
 // What one launch multiplies: up to four layers of the same K, bit width and group size (N may differ).
 // Layer l reads rows x_idx?[m] + xrow[l] of x.  With `table` set, layer l's descriptor is read on the
 // device: table[3 * *sel[l] + which[l]] (3 entries per expert: w1, w2, w3), and w[l] only gives the shape.
-// One entry of the device-side expert table (hqm_expert_table_build): the layer's descriptor and the three
-// tensor maps (packed codes, scale bytes, zero bytes) the TMA-staged kernel copies its tiles with.
+// One entry of the device-side expert table (hqm_expert_table_build): the layer's descriptor and the tensor maps (packed
+// codes, scale bytes, zero bytes) that the kernels copy their tiles with: a storage-row residue at a time, and 16 of them.
 struct alignas(128) StreamEntry {
     hqm_weight w;
     unsigned char pad[128 - sizeof(hqm_weight)];
     unsigned char maps[3][128];
+    unsigned char rows_maps[3][128];
 };
-static_assert(sizeof(StreamEntry) == 512, "table entries are 512 bytes");
+static_assert(sizeof(StreamEntry) == 896, "table entries are 896 bytes");
 
 struct StreamJob {
     const hqm_weight* w[STREAM_MAX_LAYERS];
     int xrow[STREAM_MAX_LAYERS];
     const StreamEntry* table;
+    int experts;                        // that the table holds (0: not known)
     const int32_t* sel[STREAM_MAX_LAYERS];
     int which[STREAM_MAX_LAYERS];
     // Set only when the kernel launched in front of this one lets its successor start after everything
     // before it has completed (launch_finalize_silu_mul(..., late_trigger = true)) and the indices behind
     // `sel` are older than that: the launch then reads them, and starts on the weights, without waiting.
     int sel_settled;
-    // TMA-staged launches (plan.tma) only.  counters: the zeroed header of the caller's scratch buffer (arrival
+    // STREAM_TMA launches only.  counters: the zeroed header of the caller's scratch buffer (arrival
     // counters of units split over several CTAs; left zero again).  y_out: when set, the launch writes the finished
     // row as bf16 (+ bias) there itself, and no finalize launch follows.
     uint32_t* counters;
@@ -43,6 +45,11 @@ struct StreamJob {
 // Every scratch buffer handed to the library starts with this many bytes of library state, zero when the buffer is
 // first used (hqm_scratch_init) and zero again after every call.
 constexpr size_t SCRATCH_HEADER = 64 * 1024;
+enum StreamKind {
+    STREAM_WARPS,   // gemv_stream.cu: the passes are split over warps
+    STREAM_TMA,     // gemv_tma.cu: units are (residue, block of 16 members), rho0 counts those units, and `warps` counts CTAs
+    STREAM_ROWS,    // gemv_rows.cu: units are 16 storage-row residues, rho0 counts those units, and `warps` counts CTAs
+};
 struct StreamPlan {
     int count;                          // layers in the launch
     int nbits, nb;                      // bit width, group size / 16
@@ -54,8 +61,7 @@ struct StreamPlan {
     int warps;   // warps of that grid: the units the passes are split over
     int toks;    // rows of x decoded per launch
     int slots;   // upper bound on the warps contributing to one residue: fp32 partials [slots][M][row length]
-    int tma;     // 1: the TMA-staged single-row kernel (gemv_tma.cu): units are (residue, block of 16 members),
-                 // rho0 counts those units, and `warps` counts CTAs
+    StreamKind kind;
 };
 // 2- and 4-bit layers of the streaming kernels' formats and shapes.
 bool gemv_stream_shape_ok(const hqm_weight* w, int G, int C);
@@ -79,6 +85,14 @@ bool force_generic();
 bool gemv_tma_plan(const hqm_weight* const* ws, int count, bool chained, StreamPlan* plan);
 int launch_gemv_tma(float* partial, const uint16_t* x, const int32_t* x_idx, int64_t M, const StreamJob& job,
                     const StreamPlan& plan, cudaStream_t st);
+
+// gemv_rows.cu — 2-bit layers with groups of 16, up to 8 rows.
+constexpr int STREAM_ROWS_MAX = 8;
+bool gemv_rows_shape_ok(const hqm_weight* w, int G, int C);
+bool gemv_rows_plan(const hqm_weight* const* ws, int count, int64_t M, StreamPlan* plan);
+int launch_gemv_rows(float* partial, const uint16_t* x, const int32_t* x_idx, int64_t M, const StreamJob& job,
+                     const StreamPlan& plan, cudaStream_t st);
+bool rows_cached_maps(const hqm_weight* w, int G, void* out3);        // gemv_tma.cu
 
 // router.cu — logits, top-2 indices and weights of M tokens (no per-expert lists).
 int launch_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx, const uint16_t* x,

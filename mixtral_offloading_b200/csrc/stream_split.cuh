@@ -26,6 +26,7 @@ struct Split {
 struct ColMap {
     int count, per;
     int nb;          // blocks of 16 group members that are separate units of the split (1: a unit is a whole residue)
+    int shift;       // log2 of the residues in a unit
     int col0[STREAM_MAX_LAYERS + 1];
     int rho0[STREAM_MAX_LAYERS];
     int G[STREAM_MAX_LAYERS];
@@ -50,7 +51,7 @@ __device__ __forceinline__ int partial_count(const Split& sp, const ColMap& cm, 
         G = in ? cm.G[l] : G;
     }
     const int rel = col - c0;
-    const uint32_t rho_g = (uint32_t)(r0 + ((rel % G) / cm.per) * cm.nb + ((rel / G) >> 4) % cm.nb);
+    const uint32_t rho_g = (uint32_t)(r0 + (((rel % G) / cm.per) >> cm.shift) * cm.nb + ((rel / G) >> 4) % cm.nb);
     return sp.owner(rho_g * sp.PT + sp.PT - 1) - sp.owner(rho_g * sp.PT) + 1;
 }
 
@@ -128,9 +129,10 @@ __device__ __forceinline__ void partial_sum_pair(const float* __restrict__ parti
 }
 
 // The split the CONSUMERS of a launch's sums see.  A TMA-staged launch finishes its sums itself (one fp32 row-set,
-// `grid` = 1: every element has exactly one part); the other kernel leaves one row-set per warp that touched a residue.
+// `grid` = 1: every element has exactly one part); the others leave one row-set per warp (gemv_rows.cu:
+// per CTA) that touched a residue.
 inline Split split_of(const StreamPlan& plan) {
-    return Split{plan.rho0[plan.count], plan.PT, plan.tma ? 1 : plan.warps};
+    return Split{plan.rho0[plan.count], plan.PT, plan.kind == STREAM_TMA ? 1 : plan.warps};
 }
 // The split of the passes over the launch's CTAs / warps.
 inline Split work_split_of(const StreamPlan& plan) { return Split{plan.rho0[plan.count], plan.PT, plan.warps}; }
@@ -138,7 +140,8 @@ inline ColMap colmap_of(const StreamPlan& plan) {
     ColMap cm{};
     cm.count = plan.count;
     cm.per = codes_per_word(plan.nbits);
-    cm.nb = plan.tma ? plan.nb : 1;
+    cm.nb = plan.kind == STREAM_TMA ? plan.nb : 1;
+    cm.shift = plan.kind == STREAM_ROWS ? 4 : 0;
     for (int l = 0; l < plan.count; ++l) {
         cm.col0[l] = plan.col0[l];
         cm.rho0[l] = plan.rho0[l];

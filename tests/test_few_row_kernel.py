@@ -1,0 +1,54 @@
+"""csrc/gemv_rows.cu through an expert (up to 8 rows): the remainders of its units and shares, every number of rows, layers it
+leaves to the other kernels, rows outside the range of fp16."""
+import pytest
+import torch
+
+from mixtral_offloading_b200 import _cabi
+from tests.helpers import random_layer
+from tests.test_gpu_parity import make_expert
+from tests.test_many_row_precision import weight64
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def reference(expert, x):
+    w1, w2, w3 = (weight64(layer) for layer in (expert.w1, expert.w2, expert.w3))
+    x = x.double()
+    return (torch.nn.functional.silu(x @ w1.t()) * (x @ w3.t())) @ w2.t()
+
+
+@pytest.mark.parametrize("hidden,ffn", [
+    (128, 4096),                 # one step to a unit; down: two residues of a unit's 16
+    (512, 3072),                 # fp16 values repeat after 3 residues
+    (512, 7168), (1024, 7168),   # after 7; units cut between CTAs
+    (512, 11264),                # after 11: not taken
+    (256, 768)])                 # their rows are no multiple of 128: not taken
+def test_units_and_shares(hidden, ffn):
+    ods = tuple(random_layer(n, k, 2, 16, seed=i) for i, (n, k) in enumerate(((ffn, hidden), (hidden, ffn), (ffn, hidden))))
+    expert = make_expert(hidden, ffn, ods)
+    for M in range(1, 10):
+        x = torch.randn(M, hidden, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(DEV)
+        y, want = expert(x), reference(expert, x)
+        # bf16 roundings (1.7e-3 of the value each) of gate, activation, up, h and the result: 3.8e-3; 7e-4 for the 16-bit
+        # factors of either layer; and half as much again for the scatter of 128 results
+        assert ((y.double() - want).norm() / want.norm()).item() < 6e-3, M
+        assert torch.equal(y, expert(x)), M                  # pieces of a unit are added in a fixed order
+    assert _cabi.lib().hqm_device_error() == 0
+
+
+@pytest.mark.parametrize("M", [5, 8])
+@pytest.mark.parametrize("scale", [1e-7, 3e5])
+def test_rows_outside_the_range_of_fp16(M, scale):
+    """From five rows on a row carries a power of two; its neighbours are not affected.  (Such rows make h = silu(a) * b very small
+    or, with weights this small, large but inside bf16.)"""
+    hidden, ffn = 512, 3072
+    ods = tuple(random_layer(n, k, 2, 16, seed=i, std=0.02 if scale < 1 else 1e-3)
+                for i, (n, k) in enumerate(((ffn, hidden), (hidden, ffn), (ffn, hidden))))
+    expert = make_expert(hidden, ffn, ods)
+    x = torch.randn(M, hidden, generator=torch.Generator().manual_seed(M))
+    x[M // 2] *= scale
+    x = x.to(torch.bfloat16).to(DEV)
+    y, want = expert(x).double(), reference(expert, x)
+    for m in range(M):
+        assert ((y[m] - want[m]).norm() / want[m].norm()).item() < 6e-3, m
