@@ -214,7 +214,7 @@ int hqm_expert_ffn(uint16_t* out, const uint16_t* x, int64_t M, const int32_t* t
     return HQM_OK;
 }
 
-// ---- MoE block of many tokens with every expert resident: no host read-back, seven launches --------------------------
+// ---- MoE block of many tokens with every expert resident: no host read-back, six to nine launches --------------------------
 }  // extern "C"
 
 namespace hqm {
@@ -243,12 +243,16 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(uint16_t* __restrict__
 
 struct MoePlan {
     GgPlan gg;
+    FewPlan few;
+    bool short_lists, long_lists;             // what the lists can be: up to FEW_ROWS entries (gemv_lists.cu), more (gemm_grouped.cu)
     size_t route_bytes, y_bytes;
-    size_t total() const { return route_bytes + gg.total() + y_bytes; }
+    size_t total() const { return route_bytes + (long_lists ? gg.total() : 0) + (short_lists ? few.total() : 0) + y_bytes; }
 };
 static bool moe_plan(int64_t T, int E, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3, MoePlan* mp) {
     if (T < 1 || T > (1 << 20) || E < 2 || E > GG_MAX_PROBLEMS || w2->N % 8 != 0 || w2->N != w1->K || w2->K != w1->N) return false;
     if (!gg_plan(2 * T, E, T, w1, w2, w3, &mp->gg)) return false;
+    mp->short_lists = few_plan(T, E, w1, w2, w3, &mp->few);
+    mp->long_lists = !mp->short_lists || T > FEW_ROWS;                // (a token is in a list at most once)
     mp->route_bytes = align_up((size_t)T * 2 * 4 * 5 + (size_t)(2 * E + 1) * 4, 1024);
     mp->y_bytes = align_up((size_t)T * 2 * w2->N * 2, 1024);
     return true;
@@ -286,38 +290,64 @@ int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, c
     float* token_w = (float*)(token_idx + 2 * T);                     // [2T]
     int32_t* counts = (int32_t*)(token_w + 2 * T);                    // [E]
     int32_t* offsets = counts + E;                                    // [E + 1]
-    uint8_t* xt = p + mp.route_bytes;
+    uint16_t* y = (uint16_t*)(p + mp.route_bytes);
+    uint8_t* xt = p + mp.route_bytes + mp.y_bytes;
     uint8_t* ht = xt + mp.gg.x_bytes;
     uint8_t* parts = ht + mp.gg.h_bytes;
-    uint16_t* y = (uint16_t*)(parts + mp.gg.part_bytes);
+    GgFew few{};
+    uint8_t* few_ht = nullptr;
+    float* few_part = nullptr;
+    if (mp.short_lists) {
+        uint8_t* f = mp.long_lists ? parts + mp.gg.part_bytes : xt;
+        few = GgFew{FEW_ROWS, f, (float*)(f + mp.few.x_bytes)};
+        few_ht = f + mp.few.x_bytes + mp.few.scale_bytes;
+        few_part = (float*)(few_ht + mp.few.h_bytes);
+    }
+    const FewJob fj{static_cast<const StreamEntry*>(table), counts, E, w1, w2};
     int rc = launch_router_top2(router_logits, topk_w, topk_idx, x, gate_w, T, w1->K, E, st);
     if (rc != HQM_OK) return rc;
     rc = launch_router_lists(counts, offsets, token_idx, token_w, entry_of, topk_w, topk_idx, T, E, st);
     if (rc != HQM_OK) return rc;
     const GgStaged xs = gg_staged(xt, mp.gg.xt_rows, w1->K, true), hs = gg_staged(ht, mp.gg.xt_rows, w1->N, false);
-    rc = launch_gg_stage(xs, x, 0, token_idx, counts, E, 2 * T, w1->K, w1->nbits, st);
+    rc = launch_gg_stage(xs, x, 0, token_idx, counts, E, 2 * T, w1->K, w1->nbits, st, few);
     if (rc != HQM_OK) return rc;
     GgJob up{}, down{};
     up.problems = down.problems = E;
     up.table = down.table = static_cast<const StreamEntry*>(table);
     up.counts = down.counts = counts;
     up.rows = down.rows = (int)T;
+    up.few = down.few = few.most;
     up.mode = GG_UP;
     up.shape = w1;
     up.which0 = 0;
     up.which1 = 2;
     up.x = xs;
     up.ht = ht;
-    rc = launch_gg(up, counters, parts, mp.gg.part_bytes, st);
-    if (rc != HQM_OK) return rc;
+    if (mp.short_lists) {
+        rc = launch_few_projection(fj, few.data, few_part, /*up=*/true, st);
+        if (rc != HQM_OK) return rc;
+        rc = launch_few_silu(fj, few_ht, few_part, few.scale, T, st);
+        if (rc != HQM_OK) return rc;
+    }
+    if (mp.long_lists) {
+        rc = launch_gg(up, counters, parts, mp.gg.part_bytes, st);
+        if (rc != HQM_OK) return rc;
+    }
     down.mode = GG_DOWN;
     down.shape = w2;
     down.which0 = down.which1 = 1;
     down.x = hs;
     down.out = y;
     down.row_w = token_w;
-    rc = launch_gg(down, counters, parts, mp.gg.part_bytes, st);
-    if (rc != HQM_OK) return rc;
+    if (mp.long_lists) {
+        rc = launch_gg(down, counters, parts, mp.gg.part_bytes, st);
+        if (rc != HQM_OK) return rc;
+    }
+    if (mp.short_lists) {
+        rc = launch_few_projection(fj, few_ht, few_part, /*up=*/false, st);
+        if (rc != HQM_OK) return rc;
+        return launch_few_combine(fj, out, few_part, y, entry_of, token_w, T, st);
+    }
     const int64_t work = T * (w2->N / 8);
     launch_overlapped(moe_combine_kernel, (int)((work + 255) / 256 > 148 * 8 ? 148 * 8 : (work + 255) / 256), 256, 0, st, out,
                       (const uint16_t*)y, (const int32_t*)entry_of, T, (int)(w2->N / 8));

@@ -147,7 +147,7 @@ struct Params {
     const StreamEntry* table;
     int which0, which1;
     const int32_t* counts;
-    int rows;
+    int rows, few;
     const unsigned char* xt;
     int64_t xt_rows;
     const float* row_scale;                // of the staged rows (null: 1)
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             cost = unit_cycles(p.f16, p.n);
             p.cost = cost;
             rows = r.padded();
-            units = h.tiles * r.chunks * units_k;
+            units = cnt <= prm.few ? 0 : h.tiles * r.chunks * units_k;
         }
         int row1 = rows, list1 = cnt, u1 = units;
         unsigned long long c1 = (unsigned long long)units * (unsigned)cost;
@@ -1283,22 +1283,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
 template <bool X_F16>
 __global__ void __launch_bounds__(256) gg_stage_kernel(unsigned char* __restrict__ xt, float* __restrict__ row_scale, int64_t xt_rows,
                                                        const uint16_t* __restrict__ x, const int32_t* __restrict__ idx,
-                                                       const int32_t* __restrict__ counts, int lists, int K, bool words) {
+                                                       const int32_t* __restrict__ counts, int lists, int K, bool words, GgFew few) {
     __shared__ float s_max[8];
     grid_launch_dependents();
     grid_dependency_wait();
     const int li = blockIdx.x;
-    int row = li;
+    int row = li, few_row = 0, few_cap = 0;           // (of a short list: its first staged row, and how many it has)
     if (counts) {
         int list0 = 0, row0 = 0, e = 0;
         for (; e < lists; ++e) {
-            const int c = __ldcg(counts + e);
-            if (li < list0 + c) break;
+            const int c = __ldcg(counts + e), cap = c <= few.most ? (c <= 4 ? (c ? 4 : 0) : 8) : 0;
+            if (li < list0 + c) {
+                few_cap = cap;
+                break;
+            }
             list0 += c;
             row0 += GgRows::of(c).padded();
+            few_row += cap;
         }
         if (e == lists) return;                       // the lists together are shorter than the grid
-        row = row0 + (li - list0);
+        row = few_cap ? li - list0 : row0 + (li - list0);
     }
     const uint16_t* src = x + (int64_t)(idx ? __ldcg(idx + li) : li) * K;
     auto pair = [](uint32_t v, float& lo, float& hi) {
@@ -1331,7 +1335,23 @@ __global__ void __launch_bounds__(256) gg_stage_kernel(unsigned char* __restrict
     // 2^(exponent of mx - 4); zero, tiny and infinite rows keep a finite factor
     const int e = min(max((int)(__float_as_uint(mx) >> 23), 30), 250) - 4;
     const float down = __uint_as_float((uint32_t)(254 - e) << 23);
-    if (threadIdx.x == 0) row_scale[row] = __uint_as_float((uint32_t)e << 23);
+    if (threadIdx.x == 0) (few_cap ? few.scale[li] : row_scale[row]) = __uint_as_float((uint32_t)e << 23);
+    if (few_cap) {
+        unsigned char* to = few.data + (size_t)few_row * K * 2;
+        for (int i = threadIdx.x; i < K / 8; i += 256) {
+            const uint4 v = *reinterpret_cast<const uint4*>(src + 8 * i);
+            const uint32_t o[4] = {perm(v.x, v.y, 0x5410u), perm(v.x, v.y, 0x7632u), perm(v.z, v.w, 0x5410u), perm(v.z, v.w, 0x7632u)};
+            uint32_t h[4];
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                float lo, hi;
+                pair(o[w], lo, hi);
+                h[w] = h2_of(lo * down, hi * down);
+            }
+            *reinterpret_cast<uint4*>(to + few_staged_at(8 * i, row, few_cap)) = make_uint4(h[0], h[1], h[2], h[3]);
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < K / 8; i += 256) {
         const int b = i >> 3, ch = i & 7;
         // piece ch of the staged block: words (thread column 2 (ch & 1), word ch >> 1) and the next thread column
@@ -1456,9 +1476,9 @@ GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count, siz
 }
 
 int launch_gg_stage(const GgStaged& to, const void* x, int x_f16, const int32_t* idx, const int32_t* counts, int lists, int64_t rows,
-                    int K, int nbits, cudaStream_t st) {
+                    int K, int nbits, cudaStream_t st, const GgFew& few) {
     auto kern = x_f16 ? gg::gg_stage_kernel<true> : gg::gg_stage_kernel<false>;
-    launch_overlapped(kern, (int)rows, 256, 0, st, (unsigned char*)to.data, to.scale, to.rows, (const uint16_t*)x, idx, counts, lists, K, nbits == 3);
+    launch_overlapped(kern, (int)rows, 256, 0, st, (unsigned char*)to.data, to.scale, to.rows, (const uint16_t*)x, idx, counts, lists, K, nbits == 3, few);
     HQM_LAUNCH_CHECK();
     return HQM_OK;
 }
@@ -1540,6 +1560,7 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
     p.which1 = job.which1;
     p.counts = job.counts;
     p.rows = job.rows;
+    p.few = job.few;
     p.xt = (const unsigned char*)job.x.data;
     p.row_scale = job.x.scale;
     p.xt_rows = job.x.rows;

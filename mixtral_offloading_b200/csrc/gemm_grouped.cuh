@@ -63,6 +63,7 @@ struct GgJob {
     const hqm_weight* shape;
     int which0, which1;
     const int32_t* counts;                // device: rows of every problem; null: `rows` rows, shared by all problems
+    int few;                              // (counts) lists of up to `few` rows are left out
     int rows;                             // rows (counts == null), or the most all lists hold together
     GgLayout layout;                      // (counts == null)
     GgStaged x;                           // the staged rows
@@ -91,9 +92,16 @@ size_t gg_scratch_bytes(int n);           // partial tiles of a launch with up t
 inline size_t gg_least_bytes(int K) { return gg_stage_bytes(16, K, true) + (size_t)GG_LEAST_CTAS * 2 * 16 * 128 * sizeof(float); }
 int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratch_bytes, cudaStream_t st);
 
+// Where gg_stage puts the rows of short lists (gemv_lists.cu); most = 0: there are none.
+struct GgFew {
+    int most;
+    unsigned char* data;
+    float* scale;                         // of list entry i
+};
+
 // Stages rows of x (bf16 or fp16) for layers of `nbits`.  counts == null: one list of `rows` rows, else `lists` lists of together at most `rows`;
 // idx: row of x of list entry i (null: i).
 int launch_gg_stage(const GgStaged& to, const void* x, int x_f16, const int32_t* idx, const int32_t* counts, int lists, int64_t rows,
-                    int K, int nbits, cudaStream_t st);
+                    int K, int nbits, cudaStream_t st, const GgFew& few = GgFew{});
 
 }  // namespace hqm

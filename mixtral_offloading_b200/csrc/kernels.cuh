@@ -94,6 +94,33 @@ int launch_gemv_rows(float* partial, const uint16_t* x, const int32_t* x_idx, in
                      const StreamPlan& plan, cudaStream_t st);
 bool rows_cached_maps(const hqm_weight* w, int G, void* out3);        // gemv_tma.cu
 
+// gemv_lists.cu — the experts of a MoE block whose lists are short (2-bit layers with groups of 16).
+constexpr int FEW_ROWS = 8;              // rows of a short list at most
+constexpr int FEW_MAX_LISTS = 32;
+// Tokens up to which it is asked.  A block of 8 experts, us, without / with: 2 tokens 170 / 110, 4: 204 / 129, 8: 269 / 167, 16: 301 / 205,
+// 24: 301 / 248, 33: 302 / 274, 40: 302 / 323 (both kernels run then, one after the other, on half of the lists each).
+constexpr int64_t FEW_TOKENS = 36;
+struct FewPlan {
+    size_t x_bytes, scale_bytes, h_bytes, part_bytes;
+    size_t total() const { return x_bytes + scale_bytes + h_bytes + part_bytes; }
+};
+struct FewJob {
+    const StreamEntry* table;
+    const int32_t* counts;               // device: entries of every list
+    int lists;
+    const hqm_weight *w1, *w2;           // the shapes
+};
+bool few_plan(int64_t T, int E, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3, FewPlan* fp);
+// Where columns k .. k + 7 (k a multiple of 8) of row m lie in a staged list of `cap` rows.
+__host__ __device__ inline size_t few_staged_at(int k, int m, int cap) {
+    const int c = (k >> 3) & 15;
+    return (size_t)(k >> 7) * cap * 256 + (size_t)((2 * ((c >> 1) & 1) + (c & 1)) * cap + m) * 64 + (c >> 2) * 16;
+}
+int launch_few_projection(const FewJob& job, const unsigned char* xt, float* partial, bool up, cudaStream_t st);
+int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, int64_t T, cudaStream_t st);
+int launch_few_combine(const FewJob& job, uint16_t* out, const float* partial, const uint16_t* y, const int32_t* entry_of, const float* token_w,
+                       int64_t T, cudaStream_t st);
+
 // router.cu — logits, top-2 indices and weights of M tokens (no per-expert lists).
 int launch_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx, const uint16_t* x,
                        const uint16_t* gate_w, int64_t M, int64_t K, int32_t E, cudaStream_t st);

@@ -1,11 +1,11 @@
-"""csrc/gemv_rows.cu through an expert (up to 8 rows): the remainders of its units and shares, every number of rows, layers it
-leaves to the other kernels, rows outside the range of fp16."""
+"""csrc/gemv_rows.cu through an expert (up to 8 rows) and csrc/gemv_lists.cu through a block: the remainders of their units and
+shares, every number of rows, layers they leave to the other kernels, rows outside the range of fp16."""
 import pytest
 import torch
 
-from mixtral_offloading_b200 import _cabi
+from mixtral_offloading_b200 import ResidentMoe, _cabi
 from tests.helpers import random_layer
-from tests.test_gpu_parity import make_expert
+from tests.test_gpu_parity import Cfg, make_expert
 from tests.test_many_row_precision import weight64
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +52,34 @@ def test_rows_outside_the_range_of_fp16(M, scale):
     y, want = expert(x).double(), reference(expert, x)
     for m in range(M):
         assert ((y[m] - want[m]).norm() / want[m].norm()).item() < 6e-3, m
+
+
+@pytest.mark.parametrize("hidden,ffn,n_exp", [(512, 3072, 8), (128, 4096, 3), (1024, 7168, 32)])
+@pytest.mark.parametrize("tokens", [2, 5, 8, 9, 30, 36, 37])
+def test_lists_of_every_length(hidden, ffn, n_exp, tokens):
+    """A block's lists: empty ones, up to 4, 5 to 8 and more rows in one call, units cut between CTAs, fewer steps than CTAs."""
+    ods = [tuple(random_layer(n, k, 2, 16, seed=10 * e + i) for i, (n, k) in enumerate(((ffn, hidden), (hidden, ffn), (ffn, hidden))))
+           for e in range(min(n_exp, 4))]
+    gate = torch.nn.Linear(hidden, n_exp, bias=False, dtype=torch.bfloat16, device=DEV)
+    g = torch.Generator().manual_seed(tokens)
+    gate.weight.data = (torch.randn(n_exp, hidden, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+    gate.weight.data[1] = -4.0 * gate.weight.data[0]         # lists of very different lengths
+    experts = [make_expert(hidden, ffn, ods[e % len(ods)]) for e in range(n_exp)]
+    moe = ResidentMoe(Cfg(hidden, ffn, n_exp), 0, gate, experts)
+    x = torch.randn(tokens, hidden, generator=g).to(torch.bfloat16).to(DEV)
+    y, logits = moe(x.view(1, tokens, hidden))
+    y = y.view(tokens, hidden)
+    p, idx = torch.softmax(logits.view(tokens, n_exp).float(), 1).topk(2, 1)
+    p = (p / p.sum(1, keepdim=True)).to(torch.bfloat16).double()
+    want = torch.zeros(tokens, hidden, dtype=torch.float64, device=DEV)
+    for e in range(n_exp):
+        t = (idx == e).any(1).nonzero().flatten()
+        if len(t):
+            want[t] += (p * (idx == e)).sum(1)[t].unsqueeze(1) * reference(experts[e], x[t])
+    # 5.9e-3 for the experts with more than 16 rows (bf16 weights), 4e-3 for the others, and a rounding each (1.7e-3) of the weighted
+    # outputs and of their sum: 6.4e-3; twice that for any single token, whose two outputs may partly cancel
+    error, size = (y.double() - want).norm(dim=1), want.norm(dim=1)
+    assert (error.norm() / size.norm()).item() < 7e-3
+    assert (error / size).max().item() < 1.3e-2
+    assert torch.equal(y, moe(x.view(1, tokens, hidden))[0].view(tokens, hidden))
+    assert _cabi.lib().hqm_device_error() == 0
