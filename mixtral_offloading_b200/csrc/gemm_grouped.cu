@@ -47,10 +47,15 @@
 // experts, 4096 -> 14336, 33 tokens: 201 us alone, down 103 us; the whole block 943 -> 299 us.  One expert with 512 rows
 // 325 -> 226 us: up 134, down 83.  A unit takes ~930 cycles (2500 warp instructions) at few rows, with 63 % of the issue
 // slots, 6 % of the tensor pipe and 23 % of HBM in use; without the decoding of scales and zeros, the weights' arithmetic
-// and the MMAs the same pipeline runs at ~430.  With 256 rows and whole tiles (14336 x 14336 on 112 SMs) it takes 1350, of
-// which the MMAs are 1024.  Where tiles are cut and all SMs run, the second 256 rows of an expert's up projection cost
-// 2100 per unit, and its down projection takes 79 us with 256 rows and 83 with 512; what the pieces of cut tiles, the
-// staged rows and the single accumulator contribute there has not been told apart.
+// and the MMAs the same pipeline runs at ~430.  With 256 rows a unit takes 1200 while the MMAs run (1024 their own), but a tile of
+// 256 rows has the accumulator to itself, and writing it out took 14.7 us beside the 20.5 of its 32 units; a cut tile of 256 rows
+// took another 30 to 38 us to be summed, behind everything else.  What was done about that, one expert with 512 rows, us (224 before):
+//   * a CTA takes the tiles that it shares with others first: they are summed under the MMAs of the next ones;
+//   * the pieces of a cut tile come by asynchronous copies, 16 rows of several pieces under way (a thread reads what it copied
+//     itself); with 8 rows a time 214, with 16 205, and a 4-bit layer of 16 rows 11.35 and 11.12 (11.20 before);
+//   * the next 16 rows' sums are asked for before the present ones are worked on; exponential and reciprocal without the branches
+//     for denormals, roundings before the exchange between lanes.
+// (A second group of epilogue warps, for 8 registers less in each dequantising one: no gain at 512 rows, and 3-bit layers 7 % slower.)
 //
 // 3-bit layers (ten codes of one column in 32 bits; 10 does not divide the number of groups): storage rows rho + i * P3 hold
 // the same residues in the same slots, so a tile is again 8 neighbouring residues x 16 members, from one or two rho.  The
@@ -91,6 +96,8 @@ constexpr int NA = 6;                      // A slots of 128 columns (64 TMEM co
 // raw full, raw empty, A full, A empty (even and odd rounds of the slots), B full, B empty, accumulator full, empty
 constexpr int N_BARS = 2 * MAX_RAW + 3 * NA + 2 * MAX_B_STAGES + 4;
 constexpr int TILE_BYTES = 16 * 128 * 2;   // 16 rows of a finished tile, 16 bit; two of them
+constexpr int GG_MAX_LAYERS = 4;           // of a launch without a table
+constexpr int MERGE_BYTES = 16 * 128 * 4;  // 16 rows of a piece of a cut tile, on their way to the sum
 constexpr int EPI_BYTES = 2 * TILE_BYTES + 3 * GG_MAX_ROWS * 4;     // and per row of a chunk: factor, weight, output row
 constexpr float F16_SCALE = 4.f;           // A holds a quarter of the weight in fp16 mode
 
@@ -164,10 +171,11 @@ struct Params {
 };
 
 // ---- the split of a launch's units over its CTAs -------------------------------------------------------------------
+template <int PROBLEMS>
 struct Shared {
-    Problem pr[GG_MAX_PROBLEMS];
-    int ubase[GG_MAX_PROBLEMS + 1];        // first unit of each problem
-    unsigned long long cbase[GG_MAX_PROBLEMS + 1];     // cost in front of each problem
+    Problem pr[PROBLEMS];
+    int ubase[PROBLEMS + 1];               // first unit of each problem
+    unsigned long long cbase[PROBLEMS + 1];            // cost in front of each problem
     int begin[256];                        // first unit of each CTA ([grid]: all units)
     int last;                              // epilogue: this CTA completes the tile
     uint32_t tmem;
@@ -202,12 +210,15 @@ struct Fmt {
     // Launches of up to 64 rows per chunk need few staged rows in flight and many packed bytes, others the reverse.
     __host__ __device__ static constexpr int b_ring(int n_max) { return WORDS ? 80 * 1024 : (n_max <= 64 ? 64 * 1024 : 128 * 1024); }
     // (Even: a slot is filled by one of the two copying warps then, and its phases are waited for in order.)
-    __host__ __device__ static constexpr int n_raw(int n_max) { return WORDS ? 6 : (PARTS == 4 && n_max > 64 ? 6 : 8); }
+    __host__ __device__ static constexpr int n_raw(int n_max) { return WORDS || n_max > 64 ? 6 : 8; }
+    // Pieces of 16 rows in flight while a cut tile is summed: as many as there is room for.
+    __host__ __device__ static constexpr int n_merge(int n_max) { return WORDS ? 1 : (n_max <= 64 ? 4 : (PARTS == 4 ? 1 : 3)); }
     static constexpr int ST_OFF = 0, EPI_OFF = ST_OFF + 4 * GROUPS * ST_WARP, BAR_OFF = EPI_OFF + EPI_BYTES, RING_OFF = BAR_OFF + 1024;
     __host__ __device__ static constexpr int smem(int n_max) {
-        return (RING_OFF + 1023) / 1024 * 1024 + b_ring(n_max) + n_raw(n_max) * RAW_BYTES + 1024;
+        return (RING_OFF + 1023) / 1024 * 1024 + b_ring(n_max) + n_raw(n_max) * RAW_BYTES + n_merge(n_max) * MERGE_BYTES + 1024;
     }
-    static_assert(smem(64) + (int)sizeof(Shared) <= 227 * 1024 && smem(256) + (int)sizeof(Shared) <= 227 * 1024, "shared memory");
+    static constexpr int SHARED = NBITS == 2 ? (int)sizeof(Shared<GG_MAX_PROBLEMS>) : (int)sizeof(Shared<GG_MAX_LAYERS>);
+    static_assert(smem(64) + SHARED <= 227 * 1024 && smem(256) + SHARED <= 227 * 1024, "shared memory");
     // Which row of the tile TMEM lane 32 q + 8 j + g holds (q: warp of a group, j = 0..3): part, slot of the byte, member.
     // A thread of the 16x256b store shape holds j = 0..3 at one g: four members of one quantisation group.
     __device__ __forceinline__ static int part_of(int q, int g) { return (NBITS == 4 ? 2 * (q >> 1) : 0) + (g & 1); }
@@ -409,6 +420,15 @@ __device__ __forceinline__ uint32_t bf2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// a / (1 + e^-a): the exponential and the reciprocal of the special function unit, without the branches that keep denormals (the
+// result is rounded to bf16; beyond |a| = 87 it is a or zero either way).
+__device__ __forceinline__ float silu(float a) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(a * -1.44269504f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+    return a * r;
+}
+
 __device__ __forceinline__ uint32_t bf2_mul(uint32_t a, uint32_t b) {      // one rounding, as of the fp32 product
     uint32_t d;
     asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -440,21 +460,33 @@ struct Field3 {
 // A run of this CTA's units inside one tile.
 struct Seg {
     int p, tile, chunk, k0, k1;            // problem, tile, row chunk, 128-column units [k0, k1)
-    int u0;                                // first unit, counted from the CTA's first
+    int u, u0;                             // first unit, and where it stands in the CTA's order
 };
-__device__ __forceinline__ bool next_seg(const Shared& sh, int ubegin, int uend, int at, int units_k, Seg& s) {
-    const int u = ubegin + at;
-    if (u >= uend) return false;
-    int p = s.p;
+// This CTA's share, units [begin, end), in the order in which it takes them: the first units of its last tile, where another CTA has the
+// rest, then the others.  Tiles that are cut come first this way, at about the same time in both CTAs, and are summed under the
+// units that follow instead of behind the last one.
+struct Share {
+    int begin, end, last;                  // last: units of the last tile, 0 where it is not cut or is the only one
+    __device__ __forceinline__ Share(int begin_, int end_, int units_k) : begin(begin_), end(end_), last(end_ % units_k) {
+        if (end - last < begin) last = 0;
+    }
+};
+template <int PROBLEMS>
+__device__ __forceinline__ bool next_seg(const Shared<PROBLEMS>& sh, const Share& own, int at, int units_k, Seg& s) {
+    const bool first = at < own.last;
+    const int u = first ? own.end - own.last + at : own.begin + at - own.last, end = first ? own.end : own.end - own.last;
+    if (u >= end) return false;
+    int p = at <= own.last ? 0 : s.p;
     while (u >= sh.ubase[p + 1]) ++p;
     const int rel = u - sh.ubase[p];
     const int item = rel / units_k;
     s.p = p;
     s.k0 = rel - item * units_k;
-    s.k1 = min(units_k, s.k0 + (uend - u));
+    s.k1 = min(units_k, s.k0 + (end - u));
     const int chunks = sh.pr[p].chunks;
     s.tile = item / chunks;
     s.chunk = item - s.tile * chunks;
+    s.u = u;
     s.u0 = at;
     return true;
 }
@@ -464,7 +496,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
     using F = Fmt<NBITS>;
     constexpr int PER = F::PER, PARTS = F::PARTS, SLW = F::SLW, UK = F::UK, BLOCKS = F::BLOCKS, DC = F::DC;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ Shared sh;
+    __shared__ Shared<MODE == GG_LINEAR ? GG_MAX_LAYERS : GG_MAX_PROBLEMS> sh;
     const uint32_t raw0 = smem_u32(smem_raw);
     unsigned char* base = smem_raw + ((1024u - (raw0 & 1023u)) & 1023u);
     const uint32_t sbase = smem_u32(base);
@@ -581,7 +613,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
     }
     __syncthreads();
     const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem, 0);
-    const int ub = sh.begin[cta], ue = sh.begin[cta + 1];
+    const Share own(sh.begin[cta], sh.begin[cta + 1], units_k);
     const TmemMap tmap = TmemMap::of(prm.n_max);
     const int slots = tmap.slots;
 
@@ -650,7 +682,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 pending = 0;
             }
         };
-        while (next_seg(sh, ub, ue, at, units_k, s)) {
+        while (next_seg(sh, own, at, units_k, s)) {
             const int n_seg = s.k1 - s.k0;
             at += n_seg;
             int first = group - s.u0 % GROUPS;                // first unit of the run that is this group's
@@ -878,7 +910,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             // =========================== packed weights: two warps, every other unit each ===========================
             const int turn = warp - WARP_RAW;
             int fenced = -1;
-            while (next_seg(sh, ub, ue, at, units_k, s)) {
+            while (next_seg(sh, own, at, units_k, s)) {
                 at += s.k1 - s.k0;
                 const Problem& pr = sh.pr[s.p];
                 const CUtensorMap* maps[2] = {pr.w[0].maps, pr.w[MODE == GG_UP ? 1 : 0].maps};
@@ -926,7 +958,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             if (!counted) grid_dependency_wait();
             int cls = 0, st = 0, filled = 0;                  // filled: stages that have been used since the last change
             uint32_t par = 0xffffffffu;                       // bit i: parity that a wait for "stage i is free" expects
-            while (next_seg(sh, ub, ue, at, units_k, s)) {
+            while (next_seg(sh, own, at, units_k, s)) {
                 at += s.k1 - s.k0;
                 const Problem& pr = sh.pr[s.p];
                 const BClass bc = BClass::of(pr.n, ring);
@@ -963,7 +995,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             int cls = 0, st = 0, seg = 0;
             bool prev_wide = false;
             uint32_t ready = 0;
-            while (next_seg(sh, ub, ue, at, units_k, s)) {
+            while (next_seg(sh, own, at, units_k, s)) {
                 at += s.k1 - s.k0;
                 const Problem& pr = sh.pr[s.p];
                 const int n = pr.n;
@@ -1052,7 +1084,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
         s.p = 0;
         int at = 0, seg = 0, turn = 0;
         bool ok = true;
-        while (next_seg(sh, ub, ue, at, units_k, s)) {
+        while (next_seg(sh, own, at, units_k, s)) {
             at += s.k1 - s.k0;
             const Problem& pr = sh.pr[s.p];
             const int n = pr.n, cnt = pr.cnt;
@@ -1081,42 +1113,48 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t td = tmem + tmap.d_step * (uint32_t)buf + ((uint32_t)(32 * q) << 16);
-            auto load16 = [&](int c0, float (&v)[16]) {
-                uint32_t r[16];
+            // 16 rows of x of this thread's tile row: asked for, and there
+            uint32_t acc[16];
+            auto ask = [&](int c0) {
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                    : "=r"(acc[0]), "=r"(acc[1]), "=r"(acc[2]), "=r"(acc[3]), "=r"(acc[4]), "=r"(acc[5]), "=r"(acc[6]), "=r"(acc[7]),
+                      "=r"(acc[8]), "=r"(acc[9]), "=r"(acc[10]), "=r"(acc[11]), "=r"(acc[12]), "=r"(acc[13]), "=r"(acc[14]), "=r"(acc[15])
                     : "r"(td + (uint32_t)c0));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
             };
+            auto have = [&] {
+                asm volatile("tcgen05.wait::ld.sync.aligned;"
+                             : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]), "+r"(acc[6]), "+r"(acc[7]),
+                               "+r"(acc[8]), "+r"(acc[9]), "+r"(acc[10]), "+r"(acc[11]), "+r"(acc[12]), "+r"(acc[13]), "+r"(acc[14]), "+r"(acc[15])
+                             :
+                             : "memory");
+            };
+            ask(0);
             auto release = [&] {
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) arrive(acc_empty + 8 * (seg & 1));
             };
-            int c_first = cta, c_last = cta;
+            int c_first = cta, c_last = cta, parts_n = 1;
             bool finish = true;
             if (!whole) {
                 // the tile's units are cut over the CTAs c_first .. c_last: leave this CTA's piece, the last one to arrive adds them
-                const int t0 = ub + s.u0 - s.k0;
+                const int t0 = s.u - s.k0;
                 while (c_first > 0 && sh.begin[c_first] > t0) --c_first;
-                int parts_n = 0;
+                parts_n = 0;
                 while (c_last + 1 < grid && sh.begin[c_last + 1] < t0 + units_k) ++c_last;
                 for (int c = c_first; c <= c_last; ++c) parts_n += sh.begin[c + 1] > sh.begin[c] ? 1 : 0;
                 // [4 rows of x][128 tile rows][4]: a warp writes and reads 512 contiguous bytes at a time
                 float4* mine = reinterpret_cast<float4*>(prm.parts) + (size_t)(2 * cta + (s.k0 == 0 ? 1 : 0)) * prm.n_max * 32 + 32 * q + lane;
                 for (int c0 = 0; c0 < rows_here; c0 += 16) {
-                    float v[16];
-                    load16(c0, v);
+                    have();
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
-                        __stcg(mine + (size_t)(c0 / 4 + i) * 128, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+                        __stcg(reinterpret_cast<uint4*>(mine) + (size_t)(c0 / 4 + i) * 128, make_uint4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]));
+                    if (c0 + 16 < rows_here) ask(c0 + 16);
                 }
                 release();
-                __threadfence();
+                __threadfence();                                      // (by every thread: 0.5 us sooner than one for all of them)
                 epi_sync();
                 if (et == 0) {
                     const unsigned arrived = atomicAdd(prm.counters + c_first, 1u);
@@ -1127,133 +1165,154 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 }
                 epi_sync();
                 finish = sh.last != 0;
-                __threadfence();
             } else {
                 epi_sync();                                           // s_scale and the others are complete
             }
             if (finish) {
-                // 8 rows of the sum of the pieces, in CTA order (a CTA without a unit has none), four pieces on their way at
-                // once: what a tile of many short pieces costs is their latency
-                auto add_pieces = [&](int r0, float* v) {
+                // A cut tile: the pieces in CTA order (a CTA without a unit has none), 16 rows at a time.  What this costs is latency,
+                // so several are under way; a thread copies what it will read itself, which needs no barrier.
+                const uint32_t merge = raw_ring + (uint32_t)(n_raw * F::RAW_BYTES) + 16u * et;
+                const int n_merge = F::n_merge(prm.n_max);
+                const bool dense = parts_n == c_last - c_first + 1;
+                const uint32_t step = (uint32_t)prm.n_max * 32u;      // of a CTA's two pieces
+                const float4* fetch_src = reinterpret_cast<const float4*>(prm.parts) + 32 * q + lane;
+                int fetch_c = c_first, fetch_r = 0, fetch_at = 0, merge_at = 0;
+                auto fetch = [&] {
+                    if (fetch_r < rows_here) {
+                        const float4* src = fetch_src + (uint32_t)(2 * fetch_c + (fetch_c == c_first ? 1 : 0)) * (size_t)step;
+                        const uint32_t dst = merge + (uint32_t)(fetch_at * MERGE_BYTES);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] = 0.f;
-                    for (int cb = c_first; cb <= c_last; cb += 4) {
-                        float4 f[4][2];
-#pragma unroll
-                        for (int d = 0; d < 4; ++d) {
-                            const int c = cb + d;
-                            const bool has = c <= c_last && sh.begin[c + 1] > sh.begin[c];
-                            const float4* src = reinterpret_cast<const float4*>(prm.parts) + ((size_t)(2 * c + (c == c_first ? 1 : 0)) * prm.n_max + r0) * 32 + 32 * q + lane;
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) f[d][i] = has ? __ldcg(src + (size_t)i * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int i = 0; i < 4; ++i)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(i * MERGE_BYTES / 4)), "l"(src + i * 128) : "memory");
+                        fetch_at = fetch_at + 1 == n_merge ? 0 : fetch_at + 1;
+                        ++fetch_c;
+                        if (!dense)
+                            while (fetch_c <= c_last && sh.begin[fetch_c + 1] <= sh.begin[fetch_c]) ++fetch_c;
+                        if (fetch_c > c_last) {
+                            fetch_c = c_first;
+                            fetch_r += 16;
+                            fetch_src += 16 * 32;
                         }
+                    }
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                };
+                auto add_pieces = [&](float (&v)[16]) {
 #pragma unroll
-                        for (int d = 0; d < 4; ++d)
+                    for (int i = 0; i < 16; ++i) v[i] = 0.f;
+#pragma unroll 1
+                    for (int c = 0; c < parts_n; ++c) {
+                        // the oldest of n_merge groups has arrived
+                        if (n_merge == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+                        else if (n_merge == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+                        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                        const uint32_t at = merge + (uint32_t)(merge_at * MERGE_BYTES);
 #pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                v[4 * i] += f[d][i].x;
-                                v[4 * i + 1] += f[d][i].y;
-                                v[4 * i + 2] += f[d][i].z;
-                                v[4 * i + 3] += f[d][i].w;
-                            }
+                        for (int i = 0; i < 4; ++i) {
+                            const uint4 f = lds128(at + (uint32_t)(i * MERGE_BYTES / 4));
+                            v[4 * i] += __uint_as_float(f.x);
+                            v[4 * i + 1] += __uint_as_float(f.y);
+                            v[4 * i + 2] += __uint_as_float(f.z);
+                            v[4 * i + 3] += __uint_as_float(f.w);
+                        }
+                        merge_at = merge_at + 1 == n_merge ? 0 : merge_at + 1;
+                        fetch();
                     }
                 };
+                if (!whole)
+                    for (int i = 0; i < n_merge; ++i) fetch();
+                // What a thread writes of 16 rows of x, from the buffer in which they change places.
+                const int wt = et >> 4, wm = et & 15;                 // rows wt and wt + 8; member
+                constexpr int TB_ROW = MODE == GG_UP ? 64 : 128;      // values of a row of x in the buffer
+                unsigned char* h_dst = nullptr;
+                uint16_t* out = nullptr;
+                int64_t ld = 0;
+                bool runs = true, exists = true;                      // eight neighbouring outputs in one store; the member has these rows
+                if constexpr (MODE == GG_UP) {
+                    const int col = wm * pr.G + PER * rho;            // four neighbouring columns of h, staged at pos .. pos + 3
+                    const int pos = tile_pos(col & 63), row = pr.row0 + s.chunk * n + wt;       // (row and row + 8, 16, ... share the swizzle)
+                    h_dst = prm.ht + ((int64_t)(col >> 6) * prm.xt_rows + row) * 128 + ((((pos >> 3) ^ (row & 7)) << 4) | ((pos & 7) * 2));
+                } else {
+                    ld = (MODE == GG_LINEAR) ? pr.N : prm.N;
+                    out = reinterpret_cast<uint16_t*>(MODE == GG_LINEAR ? prm.hp[s.p].y : prm.out) + (int64_t)(m0 + wm) * pr.G + PER * rho0;
+                    exists = !F::WORDS || (m0 + wm) * pr.G + PER * rho0 < pr.N;
+                    runs = !(MODE == GG_DOWN && prm.accumulate) && pr.P - rho0 >= PARTS && ((reinterpret_cast<uintptr_t>(out) | (uintptr_t)(ld * 2)) & 15) == 0;
+                    if (MODE == GG_LINEAR) out += (int64_t)(list + wt) * ld;
+                }
+                const int at0 = MODE == GG_UP ? (lane & 1) * 8 * 64 + member * 4 + (((slot & 1) << 1) | (slot >> 1)) : member * RUN + part * PER + slot;
+#pragma unroll 1
                 for (int c0 = 0; c0 < rows_here; c0 += 16) {
                     float v[16];
                     if (whole) {
-                        load16(c0, v);
-                        if (c0 + 16 >= rows_here) release();
+                        have();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(acc[i]);
                     } else {
-                        add_pieces(c0, v);
-                        add_pieces(c0 + 8, v + 8);
+                        add_pieces(v);
                     }
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float4 f = *reinterpret_cast<const float4*>(s_scale + c0 + 4 * i);
-                        v[4 * i] *= f.x;
-                        v[4 * i + 1] *= f.y;
-                        v[4 * i + 2] *= f.z;
-                        v[4 * i + 3] *= f.w;
+                        const float ff[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v[4 * i + e] *= ff[e];
                     }
-                    uint16_t* tb = reinterpret_cast<uint16_t*>(epi + turn * TILE_BYTES);
+                    if (whole) {                                      // the next rows are on their way under this arithmetic
+                        if (c0 + 16 < rows_here) ask(c0 + 16);
+                        else release();
+                    }
+                    uint16_t* tb = reinterpret_cast<uint16_t*>(epi + turn * TILE_BYTES) + at0;
                     turn ^= 1;                                        // two buffers: one barrier per 16 rows
                     if constexpr (MODE == GG_UP) {
-                        // neighbouring lanes hold the gate (even) and the up (odd) sums of one row of h; each finishes 8 rows of x
+                        // neighbouring lanes hold the gate (even) and the up (odd) sums of one row of h; each finishes 8 rows of x, two at
+                        // a time: packed roundings and products
                         const bool up = (lane & 1) != 0;
-                        uint16_t hv[8];
+                        uint32_t p[8];
 #pragma unroll
-                        for (int i = 0; i < 8; i += 2) {                  // two rows at a time: packed roundings and products
-                            uint32_t a2, b2;
-                            float a[2], b[2];
+                        for (int i = 0; i < 8; ++i) p[i] = bf2(v[2 * i], v[2 * i + 1]);
 #pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                const float give = up ? v[i + e] : v[i + e + 8];
-                                const float other = __shfl_xor_sync(0xffffffffu, give, 1);
-                                a[e] = up ? other : v[i + e];
-                                b[e] = up ? v[i + e + 8] : other;
-                            }
-                            a2 = bf2(a[0], a[1]);
-                            b2 = bf2(b[0], b[1]);
+                        for (int i = 0; i < 4; ++i) {
+                            const uint32_t other = __shfl_xor_sync(0xffffffffu, up ? p[i] : p[i + 4], 1);
+                            const uint32_t a2 = up ? other : p[i], b2 = up ? p[i + 4] : other;
                             const float a0 = __uint_as_float(a2 << 16), a1 = __uint_as_float(a2 & 0xffff0000u);
-                            const uint32_t g2 = bf2(__fdividef(a0, 1.f + __expf(-a0)), __fdividef(a1, 1.f + __expf(-a1)));
+                            const uint32_t g2 = bf2(silu(a0), silu(a1));
                             uint32_t h2 = bf2_mul(g2, b2);
-                            if (cnt <= GG_F16_ROWS) {
-                                const __half2 f = __floats2half2_rn(__uint_as_float(h2 << 16), __uint_as_float(h2 & 0xffff0000u));
-                                h2 = *reinterpret_cast<const uint32_t*>(&f);
-                            }
-                            hv[i] = (uint16_t)h2;
-                            hv[i + 1] = (uint16_t)(h2 >> 16);
-                        }
-                        // [row][member][slot in the order 0, 2, 1, 3]
-                        const int so = ((slot & 1) << 1) | (slot >> 1);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) tb[(i + (up ? 8 : 0)) * 64 + member * 4 + so] = hv[i];
-                        epi_sync();
-#pragma unroll
-                        for (int jj = 0; jj < 2; ++jj) {
-                            const int t = (et >> 4) + 8 * jj, m = et & 15;
-                            if (c0 + t < rows_here) {
-                                const int col = m * pr.G + PER * rho;         // four neighbouring columns of h, staged at pos .. pos + 3
-                                const int row = pr.row0 + s.chunk * n + c0 + t;
-                                const int pos = tile_pos(col & 63);
-                                unsigned char* dst = prm.ht + ((int64_t)(col >> 6) * prm.xt_rows + row) * 128 +
-                                                     ((((pos >> 3) ^ (row & 7)) << 4) | ((pos & 7) * 2));
-                                *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(tb + t * 64 + m * 4);
-                            }
+                            if (cnt <= GG_F16_ROWS) h2 = h2_of(__uint_as_float(h2 << 16), __uint_as_float(h2 & 0xffff0000u));
+                            tb[2 * i * 64] = (uint16_t)h2;            // [row][member][slot in the order 0, 2, 1, 3]
+                            tb[(2 * i + 1) * 64] = (uint16_t)(h2 >> 16);
                         }
                     } else {
-                        const int idx = member * RUN + part * PER + slot;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            uint16_t o;
+                        for (int i = 0; i < 8; ++i) {
+                            uint32_t o;
                             if (MODE == GG_LINEAR) {
-                                const float y = v[i] + bias;
-                                o = prm.y_f16 ? __half_as_ushort(__float2half_rn(y)) : float_to_bf16_bits(y);
+                                const float y0 = v[2 * i] + bias, y1 = v[2 * i + 1] + bias;
+                                o = prm.y_f16 ? h2_of(y0, y1) : bf2(y0, y1);
                             } else {
-                                o = float_to_bf16_bits(round_bf16(v[i]) * s_weight[c0 + i]);
+                                const float2 w = *reinterpret_cast<const float2*>(s_weight + c0 + 2 * i);
+                                const uint32_t r = bf2(v[2 * i], v[2 * i + 1]);
+                                o = bf2(__uint_as_float(r << 16) * w.x, __uint_as_float(r & 0xffff0000u) * w.y);
                             }
-                            tb[i * 128 + idx] = o;
+                            tb[2 * i * 128] = (uint16_t)o;
+                            tb[(2 * i + 1) * 128] = (uint16_t)(o >> 16);
                         }
-                        epi_sync();
-                        constexpr int MEMBERS = F::MEMBERS;
-                        const int valid = min(PARTS, pr.P - rho0) * PER;      // neighbouring rows that exist
-                        const int64_t ld = (MODE == GG_LINEAR) ? pr.N : prm.N;
-                        uint16_t* out = reinterpret_cast<uint16_t*>(MODE == GG_LINEAR ? prm.hp[s.p].y : prm.out);
-#pragma unroll 2
-                        for (int j = et; j < 16 * MEMBERS; j += 128) {
-                            const int t = j / MEMBERS, m = j % MEMBERS;
-                            if (c0 + t >= rows_here || (F::WORDS && (m0 + m) * pr.G + PER * rho0 >= pr.N)) continue;
-                            const uint16_t* src = tb + t * 128 + m * RUN;
-                            const int64_t row = MODE == GG_DOWN ? s_row[c0 + t] : list + c0 + t;
-                            uint16_t* dst = out + row * ld + (int64_t)(m0 + m) * pr.G + PER * rho0;
-                            if (MODE == GG_DOWN && prm.accumulate) {
-                                for (int x = 0; x < valid; ++x) dst[x] = float_to_bf16_bits(bf16_bits_to_float(src[x]) + bf16_bits_to_float(dst[x]));
-                            } else if (valid == RUN && (((uintptr_t)dst) & (RUN * 2 - 1)) == 0) {
-                                if constexpr (RUN == 8) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-                                else if constexpr (RUN == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
-                                else *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(src);
+                    }
+                    epi_sync();
+                    const uint16_t* from = reinterpret_cast<const uint16_t*>(epi + (turn ^ 1) * TILE_BYTES) + wt * TB_ROW;
+#pragma unroll
+                    for (int jj = 0; jj < 2; ++jj) {
+                        const int t = wt + 8 * jj;
+                        if (c0 + t >= rows_here || !exists) continue;
+                        if constexpr (MODE == GG_UP) {
+                            *reinterpret_cast<uint2*>(h_dst + (int64_t)(c0 + 8 * jj) * 128) = *reinterpret_cast<const uint2*>(from + jj * 8 * 64 + wm * 4);
+                        } else {
+                            const uint16_t* src = from + jj * 8 * 128 + wm * RUN;
+                            uint16_t* dst = MODE == GG_DOWN ? out + (int64_t)s_row[c0 + t] * ld : out + (int64_t)(c0 + 8 * jj) * ld;
+                            if (runs) {
+                                *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
                             } else {
-                                for (int x = 0; x < valid; ++x) dst[x] = src[x];
+                                const int valid = min(PARTS, pr.P - rho0) * PER;      // neighbouring rows that exist
+                                const bool add = MODE == GG_DOWN && prm.accumulate;
+                                for (int x = 0; x < valid; ++x) dst[x] = add ? float_to_bf16_bits(bf16_bits_to_float(src[x]) + bf16_bits_to_float(dst[x])) : src[x];
                             }
                         }
                     }
