@@ -19,6 +19,15 @@ def test_exact(nbits, group, N, K, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("group, N, K, std", [(16, 192, 64, 0.02), (16, 64, 1088, 3e4), (48, 384, 256, 1e-6), (5, 20, 512, 0.02)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_a_table_of_four_values(group, N, K, std, dtype):
+    """2 bit into 16-bit types: K of few columns and no multiple of a CTA's, values beyond fp16 and below its normal range."""
+    od = random_layer(N, K, 2, group, seed=7, std=std)
+    assert torch.equal(layer_from_oracle(od, DEV).dequantize(dtype).cpu(), O.dequantize(od).to(dtype))
+
+
+@pytest.mark.gpu
 def test_tensors_off_the_vector_alignment():
     od = random_layer(128, 256, 2, 16, seed=6)
     layer = layer_from_oracle(od, DEV)
