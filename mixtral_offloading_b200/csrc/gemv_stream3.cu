@@ -11,7 +11,9 @@
 // (4 columns) of members g and g+8 for each of the 4 column quarters; two words are merged
 // with PRMT and one LOP3 per slot yields the fp16 pair OFFSET + code.  Ten slot MMAs (each
 // with its own accumulator tile, columns = slots) and two correction MMAs per 16 columns.
-// One row of x per launch.
+// One row of x per launch.  14336 x 4096: 21.8 us with remainders formed in every pass and weights first asked for in their
+// pass, 21.1 so; 7168 passes of about 600 instructions and 48 MMAs (9 cycles each) on 592 schedulers are 12 each, 5 us, the rest
+// is start-up, three serial passes per warp and the finalize launch.
 #include <type_traits>
 
 #include "common.cuh"
@@ -68,8 +70,8 @@ struct Split3 {
 constexpr int ROW = 72;            // 64 columns + padding (halfs)
 constexpr int XPASS = 8;           // longest range of a warp, in passes
 constexpr int NW = 8;
-// per warp: xs[10][ROW], zz[10 + 1][ROW] (row 10 zero), x staging [XPASS * 64]
-constexpr int WARP_HALFS = 21 * ROW + XPASS * 64;
+// per warp: xs[10][ROW], zz[10 + 1][ROW] (row 10 zero), x staging [XPASS * 64], scale tasks [80] of 8 bytes
+constexpr int WARP_HALFS = 21 * ROW + XPASS * 64 + 80 * 4;
 
 // The ten fp16 pairs OFFSET + code of two words (two adjacent columns k, k+1), slot s in out[s].
 // lo = low halves of both words (slots 9..5 at bits 0,3,..,12), hi = the same of the words >> 15
@@ -101,9 +103,27 @@ gemv_stream3_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x,
     __half* xs_w = reinterpret_cast<__half*>(smem_raw) + wi * WARP_HALFS;   // [10][ROW]
     __half* zz_w = xs_w + 10 * ROW;                                          // [11][ROW], row 10 stays zero
     __half* xh = zz_w + 11 * ROW;                                            // [XPASS * 64]
+    uint2* tasks = reinterpret_cast<uint2*>(xh + XPASS * 64);
     grid_launch_dependents();                       // overlapped launch: set-up runs under the kernel in front
     for (int i = lane; i < 21 * ROW / 2; i += 32) reinterpret_cast<uint32_t*>(xs_w)[i] = 0u;
     __syncwarp();
+    const int gw = blockIdx.x * NW + wi;
+    const uint32_t L_begin = sp.begin(gw), L_end = sp.begin(gw + 1);
+    // A warp has three or four passes, loaded into registers one after the other: all their lines are asked for in L2 now, under
+    // the kernel in front (weights are never written by it), so that a pass waits for L2 instead of HBM.
+    for (uint32_t L = L_begin; L < L_end;) {
+        const int rho = (int)(L / (uint32_t)PT), pa = (int)(L - (uint32_t)rho * (uint32_t)PT);
+        const int n = min(PT, pa + (int)(L_end - L)) - pa;
+        L += (uint32_t)n;
+        for (int i = lane; i < 32 * n; i += 32) {         // 16 members, 128 bytes
+            const int64_t R = (int64_t)rho + (int64_t)(i & 15) * P3;
+            if (R < rows) prefetch_l2(reinterpret_cast<const uint32_t*>(w.W_q) + R * K + pa * 64 + (i >> 4) * 32);
+        }
+        for (int i = lane; i < 20 * n; i += 32) {         // 10 residues' scales and zeros, 64 bytes
+            const int s = i % 20;
+            prefetch_l2((s < 10 ? w.scale_q : w.zero_q) + (int64_t)((10 * rho + s % 10) % G) * K + (pa + i / 20) * 64);
+        }
+    }
     grid_dependency_wait();                         // x, the row index and the partial buffer belong to earlier kernels
 
     const uint16_t* xr = x + (int64_t)(x_idx ? x_idx[m] : m) * K;
@@ -114,8 +134,6 @@ gemv_stream3_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x,
     const uint32_t off0 = slot_offset(g) * 0x00010001u;
     const uint32_t off1 = g < 2 ? slot_offset(8 + g) * 0x00010001u : 0u;
 
-    const int gw = blockIdx.x * NW + wi;
-    const uint32_t L_begin = sp.begin(gw), L_end = sp.begin(gw + 1);
     for (uint32_t L = L_begin; L < L_end;) {
         const int rho = (int)(L / (uint32_t)PT), pa = (int)(L - (uint32_t)rho * (uint32_t)PT);
         const int pb = min(PT, pa + (int)(L_end - L));
@@ -141,6 +159,14 @@ gemv_stream3_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x,
         const uint32_t* row0 = Wq + R0 * K + 4 * t;
         const uint32_t* row1 = Wq + R1 * K + 4 * t;
 
+        // The scale tasks of a pass (slot, column octet): flat index in the segment's first pass, and its column of the fp16 values
+        // (two remainders each, which took as long as the decoding when every pass formed them).
+        for (int task = lane; task < 80; task += 32) {
+            const uint32_t idx = (uint32_t)(10 * rho + (task >> 3)) % (uint32_t)G * (uint32_t)K + (uint32_t)(pa * 64 + (task & 7) * 8);
+            tasks[task] = make_uint2(idx, idx % (uint32_t)C);
+        }
+        __syncwarp();
+
         for (int p = pa; p < pb; ++p) {
             const int k0 = p * 64;
             // ---- weight words of the pass: 4 column quarters x 2 members
@@ -156,9 +182,10 @@ gemv_stream3_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x,
                 const int task = rnd * 32 + lane;
                 if (task < 80) {
                     const int sd = task >> 3, kd = (task & 7) * 8;
-                    const uint32_t r = (uint32_t)(10 * rho + sd) % (uint32_t)G;
-                    const uint32_t idx = r * (uint32_t)K + (uint32_t)(k0 + kd);
-                    const uint32_t col = idx % (uint32_t)C;
+                    const uint2 at = tasks[task];
+                    const uint32_t ahead = (uint32_t)(p - pa) * 64u, idx = at.x + ahead;
+                    uint32_t col = at.y + ahead;
+                    while (col >= (uint32_t)C) col -= (uint32_t)C;
                     const uint2 sq = *reinterpret_cast<const uint2*>(w.scale_q + idx);
                     const uint2 zq = *reinterpret_cast<const uint2*>(w.zero_q + idx);
                     const uint4 mss = *reinterpret_cast<const uint4*>(w.ms_scale + col);
