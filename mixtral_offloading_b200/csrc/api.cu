@@ -82,6 +82,20 @@ static bool use_gg(const hqm_weight* w, int G, int C, int64_t M, bool f16 = fals
     return M >= (w->nbits == 3 ? 2 : GG_MIN_ROWS) && M <= (1 << 22) && (f16 ? gg_supported(w, G, C) : gg_takes(w, G, C, M));
 }
 
+// Large 2-bit layers with groups of 16, 2 to 5 rows, where the workspace holds the partial rows of a CTA per SM (the streaming and
+// the tensor-core kernel, which take them otherwise, make do with less).  us, those / gemv_rows.cu:
+//   rows             2            3            4            5            8
+//   14336 x 4096     15.1 / 13.6  17.9 / 13.8  18.2 / 15.2  19.1 / 16.2  19.1 / 19.3
+//   4096 x 14336     17.6 / 17.4  20.3 / 17.4  20.5 / 17.9  20.7 / 19.9  20.7 / 19.8
+//   4096 x 4096       9.9 / 10.4   9.4 / 10.5  10.1 / 11.6  10.9 / 12.5  (less than a step of the kernel for every SM)
+//   3072 x 5120       9.4 / 10.6   9.5 / 11.3   9.9 / 11.8  11.1 / 12.3  (120 steps)
+static bool use_rows(int64_t M, const hqm_weight* w, StreamPlan* plan, size_t* bytes) {
+    const hqm_weight* one[1] = {w};
+    if (M < 2 || M > 5 || force_generic() || !gemv_rows_plan(one, 1, M, plan) || plan->rho0[1] * plan->PT < 3 * plan->grid) return false;
+    *bytes = (gemv_stream_scratch_bytes(*plan, M) + 255) / 256 * 256;
+    return true;
+}
+
 // The kernels beside gemm_grouped.cu: what the one that takes the call needs.
 static size_t other_scratch_bytes(int64_t M, const hqm_weight* w, int G, int C) {
     if (gemm_tc3_supported(w, G, C, M)) return gemm_tc3_scratch_bytes(w, G, M);
@@ -99,6 +113,11 @@ static size_t other_scratch_bytes(int64_t M, const hqm_weight* w, int G, int C) 
 size_t linear_scratch_bytes(int64_t M, const hqm_weight* w, bool preferred) {
     int G, C;
     if (M <= 0 || check_weight(w, &G, &C) != HQM_OK || force_generic()) return 0;
+    if (preferred) {
+        StreamPlan plan;
+        size_t bytes;
+        if (use_rows(M, w, &plan, &bytes)) return std::max(bytes, linear_scratch_bytes(M, w));
+    }
     if (!use_gg(w, G, C, M)) return other_scratch_bytes(M, w, G, C);
     const size_t sums = w->nbits != 3 && M > STREAM_MAX_ROWS ? (size_t)M * w->N * sizeof(float) : other_scratch_bytes(M, w, G, C);
     const size_t least = std::max(gg_least_bytes(w->K), (sums + 255) / 256 * 256);
@@ -177,6 +196,14 @@ int launch_linear(uint16_t* y, const uint16_t* x, const int32_t* x_idx, int64_t 
     StreamPlan plan;
     const bool x_ok = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     if (!x_ok || force_generic()) return launch_linear_generic(y, x, x_idx, M, w, G, C, bias, st);
+    size_t rows_bytes;
+    if (scratch != nullptr && (reinterpret_cast<uintptr_t>(scratch) & 15u) == 0 && use_rows(M, w, &plan, &rows_bytes) && scratch_bytes >= rows_bytes) {
+        StreamJob job{};
+        job.w[0] = w;
+        job.counters = counters;
+        rc = launch_gemv_stream((float*)scratch, x, x_idx, M, job, plan, st);
+        return rc != HQM_OK ? rc : launch_finalize_linear(y, (const float*)scratch, bias, M, plan, st);
+    }
     if (use_gg(w, G, C, M)) {
         return linear_gg(&y, &w, &bias, 1, x, x_idx, M, counters, scratch, scratch_bytes, st);
     }

@@ -1,10 +1,12 @@
-"""csrc/gemv_rows.cu through an expert (up to 8 rows) and csrc/gemv_lists.cu through a block: the remainders of their units and
+"""csrc/gemv_rows.cu through an expert (up to 8 rows) or a layer (up to 5), and csrc/gemv_lists.cu through a block: the remainders of their units and
 shares, every number of rows, layers they leave to the other kernels, rows outside the range of fp16."""
+import ctypes as C
+
 import pytest
 import torch
 
 from mixtral_offloading_b200 import ResidentMoe, _cabi
-from tests.helpers import random_layer
+from tests.helpers import layer_from_oracle, random_layer, random_layer_fast
 from tests.test_gpu_parity import Cfg, make_expert
 from tests.test_many_row_precision import weight64
 
@@ -83,3 +85,25 @@ def test_lists_of_every_length(hidden, ffn, n_exp, tokens):
     assert (error / size).max().item() < 1.3e-2
     assert torch.equal(y, moe(x.view(1, tokens, hidden))[0].view(tokens, hidden))
     assert _cabi.lib().hqm_device_error() == 0
+
+
+@pytest.mark.parametrize("N,K", [(14336, 4096), (4096, 14336), (14336, 3072)])
+def test_large_linear_layers(N, K):
+    """Two to five rows of layers with three steps or more for every SM; with less workspace than that wants, and a bias."""
+    layer = layer_from_oracle(random_layer_fast(N, K, 2, 16, seed=3), DEV)
+    layer.bias = torch.randn(N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    lib, d, W = _cabi.lib(), layer.descriptor(), weight64(layer)
+    for M in (1, 2, 4, 5, 6):
+        x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(DEV)
+        want = x.double() @ W.t() + layer.bias.double()
+        need, wanted = lib.hqm_linear_scratch_bytes(M, C.byref(d)), lib.hqm_linear_scratch_preferred(M, C.byref(d))
+        assert wanted >= need
+        for size in (need, wanted - 1, wanted):
+            ws = torch.full((wanted + 4096,), 7, dtype=torch.uint8, device=DEV)
+            _cabi.check(lib.hqm_scratch_init(_cabi.ptr(ws), _cabi.stream_ptr(DEV)))
+            y = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+            _cabi.check(lib.hqm_linear(_cabi.ptr(y), _cabi.ptr(x), M, C.byref(d), _cabi.ptr(layer.bias), _cabi.ptr(ws), max(size, need),
+                                       _cabi.stream_ptr(DEV)))
+            assert bool((ws[max(size, need):] == 7).all())
+            # a rounding to bf16 (1.7e-3) and 16-bit factors (1e-3)
+            assert ((y.double() - want).norm() / want.norm()).item() < 2.5e-3, (M, size)
