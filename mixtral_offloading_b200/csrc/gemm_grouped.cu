@@ -40,12 +40,13 @@
 //   warp 23      issues the MMAs
 //
 // Work split: the units of all tiles of all problems follow each other, weighted by what a unit costs with its list's
-// row count, and every CTA takes an equal contiguous share.  A tile cut by a share's boundary is summed from fp32
+// row count, and every CTA takes an equal contiguous share (a launch whose rows the host knows: the layout's share, so that
+// whole tiles stay whole where their number is no multiple of the CTAs').  A tile cut by a share's boundary is summed from fp32
 // pieces in scratch memory by whichever CTA arrives last, in CTA order (no atomics on results, deterministic).
 //
 // Measured (before: the same layers through a kernel that staged A in shared memory, expert by expert): up + gate of 8
-// experts, 4096 -> 14336, 33 tokens: 201 us alone, down 103 us; the whole block 943 -> 299 us.  One expert with 512 rows
-// 325 -> 226 us: up 134, down 83.  A unit takes ~930 cycles (2500 warp instructions) at few rows, with 63 % of the issue
+// experts, 4096 -> 14336, 33 tokens: 201 us alone, down 103 us; the whole block 943 -> 299 us (lists of up to 8 rows go to
+// gemv_lists.cu by now).  One expert with 512 rows 325 -> 205 us.  A unit takes ~930 cycles (2500 warp instructions) at few rows, with 63 % of the issue
 // slots, 6 % of the tensor pipe and 23 % of HBM in use; without the decoding of scales and zeros, the weights' arithmetic
 // and the MMAs the same pipeline runs at ~430.  With 256 rows a unit takes 1200 while the MMAs run (1024 their own), but a tile of
 // 256 rows has the accumulator to itself, and writing it out took 14.7 us beside the 20.5 of its 32 units; a cut tile of 256 rows
@@ -55,6 +56,9 @@
 //     itself); with 8 rows a time 214, with 16 205, and a 4-bit layer of 16 rows 11.35 and 11.12 (11.20 before);
 //   * the next 16 rows' sums are asked for before the present ones are worked on; exponential and reciprocal without the branches
 //     for denormals, roundings before the exchange between lanes.
+//   * where whole tiles are all there is, their addresses and factors are worked out before the sums are waited for, and the room of the
+//     pieces holds packed units: 4-bit 6144 x 1024, 40 rows 10.86 -> 10.58, 3-bit 11264 x 4096, 400 rows (whole tiles that used to
+//     be cut, as their number is no multiple of the CTAs') 116 -> 106.
 // (A second group of epilogue warps, for 8 registers less in each dequantising one: no gain at 512 rows, and 3-bit layers 7 % slower.)
 //
 // 3-bit layers (ten codes of one column in 32 bits; 10 does not divide the number of groups): storage rows rho + i * P3 hold
@@ -155,6 +159,7 @@ struct Params {
     int which0, which1;
     const int32_t* counts;
     int rows, few;
+    int share, cut;                        // units of a CTA (0: shares of equal cost); some tile may be cut
     const unsigned char* xt;
     int64_t xt_rows;
     const float* row_scale;                // of the staged rows (null: 1)
@@ -210,15 +215,18 @@ struct Fmt {
     // Launches of up to 64 rows per chunk need few staged rows in flight and many packed bytes, others the reverse.
     __host__ __device__ static constexpr int b_ring(int n_max) { return WORDS ? 80 * 1024 : (n_max <= 64 ? 64 * 1024 : 128 * 1024); }
     // (Even: a slot is filled by one of the two copying warps then, and its phases are waited for in order.)
-    __host__ __device__ static constexpr int n_raw(int n_max) { return WORDS || n_max > 64 ? 6 : 8; }
+    // (2 bit, wide chunks: 8 where no tile is cut and nothing is summed: 3072 x 2048, 80 rows 12.9 us with 6, 12.6 with 8.)
+    __host__ __device__ static constexpr int n_raw(int n_max, bool cut) { return WORDS || (n_max > 64 && (cut || PARTS == 4)) ? 6 : 8; }
     // Pieces of 16 rows in flight while a cut tile is summed: as many as there is room for.
     __host__ __device__ static constexpr int n_merge(int n_max) { return WORDS ? 1 : (n_max <= 64 ? 4 : (PARTS == 4 ? 1 : 3)); }
     static constexpr int ST_OFF = 0, EPI_OFF = ST_OFF + 4 * GROUPS * ST_WARP, BAR_OFF = EPI_OFF + EPI_BYTES, RING_OFF = BAR_OFF + 1024;
-    __host__ __device__ static constexpr int smem(int n_max) {
-        return (RING_OFF + 1023) / 1024 * 1024 + b_ring(n_max) + n_raw(n_max) * RAW_BYTES + n_merge(n_max) * MERGE_BYTES + 1024;
+    __host__ __device__ static constexpr int smem(int n_max, bool cut) {
+        return (RING_OFF + 1023) / 1024 * 1024 + b_ring(n_max) + n_raw(n_max, cut) * RAW_BYTES + (cut ? n_merge(n_max) * MERGE_BYTES : 0) + 1024;
     }
+    static constexpr int max2(int a, int b) { return a > b ? a : b; }
+    static constexpr int MOST = max2(max2(smem(64, false), smem(64, true)), max2(smem(256, false), smem(256, true)));
     static constexpr int SHARED = NBITS == 2 ? (int)sizeof(Shared<GG_MAX_PROBLEMS>) : (int)sizeof(Shared<GG_MAX_LAYERS>);
-    static_assert(smem(64) + SHARED <= 227 * 1024 && smem(256) + SHARED <= 227 * 1024, "shared memory");
+    static_assert(MOST + SHARED <= 227 * 1024, "shared memory");
     // Which row of the tile TMEM lane 32 q + 8 j + g holds (q: warp of a group, j = 0..3): part, slot of the byte, member.
     // A thread of the 16x256b store shape holds j = 0..3 at one g: four members of one quantisation group.
     __device__ __forceinline__ static int part_of(int q, int g) { return (NBITS == 4 ? 2 * (q >> 1) : 0) + (g & 1); }
@@ -500,7 +508,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
     const uint32_t raw0 = smem_u32(smem_raw);
     unsigned char* base = smem_raw + ((1024u - (raw0 & 1023u)) & 1023u);
     const uint32_t sbase = smem_u32(base);
-    const int n_raw = F::n_raw(prm.n_max), ring = F::b_ring(prm.n_max);
+    const int n_raw = F::n_raw(prm.n_max, prm.cut != 0), ring = F::b_ring(prm.n_max);
     const uint32_t b_ring = sbase + (F::RING_OFF + 1023) / 1024 * 1024, raw_ring = b_ring + ring;
     const uint32_t bars = sbase + F::BAR_OFF;
     const uint32_t raw_full = bars, raw_empty = raw_full + 8 * MAX_RAW, a_full = raw_empty + 8 * MAX_RAW, a_empty = a_full + 8 * NA,
@@ -602,7 +610,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if ((int)threadIdx.x <= grid) {
+    if (prm.share > 0) {
+        if ((int)threadIdx.x <= grid) sh.begin[threadIdx.x] = min(sh.ubase[prm.problems], (int)threadIdx.x * prm.share);
+    } else if ((int)threadIdx.x <= grid) {
         const unsigned long long total = sh.cbase[prm.problems];
         const unsigned long long at = total * (unsigned long long)threadIdx.x / (unsigned)grid;
         int e = 0;
@@ -1109,6 +1119,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 const uint16_t* bp = prm.hp[s.p].bias;
                 if (bp && rho < pr.P && (!F::WORDS || (m0 + member) * pr.G + PER * rho + slot < pr.N)) bias = bf16_bits_to_float(bp[(m0 + member) * pr.G + PER * rho + slot]);
             }
+            // What a thread writes of 16 rows of x, from the buffer in which they change places.
+            const int wt = et >> 4, wm = et & 15;                 // rows wt and wt + 8; member
+            constexpr int TB_ROW = MODE == GG_UP ? 64 : 128;      // values of a row of x in the buffer
+            unsigned char* h_dst = nullptr;
+            uint16_t* out = nullptr;
+            int64_t ld = 0;
+            bool runs = true, exists = true;                      // eight neighbouring outputs in one store; the member has these rows
+            if constexpr (MODE == GG_UP) {
+                const int col = wm * pr.G + PER * rho;            // four neighbouring columns of h, staged at pos .. pos + 3
+                const int pos = tile_pos(col & 63), row = pr.row0 + s.chunk * n + wt;       // (row and row + 8, 16, ... share the swizzle)
+                h_dst = prm.ht + ((int64_t)(col >> 6) * prm.xt_rows + row) * 128 + ((((pos >> 3) ^ (row & 7)) << 4) | ((pos & 7) * 2));
+            } else {
+                ld = (MODE == GG_LINEAR) ? pr.N : prm.N;
+                out = reinterpret_cast<uint16_t*>(MODE == GG_LINEAR ? prm.hp[s.p].y : prm.out) + (int64_t)(m0 + wm) * pr.G + PER * rho0;
+                exists = !F::WORDS || (m0 + wm) * pr.G + PER * rho0 < pr.N;
+                runs = !(MODE == GG_DOWN && prm.accumulate) && pr.P - rho0 >= PARTS && ((reinterpret_cast<uintptr_t>(out) | (uintptr_t)(ld * 2)) & 15) == 0;
+                if (MODE == GG_LINEAR) out += (int64_t)(list + wt) * ld;
+            }
+            const int at0 = MODE == GG_UP ? (lane & 1) * 8 * 64 + member * 4 + (((slot & 1) << 1) | (slot >> 1)) : member * RUN + part * PER + slot;
+            epi_sync();                                               // s_scale and the others are complete
             if (!wait(acc_full + 8 * (seg & 1), (seg >> 1) & 1)) ok = false;
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1165,8 +1195,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 }
                 epi_sync();
                 finish = sh.last != 0;
-            } else {
-                epi_sync();                                           // s_scale and the others are complete
             }
             if (finish) {
                 // A cut tile: the pieces in CTA order (a CTA without a unit has none), 16 rows at a time.  What this costs is latency,
@@ -1220,25 +1248,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 };
                 if (!whole)
                     for (int i = 0; i < n_merge; ++i) fetch();
-                // What a thread writes of 16 rows of x, from the buffer in which they change places.
-                const int wt = et >> 4, wm = et & 15;                 // rows wt and wt + 8; member
-                constexpr int TB_ROW = MODE == GG_UP ? 64 : 128;      // values of a row of x in the buffer
-                unsigned char* h_dst = nullptr;
-                uint16_t* out = nullptr;
-                int64_t ld = 0;
-                bool runs = true, exists = true;                      // eight neighbouring outputs in one store; the member has these rows
-                if constexpr (MODE == GG_UP) {
-                    const int col = wm * pr.G + PER * rho;            // four neighbouring columns of h, staged at pos .. pos + 3
-                    const int pos = tile_pos(col & 63), row = pr.row0 + s.chunk * n + wt;       // (row and row + 8, 16, ... share the swizzle)
-                    h_dst = prm.ht + ((int64_t)(col >> 6) * prm.xt_rows + row) * 128 + ((((pos >> 3) ^ (row & 7)) << 4) | ((pos & 7) * 2));
-                } else {
-                    ld = (MODE == GG_LINEAR) ? pr.N : prm.N;
-                    out = reinterpret_cast<uint16_t*>(MODE == GG_LINEAR ? prm.hp[s.p].y : prm.out) + (int64_t)(m0 + wm) * pr.G + PER * rho0;
-                    exists = !F::WORDS || (m0 + wm) * pr.G + PER * rho0 < pr.N;
-                    runs = !(MODE == GG_DOWN && prm.accumulate) && pr.P - rho0 >= PARTS && ((reinterpret_cast<uintptr_t>(out) | (uintptr_t)(ld * 2)) & 15) == 0;
-                    if (MODE == GG_LINEAR) out += (int64_t)(list + wt) * ld;
-                }
-                const int at0 = MODE == GG_UP ? (lane & 1) * 8 * 64 + member * 4 + (((slot & 1) << 1) | (slot >> 1)) : member * RUN + part * PER + slot;
 #pragma unroll 1
                 for (int c0 = 0; c0 < rows_here; c0 += 16) {
                     float v[16];
@@ -1492,7 +1501,7 @@ static int64_t gg_tiles(const hqm_weight* const* ws, int count) {
     for (int i = 0; i < count; ++i) tiles += gg_tiles(ws[i]);
     return tiles;
 }
-GgLayout gg_expert_layout(int64_t M) { return GgLayout{GgRows::of((int)M), gg_sm_count(), 0}; }
+GgLayout gg_expert_layout(int64_t M) { return GgLayout{GgRows::of((int)M), gg_sm_count(), 0, 0}; }
 // Rows per chunk and CTAs of linear layers over the same rows, by what a launch costs in cycles of its longest CTA (fitted to
 // 2- and 4-bit layers of 1024 to 14336 outputs with 16 to 500 rows):
 //   its units of 128 columns:  850 + 4 n with n rows; beyond 128 rows, with one accumulator, 10 n
@@ -1522,7 +1531,7 @@ GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count, siz
             const int64_t cost = share * unit + (share + units_k - 1) / units_k * n16 * 400 + cuts * (5000 + n16 * (3000 + 400 * (pieces - 2)));
             if (cost < best_cost) {
                 best_cost = cost;
-                best = GgLayout{r, (int)std::min<int64_t>(sms, (units + share - 1) / share), cost};
+                best = GgLayout{r, (int)std::min<int64_t>(sms, (units + share - 1) / share), (int)share, cost};
             }
         };
         consider((s0 + units_k - 1) / units_k * units_k, 2, 0);                                  // whole tiles
@@ -1549,10 +1558,10 @@ static int gg_launch_one(const gg::Params& p, int grid, cudaStream_t st) {
     static bool attr_done[MAX_DEVICES];
     bool& done = attr_done[current_device_slot()];
     if (!done) {
-        HQM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem(64) > F::smem(256) ? F::smem(64) : F::smem(256)));
+        HQM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F::MOST));
         done = true;
     }
-    launch_overlapped(kern, grid, gg::NTHREADS, F::smem(p.n_max), st, p);
+    launch_overlapped(kern, grid, gg::NTHREADS, F::smem(p.n_max, p.cut != 0), st, p);
     HQM_LAUNCH_CHECK();
     return HQM_OK;
 }
@@ -1632,6 +1641,8 @@ int launch_gg(const GgJob& job, uint32_t* counters, void* scratch, size_t scratc
     p.parts = (float*)scratch;
     p.n_max = job.counts ? gg_n_max(job.rows) : job.layout.rows.n;
     p.chunks = job.layout.rows.chunks;
+    p.share = job.counts ? 0 : job.layout.share;
+    p.cut = p.share == 0 || p.share % p.units_k != 0;
     p.counters = counters;
     p.error_flag = tc_error_ptr();
     const int grid = job.counts ? gg_sm_count() : job.layout.grid;

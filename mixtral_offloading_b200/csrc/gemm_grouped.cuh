@@ -27,6 +27,7 @@ struct GgRows {
 struct GgLayout {                         // of a launch whose row count the host knows
     GgRows rows;
     int grid;
+    int share;                            // units of a CTA, the last one may have fewer (0: shares of equal cost)
     int64_t cost;                         // cycles, by the rule of gg_linear_layout
 };
 // Upper bound of the padded rows of `rows` rows spread over `lists` lists.

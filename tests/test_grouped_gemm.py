@@ -5,7 +5,7 @@ import torch
 
 from mixtral_offloading_b200 import ResidentMoe, _cabi
 from oracle import hqq_oracle as O
-from tests.helpers import layer_from_oracle, random_layer
+from tests.helpers import layer_from_oracle, random_layer, random_layer_fast
 from tests.test_gpu_parity import Cfg, make_expert
 
 pytestmark = pytest.mark.gpu
@@ -29,6 +29,21 @@ def test_linear_edges(nbits, group, N, K, std):
         want = x.double() @ W.t()
         assert ((y.double() - want).norm() / want.norm()).item() < TOL, M
         assert torch.equal(y, layer(x)), M                   # pieces of a tile are added in a fixed order
+    assert _cabi.lib().hqm_device_error() == 0
+
+
+@pytest.mark.parametrize("nbits,group,N,K,rows", [(2, 16, 13312, 512, (299, 512)), (4, 64, 13312, 512, (300,)), (3, 64, 11264, 1024, (400,))])
+def test_whole_tiles_that_the_ctas_do_not_divide(nbits, group, N, K, rows):
+    """416 and 440 tiles in shares of three: the last CTA has fewer."""
+    layer = layer_from_oracle(random_layer_fast(N, K, nbits, group, seed=nbits), DEV)
+    W = layer.dequantize(torch.float32).double()
+    for M in rows:
+        x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(torch.bfloat16).to(DEV)
+        y, want = layer(x), x.double() @ W.t()
+        assert ((y.double() - want).norm() / want.norm()).item() < TOL, M
+        # and no row or column of a tile is worse than the rest: three times the bound, as a column has some hundred values
+        assert ((y.double() - want).norm(dim=0) / want.norm(dim=0)).max().item() < 3 * TOL, M
+        assert torch.equal(y, layer(x)), M
     assert _cabi.lib().hqm_device_error() == 0
 
 
