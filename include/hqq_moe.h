@@ -130,7 +130,8 @@ size_t hqm_linear_scratch_preferred(int64_t M, const hqm_weight* w);
  * and the per-call 8-bit scale/zero decode fused in:
  *   y[M, N] = x[M, K] . W_est^T (+ bias[N]),  fp32 accumulation, bf16 in/out.
  * bias may be NULL.  scratch may be NULL when hqm_linear_scratch_bytes() is 0.
- * 1 to 4 rows (3 bit: one) take the weight-streaming kernels, more the tcgen05 kernels, formats and shapes that neither
+ * 1 to 4 rows (3 bit: one) take the weight-streaming kernels, more the tcgen05 kernels; large 2-bit layers with groups of
+ * 16 and 2 to 5 rows the few-row kernel where the workspace is of the preferred size; formats and shapes that none of them
  * covers and unaligned x the shape-agnostic one; HQM_FORCE_GENERIC=1 in the environment at load time routes everything
  * through that. */
 int hqm_linear(uint16_t* y, const uint16_t* x, int64_t M, const hqm_weight* w, const uint16_t* bias,

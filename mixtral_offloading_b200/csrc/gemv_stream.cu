@@ -1,5 +1,5 @@
-// Weight-streaming quantized linear for small row counts: the decode step's launches, layers and 2-bit experts with
-// groups of 16 up to 4 rows, other experts up to 16.  The path that
+// Weight-streaming quantized linear for small row counts: layers up to 4 rows, the decode step's 4-bit launches, experts that
+// neither gemv_rows.cu nor gemm_grouped.cu takes up to 16 rows.  The path that
 // replaces triton_matmul4_transpose / triton_matmul2_transpose of the reference
 // (triton_kernels.py:133-191, 321-380) together with the two per-call
 // Quantizer.dequantize launches in front of them (custom_layers.py:62-66).

@@ -166,7 +166,8 @@ int launch_rows_from_sums(uint16_t* y, const float* sums, const uint16_t* bias, 
 //   rows                      3            4            5            8           16
 //   2 bit 14336 x 4096   18.0 / 19.2  18.3 / 19.1  27.4 / 19.1  29.1 / 19.1  53.7 / 19.4
 //   4 bit 4096 x 4096    11.3 / 11.1  12.3 / 11.2  14.0 / 11.2  15.5 / 11.3  24.4 / 11.5
-//   expert (three 2-bit) 51.3 / 53.6  51.7 / 53.4  76.3 / 53.5  79.5 / 54.4   145 / 55.0
+// Experts whose layers gemv_rows.cu takes (2 bit, groups of 16) come here from 9 rows on (gemv_rows.cu / here: 3 rows 36.9 / 53.6, 8 rows 48.6 / 54.4).
+// 2-bit layers of three steps and more per SM leave the line to api.cu, use_rows().
 constexpr int64_t GG_MIN_ROWS = 5;
 
 // gemm_tc3.cu — tcgen05 / TMEM path for the 3-bit layers that gemm_grouped.cu does not take, from five rows on.
