@@ -82,6 +82,37 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// The two experts of a token and their weights, from p[e] = exp(logit - largest logit) and their sum: the first two of the
+// largest, renormalised and rounded to bf16.  Two different experts whatever the logits are, as row lists hold a token once per
+// expert: with a NaN or an infinity among them no comparison holds, the choice is experts 0 and 1 and the weights are the NaN
+// that softmax gives.
+template <int EMAX>
+__device__ __forceinline__ void top_two(const float (&p)[EMAX], float sum, int E, int (&idx)[2], float (&weight)[2]) {
+    int i0 = -1, i1 = -1;
+    float p0 = -1.f, p1 = -1.f;
+#pragma unroll
+    for (int e = 0; e < EMAX; ++e) {
+        if (e < E) {
+            const float pe = p[e] / sum;
+            if (pe > p0) { p1 = p0; i1 = i0; p0 = pe; i0 = e; }
+            else if (pe > p1) { p1 = pe; i1 = e; }
+        }
+    }
+    if (i0 < 0) {
+        i0 = 0;
+        i1 = E > 1 ? 1 : 0;
+        p0 = p1 = p[0] / sum;
+    } else if (i1 < 0) {                 // E == 1
+        i1 = i0;
+        p1 = 0.f;
+    }
+    const float norm = p0 + p1;
+    idx[0] = i0;
+    idx[1] = i1;
+    weight[0] = round_bf16(p0 / norm);
+    weight[1] = round_bf16(p1 / norm);
+}
+
 // Streaming 16-byte load that does not pollute L1 (weights are read exactly once).
 __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
     uint4 v;

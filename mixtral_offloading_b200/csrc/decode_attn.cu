@@ -322,20 +322,12 @@ __global__ void __launch_bounds__(NORM_THREADS) finalize_add_rmsnorm_router_kern
             p[e] = (e < E) ? expf(acc[e] - mx) : 0.f;
             sum += p[e];
         }
-        int i0 = 0, i1 = -1;
-        float p0 = -1.f, p1 = -1.f;
-#pragma unroll
-        for (int e = 0; e < ROUTER_EMAX; ++e) {
-            if (e < E) {
-                const float pe = p[e] / sum;
-                if (pe > p0) { p1 = p0; i1 = i0; p0 = pe; i0 = e; }
-                else if (pe > p1) { p1 = pe; i1 = e; }
-            }
-        }
+        int idx[2];
+        float wgt[2];
+        top_two(p, sum, E, idx, wgt);
+        const int i0 = idx[0], i1 = idx[1];
+        const float w0 = wgt[0], w1 = wgt[1];
         if (lane < E) logits_out[lane] = float_to_bf16_bits(mine_e);
-        if (i1 < 0) { i1 = i0; p1 = 0.f; }
-        const float norm = p0 + p1;
-        const float w0 = round_bf16(p0 / norm), w1 = round_bf16(p1 / norm);
         if (lane == 0) {
             topk_w[0] = w0;
             topk_w[1] = w1;

@@ -29,23 +29,16 @@ __device__ __forceinline__ void finish_token(const float (&acc)[EMAX], float mx,
         p[e] = (e < E) ? expf(acc[e] - mx) : 0.f;
         sum += p[e];
     }
-    int i0 = 0, i1 = -1;
-    float p0 = -1.f, p1 = -1.f;
 #pragma unroll
-    for (int e = 0; e < EMAX; ++e) {
-        if (e < E) {
-            const float pe = p[e] / sum;
-            logits_out[(int64_t)t * E + e] = float_to_bf16_bits(acc[e]);
-            if (pe > p0) { p1 = p0; i1 = i0; p0 = pe; i0 = e; }
-            else if (pe > p1) { p1 = pe; i1 = e; }
-        }
-    }
-    if (i1 < 0) { i1 = i0; p1 = 0.f; }   // E == 1
-    const float norm = p0 + p1;
-    topk_w[2 * t] = round_bf16(p0 / norm);
-    topk_w[2 * t + 1] = round_bf16(p1 / norm);
-    topk_idx[2 * t] = i0;
-    topk_idx[2 * t + 1] = i1;
+    for (int e = 0; e < EMAX; ++e)
+        if (e < E) logits_out[(int64_t)t * E + e] = float_to_bf16_bits(acc[e]);
+    int idx[2];
+    float w[2];
+    top_two(p, sum, E, idx, w);
+    topk_w[2 * t] = w[0];
+    topk_w[2 * t + 1] = w[1];
+    topk_idx[2 * t] = idx[0];
+    topk_idx[2 * t + 1] = idx[1];
 }
 
 // Up to 8 experts and 4096 columns: a CTA per token, a thread per 8 columns; the sums are formed in the order of the kernel
