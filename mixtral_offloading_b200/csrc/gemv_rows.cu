@@ -29,6 +29,7 @@
 #include <algorithm>
 
 #include "gemv_rows.cuh"
+#include "shared_limit.h"
 #include "stream_split.cuh"
 
 namespace hqm {
@@ -341,15 +342,8 @@ static int stages_for(int toks, int period, int steps) {
 
 template <int TOKS>
 static bool prepare(size_t smem) {
-    static size_t configured[MAX_DEVICES];
-    size_t& have = configured[current_device_slot()];
-    if (have >= smem) return true;
-    if (cudaFuncSetAttribute(gemv_rows_kernel<TOKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    have = smem;
-    return true;
+    static SharedLimits limits;
+    return allow_shared(gemv_rows_kernel<TOKS>, limits, smem);
 }
 
 }  // namespace rows

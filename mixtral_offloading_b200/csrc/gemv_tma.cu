@@ -37,6 +37,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "shared_limit.h"
 #include "stream_split.cuh"
 
 namespace hqm {
@@ -771,15 +772,8 @@ bool tma_disabled() { return tma_mode() == 0; }
 
 template <int NBITS, int DEPTH>
 bool prepare_kernel(size_t smem) {
-    static size_t configured[MAX_DEVICES];
-    size_t& have = configured[current_device_slot()];
-    if (have >= smem) return true;
-    if (cudaFuncSetAttribute(gemv_tma_kernel<NBITS, DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    have = smem;
-    return true;
+    static SharedLimits limits;
+    return allow_shared(gemv_tma_kernel<NBITS, DEPTH>, limits, smem);
 }
 
 }  // namespace
