@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
         // =========================== computing warps ===========================
         int st = 0, e = 0;
         uint32_t par = 0;
-        bool ok = true;
+        bool ok = true, again = false;
         const int row_len = prm.layers * prm.N;
         for (uint32_t u = ub; u < ue && ok;) {
             const Run r = run_at(u, e);
@@ -206,8 +206,29 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
                              (PER * rho + (lane >> 3)) % prm.period, sp.n[e], prm.G, row_len, rho * PER < prm.G};
             float* dst = prm.partial + ((size_t)piece * sp.R + sp.row0[e]) * row_len + layer * prm.N + PER * rho;
             const auto one = [](int) { return 1.f; };
-            if (sg.M <= 4) ok = rows_segment<4, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one);
-            else ok = rows_segment<8, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one);
+            if (sg.M <= 4) ok = rows_segment<4, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again);
+            else ok = rows_segment<8, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again);
+        }
+        if (__all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, again)) {
+            for (uint32_t u = ub; u < ue;) {
+                const Run r = run_at(u, 0);
+                u += (uint32_t)(r.pb - r.pa);
+                const int layer = r.unit / prm.units, rho = (r.unit - layer * prm.units) * CW + warp;
+                if (rho * PER >= prm.G) continue;
+                const int piece = r.pa ? cta - sp.owner(r.e, (uint32_t)(r.unit * PT)) : 0;
+                Again a{};
+                a.layer(prm.table[3 * r.e + (layer ? prm.which1 : prm.which0)].w);
+                a.K = K;
+                a.G = prm.G;
+                a.C = prm.C;
+                a.rho = rho;
+                a.k0 = r.pa * KC;
+                a.k1 = r.pb * KC;
+                a.staged = prm.xt + (size_t)sp.xrow0[r.e] * K * 2;
+                a.cap = ListSplit::cap(sp.n[r.e]);
+                for (a.m = 0; a.m < sp.n[r.e]; ++a.m)
+                    sum_again(a, prm.partial + ((size_t)piece * sp.R + sp.row0[r.e] + a.m) * row_len + layer * prm.N + PER * rho, 1.f);
+            }
         }
         if (!ok) s_failed = 1;
     }

@@ -38,6 +38,7 @@ namespace rows {
 
 struct LayerParams {
     const uint16_t* meta[4];                            // ms_scale, mz_scale, ms_zero, mz_zero
+    const uint8_t* data[3];                             // codes, scale bytes, zero bytes
     CUtensorMap maps[3];
 };
 struct Params {
@@ -199,7 +200,7 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
         uint32_t x_at = x_area;                                     // of the present step
         int st = 0;
         uint32_t par = 0;
-        bool ok = true;
+        bool ok = true, again = false;
         for (int unit = unit0, pa = pa0, left = n_steps; left > 0 && ok; ++unit, pa = 0) {
             const int pb_all = min(PT, pa + left);
             left -= pb_all - pa;
@@ -316,9 +317,27 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
                 ok = rows_segment<TOKS, S::FINE_Z>(sg, pb - pa, st, par, x_at, S::X_STEP,
                                                    partial + (int64_t)slot_idx * M_total * sg.row_len + prm.col0[l] + PER * rho, [&](int m) {
                     return S::SCALED ? __uint_as_float((uint32_t)row_exponent(m) << 23) : 1.f;
-                });
+                }, again);
             }
             x_at += (uint32_t)(pb_all - pa) * S::X_STEP;
+        }
+        if (TOKS > 1 && __all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, again)) {
+            for (int unit = unit0, pa = pa0, left = n_steps; left > 0; ++unit, pa = 0) {
+                const int pb = min(PT, pa + left);
+                left -= pb - pa;
+                const int l = layer_of(unit), rho = (unit - prm.unit0[l]) * CW + warp;
+                if (rho * PER >= prm.G[l] || (prm.table && s_absent[l])) continue;
+                const LayerParams& ly = prm.ly[l];
+                Again a{ly.data[0], ly.data[1], ly.data[2], ly.meta[0], ly.meta[1], ly.meta[2], ly.meta[3], K, prm.G[l], prm.C[l], rho, pa * KC, pb * KC};
+                if (prm.table) a.layer(prm.table[3 * __ldcg(prm.sel[l]) + prm.which[l]].w);
+                const int64_t row_len = prm.col0[prm.count], slot_idx = unit == unit0 ? slot0 : 0;
+                for (int m = 0; m < M; ++m) {
+                    a.x = x + ((x_idx ? x_idx[m] : m) + prm.xrow[l]) * (int64_t)K;
+                    a.down = S::SCALED ? __uint_as_float((uint32_t)(254 - row_exponent(m)) << 23) : 1.f;
+                    sum_again(a, partial + (slot_idx * M_total + m) * row_len + prm.col0[l] + PER * rho,
+                              S::SCALED ? __uint_as_float((uint32_t)row_exponent(m) << 23) : 1.f);
+                }
+            }
         }
         if (!ok) s_failed = 1;
     }
@@ -404,6 +423,9 @@ int launch_gemv_rows(float* partial, const uint16_t* x, const int32_t* x_idx, in
             prm.ly[l].meta[1] = w->mz_scale;
             prm.ly[l].meta[2] = w->ms_zero;
             prm.ly[l].meta[3] = w->mz_zero;
+            prm.ly[l].data[0] = static_cast<const uint8_t*>(w->W_q);
+            prm.ly[l].data[1] = w->scale_q;
+            prm.ly[l].data[2] = w->zero_q;
             if (!rows_cached_maps(w, plan.G[l], prm.ly[l].maps)) {
                 set_error("gemv_rows: cuTensorMapEncodeTiled failed for a %dx%d layer", w->N, w->K);
                 return HQM_ERR_CUDA;

@@ -128,11 +128,79 @@ struct Segment {
     bool live;                                 // the warp has a storage-row residue
 };
 
+// A layer as it lies in memory, a run of steps of one unit, and the rows of x: what sum_again() reads.
+struct Again {
+    const uint8_t *codes, *scale_q, *zero_q;
+    const uint16_t *ms_scale, *mz_scale, *ms_zero, *mz_zero;
+    int K, G, C, rho, k0, k1;                  // the warp's storage-row residue; columns of the run
+    const uint16_t* x;                         // a bf16 row, multiplied with `down` ...
+    float down;
+    const unsigned char* staged;               // ... or (not null) row m of a staged list of `cap` rows
+    int m, cap;
+    __device__ __forceinline__ void layer(const hqm_weight& w) {
+        codes = static_cast<const uint8_t*>(w.W_q);
+        scale_q = w.scale_q;
+        zero_q = w.zero_q;
+        ms_scale = w.ms_scale;
+        mz_scale = w.mz_scale;
+        ms_zero = w.ms_zero;
+        mz_zero = w.mz_zero;
+    }
+};
+// One row's sums over a run of steps once more, with the weights that dequantize() makes and fp32 products, where a sum that
+// rows_segment() left at `to` (16 members, G apart, of 4 residues) is not finite.  With the tensor cores' factors that happens for
+// inputs that are fine: x * s leaves fp16 where a scale is 2048 or more (x is staged below 32), and an infinite x meets codes of 0
+// and makes the zeros' sum a difference of infinities, though its products with the weights have a sign.  A warp comes here behind
+// all of its steps, when it has seen such a sum: beside them the call would cost the steps 60 to 190 bytes of spilled registers.
+__device__ __noinline__ static void sum_again(const Again& a, float* to, float up) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();                                  // other lanes have stored some of the sums
+    const float2 have = *reinterpret_cast<const float2*>(to + (int64_t)(lane >> 1) * a.G + 2 * (lane & 1));
+    if (__all_sync(0xffffffffu, isfinite(have.x) && isfinite(have.y))) return;
+    for (int s = 0; s < PER; ++s) {
+        float sum[MEMBERS];
+#pragma unroll
+        for (int j = 0; j < MEMBERS; ++j) sum[j] = 0.f;
+        for (int k = a.k0 + 4 * lane; k < a.k1; k += 128) {
+            const uint8_t* codes = a.codes + (int64_t)a.rho * a.K + k;
+            uint32_t q[MEMBERS];
+#pragma unroll
+            for (int j = 0; j < MEMBERS; ++j) q[j] = *reinterpret_cast<const uint32_t*>(codes + (int64_t)j * (a.G / PER) * a.K) >> (6 - 2 * s);
+            const int64_t at = (int64_t)(PER * a.rho + s) * a.K + k;
+            const uint32_t sq = *reinterpret_cast<const uint32_t*>(a.scale_q + at), zq = *reinterpret_cast<const uint32_t*>(a.zero_q + at);
+            const int col = (int)(at % a.C);
+            float x[4];
+            if (a.staged) {
+                const uint2 v = *reinterpret_cast<const uint2*>(a.staged + few_staged_at(k & ~7, a.m, a.cap) + (k & 4) * 2);
+                const uint32_t w[2] = {v.x, v.y};                                 // columns (0, 2), (1, 3)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) x[c] = f16_bits_to_float((uint16_t)(w[c & 1] >> (8 * (c & 2))));
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) x[c] = bf16_bits_to_float(a.x[k + c]) * a.down;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float scale = __fmul_rn(__fsub_rn((float)((sq >> (8 * c)) & 255u), f16_bits_to_float(a.mz_scale[col + c])), f16_bits_to_float(a.ms_scale[col + c]));
+                const float zero = __fmul_rn(__fsub_rn((float)((zq >> (8 * c)) & 255u), f16_bits_to_float(a.mz_zero[col + c])), f16_bits_to_float(a.ms_zero[col + c]));
+#pragma unroll
+                for (int j = 0; j < MEMBERS; ++j) sum[j] = fmaf(x[c], __fmul_rn(__fsub_rn((float)((q[j] >> (8 * c)) & 3u), zero), scale), sum[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < MEMBERS; ++j) {
+            const float v = warp_sum(sum[j]);
+            if (lane == 0) to[(int64_t)j * a.G + s] = v * up;
+        }
+    }
+}
+
 // TOKS > 1 rows over `steps` steps, from stage st (phase par) on.  x: at x0, x_step bytes further with every step, or (x_step 0) at x0 of
-// the stage.  dst: the warp's first column of row 0; up(m): factor of row m.  False where a wait ran out.
+// the stage.  dst: the warp's first column of row 0; up(m): factor of row m; again: set where a sum is not finite (see sum_again()).
+// False where a wait ran out.
 template <int TOKS, bool FINE_Z, typename Up>
 __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& st, uint32_t& par, uint32_t x0, uint32_t x_step, float* dst,
-                                             const Up& up) {
+                                             const Up& up, bool& again) {
     using S = Shape<TOKS>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t code_off = (uint32_t)(warp * MEMBERS * KC + g * KC), sw = (uint32_t)g;
@@ -307,6 +375,8 @@ __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& 
                     float y[4];
 #pragma unroll
                     for (int s = 0; s < 4; ++s) y[s] = (acc[s][2 * half + e] * (float)(1 << (18 + 2 * s)) - z[s]) * f;
+                    // 0 * y is 0, or NaN where y is not finite.  (Of two lanes with the same sums each writes half: both look at all.)
+                    again |= !(fmaf(0.f, y[0], fmaf(0.f, y[1], fmaf(0.f, y[2], 0.f * y[3]))) == 0.f);
                     float* at = to + (int64_t)8 * half * sg.G;
                     if constexpr (TOKS == 4) {          // lanes t < 2 hold slots 0 and 2, the others 1 and 3
                         at[t >> 1] = t < 2 ? y[0] : y[1];
