@@ -82,11 +82,14 @@ int hqm_device_error(void);
  * setting.  Process wide. */
 int hqm_set_overlap(int on);
 
-/* No counterpart in the reference.  Which single-row launches use the TMA-staged streaming kernel (tiled
- * cp.async.bulk.tensor copies of the packed tiles into per-warp stage rings, rows finished inside the kernel):
- * 0 = none, 1 = a linear that stands alone (hqm_linear, the default), 2 = also the multi-layer and table-driven
- * launches of hqm_expert_ffn / hqm_moe_decode / hqm_attn_decode / hqm_decode_layer.  HQM_TMA=0|1|2 in the
- * environment sets the initial value.  Returns the previous mode.  Process wide. */
+/* No counterpart in the reference.  Which single-row launches bring their packed tiles by tiled copies
+ * (cp.async.bulk.tensor): 0 = none; 1 (the default) = a linear that stands alone (hqm_linear) through the TMA-staged
+ * streaming kernel (per-warp stage rings, rows finished inside the kernel), and the 2-bit experts with groups of 16 of
+ * hqm_expert_ffn / hqm_moe_decode / hqm_decode_layer through the few-row kernel; 2 = every single-row launch through the
+ * TMA-staged streaming kernel, the multi-layer and table-driven ones of hqm_expert_ffn / hqm_moe_decode /
+ * hqm_attn_decode / hqm_decode_layer included.  Launches of several rows do not depend on it.  Workspaces differ between
+ * the modes: ask for their sizes again after a change.  HQM_TMA=0|1|2 in the environment sets the initial value.  Returns
+ * the previous mode.  Process wide. */
 int hqm_set_tma_mode(int mode);
 
 /* ---- bit packing: src/packing.py --------------------------------------- */

@@ -738,7 +738,8 @@ bool gemv_stream_shape_ok(const hqm_weight* w, int G, int C) {
 
 bool gemv_stream_plan(const hqm_weight* const* ws, int count, int64_t M, StreamPlan* plan, bool chained) {
     if (count < 1 || count > STREAM_MAX_LAYERS || force_generic()) return false;
-    if (chained && gemv_rows_plan(ws, count, M, plan)) return true;
+    // (several rows of the experts' layers have this one kernel; a single row has three, and the caller a say: hqm_set_tma_mode)
+    if (chained && (M > 1 || tma_mode() == 1) && gemv_rows_plan(ws, count, M, plan)) return true;
     if (M == 1 && gemv_tma_plan(ws, count, chained, plan)) return true;
     plan->kind = STREAM_WARPS;
     const hqm_weight* w = ws[0];

@@ -755,10 +755,20 @@ int distinct_xrows(const int* xrow, int count, int* xslot) {
     return nx;
 }
 
-// 0: never; 1: launches of a single layer that finish their row themselves (hqm_linear, hqm_expert_ffn); 2: every
-// single-row launch, the decode step's multi-layer and table-driven ones included.  HQM_TMA in the environment
-// gives the initial value (default 1); hqm_set_tma_mode changes it.
 std::atomic<int> g_tma_mode{-1};
+
+template <int NBITS, int DEPTH>
+bool prepare_kernel(size_t smem) {
+    static SharedLimits limits;
+    return allow_shared(gemv_tma_kernel<NBITS, DEPTH>, limits, smem);
+}
+
+}  // namespace
+
+// Which single-row launches copy whole tiles.  0: none; 1: this file's kernel takes a layer that stands alone (hqm_linear), and
+// gemv_rows.cu the launches of 2-bit experts with groups of 16; 2: this file's kernel takes every single-row launch, the experts'
+// and the decode step's multi-layer and table-driven ones included.  HQM_TMA in the environment gives the initial value
+// (default 1); hqm_set_tma_mode changes it.
 int tma_mode() {
     int v = g_tma_mode.load(std::memory_order_relaxed);
     if (v < 0) {
@@ -768,15 +778,6 @@ int tma_mode() {
     }
     return v;
 }
-bool tma_disabled() { return tma_mode() == 0; }
-
-template <int NBITS, int DEPTH>
-bool prepare_kernel(size_t smem) {
-    static SharedLimits limits;
-    return allow_shared(gemv_tma_kernel<NBITS, DEPTH>, limits, smem);
-}
-
-}  // namespace
 
 // The tensor maps of a layer for the other TMA users (three CUtensorMaps; the codes' box is 128 columns x 16 members).
 bool stream_cached_maps(const hqm_weight* w, int G, void* out3) {
@@ -833,7 +834,7 @@ size_t gemv_tma_scratch_bytes(const StreamPlan& plan, int64_t M) {
 }
 
 bool gemv_tma_plan(const hqm_weight* const* ws, int count, bool chained, StreamPlan* plan) {
-    if (count < 1 || count > STREAM_MAX_LAYERS || tma_disabled() || encode_fn() == nullptr) return false;
+    if (count < 1 || count > STREAM_MAX_LAYERS || tma_mode() == 0 || encode_fn() == nullptr) return false;
     if ((chained || count > 1) && tma_mode() < 2) return false;
     const hqm_weight* w = ws[0];
     const int per = codes_per_word(w->nbits);

@@ -83,6 +83,7 @@ int launch_finalize_scatter(uint16_t* out, const float* partial, const int32_t* 
 bool force_generic();
 // gemv_tma.cu — the same for ONE row of x, tiles staged by TMA.
 bool gemv_tma_plan(const hqm_weight* const* ws, int count, bool chained, StreamPlan* plan);
+int tma_mode();
 int launch_gemv_tma(float* partial, const uint16_t* x, const int32_t* x_idx, int64_t M, const StreamJob& job,
                     const StreamPlan& plan, cudaStream_t st);
 
