@@ -118,7 +118,7 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
                 for (int i = 0; i < 3 * (int)sizeof(StreamEntry); i += 128)
                     prefetch_l2(reinterpret_cast<const unsigned char*>(prm.table + 3 * idx) + i);
         }
-        int st = 0, fenced = -1;
+        int st = 0, fenced = -1, ahead = stages;
         uint32_t par = 1;
         bool ok = true;
         for (int unit = unit0, pa = pa0, left = n_steps; left > 0 && ok; ++unit, pa = 0) {
@@ -145,6 +145,9 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
             const int rho = (unit - prm.unit0[l]) * CW;
             uint32_t col = pa ? pa_col : 0u;                  // of class 0
             for (int p = pa; p < pb; ++p) {
+                // Stages are freed by warps that wait for the kernel in front.  So does this one before it waits for them: the
+                // limit of a wait covers this kernel's own steps, not what is left of the other's.
+                if (ahead-- == 0) grid_dependency_wait();
                 if (!wait(empty + 8 * st, par)) {
                     ok = false;
                     break;
