@@ -9,6 +9,7 @@ from mixtral_offloading_b200 import ResidentMoe, _cabi
 from tests.helpers import layer_from_oracle, random_layer, random_layer_fast
 from tests.test_gpu_parity import Cfg, make_expert
 from tests.test_many_row_precision import weight64
+from tests.test_tma_mode import kernels_of
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda:0")
@@ -87,9 +88,12 @@ def test_lists_of_every_length(hidden, ffn, n_exp, tokens):
     assert _cabi.lib().hqm_device_error() == 0
 
 
-@pytest.mark.parametrize("N,K", [(14336, 4096), (4096, 14336), (14336, 3072)])
-def test_large_linear_layers(N, K):
-    """Two to five rows of layers with three steps or more for every SM; with less workspace than that wants, and a bias."""
+@pytest.mark.parametrize("N,K,few", [(14336, 4096, True), (4096, 14336, True), (14336, 14336, True), (14336, 3072, False)])
+def test_large_linear_layers(N, K, few):
+    """Two to five rows of layers with three steps or more for every SM (one with less, which the other kernels keep); with less
+    workspace than that wants, and a bias."""
+    steps = -(-N // 16 // 4 // 16) * (K // 128)
+    assert few == (steps >= 3 * torch.cuda.get_device_properties(0).multi_processor_count)
     layer = layer_from_oracle(random_layer_fast(N, K, 2, 16, seed=3), DEV)
     layer.bias = torch.randn(N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
     lib, d, W = _cabi.lib(), layer.descriptor(), weight64(layer)
@@ -98,12 +102,27 @@ def test_large_linear_layers(N, K):
         want = x.double() @ W.t() + layer.bias.double()
         need, wanted = lib.hqm_linear_scratch_bytes(M, C.byref(d)), lib.hqm_linear_scratch_preferred(M, C.byref(d))
         assert wanted >= need
-        for size in (need, wanted - 1, wanted):
+        if M < 5:
+            assert (wanted > need) == (few and M > 1)
+        for size in sorted({need, max(need, wanted - 1), wanted}):
             ws = torch.full((wanted + 4096,), 7, dtype=torch.uint8, device=DEV)
             _cabi.check(lib.hqm_scratch_init(_cabi.ptr(ws), _cabi.stream_ptr(DEV)))
             y = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
-            _cabi.check(lib.hqm_linear(_cabi.ptr(y), _cabi.ptr(x), M, C.byref(d), _cabi.ptr(layer.bias), _cabi.ptr(ws), max(size, need),
-                                       _cabi.stream_ptr(DEV)))
-            assert bool((ws[max(size, need):] == 7).all())
+            run = lambda: _cabi.check(lib.hqm_linear(_cabi.ptr(y), _cabi.ptr(x), M, C.byref(d), _cabi.ptr(layer.bias), _cabi.ptr(ws), size,
+                                                     _cabi.stream_ptr(DEV)))
+            assert ("gemv_rows_kernel" in kernels_of(run)) == (few and 2 <= M <= 5 and size == wanted), (M, size)
+            assert bool((ws[size:] == 7).all())
             # a rounding to bf16 (1.7e-3) and 16-bit factors (1e-3)
             assert ((y.double() - want).norm() / want.norm()).item() < 2.5e-3, (M, size)
+
+
+def test_what_the_factors_add():
+    """Five rows, one of them with a bias that takes its value away, so that the rounding of the result is small: what is left are
+    three roundings to fp16 of x * s (1e-4 each, together 1.8e-4).  Zeros of 11 bits would add two of the zeros, which are 1.4 times
+    the weights: 2.6e-4."""
+    layer = layer_from_oracle(random_layer(14336, 4096, 2, 16, seed=3), DEV)
+    x = torch.randn(5, 4096, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).to(DEV)
+    want = x.double() @ weight64(layer).t()
+    layer.bias = (-want[0]).to(torch.bfloat16)
+    y = layer(x)[0].double() - layer.bias.double()
+    assert ((y - want[0]).norm() / want[0].norm()).item() < 2.2e-4
