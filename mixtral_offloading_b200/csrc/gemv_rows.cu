@@ -53,12 +53,47 @@ struct Params {
     int sel_settled, experts;
     int M;
     int* error_flag;
+    __device__ __forceinline__ int layer_of(int unit) const {
+        int l = 0;
+#pragma unroll
+        for (int i = 1; i < STREAM_MAX_LAYERS; ++i) l += (i < count && unit >= unit0[i]) ? 1 : 0;
+        return l;
+    }
 };
+// Of a row's factor, biased, from the row's largest |x| as bf16.
+__device__ __forceinline__ int exponent_of(uint32_t largest) { return min(max((int)(largest >> 7), 30), 250) - 4; }
+
+// sum_again() for the runs of this warp.  (A function of its own that finds them anew: what they are known by would otherwise stay in
+// registers beside the steps, 4 % of the time at 8 rows.)
+template <bool SCALED>
+__device__ __noinline__ void rows_again(const Params& prm, const Split& sp, float* partial, const uint16_t* x, const int32_t* x_idx, int M_total,
+                                        const uint32_t* s_max, const int* s_absent) {
+    const int warp = threadIdx.x >> 5, K = prm.K, PT = prm.PT;
+    const uint32_t first = sp.begin(blockIdx.x);
+    const int unit0 = (int)(first / (uint32_t)PT), slot0 = (int)blockIdx.x - sp.owner((uint32_t)unit0 * (uint32_t)PT);
+    int pa = (int)(first - (uint32_t)unit0 * (uint32_t)PT), left = (int)(sp.begin(blockIdx.x + 1) - first);
+    for (int unit = unit0; left > 0; ++unit, pa = 0) {
+        const int pb = min(PT, pa + left);
+        left -= pb - pa;
+        const int l = prm.layer_of(unit), rho = (unit - prm.unit0[l]) * CW + warp;
+        if (rho * PER >= prm.G[l] || (prm.table && s_absent[l])) continue;
+        const LayerParams& ly = prm.ly[l];
+        Again a{ly.data[0], ly.data[1], ly.data[2], ly.meta[0], ly.meta[1], ly.meta[2], ly.meta[3], K, prm.G[l], prm.C[l], rho, pa * KC, pb * KC};
+        if (prm.table) a.layer(prm.table[3 * __ldcg(prm.sel[l]) + prm.which[l]].w);
+        const int64_t row_len = prm.col0[prm.count], slot = unit == unit0 ? slot0 : 0;
+        for (int m = 0; m < prm.M; ++m) {
+            const int e = SCALED ? exponent_of(s_max[m]) : 127;
+            a.x = x + ((x_idx ? x_idx[m] : m) + prm.xrow[l]) * (int64_t)K;
+            a.down = __uint_as_float((uint32_t)(254 - e) << 23);
+            sum_again(a, partial + (slot * M_total + m) * row_len + prm.col0[l] + PER * rho, __uint_as_float((uint32_t)e << 23));
+        }
+    }
+}
 
 template <int TOKS>
 __global__ void __launch_bounds__(THREADS, 1)
 gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, const int32_t* __restrict__ x_idx, int M_total,
-                 const __grid_constant__ Params prm, Split sp) {
+                 const __grid_constant__ Params prm, const __grid_constant__ Split sp) {
     using S = Shape<TOKS>;
     extern __shared__ unsigned char smem_raw[];
     __shared__ int s_absent[STREAM_MAX_LAYERS];
@@ -84,14 +119,8 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
     const uint32_t L0 = sp.begin(blockIdx.x), L1 = sp.begin(blockIdx.x + 1);
     const int unit0 = (int)(L0 / (uint32_t)PT), pa0 = (int)(L0 - (uint32_t)unit0 * (uint32_t)PT), n_steps = (int)(L1 - L0);
     const int slot0 = (int)blockIdx.x - sp.owner((uint32_t)unit0 * (uint32_t)PT);
-    auto layer_of = [&](int unit) {
-        int l = 0;
-#pragma unroll
-        for (int i = 1; i < STREAM_MAX_LAYERS; ++i) l += (i < prm.count && unit >= prm.unit0[i]) ? 1 : 0;
-        return l;
-    };
-
-    auto row_exponent = [&](int m) { return min(max((int)(s_max[m] >> 7), 30), 250) - 4; };     // of the factor, biased
+    auto layer_of = [&](int unit) { return prm.layer_of(unit); };
+    auto row_exponent = [&](int m) { return exponent_of(s_max[m]); };
 
     if (warp == CW) {
         // =========================== copies ===========================
@@ -324,24 +353,8 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
             }
             x_at += (uint32_t)(pb_all - pa) * S::X_STEP;
         }
-        if (TOKS > 1 && __all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, again)) {
-            for (int unit = unit0, pa = pa0, left = n_steps; left > 0; ++unit, pa = 0) {
-                const int pb = min(PT, pa + left);
-                left -= pb - pa;
-                const int l = layer_of(unit), rho = (unit - prm.unit0[l]) * CW + warp;
-                if (rho * PER >= prm.G[l] || (prm.table && s_absent[l])) continue;
-                const LayerParams& ly = prm.ly[l];
-                Again a{ly.data[0], ly.data[1], ly.data[2], ly.meta[0], ly.meta[1], ly.meta[2], ly.meta[3], K, prm.G[l], prm.C[l], rho, pa * KC, pb * KC};
-                if (prm.table) a.layer(prm.table[3 * __ldcg(prm.sel[l]) + prm.which[l]].w);
-                const int64_t row_len = prm.col0[prm.count], slot_idx = unit == unit0 ? slot0 : 0;
-                for (int m = 0; m < M; ++m) {
-                    a.x = x + ((x_idx ? x_idx[m] : m) + prm.xrow[l]) * (int64_t)K;
-                    a.down = S::SCALED ? __uint_as_float((uint32_t)(254 - row_exponent(m)) << 23) : 1.f;
-                    sum_again(a, partial + (slot_idx * M_total + m) * row_len + prm.col0[l] + PER * rho,
-                              S::SCALED ? __uint_as_float((uint32_t)row_exponent(m) << 23) : 1.f);
-                }
-            }
-        }
+        if (TOKS > 1 && __all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, again))
+            rows_again<S::SCALED>(prm, sp, partial, x, x_idx, M_total, s_max, s_absent);
         if (!ok) s_failed = 1;
     }
     // ---- a wait ran out: copies may still be on their way to this CTA's shared memory

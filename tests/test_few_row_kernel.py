@@ -102,8 +102,7 @@ def test_large_linear_layers(N, K, few):
         want = x.double() @ W.t() + layer.bias.double()
         need, wanted = lib.hqm_linear_scratch_bytes(M, C.byref(d)), lib.hqm_linear_scratch_preferred(M, C.byref(d))
         assert wanted >= need
-        if M < 5:
-            assert (wanted > need) == (few and M > 1)
+        header = lib.hqm_scratch_header_bytes()                  # (where nothing is needed the buffer still has one)
         for size in sorted({need, max(need, wanted - 1), wanted}):
             ws = torch.full((wanted + 4096,), 7, dtype=torch.uint8, device=DEV)
             _cabi.check(lib.hqm_scratch_init(_cabi.ptr(ws), _cabi.stream_ptr(DEV)))
@@ -111,18 +110,19 @@ def test_large_linear_layers(N, K, few):
             run = lambda: _cabi.check(lib.hqm_linear(_cabi.ptr(y), _cabi.ptr(x), M, C.byref(d), _cabi.ptr(layer.bias), _cabi.ptr(ws), size,
                                                      _cabi.stream_ptr(DEV)))
             assert ("gemv_rows_kernel" in kernels_of(run)) == (few and 2 <= M <= 5 and size == wanted), (M, size)
-            assert bool((ws[size:] == 7).all())
+            assert bool((ws[max(size, header):] == 7).all())
             # a rounding to bf16 (1.7e-3) and 16-bit factors (1e-3)
             assert ((y.double() - want).norm() / want.norm()).item() < 2.5e-3, (M, size)
 
 
 def test_what_the_factors_add():
     """Five rows, one of them with a bias that takes its value away, so that the rounding of the result is small: what is left are
-    three roundings to fp16 of x * s (1e-4 each, together 1.8e-4).  Zeros of 11 bits would add two of the zeros, which are 1.4 times
-    the weights: 2.6e-4."""
+    the roundings to fp16 of a scale (3.0e-4: of byte - zero and of the product) and of x * s (2.1e-4), 3.7e-4 together.  (These
+    layers with the same roundings in 64 bits: 3.65e-4.)  Zeros of 11 bits have two more, relative to z, which is 1.7 times q - z:
+    6.2e-4."""
     layer = layer_from_oracle(random_layer(14336, 4096, 2, 16, seed=3), DEV)
     x = torch.randn(5, 4096, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).to(DEV)
     want = x.double() @ weight64(layer).t()
     layer.bias = (-want[0]).to(torch.bfloat16)
     y = layer(x)[0].double() - layer.bias.double()
-    assert ((y - want[0]).norm() / want[0].norm()).item() < 2.2e-4
+    assert ((y - want[0]).norm() / want[0].norm()).item() < 4.5e-4
