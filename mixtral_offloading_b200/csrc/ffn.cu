@@ -326,7 +326,7 @@ int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, c
     if (mp.short_lists) {
         rc = launch_few_projection(fj, few.data, few_part, /*up=*/true, st);
         if (rc != HQM_OK) return rc;
-        rc = launch_few_silu(fj, few_ht, few_part, few.scale, T, st);
+        rc = launch_few_silu(fj, few_ht, few_part, few.scale, few.scale + 2 * T, T, st);
         if (rc != HQM_OK) return rc;
     }
     if (mp.long_lists) {
@@ -346,7 +346,7 @@ int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, c
     if (mp.short_lists) {
         rc = launch_few_projection(fj, few_ht, few_part, /*up=*/false, st);
         if (rc != HQM_OK) return rc;
-        return launch_few_combine(fj, out, few_part, y, entry_of, token_w, T, st);
+        return launch_few_combine(fj, out, few_part, y, entry_of, token_w, few.scale + 2 * T, T, st);
     }
     const int64_t work = T * (w2->N / 8);
     launch_overlapped(moe_combine_kernel, (int)((work + 255) / 256 > 148 * 8 ? 148 * 8 : (work + 255) / 256), 256, 0, st, out,

@@ -9,11 +9,13 @@
 // the share depends on the lists' lengths, every kernel computes the split anew (ListSplit, a warp's prefix sums).
 //
 // The rows of a list are staged by gg_stage_kernel, h by few_silu_kernel: fp16 in the order in which a step reads them,
-// [step][half][16-byte piece][row][thread column], with a power of two per row of x.
+// [step][half][16-byte piece][row][thread column], with a power of two per row.
 //
 // Measured on B200, 8 experts 4096 -> 14336 -> 4096, 8 tokens, up + gate / down: 202 / 98 us through the tensor-core kernel (whose
 // dequantisation takes 1345 warp instructions for 8192 codes), 95 / 49 here: 560 warp instructions, 59 % of the issue slots and 62 % of
 // shared memory's cycles in use; the copies alone take 56 / 30.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "gemv_rows.cuh"
@@ -255,36 +257,62 @@ __device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* p
     return v;
 }
 
-// h = bf16(bf16(silu(bf16(gate))) * bf16(up)) of the short lists, staged for the down projections.  A thread: four columns of
-// list entry blockIdx.y.
+// h = bf16(bf16(silu(bf16(gate))) * bf16(up)) of the short lists, staged for the down projections as fp16 with a power of two per
+// row, as the rows of x are: h of 1e-6 times a scale of 0.02 would be a denormal in fp16 (a block of weights of 1e-4: 0.24 from 64
+// bits without the factor, 3e-3 with it).  A cluster of SILU_CTAS CTAs takes list entry blockIdx.y, a thread four columns at a time.
+constexpr int SILU_CTAS = 8, SILU_COLS = SILU_CTAS * 256 * 4;
 __global__ void __launch_bounds__(256) few_silu_kernel(unsigned char* __restrict__ ht, const float* __restrict__ partial,
-                                                       const int32_t* __restrict__ counts, const float* __restrict__ row_scale, int lists,
-                                                       int ctas, int units, int PT, int F, int G) {
+                                                       const int32_t* __restrict__ counts, const float* __restrict__ row_scale,
+                                                       float* __restrict__ h_scale, int lists, int ctas, int units, int PT, int F, int G) {
     __shared__ ListSplit sp;
+    __shared__ uint32_t s_max;                          // largest |h| of this CTA's columns, as bf16
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     grid_launch_dependents();
+    if (threadIdx.x == 0) s_max = 0u;
     grid_dependency_wait();
     if (threadIdx.x < 32) sp.make(counts, lists, (uint32_t)(2 * units * PT), ctas);
     __syncthreads();
-    const int entry = blockIdx.y, f = 4 * (blockIdx.x * 256 + threadIdx.x);
+    const int entry = blockIdx.y;
     const int e = sp.list_of(entry), m = entry - sp.list0[e], cap = ListSplit::cap(sp.n[e]);
-    if (cap == 0 || m >= sp.n[e] || f >= F) return;
-    const int unit = f % G / PER / CW;
+    if (cap == 0 || m >= sp.n[e]) return;               // (all CTAs of a cluster alike)
     const float scale = __ldcg(row_scale + entry);
-    const float4 a = sum_pieces(sp, partial, e, m, unit, PT, f, 2 * F), b = sum_pieces(sp, partial, e, m, units + unit, PT, F + f, 2 * F);
     auto act = [scale](float x, float y) {
         const float g = round_bf16(x * scale);
-        return round_bf16(round_bf16(g / (1.f + __expf(-g))) * round_bf16(y * scale));
+        return float_to_bf16_bits(round_bf16(g / (1.f + __expf(-g))) * round_bf16(y * scale));
     };
-    const uint32_t lo = h2_of(act(a.x, b.x), act(a.z, b.z)), hi = h2_of(act(a.y, b.y), act(a.w, b.w));
-    *reinterpret_cast<uint2*>(ht + (size_t)sp.xrow0[e] * F * 2 + few_staged_at(f, m, cap) + ((f >> 2) & 1) * 8) = make_uint2(lo, hi);
+    // as bf16 where the fp16 values will be
+    auto place = [&](int f) { return reinterpret_cast<uint2*>(ht + (size_t)sp.xrow0[e] * F * 2 + few_staged_at(f, m, cap) + ((f >> 2) & 1) * 8); };
+    uint32_t mx = 0;
+    for (int f = 4 * (blockIdx.x * 256 + threadIdx.x); f < F; f += SILU_COLS) {
+        const int unit = f % G / PER / CW;
+        const float4 a = sum_pieces(sp, partial, e, m, unit, PT, f, 2 * F), b = sum_pieces(sp, partial, e, m, units + unit, PT, F + f, 2 * F);
+        const uint32_t lo = act(a.x, b.x) | ((uint32_t)act(a.z, b.z) << 16), hi = act(a.y, b.y) | ((uint32_t)act(a.w, b.w) << 16);
+        mx = __vmaxu2(mx, __vmaxu2(lo & 0x7fff7fffu, hi & 0x7fff7fffu));
+        *place(f) = make_uint2(lo, hi);
+    }
+    mx = __reduce_max_sync(0xffffffffu, max(mx & 0xffffu, mx >> 16));
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, mx);
+    cluster.sync();
+    mx = 0;
+#pragma unroll
+    for (int r = 0; r < SILU_CTAS; ++r) mx = max(mx, *cluster.map_shared_rank(&s_max, r));
+    const int ex = exponent_of(mx);
+    const float down = __uint_as_float((uint32_t)(254 - ex) << 23);
+    if (blockIdx.x == 0 && threadIdx.x == 0) h_scale[entry] = __uint_as_float((uint32_t)ex << 23);
+    for (int f = 4 * (blockIdx.x * 256 + threadIdx.x); f < F; f += SILU_COLS) {
+        const uint2 v = *place(f);
+        auto half = [down](uint32_t w) { return h2_of(__uint_as_float(w << 16) * down, __uint_as_float(w & 0xffff0000u) * down); };
+        *place(f) = make_uint2(half(v.x), half(v.y));
+    }
+    cluster.sync();                                     // nobody leaves while its shared memory may still be read
 }
 
 // out[t] = bf16(bf16(w_i * y_i) + bf16(w_j * y_j)) of the two list entries of token t: sums of pieces where the list is short, else
 // the finished rows `y` of the tensor-core kernel.  A thread: four columns of token blockIdx.y.
 __global__ void __launch_bounds__(256) few_combine_kernel(uint16_t* __restrict__ out, const float* __restrict__ partial,
                                                           const uint16_t* __restrict__ y, const int32_t* __restrict__ counts,
-                                                          const int32_t* __restrict__ entry_of, const float* __restrict__ token_w, int lists,
-                                                          int ctas, int units, int PT, int H, int G) {
+                                                          const int32_t* __restrict__ entry_of, const float* __restrict__ token_w,
+                                                          const float* __restrict__ h_scale, int lists, int ctas, int units, int PT, int H, int G) {
     __shared__ ListSplit sp;
     grid_launch_dependents();
     grid_dependency_wait();
@@ -297,12 +325,12 @@ __global__ void __launch_bounds__(256) few_combine_kernel(uint16_t* __restrict__
     for (int j = 0; j < 2; ++j) {
         const int entry = __ldcg(entry_of + 2 * t + j), e = sp.list_of(entry);
         if (sp.n[e] <= FEW_ROWS) {
-            const float w = __ldcg(token_w + entry);
+            const float w = __ldcg(token_w + entry), up = __ldcg(h_scale + entry);
             const float4 s = sum_pieces(sp, partial, e, entry - sp.list0[e], c % G / PER / CW, PT, c, H);
-            v[j][0] = round_bf16(round_bf16(s.x) * w);
-            v[j][1] = round_bf16(round_bf16(s.y) * w);
-            v[j][2] = round_bf16(round_bf16(s.z) * w);
-            v[j][3] = round_bf16(round_bf16(s.w) * w);
+            v[j][0] = round_bf16(round_bf16(s.x * up) * w);
+            v[j][1] = round_bf16(round_bf16(s.y * up) * w);
+            v[j][2] = round_bf16(round_bf16(s.z * up) * w);
+            v[j][3] = round_bf16(round_bf16(s.w * up) * w);
         } else {
             const uint2 r = *reinterpret_cast<const uint2*>(y + (size_t)entry * H + c);
             v[j][0] = __uint_as_float(r.x << 16);
@@ -359,7 +387,7 @@ bool few_plan(int64_t T, int E, const hqm_weight* w1, const hqm_weight* w2, cons
     const int64_t u1 = (w1->N / 16 / PER + CW - 1) / CW, u2 = (w2->N / 16 / PER + CW - 1) / CW;
     auto align = [](size_t v) { return (v + 1023) / 1024 * 1024; };
     fp->x_bytes = align(staged_rows * w1->K * 2);
-    fp->scale_bytes = align((size_t)2 * T * sizeof(float));
+    fp->scale_bytes = align((size_t)4 * T * sizeof(float));                          // of x, of h
     fp->h_bytes = align(staged_rows * w1->N * 2);
     fp->part_bytes = align(std::max(partial_bytes(T, E, 2 * u1, w1->K / KC, 2 * (int64_t)w1->N, sms), partial_bytes(T, E, u2, w2->K / KC, w2->N, sms)));
     return true;
@@ -401,21 +429,21 @@ int launch_few_projection(const FewJob& job, const unsigned char* xt, float* par
     return HQM_OK;
 }
 
-int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, int64_t T, cudaStream_t st) {
+int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, float* h_scale, int64_t T, cudaStream_t st) {
     using namespace rows;
     const int F = job.w1->N, G = F / 16, units = (G / PER + CW - 1) / CW;
-    launch_overlapped(few_silu_kernel, dim3((F / 4 + 255) / 256, (unsigned)(2 * T)), 256, 0, st, ht, partial, job.counts, row_scale, job.lists,
-                      sm_count(), units, job.w1->K / KC, F, G);
+    launch_overlapped_cluster(few_silu_kernel, dim3(SILU_CTAS, (unsigned)(2 * T)), 256, 0, SILU_CTAS, st, ht, partial, job.counts, row_scale, h_scale,
+                              job.lists, sm_count(), units, job.w1->K / KC, F, G);
     HQM_LAUNCH_CHECK();
     return HQM_OK;
 }
 
 int launch_few_combine(const FewJob& job, uint16_t* out, const float* partial, const uint16_t* y, const int32_t* entry_of, const float* token_w,
-                       int64_t T, cudaStream_t st) {
+                       const float* h_scale, int64_t T, cudaStream_t st) {
     using namespace rows;
     const int H = job.w2->N, G = H / 16, units = (G / PER + CW - 1) / CW;
     launch_overlapped(few_combine_kernel, dim3((H / 4 + 255) / 256, (unsigned)T), 256, 0, st, out, partial, y, job.counts, entry_of, token_w,
-                      job.lists, sm_count(), units, job.w2->K / KC, H, G);
+                      h_scale, job.lists, sm_count(), units, job.w2->K / KC, H, G);
     HQM_LAUNCH_CHECK();
     return HQM_OK;
 }

@@ -60,8 +60,6 @@ struct Params {
         return l;
     }
 };
-// Of a row's factor, biased, from the row's largest |x| as bf16.
-__device__ __forceinline__ int exponent_of(uint32_t largest) { return min(max((int)(largest >> 7), 30), 250) - 4; }
 
 // sum_again() for the runs of this warp.  (A function of its own that finds them anew: what they are known by would otherwise stay in
 // registers beside the steps, 4 % of the time at 8 rows.)

@@ -107,6 +107,9 @@ __device__ __forceinline__ uint4 stage8(uint4 v, float f) {
     return make_uint4(h2_of(lo(v.x), lo(v.y)), h2_of(hi(v.x), hi(v.y)), h2_of(lo(v.z), lo(v.w)), h2_of(hi(v.z), hi(v.w)));
 }
 
+// Of a row's factor, biased, from the row's largest |x| as bf16: the factor brings it into [16, 32).
+__device__ __forceinline__ int exponent_of(uint32_t largest) { return min(max((int)(largest >> 7), 30), 250) - 4; }
+
 // TOKS: rows of x computed together.  1: the four slots of a byte are B columns 0-3.  4: a B fragment holds two slots of four
 // rows; 8: one slot of eight.
 template <int TOKS>

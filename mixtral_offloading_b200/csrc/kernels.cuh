@@ -118,9 +118,10 @@ __host__ __device__ inline size_t few_staged_at(int k, int m, int cap) {
     return (size_t)(k >> 7) * cap * 256 + (size_t)((2 * ((c >> 1) & 1) + (c & 1)) * cap + m) * 64 + (c >> 2) * 16;
 }
 int launch_few_projection(const FewJob& job, const unsigned char* xt, float* partial, bool up, cudaStream_t st);
-int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, int64_t T, cudaStream_t st);
+int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, float* h_scale, int64_t T,
+                    cudaStream_t st);
 int launch_few_combine(const FewJob& job, uint16_t* out, const float* partial, const uint16_t* y, const int32_t* entry_of, const float* token_w,
-                       int64_t T, cudaStream_t st);
+                       const float* h_scale, int64_t T, cudaStream_t st);
 
 // router.cu — logits, top-2 indices and weights of M tokens (no per-expert lists).
 int launch_router_top2(uint16_t* router_logits, float* topk_w, int32_t* topk_idx, const uint16_t* x,

@@ -47,6 +47,22 @@ def test_large_scales_of_a_block(std, tokens):
     assert _cabi.lib().hqm_device_error() == 0
 
 
+@pytest.mark.parametrize("std", [1e-6, 1e-4, 3e-3])
+@pytest.mark.parametrize("tokens", [2, 8])
+def test_small_h_of_a_block(std, tokens):
+    """h of 1e-10 to 1e-3: as fp16 without a factor of its row, and times a scale, below fp16's smallest."""
+    experts = [make_expert(512, 3072, layers(512, 3072, std)) for _ in range(4)]
+    gate = torch.nn.Linear(512, 4, bias=False, dtype=torch.bfloat16, device=DEV)
+    gate.weight.data = (torch.randn(4, 512, generator=torch.Generator().manual_seed(1)) * 0.1).to(torch.bfloat16).to(DEV)
+    moe = ResidentMoe(Cfg(512, 3072, 4), 0, gate, experts)
+    x = rows(tokens, 512, 1.0, tokens)
+    y, logits = moe(x.view(1, tokens, 512))
+    p = torch.softmax(logits.view(tokens, 4).float(), 1).topk(2, 1).values
+    p = (p / p.sum(1, keepdim=True)).to(torch.bfloat16).double()
+    want = reference(experts[0], x) * p.sum(1, keepdim=True)                  # (the experts are alike)
+    assert ((y.view(tokens, 512).double() - want).norm() / want.norm()).item() < 7e-3
+
+
 @pytest.mark.parametrize("N,K", [(14336, 4096), (4096, 14336)])
 @pytest.mark.parametrize("value", [float("inf"), -float("inf")])
 def test_an_infinite_x_has_the_sign_of_the_weight(N, K, value):
