@@ -373,7 +373,7 @@ static size_t partial_bytes(int64_t T, int E, int64_t units, int64_t PT, int64_t
 
 bool few_plan(int64_t T, int E, const hqm_weight* w1, const hqm_weight* w2, const hqm_weight* w3, FewPlan* fp) {
     using namespace rows;
-    if (T < 1 || T > FEW_TOKENS || E < 2 || E > FEW_MAX_LISTS || force_generic() || tma_encode_entry() == nullptr) return false;
+    if (T < 1 || E < 2 || !few_tokens_ok(T, E) || E > FEW_MAX_LISTS || force_generic() || tma_encode_entry() == nullptr) return false;
     const hqm_weight* ws[3] = {w1, w3, w2};
     for (const hqm_weight* w : ws) {
         int G, C;

@@ -98,9 +98,15 @@ bool rows_cached_maps(const hqm_weight* w, int G, void* out3);        // gemv_tm
 // gemv_lists.cu — the experts of a MoE block whose lists are short (2-bit layers with groups of 16).
 constexpr int FEW_ROWS = 8;              // rows of a short list at most
 constexpr int FEW_MAX_LISTS = 32;
-// Tokens up to which it is asked.  A block of 8 experts, us, without / with: 2 tokens 170 / 110, 4: 204 / 129, 8: 269 / 167, 16: 301 / 205,
-// 24: 301 / 248, 33: 302 / 274, 40: 302 / 323 (both kernels run then, one after the other, on half of the lists each).
-constexpr int64_t FEW_TOKENS = 36;
+// Whether it is asked: what decides is how long the lists are, 2 T / E entries on average.  Where many are longer than FEW_ROWS both
+// kernels run, one after the other; with two experts every list has all T tokens.  A block of 4096 -> 14336 -> 4096, us, without / with:
+//    2 experts   2 tokens  96 /  74   8  98 /  83  12  98 / 104  24 106 / 114
+//    4           4 tokens 130 /  92  12 164 / 130  16 164 / 160  24 164 / 172
+//    8           8 tokens 262 / 160  16 295 / 205  36 295 / 282  48 296 / 319
+//   16          16 tokens 505 / 307  36 545 / 374  64 593 / 514  96 638 / 605  128 677 / 695
+//   32          16 tokens 740 / 425  36 1044 / 602  96 1176 / 863  128 1193 / 1025
+constexpr int64_t FEW_MEAN = 9;
+inline bool few_tokens_ok(int64_t T, int E) { return T <= FEW_ROWS || (E > 2 && 2 * T <= FEW_MEAN * E); }
 struct FewPlan {
     size_t x_bytes, scale_bytes, h_bytes, part_bytes;
     size_t total() const { return x_bytes + scale_bytes + h_bytes + part_bytes; }

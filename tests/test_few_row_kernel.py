@@ -88,6 +88,26 @@ def test_lists_of_every_length(hidden, ffn, n_exp, tokens):
     assert _cabi.lib().hqm_device_error() == 0
 
 
+@pytest.mark.parametrize("n_exp,tokens,few", [(2, 8, True), (2, 9, False), (3, 13, True), (3, 14, False), (4, 18, True), (4, 19, False),
+                                              (8, 36, True), (8, 37, False), (32, 144, True), (32, 145, False)])
+def test_which_blocks_have_short_lists(n_exp, tokens, few):
+    """Up to nine entries per list on average; with two experts no list is shorter than the block."""
+    hidden, ffn = 128, 4096
+    ods = tuple(random_layer(n, k, 2, 16, seed=i) for i, (n, k) in enumerate(((ffn, hidden), (hidden, ffn), (ffn, hidden))))
+    gate = torch.nn.Linear(hidden, n_exp, bias=False, dtype=torch.bfloat16, device=DEV)
+    gate.weight.data = (torch.randn(n_exp, hidden, generator=torch.Generator().manual_seed(1)) * 0.1).to(torch.bfloat16).to(DEV)
+    expert = make_expert(hidden, ffn, ods)
+    moe = ResidentMoe(Cfg(hidden, ffn, n_exp), 0, gate, [expert] * n_exp)
+    x = torch.randn(1, tokens, hidden, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16).to(DEV)
+    assert ("gemv_lists_kernel" in kernels_of(lambda: moe(x))) == few
+    y, logits = moe(x)
+    p = torch.softmax(logits.view(tokens, n_exp).float(), 1).topk(2, 1).values
+    p = (p / p.sum(1, keepdim=True)).to(torch.bfloat16).double()
+    want = reference(expert, x[0]) * p.sum(1, keepdim=True)                   # (the experts are alike)
+    assert ((y[0].double() - want).norm() / want.norm()).item() < 7e-3        # as in test_lists_of_every_length
+    assert _cabi.lib().hqm_device_error() == 0
+
+
 @pytest.mark.parametrize("N,K,few", [(14336, 4096, True), (4096, 14336, True), (14336, 14336, True), (14336, 3072, False)])
 def test_large_linear_layers(N, K, few):
     """Two to five rows of layers with three steps or more for every SM (one with less, which the other kernels keep); with less

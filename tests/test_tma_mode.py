@@ -20,7 +20,7 @@ def kernels_of(run):
         run()
         torch.cuda.synchronize()
     names = " ".join(e.key for e in prof.key_averages())
-    return {k for k in KERNELS.values() if k in names}
+    return {k for k in (*KERNELS.values(), "gemv_lists_kernel") if k in names}
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
