@@ -217,9 +217,7 @@ struct Fmt {
     // (Even: a slot is filled by one of the two copying warps then, and its phases are waited for in order.)
     // (2 bit, wide chunks: 8 where no tile is cut and nothing is summed: 3072 x 2048, 80 rows 12.9 us with 6, 12.6 with 8.)
     __host__ __device__ static constexpr int n_raw(int n_max, bool cut) { return WORDS || (n_max > 64 && (cut || PARTS == 4)) ? 6 : 8; }
-    // Pieces of 16 rows on their way to shared memory while a cut tile is summed: as many as there is room for.  (One more is on
-    // its way to registers: with one piece in flight, as wide 4-bit and all 3-bit launches then had, 3-bit 1024 x 2048, 90 rows
-    // took @16.17@ us, 4-bit 2048 x 9216, 192 rows 33.0.)
+    // Pieces of 16 rows in flight while a cut tile is summed: as many as there is room for.
     __host__ __device__ static constexpr int n_merge(int n_max) { return WORDS ? 1 : (n_max <= 64 ? 4 : (PARTS == 4 ? 1 : 3)); }
     static constexpr int ST_OFF = 0, EPI_OFF = ST_OFF + 4 * GROUPS * ST_WARP, BAR_OFF = EPI_OFF + EPI_BYTES, RING_OFF = BAR_OFF + 1024;
     __host__ __device__ static constexpr int smem(int n_max, bool cut) {
@@ -1200,8 +1198,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
             }
             if (finish) {
                 // A cut tile: the pieces in CTA order (a CTA without a unit has none), 16 rows at a time.  What this costs is latency,
-                // so several are under way: n_merge in shared memory, where a thread copies what it will read itself, which needs no
-                // barrier, and one in the registers that the tile's own piece has left.
+                // so several are under way; a thread copies what it will read itself, which needs no barrier.
                 const uint32_t merge = raw_ring + (uint32_t)(n_raw * F::RAW_BYTES) + 16u * et;
                 const int n_merge = F::n_merge(prm.n_max);
                 const bool dense = parts_n == c_last - c_first + 1;
@@ -1211,23 +1208,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                 auto fetch = [&] {
                     if (fetch_r < rows_here) {
                         const float4* src = fetch_src + (uint32_t)(2 * fetch_c + (fetch_c == c_first ? 1 : 0)) * (size_t)step;
-                        if (fetch_at == n_merge) {
+                        const uint32_t dst = merge + (uint32_t)(fetch_at * MERGE_BYTES);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const uint4 f = __ldcg(reinterpret_cast<const uint4*>(src + i * 128));
-                                acc[4 * i] = f.x;
-                                acc[4 * i + 1] = f.y;
-                                acc[4 * i + 2] = f.z;
-                                acc[4 * i + 3] = f.w;
-                            }
-                            fetch_at = -1;
-                        } else {
-                            const uint32_t dst = merge + (uint32_t)(fetch_at * MERGE_BYTES);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(i * MERGE_BYTES / 4)), "l"(src + i * 128) : "memory");
-                        }
-                        ++fetch_at;
+                        for (int i = 0; i < 4; ++i)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(i * MERGE_BYTES / 4)), "l"(src + i * 128) : "memory");
+                        fetch_at = fetch_at + 1 == n_merge ? 0 : fetch_at + 1;
                         ++fetch_c;
                         if (!dense)
                             while (fetch_c <= c_last && sh.begin[fetch_c + 1] <= sh.begin[fetch_c]) ++fetch_c;
@@ -1244,31 +1229,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) gg_kernel(const __grid_constant__
                     for (int i = 0; i < 16; ++i) v[i] = 0.f;
 #pragma unroll 1
                     for (int c = 0; c < parts_n; ++c) {
-                        if (merge_at == n_merge) {
+                        // the oldest of n_merge groups has arrived
+                        if (n_merge == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+                        else if (n_merge == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+                        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                        const uint32_t at = merge + (uint32_t)(merge_at * MERGE_BYTES);
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) v[i] += __uint_as_float(acc[i]);
-                            merge_at = -1;
-                        } else {
-                            // the oldest of n_merge + 1 groups has arrived (that of the registers is empty)
-                            if (n_merge == 4) asm volatile("cp.async.wait_group 4;" ::: "memory");
-                            else if (n_merge == 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
-                            else asm volatile("cp.async.wait_group 1;" ::: "memory");
-                            const uint32_t at = merge + (uint32_t)(merge_at * MERGE_BYTES);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const uint4 f = lds128(at + (uint32_t)(i * MERGE_BYTES / 4));
-                                v[4 * i] += __uint_as_float(f.x);
-                                v[4 * i + 1] += __uint_as_float(f.y);
-                                v[4 * i + 2] += __uint_as_float(f.z);
-                                v[4 * i + 3] += __uint_as_float(f.w);
-                            }
+                        for (int i = 0; i < 4; ++i) {
+                            const uint4 f = lds128(at + (uint32_t)(i * MERGE_BYTES / 4));
+                            v[4 * i] += __uint_as_float(f.x);
+                            v[4 * i + 1] += __uint_as_float(f.y);
+                            v[4 * i + 2] += __uint_as_float(f.z);
+                            v[4 * i + 3] += __uint_as_float(f.w);
                         }
-                        ++merge_at;
+                        merge_at = merge_at + 1 == n_merge ? 0 : merge_at + 1;
                         fetch();
                     }
                 };
                 if (!whole)
-                    for (int i = 0; i <= n_merge; ++i) fetch();
+                    for (int i = 0; i < n_merge; ++i) fetch();
 #pragma unroll 1
                 for (int c0 = 0; c0 < rows_here; c0 += 16) {
                     float v[16];
