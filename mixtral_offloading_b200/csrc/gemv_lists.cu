@@ -260,15 +260,18 @@ __device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* p
 // h = bf16(bf16(silu(bf16(gate))) * bf16(up)) of the short lists, staged for the down projections as fp16 with a power of two per
 // row, as the rows of x are: h of 1e-6 times a scale of 0.02 would be a denormal in fp16 (a block of weights of 1e-4: 0.24 from 64
 // bits without the factor, 3e-3 with it).  A cluster of SILU_CTAS CTAs takes list entry blockIdx.y, a thread four columns at a time.
-constexpr int SILU_CTAS = 8, SILU_COLS = SILU_CTAS * 256 * 4;
-__global__ void __launch_bounds__(256) few_silu_kernel(unsigned char* __restrict__ ht, const float* __restrict__ partial,
-                                                       const int32_t* __restrict__ counts, const float* __restrict__ row_scale,
-                                                       float* __restrict__ h_scale, int lists, int ctas, int units, int PT, int F, int G) {
+// The CTAs leave their largest values in each other's shared memory, so that one cluster barrier stands between the sums and the
+// stores; the one in front of the sums (every CTA is there to be written to) passes under the kernel in front.
+constexpr int SILU_CTAS = 8, SILU_THREADS = 512, SILU_COLS = SILU_CTAS * SILU_THREADS * 4;
+__global__ void __launch_bounds__(SILU_THREADS) few_silu_kernel(unsigned char* __restrict__ ht, const float* __restrict__ partial,
+                                                                const int32_t* __restrict__ counts, const float* __restrict__ row_scale,
+                                                                float* __restrict__ h_scale, int lists, int ctas, int units, int PT, int F, int G) {
     __shared__ ListSplit sp;
-    __shared__ uint32_t s_max;                          // largest |h| of this CTA's columns, as bf16
+    __shared__ uint32_t s_max, s_all[SILU_CTAS];        // largest |h| of this CTA's columns, of every CTA's, as bf16
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     grid_launch_dependents();
     if (threadIdx.x == 0) s_max = 0u;
+    cluster.sync();
     grid_dependency_wait();
     if (threadIdx.x < 32) sp.make(counts, lists, (uint32_t)(2 * units * PT), ctas);
     __syncthreads();
@@ -278,33 +281,37 @@ __global__ void __launch_bounds__(256) few_silu_kernel(unsigned char* __restrict
     const float scale = __ldcg(row_scale + entry);
     auto act = [scale](float x, float y) {
         const float g = round_bf16(x * scale);
-        return float_to_bf16_bits(round_bf16(g / (1.f + __expf(-g))) * round_bf16(y * scale));
+        return (uint32_t)float_to_bf16_bits(round_bf16(g / (1.f + __expf(-g))) * round_bf16(y * scale));
     };
-    // as bf16 where the fp16 values will be
     auto place = [&](int f) { return reinterpret_cast<uint2*>(ht + (size_t)sp.xrow0[e] * F * 2 + few_staged_at(f, m, cap) + ((f >> 2) & 1) * 8); };
+    // bf16 values of four columns: a thread's first ones stay in registers, others wait where the fp16 values will be
+    const int f0 = 4 * (blockIdx.x * SILU_THREADS + threadIdx.x);
+    uint2 first = make_uint2(0u, 0u);
     uint32_t mx = 0;
-    for (int f = 4 * (blockIdx.x * 256 + threadIdx.x); f < F; f += SILU_COLS) {
+    for (int f = f0; f < F; f += SILU_COLS) {
         const int unit = f % G / PER / CW;
         const float4 a = sum_pieces(sp, partial, e, m, unit, PT, f, 2 * F), b = sum_pieces(sp, partial, e, m, units + unit, PT, F + f, 2 * F);
-        const uint32_t lo = act(a.x, b.x) | ((uint32_t)act(a.z, b.z) << 16), hi = act(a.y, b.y) | ((uint32_t)act(a.w, b.w) << 16);
-        mx = __vmaxu2(mx, __vmaxu2(lo & 0x7fff7fffu, hi & 0x7fff7fffu));
-        *place(f) = make_uint2(lo, hi);
+        const uint2 v = make_uint2(act(a.x, b.x) | (act(a.z, b.z) << 16), act(a.y, b.y) | (act(a.w, b.w) << 16));
+        mx = __vmaxu2(mx, __vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu));
+        if (f == f0) first = v;
+        else *place(f) = v;
     }
     mx = __reduce_max_sync(0xffffffffu, max(mx & 0xffffu, mx >> 16));
     if ((threadIdx.x & 31) == 0) atomicMax(&s_max, mx);
+    __syncthreads();
+    if (threadIdx.x < SILU_CTAS) *cluster.map_shared_rank(&s_all[blockIdx.x], threadIdx.x) = s_max;
     cluster.sync();
     mx = 0;
 #pragma unroll
-    for (int r = 0; r < SILU_CTAS; ++r) mx = max(mx, *cluster.map_shared_rank(&s_max, r));
+    for (int r = 0; r < SILU_CTAS; ++r) mx = max(mx, s_all[r]);
     const int ex = exponent_of(mx);
     const float down = __uint_as_float((uint32_t)(254 - ex) << 23);
     if (blockIdx.x == 0 && threadIdx.x == 0) h_scale[entry] = __uint_as_float((uint32_t)ex << 23);
-    for (int f = 4 * (blockIdx.x * 256 + threadIdx.x); f < F; f += SILU_COLS) {
-        const uint2 v = *place(f);
+    for (int f = f0; f < F; f += SILU_COLS) {
+        const uint2 v = f == f0 ? first : *place(f);
         auto half = [down](uint32_t w) { return h2_of(__uint_as_float(w << 16) * down, __uint_as_float(w & 0xffff0000u) * down); };
         *place(f) = make_uint2(half(v.x), half(v.y));
     }
-    cluster.sync();                                     // nobody leaves while its shared memory may still be read
 }
 
 // out[t] = bf16(bf16(w_i * y_i) + bf16(w_j * y_j)) of the two list entries of token t: sums of pieces where the list is short, else
@@ -432,7 +439,7 @@ int launch_few_projection(const FewJob& job, const unsigned char* xt, float* par
 int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, float* h_scale, int64_t T, cudaStream_t st) {
     using namespace rows;
     const int F = job.w1->N, G = F / 16, units = (G / PER + CW - 1) / CW;
-    launch_overlapped_cluster(few_silu_kernel, dim3(SILU_CTAS, (unsigned)(2 * T)), 256, 0, SILU_CTAS, st, ht, partial, job.counts, row_scale, h_scale,
+    launch_overlapped_cluster(few_silu_kernel, dim3(SILU_CTAS, (unsigned)(2 * T)), SILU_THREADS, 0, SILU_CTAS, st, ht, partial, job.counts, row_scale, h_scale,
                               job.lists, sm_count(), units, job.w1->K / KC, F, G);
     HQM_LAUNCH_CHECK();
     return HQM_OK;
