@@ -97,11 +97,51 @@ struct ListParams {
     int* error_flag;
 };
 
+// A run of steps of one unit: list, unit of the list, steps [pa, pb) of it.
+struct Run {
+    int e, unit, pa, pb;
+    // That of step u; the caller's steps end at ue, and list `from` does not lie behind the step's.
+    __device__ __forceinline__ static Run at(const ListSplit& sp, int PT, uint32_t ue, uint32_t u, int from) {
+        Run r;
+        r.e = from;
+        while (u >= sp.step0[r.e + 1]) ++r.e;
+        const uint32_t rel = u - sp.step0[r.e];
+        r.unit = (int)(rel / (uint32_t)PT);
+        r.pa = (int)(rel - (uint32_t)r.unit * (uint32_t)PT);
+        r.pb = (int)min((uint32_t)PT, (uint32_t)r.pa + (ue - u));
+        return r;
+    }
+};
+
+// sum_again() for the runs of this warp in the steps [u, ue).
+__device__ __noinline__ void lists_again(const ListParams& prm, const ListSplit& sp, uint32_t u, uint32_t ue) {
+    const int warp = threadIdx.x >> 5, K = prm.K, row_len = prm.layers * prm.N;
+    while (u < ue) {
+        const Run r = Run::at(sp, prm.PT, ue, u, 0);
+        u += (uint32_t)(r.pb - r.pa);
+        const int layer = r.unit / prm.units, rho = (r.unit - layer * prm.units) * CW + warp;
+        if (rho * PER >= prm.G) continue;
+        const int piece = r.pa ? (int)blockIdx.x - sp.owner(r.e, (uint32_t)(r.unit * prm.PT)) : 0;
+        Again a{};
+        a.layer(prm.table[3 * r.e + (layer ? prm.which1 : prm.which0)].w);
+        a.K = K;
+        a.G = prm.G;
+        a.C = prm.C;
+        a.rho = rho;
+        a.k0 = r.pa * KC;
+        a.k1 = r.pb * KC;
+        a.staged = prm.xt + (size_t)sp.xrow0[r.e] * K * 2;
+        a.cap = ListSplit::cap(sp.n[r.e]);
+        for (a.m = 0; a.m < sp.n[r.e]; ++a.m)
+            sum_again(a, prm.partial + ((size_t)piece * sp.R + sp.row0[r.e] + a.m) * row_len + layer * prm.N + PER * rho, 1.f);
+    }
+}
+
 __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_constant__ ListParams prm) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ ListSplit sp;
     __shared__ uint32_t s_begin[2];
-    __shared__ int s_failed;
+    __shared__ int s_failed, s_again;
     __shared__ __align__(8) uint64_t s_bars[2 * MAX_STAGES];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t exch = ring + prm.stages * prm.stage_bytes;
@@ -112,7 +152,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
     grid_launch_dependents();
     if (threadIdx.x == 0) {
         init_barriers(full, empty, prm.stages);
-        s_failed = 0;
+        s_failed = s_again = 0;
     }
     // the table's entries in L2 by the time the lists are known
     for (int i = threadIdx.x; i < 4 * prm.layers * prm.lists; i += THREADS) {
@@ -128,20 +168,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
     __syncthreads();
     const uint32_t ub = s_begin[0], ue = s_begin[1];
 
-    // The runs of steps of one unit: list, unit of the list, steps [pa, pb) of it.
-    struct Run {
-        int e, unit, pa, pb;
-    };
-    auto run_at = [&](uint32_t u, int from) {
-        Run r;
-        r.e = from;
-        while (u >= sp.step0[r.e + 1]) ++r.e;
-        const uint32_t rel = u - sp.step0[r.e];
-        r.unit = (int)(rel / (uint32_t)PT);
-        r.pa = (int)(rel - (uint32_t)r.unit * (uint32_t)PT);
-        r.pb = (int)min((uint32_t)PT, (uint32_t)r.pa + (ue - u));
-        return r;
-    };
+    auto run_at = [&](uint32_t u, int from) { return Run::at(sp, PT, ue, u, from); };
 
     if (warp == CW) {
         // =========================== copies ===========================
@@ -211,31 +238,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
             if (sg.M <= 4) ok = rows_segment<4, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again);
             else ok = rows_segment<8, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again);
         }
-        if (__all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, again)) {
-            for (uint32_t u = ub; u < ue;) {
-                const Run r = run_at(u, 0);
-                u += (uint32_t)(r.pb - r.pa);
-                const int layer = r.unit / prm.units, rho = (r.unit - layer * prm.units) * CW + warp;
-                if (rho * PER >= prm.G) continue;
-                const int piece = r.pa ? cta - sp.owner(r.e, (uint32_t)(r.unit * PT)) : 0;
-                Again a{};
-                a.layer(prm.table[3 * r.e + (layer ? prm.which1 : prm.which0)].w);
-                a.K = K;
-                a.G = prm.G;
-                a.C = prm.C;
-                a.rho = rho;
-                a.k0 = r.pa * KC;
-                a.k1 = r.pb * KC;
-                a.staged = prm.xt + (size_t)sp.xrow0[r.e] * K * 2;
-                a.cap = ListSplit::cap(sp.n[r.e]);
-                for (a.m = 0; a.m < sp.n[r.e]; ++a.m)
-                    sum_again(a, prm.partial + ((size_t)piece * sp.R + sp.row0[r.e] + a.m) * row_len + layer * prm.N + PER * rho, 1.f);
-            }
-        }
+        if (again) s_again = 1;
         if (!ok) s_failed = 1;
     }
-    // ---- a wait ran out: copies may still be on their way to this CTA's shared memory
     __syncthreads();
+    if (s_again && !s_failed && warp < CW) lists_again(prm, sp, ub, ue);
+    // ---- a wait ran out: copies may still be on their way to this CTA's shared memory
     if (s_failed) {
         for (int i = 0; i < 200; ++i) __nanosleep(1000);
         if (threadIdx.x == 0 && prm.error_flag) atomicExch(prm.error_flag, 1);

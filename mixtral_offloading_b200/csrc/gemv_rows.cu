@@ -61,8 +61,8 @@ struct Params {
     }
 };
 
-// sum_again() for the runs of this warp.  (A function of its own that finds them anew: what they are known by would otherwise stay in
-// registers beside the steps, 4 % of the time at 8 rows.)
+// sum_again() for the runs of this warp.  (A function of its own that finds them anew, called where the warps' roles have come
+// together: what the runs are known by would otherwise stay in registers beside the steps, 3 to 4 % of the time at 5 to 8 rows.)
 template <bool SCALED>
 __device__ __noinline__ void rows_again(const Params& prm, const Split& sp, float* partial, const uint16_t* x, const int32_t* x_idx, int M_total,
                                         const uint32_t* s_max, const int* s_absent) {
@@ -95,7 +95,7 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
     using S = Shape<TOKS>;
     extern __shared__ unsigned char smem_raw[];
     __shared__ int s_absent[STREAM_MAX_LAYERS];
-    __shared__ int s_failed;
+    __shared__ int s_failed, s_again;
     __shared__ uint32_t s_max[8];                       // largest |x| of a row's columns, as bf16
     __shared__ __align__(8) uint64_t s_bars[2 * MAX_STAGES];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -109,7 +109,7 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
     grid_launch_dependents();
     if (threadIdx.x == 0) {
         init_barriers(full, empty, stages);
-        s_failed = 0;
+        s_failed = s_again = 0;
     }
     if (threadIdx.x < 8) s_max[threadIdx.x] = 0u;
     __syncthreads();
@@ -145,7 +145,7 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
                 for (int i = 0; i < 3 * (int)sizeof(StreamEntry); i += 128)
                     prefetch_l2(reinterpret_cast<const unsigned char*>(prm.table + 3 * idx) + i);
         }
-        int st = 0, fenced = -1, ahead = stages;
+        int st = 0, fenced = -1;
         uint32_t par = 1;
         bool ok = true;
         for (int unit = unit0, pa = pa0, left = n_steps; left > 0 && ok; ++unit, pa = 0) {
@@ -172,12 +172,14 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
             const int rho = (unit - prm.unit0[l]) * CW;
             uint32_t col = pa ? pa_col : 0u;                  // of class 0
             for (int p = pa; p < pb; ++p) {
-                // Stages are freed by warps that wait for the kernel in front.  So does this one before it waits for them: the
-                // limit of a wait covers this kernel's own steps, not what is left of the other's.
-                if (ahead-- == 0) grid_dependency_wait();
                 if (!wait(empty + 8 * st, par)) {
-                    ok = false;
-                    break;
+                    // The warps that free a stage may still be waiting for the kernel in front, which has no limit: its time does not
+                    // count.  (Waiting for it ahead of the first stage that is not free instead: 0.4 us of 30.5 at one row.)
+                    grid_dependency_wait();
+                    if (!wait(empty + 8 * st, par)) {
+                        ok = false;
+                        break;
+                    }
                 }
                 copy(ring + st * stage_bytes, full + 8 * st, maps, p * KC, rho, src0, src1, col);
                 col += KC;
@@ -351,12 +353,12 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
             }
             x_at += (uint32_t)(pb_all - pa) * S::X_STEP;
         }
-        if (TOKS > 1 && __all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, again))
-            rows_again<S::SCALED>(prm, sp, partial, x, x_idx, M_total, s_max, s_absent);
+        if (again) s_again = 1;
         if (!ok) s_failed = 1;
     }
-    // ---- a wait ran out: copies may still be on their way to this CTA's shared memory
     __syncthreads();
+    if (TOKS > 1 && s_again && !s_failed && warp < CW) rows_again<S::SCALED>(prm, sp, partial, x, x_idx, M_total, s_max, s_absent);
+    // ---- a wait ran out: copies may still be on their way to this CTA's shared memory
     if (s_failed) {
         for (int i = 0; i < 200; ++i) __nanosleep(1000);
         if (threadIdx.x == 0 && prm.error_flag) atomicExch(prm.error_flag, 1);

@@ -154,8 +154,9 @@ struct Again {
 // One row's sums over a run of steps once more, with the weights that dequantize() makes and fp32 products, where a sum that
 // rows_segment() left at `to` (16 members, G apart, of 4 residues) is not finite.  With the tensor cores' factors that happens for
 // inputs that are fine: x * s leaves fp16 where a scale is 2048 or more (x is staged below 32), and an infinite x meets codes of 0
-// and makes the zeros' sum a difference of infinities, though its products with the weights have a sign.  A warp comes here behind
-// all of its steps, when it has seen such a sum: beside them the call would cost the steps 60 to 190 bytes of spilled registers.
+// and makes the zeros' sum a difference of infinities, though its products with the weights have a sign.  The warps come
+// here behind all of their steps, when one has seen such a sum: beside them the call would cost the steps 60 to 190 bytes of spilled
+// registers.
 __device__ __noinline__ static void sum_again(const Again& a, float* to, float up) {
     const int lane = threadIdx.x & 31;
     __syncwarp();                                  // other lanes have stored some of the sums

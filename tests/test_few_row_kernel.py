@@ -88,10 +88,10 @@ def test_lists_of_every_length(hidden, ffn, n_exp, tokens):
     assert _cabi.lib().hqm_device_error() == 0
 
 
-@pytest.mark.parametrize("n_exp,tokens,few", [(2, 8, True), (2, 9, False), (3, 13, True), (3, 14, False), (4, 18, True), (4, 19, False),
+@pytest.mark.parametrize("n_exp,tokens,few", [(2, 8, True), (2, 9, False), (3, 12, True), (3, 13, False), (4, 16, True), (4, 17, False),
                                               (8, 36, True), (8, 37, False), (32, 144, True), (32, 145, False)])
 def test_which_blocks_have_short_lists(n_exp, tokens, few):
-    """Up to nine entries per list on average; with two experts no list is shorter than the block."""
+    """Up to nine entries per list on average, up to eight with four experts or less."""
     hidden, ffn = 128, 4096
     ods = tuple(random_layer(n, k, 2, 16, seed=i) for i, (n, k) in enumerate(((ffn, hidden), (hidden, ffn), (ffn, hidden))))
     gate = torch.nn.Linear(hidden, n_exp, bias=False, dtype=torch.bfloat16, device=DEV)
