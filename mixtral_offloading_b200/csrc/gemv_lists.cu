@@ -250,11 +250,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
     }
 }
 
-// Sum of the pieces of four neighbouring columns of a row.
-__device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* partial, int e, int m, int unit, int PT, int col, int row_len) {
-    const int cnt = sp.owner(e, (uint32_t)(unit * PT + PT - 1)) - sp.owner(e, (uint32_t)(unit * PT)) + 1;
+// CTAs that left a piece of a unit of list e, and the sum of the pieces of four neighbouring columns of row m.
+__device__ __forceinline__ int pieces_of(const ListSplit& sp, int e, int unit, int PT) {
+    return sp.owner(e, (uint32_t)(unit * PT + PT - 1)) - sp.owner(e, (uint32_t)(unit * PT)) + 1;
+}
+__device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* partial, int e, int m, int cnt, int col, int row_len) {
     const float* at = partial + (size_t)(sp.row0[e] + m) * row_len + col;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
     for (int i = 0; i < cnt; ++i) {
         const float4 p = *reinterpret_cast<const float4*>(at + (size_t)i * sp.R * row_len);
         v.x += p.x;
@@ -269,13 +272,16 @@ __device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* p
 // row, as the rows of x are: h of 1e-6 times a scale of 0.02 would be a denormal in fp16 (a block of weights of 1e-4: 0.24 from 64
 // bits without the factor, 3e-3 with it).  A cluster of SILU_CTAS CTAs takes list entry blockIdx.y, a thread four columns at a time.
 // The CTAs leave their largest values in each other's shared memory, so that one cluster barrier stands between the sums and the
-// stores; the one in front of the sums (every CTA is there to be written to) passes under the kernel in front.
-constexpr int SILU_CTAS = 8, SILU_THREADS = 512, SILU_COLS = SILU_CTAS * SILU_THREADS * 4;
-__global__ void __launch_bounds__(SILU_THREADS) few_silu_kernel(unsigned char* __restrict__ ht, const float* __restrict__ partial,
-                                                                const int32_t* __restrict__ counts, const float* __restrict__ row_scale,
-                                                                float* __restrict__ h_scale, int lists, int ctas, int units, int PT, int F, int G) {
+// stores; the one in front of the sums (every CTA is there to be written to) passes under the kernel in front.  Few threads and
+// registers, as the launch in front leaves an SM 13312 of them: with 512 threads a block of 16 tokens took 5.7 us more than without
+// factors, of which this launch alone explains 1.6.
+constexpr int SILU_CTAS = 8, SILU_THREADS = 256, SILU_COLS = SILU_CTAS * SILU_THREADS * 4, SILU_KEPT = 2, SILU_UNITS = 64;
+__global__ void __launch_bounds__(SILU_THREADS, 5) few_silu_kernel(unsigned char* __restrict__ ht, const float* __restrict__ partial,
+                                                                   const int32_t* __restrict__ counts, const float* __restrict__ row_scale,
+                                                                   float* __restrict__ h_scale, int lists, int ctas, int units, int PT, int F, int G) {
     __shared__ ListSplit sp;
     __shared__ uint32_t s_max, s_all[SILU_CTAS];        // largest |h| of this CTA's columns, of every CTA's, as bf16
+    __shared__ int s_cnt[2 * SILU_UNITS];               // pieces of the units of this entry's list
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     grid_launch_dependents();
     if (threadIdx.x == 0) s_max = 0u;
@@ -286,24 +292,31 @@ __global__ void __launch_bounds__(SILU_THREADS) few_silu_kernel(unsigned char* _
     const int entry = blockIdx.y;
     const int e = sp.list_of(entry), m = entry - sp.list0[e], cap = ListSplit::cap(sp.n[e]);
     if (cap == 0 || m >= sp.n[e]) return;               // (all CTAs of a cluster alike)
+    // (four 64-bit divisions for a unit: once for all threads)
+    for (int u = threadIdx.x; u < 2 * units; u += SILU_THREADS) s_cnt[u] = pieces_of(sp, e, u, PT);
     const float scale = __ldcg(row_scale + entry);
+    __syncthreads();
     auto act = [scale](float x, float y) {
         const float g = round_bf16(x * scale);
         return (uint32_t)float_to_bf16_bits(round_bf16(g / (1.f + __expf(-g))) * round_bf16(y * scale));
     };
-    auto place = [&](int f) { return reinterpret_cast<uint2*>(ht + (size_t)sp.xrow0[e] * F * 2 + few_staged_at(f, m, cap) + ((f >> 2) & 1) * 8); };
-    // bf16 values of four columns: a thread's first ones stay in registers, others wait where the fp16 values will be
-    const int f0 = 4 * (blockIdx.x * SILU_THREADS + threadIdx.x);
-    uint2 first = make_uint2(0u, 0u);
     uint32_t mx = 0;
-    for (int f = f0; f < F; f += SILU_COLS) {
+    auto values = [&](int f) {                          // of four columns, as bf16
+        if (f >= F) return make_uint2(0u, 0u);
         const int unit = f % G / PER / CW;
-        const float4 a = sum_pieces(sp, partial, e, m, unit, PT, f, 2 * F), b = sum_pieces(sp, partial, e, m, units + unit, PT, F + f, 2 * F);
+        const float4 a = sum_pieces(sp, partial, e, m, s_cnt[unit], f, 2 * F);
+        const float4 b = sum_pieces(sp, partial, e, m, s_cnt[units + unit], F + f, 2 * F);
         const uint2 v = make_uint2(act(a.x, b.x) | (act(a.z, b.z) << 16), act(a.y, b.y) | (act(a.w, b.w) << 16));
         mx = __vmaxu2(mx, __vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu));
-        if (f == f0) first = v;
-        else *place(f) = v;
-    }
+        return v;
+    };
+    auto place = [&](int f) { return reinterpret_cast<uint2*>(ht + (size_t)sp.xrow0[e] * F * 2 + few_staged_at(f, m, cap) + ((f >> 2) & 1) * 8); };
+    // a thread's first values stay in registers, others wait where the fp16 values will be
+    const int f0 = 4 * (blockIdx.x * SILU_THREADS + threadIdx.x);
+    uint2 kept[SILU_KEPT];
+#pragma unroll
+    for (int j = 0; j < SILU_KEPT; ++j) kept[j] = values(f0 + j * SILU_COLS);
+    for (int f = f0 + SILU_KEPT * SILU_COLS; f < F; f += SILU_COLS) *place(f) = values(f);
     mx = __reduce_max_sync(0xffffffffu, max(mx & 0xffffu, mx >> 16));
     if ((threadIdx.x & 31) == 0) atomicMax(&s_max, mx);
     __syncthreads();
@@ -315,9 +328,12 @@ __global__ void __launch_bounds__(SILU_THREADS) few_silu_kernel(unsigned char* _
     const int ex = exponent_of(mx);
     const float down = __uint_as_float((uint32_t)(254 - ex) << 23);
     if (blockIdx.x == 0 && threadIdx.x == 0) h_scale[entry] = __uint_as_float((uint32_t)ex << 23);
-    for (int f = f0; f < F; f += SILU_COLS) {
-        const uint2 v = f == f0 ? first : *place(f);
-        auto half = [down](uint32_t w) { return h2_of(__uint_as_float(w << 16) * down, __uint_as_float(w & 0xffff0000u) * down); };
+    auto half = [down](uint32_t w) { return h2_of(__uint_as_float(w << 16) * down, __uint_as_float(w & 0xffff0000u) * down); };
+#pragma unroll
+    for (int j = 0; j < SILU_KEPT; ++j)
+        if (f0 + j * SILU_COLS < F) *place(f0 + j * SILU_COLS) = make_uint2(half(kept[j].x), half(kept[j].y));
+    for (int f = f0 + SILU_KEPT * SILU_COLS; f < F; f += SILU_COLS) {
+        const uint2 v = *place(f);
         *place(f) = make_uint2(half(v.x), half(v.y));
     }
 }
@@ -341,7 +357,7 @@ __global__ void __launch_bounds__(256) few_combine_kernel(uint16_t* __restrict__
         const int entry = __ldcg(entry_of + 2 * t + j), e = sp.list_of(entry);
         if (sp.n[e] <= FEW_ROWS) {
             const float w = __ldcg(token_w + entry), up = __ldcg(h_scale + entry);
-            const float4 s = sum_pieces(sp, partial, e, entry - sp.list0[e], c % G / PER / CW, PT, c, H);
+            const float4 s = sum_pieces(sp, partial, e, entry - sp.list0[e], pieces_of(sp, e, c % G / PER / CW, PT), c, H);
             v[j][0] = round_bf16(round_bf16(s.x * up) * w);
             v[j][1] = round_bf16(round_bf16(s.y * up) * w);
             v[j][2] = round_bf16(round_bf16(s.z * up) * w);
@@ -400,6 +416,7 @@ bool few_plan(int64_t T, int E, const hqm_weight* w1, const hqm_weight* w2, cons
     const int sms = sm_count();
     const size_t staged_rows = (size_t)std::min<int64_t>(8 * E, 8 * T);              // (a list of one row takes four)
     const int64_t u1 = (w1->N / 16 / PER + CW - 1) / CW, u2 = (w2->N / 16 / PER + CW - 1) / CW;
+    if (u1 > SILU_UNITS) return false;
     auto align = [](size_t v) { return (v + 1023) / 1024 * 1024; };
     fp->x_bytes = align(staged_rows * w1->K * 2);
     fp->scale_bytes = align((size_t)4 * T * sizeof(float));                          // of x, of h
