@@ -1507,7 +1507,10 @@ GgLayout gg_expert_layout(int64_t M) { return GgLayout{GgRows::of((int)M), gg_sm
 //   its units of 128 columns:  850 + 4 n with n rows; beyond 128 rows, with one accumulator, 10 n
 //   a finished tile:           400 for every 16 rows
 //   a tile cut into p pieces:  5000 until the last CTA has seen that it is the last, and 3000 + 400 (p - 2) for every 16 rows;
-//                              twice where shares and tiles are not aligned, as a CTA then holds pieces of two tiles
+//                              twice where shares and tiles are not aligned, as a CTA then holds pieces of two tiles.
+//                              4-bit chunks of more than 64 rows have one piece in flight: 1200 (p - 2).  (4-bit 2048 x 9216, 192
+//                              rows 31.2 -> 29.9 us, 4096 x 9216, 100 rows 32.0 -> 29.2, 1024 x 9216, 300 rows 29.5 -> 27.9; 3-bit
+//                              launches have one as well, but 1024 x 9216, 192 rows 28.4 -> 37.7, as whole tiles are all they have left.)
 // Wide chunks dequantise the weights less often; narrow ones give every SM whole tiles, and need less scratch.
 GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count, size_t bytes) {
     const int64_t tiles = gg_tiles(ws, count), units_k = (ws[0]->K + 127) / 128;
@@ -1527,8 +1530,9 @@ GgLayout gg_linear_layout(int64_t M, const hqm_weight* const* ws, int count, siz
         }
         const int64_t units = tiles * r.chunks * units_k, n16 = r.n / 16, s0 = (units + sms - 1) / sms;
         const int64_t unit = std::max<int64_t>(850 + 4 * r.n, r.n > 128 ? 10 * r.n : 0);
+        const int64_t more = ws[0]->nbits == 4 && r.n > 64 ? 1200 : 400;
         auto consider = [&](int64_t share, int64_t pieces, int cuts) {
-            const int64_t cost = share * unit + (share + units_k - 1) / units_k * n16 * 400 + cuts * (5000 + n16 * (3000 + 400 * (pieces - 2)));
+            const int64_t cost = share * unit + (share + units_k - 1) / units_k * n16 * 400 + cuts * (5000 + n16 * (3000 + more * (pieces - 2)));
             if (cost < best_cost) {
                 best_cost = cost;
                 best = GgLayout{r, (int)std::min<int64_t>(sms, (units + share - 1) / share), (int)share, cost};
