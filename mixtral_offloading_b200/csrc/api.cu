@@ -87,8 +87,15 @@ static bool use_gg(const hqm_weight* w, int G, int C, int64_t M, bool f16 = fals
 //   rows             2            3            4            5            8
 //   14336 x 4096     15.1 / 13.6  17.9 / 13.8  18.2 / 15.2  19.1 / 16.2  19.1 / 19.3
 //   4096 x 14336     17.6 / 17.4  20.3 / 17.4  20.5 / 17.9  20.7 / 19.9  20.7 / 19.8
-//   4096 x 4096       9.9 / 10.4   9.4 / 10.5  10.1 / 11.6  10.9 / 12.5  (less than a step of the kernel for every SM)
-//   3072 x 5120       9.4 / 10.6   9.5 / 11.3   9.9 / 11.8  11.1 / 12.3  (120 steps)
+//   8192 x 8192      16.3 / 14.8  19.5 / 15.6  19.5 / 15.6  20.8 / 17.4  20.9 / 18.2
+//   14336 x 14336     295 / 24.3  48.1 / 25.0  48.3 / 25.8  48.6 / 32.1  50.6 / 36.0  (two rows: the general kernel)
+// and below three steps for every SM (448 and more above):
+//   12288 x 4096     13.0 / 11.6  16.0 / 12.2  16.1 / 12.3  18.3 / 13.5  18.4 / 15.1  (384 steps)
+//   8192 x 5120      15.0 / 12.8  15.2 / 13.9  15.2 / 14.8  15.8 / 15.5  15.9 / 16.6  (320)
+//   6144 x 6144      14.9 / 12.5  13.5 / 12.8  13.5 / 13.9  17.0 / 14.1  17.2 / 15.5  (288)
+//   4096 x 4096       9.9 / 10.4   9.4 / 10.5  10.1 / 11.6  10.9 / 12.5  (128)
+//   3072 x 5120       9.4 / 10.6   9.5 / 11.3   9.9 / 11.8  11.1 / 12.3  (120)
+// The line is on the safe side of where the two meet, somewhere between 130 and 290 steps.
 static bool use_rows(int64_t M, const hqm_weight* w, StreamPlan* plan, size_t* bytes) {
     const hqm_weight* one[1] = {w};
     if (M < 2 || M > 5 || force_generic() || !gemv_rows_plan(one, 1, M, plan) || plan->rho0[1] * plan->PT < 3 * plan->grid) return false;
