@@ -299,7 +299,8 @@ int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, c
     float* few_part = nullptr;
     if (mp.short_lists) {
         uint8_t* f = mp.long_lists ? parts + mp.gg.part_bytes : xt;
-        few = GgFew{FEW_ROWS, f, (float*)(f + mp.few.x_bytes)};
+        float* scales = (float*)(f + mp.few.x_bytes);                // [2T] of x, [2T] of h, [2T][2] largest pieces
+        few = GgFew{FEW_ROWS, f, scales, (uint32_t*)(scales + 4 * T)};
         few_ht = f + mp.few.x_bytes + mp.few.scale_bytes;
         few_part = (float*)(few_ht + mp.few.h_bytes);
     }
@@ -324,9 +325,9 @@ int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, c
     up.x = xs;
     up.ht = ht;
     if (mp.short_lists) {
-        rc = launch_few_projection(fj, few.data, few_part, /*up=*/true, st);
+        rc = launch_few_projection(fj, few.data, few_part, few.largest, st);
         if (rc != HQM_OK) return rc;
-        rc = launch_few_silu(fj, few_ht, few_part, few.scale, few.scale + 2 * T, T, st);
+        rc = launch_few_silu(fj, few_ht, few_part, few.scale, few.largest, few.scale + 2 * T, T, st);
         if (rc != HQM_OK) return rc;
     }
     if (mp.long_lists) {
@@ -344,7 +345,7 @@ int hqm_moe_forward(uint16_t* out, uint16_t* router_logits, const uint16_t* x, c
         if (rc != HQM_OK) return rc;
     }
     if (mp.short_lists) {
-        rc = launch_few_projection(fj, few_ht, few_part, /*up=*/false, st);
+        rc = launch_few_projection(fj, few_ht, few_part, nullptr, st);
         if (rc != HQM_OK) return rc;
         return launch_few_combine(fj, out, few_part, y, entry_of, token_w, few.scale + 2 * T, T, st);
     }

@@ -1404,6 +1404,7 @@ __global__ void __launch_bounds__(256) gg_stage_kernel(unsigned char* __restrict
     const int e = min(max((int)(__float_as_uint(mx) >> 23), 30), 250) - 4;
     const float down = __uint_as_float((uint32_t)(254 - e) << 23);
     if (threadIdx.x == 0) (few_cap ? few.scale[li] : row_scale[row]) = __uint_as_float((uint32_t)e << 23);
+    if (few_cap && threadIdx.x < 2) few.largest[2 * li + threadIdx.x] = 0u;
     if (few_cap) {
         unsigned char* to = few.data + (size_t)few_row * K * 2;
         for (int i = threadIdx.x; i < K / 8; i += 256) {

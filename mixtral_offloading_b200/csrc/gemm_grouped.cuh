@@ -98,6 +98,7 @@ struct GgFew {
     int most;
     unsigned char* data;
     float* scale;                         // of list entry i
+    uint32_t* largest;                    // of list entry i, cleared: [2 i] and [2 i + 1], the largest |gate| and |up| of any piece
 };
 
 // Stages rows of x (bf16 or fp16) for layers of `nbits`.  counts == null: one list of `rows` rows, else `lists` lists of together at most `rows`;

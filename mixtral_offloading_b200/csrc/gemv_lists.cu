@@ -14,8 +14,6 @@
 // Measured on B200, 8 experts 4096 -> 14336 -> 4096, 8 tokens, up + gate / down: 202 / 98 us through the tensor-core kernel (whose
 // dequantisation takes 1345 warp instructions for 8192 codes), 95 / 49 here: 560 warp instructions, 59 % of the issue slots and 62 % of
 // shared memory's cycles in use; the copies alone take 56 / 30.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 
 #include "gemv_rows.cuh"
@@ -94,6 +92,7 @@ struct ListParams {
     int K, PT, N, G, C, units, period, stages, stage_bytes, x_off;      // units: of a layer
     const unsigned char* xt;
     float* partial;
+    uint32_t* largest;                                  // (two layers) see GgFew
     int* error_flag;
 };
 
@@ -132,8 +131,10 @@ __device__ __noinline__ void lists_again(const ListParams& prm, const ListSplit&
         a.k1 = r.pb * KC;
         a.staged = prm.xt + (size_t)sp.xrow0[r.e] * K * 2;
         a.cap = ListSplit::cap(sp.n[r.e]);
-        for (a.m = 0; a.m < sp.n[r.e]; ++a.m)
-            sum_again(a, prm.partial + ((size_t)piece * sp.R + sp.row0[r.e] + a.m) * row_len + layer * prm.N + PER * rho, 1.f);
+        for (a.m = 0; a.m < sp.n[r.e]; ++a.m) {
+            const float v = sum_again(a, prm.partial + ((size_t)piece * sp.R + sp.row0[r.e] + a.m) * row_len + layer * prm.N + PER * rho, 1.f);
+            if (prm.layers == 2 && v > 0.f && (threadIdx.x & 31) == 0) atomicMax(prm.largest + 2 * (sp.list0[r.e] + a.m) + layer, __float_as_uint(v));
+        }
     }
 }
 
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
     __shared__ ListSplit sp;
     __shared__ uint32_t s_begin[2];
     __shared__ int s_failed, s_again;
+    __shared__ uint32_t s_largest[FEW_MAX_LISTS * 2 * FEW_ROWS];        // of [list][layer][row], this CTA's
     __shared__ __align__(8) uint64_t s_bars[2 * MAX_STAGES];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t exch = ring + prm.stages * prm.stage_bytes;
@@ -154,6 +156,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
         init_barriers(full, empty, prm.stages);
         s_failed = s_again = 0;
     }
+    for (int i = threadIdx.x; i < FEW_MAX_LISTS * 2 * FEW_ROWS; i += THREADS) s_largest[i] = 0u;
     // the table's entries in L2 by the time the lists are known
     for (int i = threadIdx.x; i < 4 * prm.layers * prm.lists; i += THREADS) {
         const StreamEntry* en = prm.table + 3 * ((i >> 2) / prm.layers) + ((i >> 2) % prm.layers ? prm.which1 : prm.which0);
@@ -235,13 +238,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
                              (PER * rho + (lane >> 3)) % prm.period, sp.n[e], prm.G, row_len, rho * PER < prm.G};
             float* dst = prm.partial + ((size_t)piece * sp.R + sp.row0[e]) * row_len + layer * prm.N + PER * rho;
             const auto one = [](int) { return 1.f; };
-            if (sg.M <= 4) ok = rows_segment<4, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again);
-            else ok = rows_segment<8, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again);
+            uint32_t* largest = prm.layers == 2 ? s_largest + (2 * e + layer) * FEW_ROWS : nullptr;
+            if (sg.M <= 4) ok = rows_segment<4, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again, largest);
+            else ok = rows_segment<8, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again, largest);
         }
         if (again) s_again = 1;
         if (!ok) s_failed = 1;
     }
     __syncthreads();
+    if (prm.layers == 2)
+        for (int i = threadIdx.x; i < FEW_MAX_LISTS * 2 * FEW_ROWS; i += THREADS)
+            if (const uint32_t v = s_largest[i])
+                atomicMax(prm.largest + 2 * (sp.list0[i / (2 * FEW_ROWS)] + i % FEW_ROWS) + i / FEW_ROWS % 2, v);
     if (s_again && !s_failed && warp < CW) lists_again(prm, sp, ub, ue);
     // ---- a wait ran out: copies may still be on their way to this CTA's shared memory
     if (s_failed) {
@@ -250,14 +258,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
     }
 }
 
-// CTAs that left a piece of a unit of list e, and the sum of the pieces of four neighbouring columns of row m.
-__device__ __forceinline__ int pieces_of(const ListSplit& sp, int e, int unit, int PT) {
-    return sp.owner(e, (uint32_t)(unit * PT + PT - 1)) - sp.owner(e, (uint32_t)(unit * PT)) + 1;
-}
-__device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* partial, int e, int m, int cnt, int col, int row_len) {
+// Sum of the pieces of four neighbouring columns of a row.
+__device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* partial, int e, int m, int unit, int PT, int col, int row_len) {
+    const int cnt = sp.owner(e, (uint32_t)(unit * PT + PT - 1)) - sp.owner(e, (uint32_t)(unit * PT)) + 1;
     const float* at = partial + (size_t)(sp.row0[e] + m) * row_len + col;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
     for (int i = 0; i < cnt; ++i) {
         const float4 p = *reinterpret_cast<const float4*>(at + (size_t)i * sp.R * row_len);
         v.x += p.x;
@@ -269,73 +274,38 @@ __device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* p
 }
 
 // h = bf16(bf16(silu(bf16(gate))) * bf16(up)) of the short lists, staged for the down projections as fp16 with a power of two per
-// row, as the rows of x are: h of 1e-6 times a scale of 0.02 would be a denormal in fp16 (a block of weights of 1e-4: 0.24 from 64
-// bits without the factor, 3e-3 with it).  A cluster of SILU_CTAS CTAs takes list entry blockIdx.y, a thread four columns at a time.
-// The CTAs leave their largest values in each other's shared memory, so that one cluster barrier stands between the sums and the
-// stores; the one in front of the sums (every CTA is there to be written to) passes under the kernel in front.  Few threads and
-// registers, as the launch in front leaves an SM 13312 of them: with 512 threads a block of 16 tokens took 5.7 us more than without
-// factors, of which this launch alone explains 1.6.
-constexpr int SILU_CTAS = 8, SILU_THREADS = 256, SILU_COLS = SILU_CTAS * SILU_THREADS * 4, SILU_KEPT = 2, SILU_UNITS = 64;
-__global__ void __launch_bounds__(SILU_THREADS, 5) few_silu_kernel(unsigned char* __restrict__ ht, const float* __restrict__ partial,
-                                                                   const int32_t* __restrict__ counts, const float* __restrict__ row_scale,
-                                                                   float* __restrict__ h_scale, int lists, int ctas, int units, int PT, int F, int G) {
+// row: h of 1e-6 times a scale of 0.02 would be a denormal in fp16 (a block of weights of 1e-4: 0.24 from 64 bits without the factor).
+// What decides the factor is a bound of |h| that no CTA has to wait for: the pieces of a sum times the largest of them, of gate and of
+// up (the launch in front leaves both; |silu(a)| <= |a|).  The bound comes into [2^11, 2^12): h lies some 2^5 below it, typically
+// between 1 and 100, far from either end of fp16.  (The row's true maximum instead, by a cluster per row: 1.3 to 5.7 us of a
+// block of 2 to 24 tokens; with the bound -- see the figures in kernels.cuh.)
+// A thread: four columns of list entry blockIdx.y.
+__global__ void __launch_bounds__(256) few_silu_kernel(unsigned char* __restrict__ ht, const float* __restrict__ partial,
+                                                       const int32_t* __restrict__ counts, const float* __restrict__ row_scale,
+                                                       const uint32_t* __restrict__ largest, float* __restrict__ h_scale, int lists, int ctas,
+                                                       int units, int PT, int F, int G) {
     __shared__ ListSplit sp;
-    __shared__ uint32_t s_max, s_all[SILU_CTAS];        // largest |h| of this CTA's columns, of every CTA's, as bf16
-    __shared__ int s_cnt[2 * SILU_UNITS];               // pieces of the units of this entry's list
-    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     grid_launch_dependents();
-    if (threadIdx.x == 0) s_max = 0u;
-    cluster.sync();
     grid_dependency_wait();
     if (threadIdx.x < 32) sp.make(counts, lists, (uint32_t)(2 * units * PT), ctas);
     __syncthreads();
-    const int entry = blockIdx.y;
+    const int entry = blockIdx.y, f = 4 * (blockIdx.x * 256 + threadIdx.x);
     const int e = sp.list_of(entry), m = entry - sp.list0[e], cap = ListSplit::cap(sp.n[e]);
-    if (cap == 0 || m >= sp.n[e]) return;               // (all CTAs of a cluster alike)
-    // (four 64-bit divisions for a unit: once for all threads)
-    for (int u = threadIdx.x; u < 2 * units; u += SILU_THREADS) s_cnt[u] = pieces_of(sp, e, u, PT);
+    if (cap == 0 || m >= sp.n[e] || f >= F) return;
+    const int unit = f % G / PER / CW;
     const float scale = __ldcg(row_scale + entry);
-    __syncthreads();
-    auto act = [scale](float x, float y) {
-        const float g = round_bf16(x * scale);
-        return (uint32_t)float_to_bf16_bits(round_bf16(g / (1.f + __expf(-g))) * round_bf16(y * scale));
-    };
-    uint32_t mx = 0;
-    auto values = [&](int f) {                          // of four columns, as bf16
-        if (f >= F) return make_uint2(0u, 0u);
-        const int unit = f % G / PER / CW;
-        const float4 a = sum_pieces(sp, partial, e, m, s_cnt[unit], f, 2 * F);
-        const float4 b = sum_pieces(sp, partial, e, m, s_cnt[units + unit], F + f, 2 * F);
-        const uint2 v = make_uint2(act(a.x, b.x) | (act(a.z, b.z) << 16), act(a.y, b.y) | (act(a.w, b.w) << 16));
-        mx = __vmaxu2(mx, __vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu));
-        return v;
-    };
-    auto place = [&](int f) { return reinterpret_cast<uint2*>(ht + (size_t)sp.xrow0[e] * F * 2 + few_staged_at(f, m, cap) + ((f >> 2) & 1) * 8); };
-    // a thread's first values stay in registers, others wait where the fp16 values will be
-    const int f0 = 4 * (blockIdx.x * SILU_THREADS + threadIdx.x);
-    uint2 kept[SILU_KEPT];
-#pragma unroll
-    for (int j = 0; j < SILU_KEPT; ++j) kept[j] = values(f0 + j * SILU_COLS);
-    for (int f = f0 + SILU_KEPT * SILU_COLS; f < F; f += SILU_COLS) *place(f) = values(f);
-    mx = __reduce_max_sync(0xffffffffu, max(mx & 0xffffu, mx >> 16));
-    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, mx);
-    __syncthreads();
-    if (threadIdx.x < SILU_CTAS) *cluster.map_shared_rank(&s_all[blockIdx.x], threadIdx.x) = s_max;
-    cluster.sync();
-    mx = 0;
-#pragma unroll
-    for (int r = 0; r < SILU_CTAS; ++r) mx = max(mx, s_all[r]);
-    const int ex = exponent_of(mx);
+    const float pieces = (float)((uint32_t)PT * sp.cost(e) / (sp.cost0[sp.lists] / (uint32_t)sp.grid) + 2u) * scale;
+    const float most = (pieces * __uint_as_float(__ldcg(largest + 2 * entry))) * (pieces * __uint_as_float(__ldcg(largest + 2 * entry + 1)));
+    const int ex = min(max((int)(__float_as_uint(most) >> 23), 30), 250) - 11;      // biased
     const float down = __uint_as_float((uint32_t)(254 - ex) << 23);
-    if (blockIdx.x == 0 && threadIdx.x == 0) h_scale[entry] = __uint_as_float((uint32_t)ex << 23);
-    auto half = [down](uint32_t w) { return h2_of(__uint_as_float(w << 16) * down, __uint_as_float(w & 0xffff0000u) * down); };
-#pragma unroll
-    for (int j = 0; j < SILU_KEPT; ++j)
-        if (f0 + j * SILU_COLS < F) *place(f0 + j * SILU_COLS) = make_uint2(half(kept[j].x), half(kept[j].y));
-    for (int f = f0 + SILU_KEPT * SILU_COLS; f < F; f += SILU_COLS) {
-        const uint2 v = *place(f);
-        *place(f) = make_uint2(half(v.x), half(v.y));
-    }
+    if (f == 0) h_scale[entry] = __uint_as_float((uint32_t)ex << 23);
+    const float4 a = sum_pieces(sp, partial, e, m, unit, PT, f, 2 * F), b = sum_pieces(sp, partial, e, m, units + unit, PT, F + f, 2 * F);
+    auto act = [scale, down](float x, float y) {
+        const float g = round_bf16(x * scale);
+        return round_bf16(round_bf16(g / (1.f + __expf(-g))) * round_bf16(y * scale)) * down;
+    };
+    const uint32_t lo = h2_of(act(a.x, b.x), act(a.z, b.z)), hi = h2_of(act(a.y, b.y), act(a.w, b.w));
+    *reinterpret_cast<uint2*>(ht + (size_t)sp.xrow0[e] * F * 2 + few_staged_at(f, m, cap) + ((f >> 2) & 1) * 8) = make_uint2(lo, hi);
 }
 
 // out[t] = bf16(bf16(w_i * y_i) + bf16(w_j * y_j)) of the two list entries of token t: sums of pieces where the list is short, else
@@ -357,7 +327,7 @@ __global__ void __launch_bounds__(256) few_combine_kernel(uint16_t* __restrict__
         const int entry = __ldcg(entry_of + 2 * t + j), e = sp.list_of(entry);
         if (sp.n[e] <= FEW_ROWS) {
             const float w = __ldcg(token_w + entry), up = __ldcg(h_scale + entry);
-            const float4 s = sum_pieces(sp, partial, e, entry - sp.list0[e], pieces_of(sp, e, c % G / PER / CW, PT), c, H);
+            const float4 s = sum_pieces(sp, partial, e, entry - sp.list0[e], c % G / PER / CW, PT, c, H);
             v[j][0] = round_bf16(round_bf16(s.x * up) * w);
             v[j][1] = round_bf16(round_bf16(s.y * up) * w);
             v[j][2] = round_bf16(round_bf16(s.z * up) * w);
@@ -385,7 +355,7 @@ static int sm_count() {
 static size_t lists_smem(int period, int stages) { return 1024 + (size_t)stages * (meta_end(period) + FEW_ROWS * KC * 2) + (size_t)CW * EXCH_BYTES; }
 static int lists_stages(int period) {
     for (int s = MAX_STAGES; s >= 2; --s)
-        if (lists_smem(period, s) <= 225 * 1024) return s;
+        if (lists_smem(period, s) <= 224 * 1024) return s;
     return 0;
 }
 // Bytes of the partial row-sets of a launch, whatever the lists' lengths: A short lists have at most min(8 A, 2 T) rows, and a unit
@@ -416,16 +386,16 @@ bool few_plan(int64_t T, int E, const hqm_weight* w1, const hqm_weight* w2, cons
     const int sms = sm_count();
     const size_t staged_rows = (size_t)std::min<int64_t>(8 * E, 8 * T);              // (a list of one row takes four)
     const int64_t u1 = (w1->N / 16 / PER + CW - 1) / CW, u2 = (w2->N / 16 / PER + CW - 1) / CW;
-    if (u1 > SILU_UNITS) return false;
     auto align = [](size_t v) { return (v + 1023) / 1024 * 1024; };
     fp->x_bytes = align(staged_rows * w1->K * 2);
-    fp->scale_bytes = align((size_t)4 * T * sizeof(float));                          // of x, of h
+    fp->scale_bytes = align((size_t)8 * T * sizeof(float));                          // factors of x and of h, GgFew::largest
     fp->h_bytes = align(staged_rows * w1->N * 2);
     fp->part_bytes = align(std::max(partial_bytes(T, E, 2 * u1, w1->K / KC, 2 * (int64_t)w1->N, sms), partial_bytes(T, E, u2, w2->K / KC, w2->N, sms)));
     return true;
 }
 
-int launch_few_projection(const FewJob& job, const unsigned char* xt, float* partial, bool up, cudaStream_t st) {
+int launch_few_projection(const FewJob& job, const unsigned char* xt, float* partial, uint32_t* largest, cudaStream_t st) {
+    const bool up = largest != nullptr;
     using namespace rows;
     const hqm_weight* w = up ? job.w1 : job.w2;
     ListParams p{};
@@ -449,11 +419,12 @@ int launch_few_projection(const FewJob& job, const unsigned char* xt, float* par
     p.stage_bytes = p.x_off + FEW_ROWS * KC * 2;
     p.xt = xt;
     p.partial = partial;
+    p.largest = largest;
     p.error_flag = tc_error_ptr();
     static bool done[MAX_DEVICES];
     bool& d = done[current_device_slot()];
     if (!d) {
-        HQM_CUDA(cudaFuncSetAttribute(gemv_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024));
+        HQM_CUDA(cudaFuncSetAttribute(gemv_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
         d = true;
     }
     launch_overlapped(gemv_lists_kernel, sm_count(), THREADS, lists_smem(p.period, p.stages), st, p);
@@ -461,11 +432,12 @@ int launch_few_projection(const FewJob& job, const unsigned char* xt, float* par
     return HQM_OK;
 }
 
-int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, float* h_scale, int64_t T, cudaStream_t st) {
+int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, const uint32_t* largest, float* h_scale,
+                    int64_t T, cudaStream_t st) {
     using namespace rows;
     const int F = job.w1->N, G = F / 16, units = (G / PER + CW - 1) / CW;
-    launch_overlapped_cluster(few_silu_kernel, dim3(SILU_CTAS, (unsigned)(2 * T)), SILU_THREADS, 0, SILU_CTAS, st, ht, partial, job.counts, row_scale, h_scale,
-                              job.lists, sm_count(), units, job.w1->K / KC, F, G);
+    launch_overlapped(few_silu_kernel, dim3((F / 4 + 255) / 256, (unsigned)(2 * T)), 256, 0, st, ht, partial, job.counts, row_scale, largest, h_scale,
+                      job.lists, sm_count(), units, job.w1->K / KC, F, G);
     HQM_LAUNCH_CHECK();
     return HQM_OK;
 }

@@ -156,12 +156,13 @@ struct Again {
 // inputs that are fine: x * s leaves fp16 where a scale is 2048 or more (x is staged below 32), and an infinite x meets codes of 0
 // and makes the zeros' sum a difference of infinities, though its products with the weights have a sign.  The warps come
 // here behind all of their steps, when one has seen such a sum: beside them the call would cost the steps 60 to 190 bytes of spilled
-// registers.
-__device__ __noinline__ static void sum_again(const Again& a, float* to, float up) {
+// registers.  Returns the largest finite |sum| it formed.
+__device__ __noinline__ static float sum_again(const Again& a, float* to, float up) {
     const int lane = threadIdx.x & 31;
     __syncwarp();                                  // other lanes have stored some of the sums
     const float2 have = *reinterpret_cast<const float2*>(to + (int64_t)(lane >> 1) * a.G + 2 * (lane & 1));
-    if (__all_sync(0xffffffffu, isfinite(have.x) && isfinite(have.y))) return;
+    if (__all_sync(0xffffffffu, isfinite(have.x) && isfinite(have.y))) return 0.f;
+    float largest = 0.f;
     for (int s = 0; s < PER; ++s) {
         float sum[MEMBERS];
 #pragma unroll
@@ -194,18 +195,20 @@ __device__ __noinline__ static void sum_again(const Again& a, float* to, float u
         }
 #pragma unroll
         for (int j = 0; j < MEMBERS; ++j) {
-            const float v = warp_sum(sum[j]);
-            if (lane == 0) to[(int64_t)j * a.G + s] = v * up;
+            const float v = warp_sum(sum[j]) * up;
+            if (lane == 0) to[(int64_t)j * a.G + s] = v;
+            if (isfinite(v)) largest = fmaxf(largest, fabsf(v));
         }
     }
+    return largest;
 }
 
 // TOKS > 1 rows over `steps` steps, from stage st (phase par) on.  x: at x0, x_step bytes further with every step, or (x_step 0) at x0 of
-// the stage.  dst: the warp's first column of row 0; up(m): factor of row m; again: set where a sum is not finite (see sum_again()).
-// False where a wait ran out.
+// the stage.  dst: the warp's first column of row 0; up(m): factor of row m; again: set where a sum is not finite (see sum_again());
+// largest (null: not asked for): of row m in shared memory, the largest finite |sum|.  False where a wait ran out.
 template <int TOKS, bool FINE_Z, typename Up>
 __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& st, uint32_t& par, uint32_t x0, uint32_t x_step, float* dst,
-                                             const Up& up, bool& again) {
+                                             const Up& up, bool& again, uint32_t* largest = nullptr) {
     using S = Shape<TOKS>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t code_off = (uint32_t)(warp * MEMBERS * KC + g * KC), sw = (uint32_t)g;
@@ -372,6 +375,7 @@ __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& 
                 const float v = TOKS == 8 ? cor[(s >> 1) % CORS][3 * (s & 1)] : (FINE_Z ? cor[0][s >> 1] : cor[(s >> 1) % CORS][0]);
                 z[s] = __shfl_sync(0xffffffffu, v, (TOKS == 4 ? ((s & 1) * 4 + m) * 4 : m * 4) + (s >> 1));
             }
+            float most = 0.f;
             if (m < sg.M) {
                 const float f = up(m);
                 float* to = dst + (int64_t)m * sg.row_len + (int64_t)g * sg.G;
@@ -383,6 +387,11 @@ __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& 
                     // 0 * y is 0, or NaN where y is not finite.  (Of two lanes with the same sums each writes half: both look at all.)
                     again |= !(fmaf(0.f, y[0], fmaf(0.f, y[1], fmaf(0.f, y[2], 0.f * y[3]))) == 0.f);
                     float* at = to + (int64_t)8 * half * sg.G;
+                    if (largest) {
+#pragma unroll
+                        for (int s = 0; s < 4; ++s)
+                            if ((TOKS != 4 || (s & 1) == (t >> 1)) && isfinite(y[s])) most = fmaxf(most, fabsf(y[s]));
+                    }
                     if constexpr (TOKS == 4) {          // lanes t < 2 hold slots 0 and 2, the others 1 and 3
                         at[t >> 1] = t < 2 ? y[0] : y[1];
                         at[2 + (t >> 1)] = t < 2 ? y[2] : y[3];
@@ -390,6 +399,11 @@ __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& 
                         *reinterpret_cast<float4*>(at) = make_float4(y[0], y[1], y[2], y[3]);
                     }
                 }
+            }
+            if (largest) {                          // lanes of one row: same t (TOKS 4: and t + 2)
+#pragma unroll
+                for (int o = TOKS == 4 ? 2 : 4; o < 32; o <<= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+                if (lane < (TOKS == 4 ? 2 : 4) && m < sg.M) atomicMax(largest + m, __float_as_uint(most));
             }
         }
     }

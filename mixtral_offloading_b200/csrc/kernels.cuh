@@ -123,9 +123,10 @@ __host__ __device__ inline size_t few_staged_at(int k, int m, int cap) {
     const int c = (k >> 3) & 15;
     return (size_t)(k >> 7) * cap * 256 + (size_t)((2 * ((c >> 1) & 1) + (c & 1)) * cap + m) * 64 + (c >> 2) * 16;
 }
-int launch_few_projection(const FewJob& job, const unsigned char* xt, float* partial, bool up, cudaStream_t st);
-int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, float* h_scale, int64_t T,
-                    cudaStream_t st);
+// Gate and up projections where `largest` (GgFew) is given, else the down projections.
+int launch_few_projection(const FewJob& job, const unsigned char* xt, float* partial, uint32_t* largest, cudaStream_t st);
+int launch_few_silu(const FewJob& job, unsigned char* ht, const float* partial, const float* row_scale, const uint32_t* largest, float* h_scale,
+                    int64_t T, cudaStream_t st);
 int launch_few_combine(const FewJob& job, uint16_t* out, const float* partial, const uint16_t* y, const int32_t* entry_of, const float* token_w,
                        const float* h_scale, int64_t T, cudaStream_t st);
 
