@@ -156,7 +156,7 @@ struct Again {
 // inputs that are fine: x * s leaves fp16 where a scale is 2048 or more (x is staged below 32), and an infinite x meets codes of 0
 // and makes the zeros' sum a difference of infinities, though its products with the weights have a sign.  The warps come
 // here behind all of their steps, when one has seen such a sum: beside them the call would cost the steps 60 to 190 bytes of spilled
-// registers.  Returns the largest finite |sum| it formed.
+// registers.  Returns the largest finite |sum| it formed, 0 where all were finite as they were.
 __device__ __noinline__ static float sum_again(const Again& a, float* to, float up) {
     const int lane = threadIdx.x & 31;
     __syncwarp();                                  // other lanes have stored some of the sums
@@ -205,7 +205,7 @@ __device__ __noinline__ static float sum_again(const Again& a, float* to, float 
 
 // TOKS > 1 rows over `steps` steps, from stage st (phase par) on.  x: at x0, x_step bytes further with every step, or (x_step 0) at x0 of
 // the stage.  dst: the warp's first column of row 0; up(m): factor of row m; again: set where a sum is not finite (see sum_again());
-// largest (null: not asked for): of row m in shared memory, the largest finite |sum|.  False where a wait ran out.
+// largest (null: not asked for): of row m in shared memory, the largest |sum| as bits, but for rows that are formed again.  False where a wait ran out.
 template <int TOKS, bool FINE_Z, typename Up>
 __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& st, uint32_t& par, uint32_t x0, uint32_t x_step, float* dst,
                                              const Up& up, bool& again, uint32_t* largest = nullptr) {
@@ -375,7 +375,7 @@ __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& 
                 const float v = TOKS == 8 ? cor[(s >> 1) % CORS][3 * (s & 1)] : (FINE_Z ? cor[0][s >> 1] : cor[(s >> 1) % CORS][0]);
                 z[s] = __shfl_sync(0xffffffffu, v, (TOKS == 4 ? ((s & 1) * 4 + m) * 4 : m * 4) + (s >> 1));
             }
-            float most = 0.f;
+            uint32_t most = 0;                      // of the |sums| this lane writes, as bits: infinities and NaN are the largest
             if (m < sg.M) {
                 const float f = up(m);
                 float* to = dst + (int64_t)m * sg.row_len + (int64_t)g * sg.G;
@@ -384,26 +384,24 @@ __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& 
                     float y[4];
 #pragma unroll
                     for (int s = 0; s < 4; ++s) y[s] = (acc[s][2 * half + e] * (float)(1 << (18 + 2 * s)) - z[s]) * f;
-                    // 0 * y is 0, or NaN where y is not finite.  (Of two lanes with the same sums each writes half: both look at all.)
-                    again |= !(fmaf(0.f, y[0], fmaf(0.f, y[1], fmaf(0.f, y[2], 0.f * y[3]))) == 0.f);
+                    auto bits = [](float v) { return __float_as_uint(v) & 0x7fffffffu; };
                     float* at = to + (int64_t)8 * half * sg.G;
-                    if (largest) {
-#pragma unroll
-                        for (int s = 0; s < 4; ++s)
-                            if ((TOKS != 4 || (s & 1) == (t >> 1)) && isfinite(y[s])) most = fmaxf(most, fabsf(y[s]));
-                    }
                     if constexpr (TOKS == 4) {          // lanes t < 2 hold slots 0 and 2, the others 1 and 3
-                        at[t >> 1] = t < 2 ? y[0] : y[1];
-                        at[2 + (t >> 1)] = t < 2 ? y[2] : y[3];
+                        const float a = t < 2 ? y[0] : y[1], b = t < 2 ? y[2] : y[3];
+                        at[t >> 1] = a;
+                        at[2 + (t >> 1)] = b;
+                        most = max(most, max(bits(a), bits(b)));
                     } else {
                         *reinterpret_cast<float4*>(at) = make_float4(y[0], y[1], y[2], y[3]);
+                        most = max(max(most, max(bits(y[0]), bits(y[1]))), max(bits(y[2]), bits(y[3])));
                     }
                 }
             }
+            again |= most >= 0x7f800000u;
             if (largest) {                          // lanes of one row: same t (TOKS 4: and t + 2)
 #pragma unroll
-                for (int o = TOKS == 4 ? 2 : 4; o < 32; o <<= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-                if (lane < (TOKS == 4 ? 2 : 4) && m < sg.M) atomicMax(largest + m, __float_as_uint(most));
+                for (int o = TOKS == 4 ? 2 : 4; o < 32; o <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+                if (lane < (TOKS == 4 ? 2 : 4) && m < sg.M && most < 0x7f800000u) atomicMax(largest + m, most);
             }
         }
     }
