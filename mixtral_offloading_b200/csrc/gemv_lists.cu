@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
     __shared__ uint32_t s_begin[2];
     __shared__ int s_failed, s_again;
     __shared__ uint32_t s_largest[FEW_MAX_LISTS * 2 * FEW_ROWS];        // of [list][layer][row], this CTA's
+    __shared__ int s_largest_at[CW];                                    // of each computing warp's run
     __shared__ __align__(8) uint64_t s_bars[2 * MAX_STAGES];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t exch = ring + prm.stages * prm.stage_bytes;
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
         // =========================== computing warps ===========================
         int st = 0, e = 0;
         uint32_t par = 0;
-        bool ok = true, again = false;
+        bool ok = true;
         const int row_len = prm.layers * prm.N;
         for (uint32_t u = ub; u < ue && ok;) {
             const Run r = run_at(u, e);
@@ -238,11 +239,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
                              (PER * rho + (lane >> 3)) % prm.period, sp.n[e], prm.G, row_len, rho * PER < prm.G};
             float* dst = prm.partial + ((size_t)piece * sp.R + sp.row0[e]) * row_len + layer * prm.N + PER * rho;
             const auto one = [](int) { return 1.f; };
-            uint32_t* largest = prm.layers == 2 ? s_largest + (2 * e + layer) * FEW_ROWS : nullptr;
-            if (sg.M <= 4) ok = rows_segment<4, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again, largest);
-            else ok = rows_segment<8, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, again, largest);
+            uint32_t* largest = prm.layers == 2 ? s_largest : nullptr;
+            __syncwarp();                               // (the last run's has been read)
+            if (lane == 0) s_largest_at[warp] = (2 * e + layer) * FEW_ROWS;
+            __syncwarp();
+            if (sg.M <= 4) ok = rows_segment<4, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, s_again, largest, s_largest_at + warp);
+            else ok = rows_segment<8, true>(sg, r.pb - r.pa, st, par, (uint32_t)prm.x_off, 0u, dst, one, s_again, largest, s_largest_at + warp);
         }
-        if (again) s_again = 1;
         if (!ok) s_failed = 1;
     }
     __syncthreads();
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_lists_kernel(const __grid_con
         for (int i = threadIdx.x; i < FEW_MAX_LISTS * 2 * FEW_ROWS; i += THREADS)
             if (const uint32_t v = s_largest[i])
                 atomicMax(prm.largest + 2 * (sp.list0[i / (2 * FEW_ROWS)] + i % FEW_ROWS) + i / FEW_ROWS % 2, v);
-    if (s_again && !s_failed && warp < CW) lists_again(prm, sp, ub, ue);
+    if (s_again && !s_failed && warp < CW) lists_again(prm, sp, s_begin[0], s_begin[1]);
     // ---- a wait ran out: copies may still be on their way to this CTA's shared memory
     if (s_failed) {
         for (int i = 0; i < 200; ++i) __nanosleep(1000);

@@ -232,7 +232,7 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
         uint32_t x_at = x_area;                                     // of the present step
         int st = 0;
         uint32_t par = 0;
-        bool ok = true, again = false;
+        bool ok = true;
         for (int unit = unit0, pa = pa0, left = n_steps; left > 0 && ok; ++unit, pa = 0) {
             const int pb_all = min(PT, pa + left);
             left -= pb_all - pa;
@@ -349,11 +349,10 @@ gemv_rows_kernel(float* __restrict__ partial, const uint16_t* __restrict__ x, co
                 ok = rows_segment<TOKS, S::FINE_Z>(sg, pb - pa, st, par, x_at, S::X_STEP,
                                                    partial + (int64_t)slot_idx * M_total * sg.row_len + prm.col0[l] + PER * rho, [&](int m) {
                     return S::SCALED ? __uint_as_float((uint32_t)row_exponent(m) << 23) : 1.f;
-                }, again);
+                }, s_again);
             }
             x_at += (uint32_t)(pb_all - pa) * S::X_STEP;
         }
-        if (again) s_again = 1;
         if (!ok) s_failed = 1;
     }
     __syncthreads();

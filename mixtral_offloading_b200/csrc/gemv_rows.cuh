@@ -204,11 +204,12 @@ __device__ __noinline__ static float sum_again(const Again& a, float* to, float 
 }
 
 // TOKS > 1 rows over `steps` steps, from stage st (phase par) on.  x: at x0, x_step bytes further with every step, or (x_step 0) at x0 of
-// the stage.  dst: the warp's first column of row 0; up(m): factor of row m; again: set where a sum is not finite (see sum_again());
-// largest (null: not asked for): of row m in shared memory, the largest |sum| as bits, but for rows that are formed again.  False where a wait ran out.
+// the stage.  dst: the warp's first column of row 0; up(m): factor of row m; again (shared memory): set to 1 where a sum is not finite (see sum_again());
+// largest + *largest_at (shared memory; null: not asked for): of row m, the largest |sum| as bits, but for rows that are formed again.
+// (What is needed behind the steps only waits in shared memory, as they want all registers.)  False where a wait ran out.
 template <int TOKS, bool FINE_Z, typename Up>
 __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& st, uint32_t& par, uint32_t x0, uint32_t x_step, float* dst,
-                                             const Up& up, bool& again, uint32_t* largest = nullptr) {
+                                             const Up& up, int& again, uint32_t* largest = nullptr, const int* largest_at = nullptr) {
     using S = Shape<TOKS>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t code_off = (uint32_t)(warp * MEMBERS * KC + g * KC), sw = (uint32_t)g;
@@ -397,11 +398,11 @@ __device__ __forceinline__ bool rows_segment(const Segment& sg, int steps, int& 
                     }
                 }
             }
-            again |= most >= 0x7f800000u;
+            if (most >= 0x7f800000u) again = 1;
             if (largest) {                          // lanes of one row: same t (TOKS 4: and t + 2)
 #pragma unroll
                 for (int o = TOKS == 4 ? 2 : 4; o < 32; o <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-                if (lane < (TOKS == 4 ? 2 : 4) && m < sg.M && most < 0x7f800000u) atomicMax(largest + m, most);
+                if (lane < (TOKS == 4 ? 2 : 4) && m < sg.M && most < 0x7f800000u) atomicMax(largest + *largest_at + m, most);
             }
         }
     }
