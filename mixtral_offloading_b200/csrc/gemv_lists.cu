@@ -12,7 +12,7 @@
 // [step][half][16-byte piece][row][thread column], with a power of two per row.
 //
 // Measured on B200, 8 experts 4096 -> 14336 -> 4096, 8 tokens, up + gate / down: 202 / 98 us through the tensor-core kernel (whose
-// dequantisation takes 1345 warp instructions for 8192 codes), 95 / 49 here: 560 warp instructions, 59 % of the issue slots and 62 % of
+// dequantisation takes 1345 warp instructions for 8192 codes), 95 / 49 here: 565 warp instructions, 60 % of the issue slots and 59 % of
 // shared memory's cycles in use; the copies alone take 56 / 30.
 #include <algorithm>
 
@@ -280,8 +280,9 @@ __device__ __forceinline__ float4 sum_pieces(const ListSplit& sp, const float* p
 // row: h of 1e-6 times a scale of 0.02 would be a denormal in fp16 (a block of weights of 1e-4: 0.24 from 64 bits without the factor).
 // What decides the factor is a bound of |h| that no CTA has to wait for: the pieces of a sum times the largest of them, of gate and of
 // up (the launch in front leaves both; |silu(a)| <= |a|).  The bound comes into [2^11, 2^12): h lies some 2^5 below it, typically
-// between 1 and 100, far from either end of fp16.  (The row's true maximum instead, by a cluster per row: 1.3 to 5.7 us of a
-// block of 2 to 24 tokens; with the bound -- see the figures in kernels.cuh.)
+// between 1 and 100, far from either end of fp16.  (Blocks of 8 experts with 2 / 8 / 24 / 36 tokens, us, without
+// a factor 107.3 / 158.8 / 243.8 / 281.7, so 108.6 / 159.9 / 247.3 / 283.0, and with a row's true maximum, by a cluster of CTAs per row, 108.8 /
+// 160.6 / 252.8 / 288.3.)
 // A thread: four columns of list entry blockIdx.y.
 __global__ void __launch_bounds__(256) few_silu_kernel(unsigned char* __restrict__ ht, const float* __restrict__ partial,
                                                        const int32_t* __restrict__ counts, const float* __restrict__ row_scale,
